@@ -14,9 +14,12 @@
 //   codec    optional s4-bp128 encode + decode of the sorted queue; the
 //            decoded queue feeds the next top-down level
 //
-// The level loop is one CUDA graph with a conditional while node, so a
-// search costs one graph launch and one small read-back at the end (the
-// reference copies the visited mask and the queue across PCIe every level,
+// A search without codec whose parents come from atomicMin (the default) runs
+// as one kernel instead, g5_search.cuh; the level loop above serves the
+// searches that need a level's sorted queue or a fix-up sweep, as one CUDA
+// graph with a conditional while node, and the host-driven ones.  Either way a
+// search costs one launch and one small read-back at the end (the reference
+// copies the visited mask and the queue across PCIe every level,
 // cuda_bfs.cu:252-269,397-450,524-529).
 //
 // Parent choice: a vertex discovered at level L+1 gets the smallest adjacent
@@ -36,6 +39,7 @@
 #include "g5_codec_dev.cuh"
 #include "g5_common.cuh"
 #include "g5_internal.h"
+#include "g5_search.cuh"
 
 namespace {
 
@@ -65,16 +69,6 @@ constexpr uint32_t kHeavy = 64;    // degree above which top-down sets the paren
 constexpr uint32_t kSparseCap = 4096;
 constexpr uint64_t kSparseEdges = 65536;
 constexpr int kSparseRound = 4;  // list entries per thread per round of the finish
-
-enum : int32_t { DIR_TD = 0, DIR_BU = 1 };
-
-struct LevelRec {
-    int32_t dir;        // direction used to expand this level's frontier
-    int32_t pad;
-    uint64_t nf;        // frontier vertices
-    uint64_t mf;        // their adjacency entries
-    uint64_t examined;  // adjacency entries read while expanding
-};
 
 struct BfsState {
     int32_t level;      // index L of the frontier currently held
@@ -155,13 +149,6 @@ struct BfsArgs {
     cudaGraphConditionalHandle cond;
     int use_cond;
 };
-
-__device__ __forceinline__ uint64_t warp_sum_u64(uint64_t v)
-{
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    return v;
-}
 
 // Whether the next top-down level, whose frontier has tm adjacency entries,
 // appends its discoveries to the sparse list (it discovers at most tm
@@ -342,95 +329,6 @@ __device__ void expand_td(const BfsArgs &a, uint64_t &examined)
     }
 }
 
-// One warp per 32-vertex word.  BOTTOM_UP: the candidates are the unvisited
-// vertices; a candidate with a neighbour in the frontier joins the next
-// frontier with the first such neighbour of its ascending adjacency as parent.
-// FIXUP (after a top-down level): the candidates are the vertices top-down
-// just discovered; each takes the first frontier neighbour of its adjacency.
-// Either way the parent is the smallest neighbour in the frontier.
-// Warp-collective search of each active lane's adjacency [s, e) for its
-// first vertex in the frontier: every lane scans its first bu_serial entries
-// alone (four independent loads at a time), then the warp finishes the longer
-// lists one at a time, 32 entries per step (the first set ballot bit is the
-// smallest index).  Returns found / par per lane and the entries read.
-template <typename Off>
-__device__ __forceinline__ void first_hit(const BfsArgs &a, bool mine, Off s, Off e, uint32_t u0, bool &found,
-                                          uint32_t &par, uint64_t &ex)
-{
-    const int lane = g5_lane();
-    const uint32_t *__restrict__ front = a.front;
-    const uint32_t *__restrict__ col = a.col;
-    found = false;
-    par = 0;
-    Off j = s;
-    // the first neighbour comes from the dense copy (loaded with the offsets,
-    // coalesced), so a vertex whose first neighbour is in the frontier never
-    // touches its row
-    if (mine && s < e) {
-        if ((__ldg(front + (u0 >> 5)) >> (u0 & 31)) & 1u) {
-            found = true;
-            par = u0;
-        }
-        j = s + 1;
-    }
-    // (callers pass s = e = 0 on lanes without a candidate, so those lanes
-    // scan nothing here)
-    const Off lim = min(e, (Off)(s + a.bu_serial));
-    while (j < lim && !found) {
-        uint32_t u[4];
-        bool h[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) u[k] = (j + k < lim) ? __ldg(col + j + k) : 0u;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            h[k] = (j + k < lim) && ((__ldg(front + (u[k] >> 5)) >> (u[k] & 31)) & 1u);
-        int k = 0;
-        while (k < 4 && j + k < lim && !h[k]) ++k;
-        if (k < 4 && j + k < lim) {
-            found = true;
-            par = u[k];
-            j += k + 1;
-        } else {
-            j = min((Off)(j + 4), lim);
-        }
-    }
-    ex = mine ? (uint64_t)(j - s) : 0;
-    unsigned pend = __ballot_sync(0xFFFFFFFFu, mine && !found && j < e);
-    while (pend) {
-        const int l = __ffs(pend) - 1;
-        pend &= pend - 1;
-        Off jj = __shfl_sync(0xFFFFFFFFu, j, l);
-        const Off ee = __shfl_sync(0xFFFFFFFFu, e, l);
-        const Off st = jj;
-        bool got = false;
-        uint32_t gpar = 0;
-        while (jj < ee) {
-            const Off idx = jj + (Off)lane;
-            uint32_t u = 0;
-            bool hit = false;
-            if (idx < ee) {
-                u = __ldg(col + idx);
-                hit = (__ldg(front + (u >> 5)) >> (u & 31)) & 1u;
-            }
-            const unsigned m = __ballot_sync(0xFFFFFFFFu, hit);
-            if (m) {
-                const int f = __ffs(m) - 1;
-                gpar = __shfl_sync(0xFFFFFFFFu, u, f);
-                got = true;
-                jj += f + 1;
-                break;
-            }
-            jj += 32;
-        }
-        jj = min(jj, ee);
-        if (lane == l) {
-            found = got;
-            par = gpar;
-            ex += (uint64_t)(jj - st);
-        }
-    }
-}
-
 // Row offsets of v: the uint32 copy when nnz < 2^32 (half the bytes, and
 // 32-bit loop indices), else the int64 array.
 __device__ __forceinline__ void load_offsets(const BfsArgs &a, uint64_t v, uint32_t &s, uint32_t &e)
@@ -495,7 +393,7 @@ __device__ void sweep(const BfsArgs &a, uint64_t &examined)
         bool found;
         uint32_t par;
         uint64_t ex;
-        first_hit<Off>(a, mine, s, e, u0, found, par, ex);
+        first_hit<Off, true>(a.front, a.col, a.bu_serial, mine, s, e, u0, found, par, ex);
         if (found) a.pred[v] = (int64_t)par;
         if (FIXUP) {
             if (mine && !found) atomicOr(&a.st->err, G5_DEVERR_CAPACITY);  // cannot happen on a symmetric CSR
@@ -557,7 +455,7 @@ __device__ void sweep_bu(const BfsArgs &a, uint64_t &examined)
         bool found;
         uint32_t par;
         uint64_t ex;
-        first_hit<Off>(a, mine, s, e, u0, found, par, ex);
+        first_hit<Off, true>(a.front, a.col, a.bu_serial, mine, s, e, u0, found, par, ex);
         if (found) a.pred[v] = (int64_t)par;
         const unsigned fm = __ballot_sync(0xFFFFFFFFu, found);
         if (fm) {
@@ -614,7 +512,7 @@ __device__ void bottom_up_list(const BfsArgs &a, uint64_t &examined)
         bool found;
         uint32_t par;
         uint64_t ex;
-        first_hit<Off>(a, mine, s, e, u0, found, par, ex);
+        first_hit<Off, true>(a.front, a.col, a.bu_serial, mine, s, e, u0, found, par, ex);
         if (found) a.pred[v] = (int64_t)par;
         // the list is sorted, so lanes holding vertices of one bitmap word
         // are adjacent: a segmented scan gives the last lane of each word
@@ -1401,6 +1299,17 @@ struct g5_bfs {
     int64_t *cur_pred = nullptr;    // parent array of the last search
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     Prof prof;
+    // one-launch search (k_search): work items, barrier and results
+    bool one = false;             // searches run as one launch
+    int sform = SEARCH_BLOCK;     // its form
+    int sgrid = 0;                // its blocks
+    int aform = SEARCH_BLOCK, agrid = 0;  // form and blocks of an asynchronous search (g5_bfs_launch)
+    size_t ssmem = 0;             // its shared memory per block
+    SearchArgs sargs;
+    Item *items = nullptr;        // two claimed buffers and the built one
+    LevelSum *sums = nullptr;     // the ring of level sums, then its place and the abort flag
+    SearchState *h_out = nullptr; // pinned: the last search's result
+    SearchState *h_outs = nullptr;  // pinned: one per search of a run_many call
     int64_t with_edges = 0;  // vertices of degree > 0
     bool ran = false;
     int64_t last_root = -1;
@@ -1498,6 +1407,106 @@ g5_status build_graph(g5_bfs *b, int64_t *pred, cudaGraphExec_t *exec_out, cudaG
     return G5_OK;
 }
 
+// The kernel of a form of the one-launch search.
+template <typename Off>
+void (*search_kernel(int form))(const SearchArgs)
+{
+    return form == SEARCH_BLOCK     ? k_search<Off, SEARCH_BLOCK>
+           : form == SEARCH_CLUSTER ? k_search<Off, SEARCH_CLUSTER>
+           : form == SEARCH_GRID1   ? k_search<Off, SEARCH_GRID1>
+                                    : k_search<Off, SEARCH_GRID2>;
+}
+
+// Launches the search of `root` on s as one kernel: parents to `pred`, its
+// result to `out` (pinned).
+cudaError_t launch_search(g5_bfs *b, int64_t root, int64_t *pred, SearchState *out, cudaStream_t s, bool async = false)
+{
+    const int form = async ? b->aform : b->sform, grid = async ? b->agrid : b->sgrid;
+    SearchArgs a = b->sargs;
+    a.root = root;
+    a.pred = pred;
+    a.out = out;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kSB);
+    cfg.dynamicSmemBytes = b->ssmem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    cfg.attrs = at;
+    cfg.numAttrs = form == SEARCH_BLOCK ? 0 : 1;
+    if (form == SEARCH_CLUSTER) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = grid;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    } else {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    return cudaLaunchKernelEx(&cfg, a.ro32 ? search_kernel<uint32_t>(form) : search_kernel<int64_t>(form), a);
+}
+
+// Sets the form, grid and shared memory of the one-launch search; false if
+// the device holds none of them.
+template <typename Off>
+bool plan_search(g5_bfs *b)
+{
+    for (int form = search_form(b->g->n, b->g->nnz); form <= SEARCH_GRID2; ++form) {
+        auto kern = search_kernel<Off>(form);
+        // (the same for every graph of a form: the attribute set below is the
+        // kernel's, shared by all workspaces)
+        b->ssmem = sizeof(SearchShared) + (form == SEARCH_BLOCK ? (size_t)kBlockVertices / 8 * 4 : 0);
+        int per_sm = 0;
+        if ((form == SEARCH_CLUSTER &&
+             cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->ssmem) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSB, b->ssmem) != cudaSuccess || per_sm < 1) {
+            cudaGetLastError();
+            continue;
+        }
+        b->sform = form;
+        b->sgrid = form == SEARCH_BLOCK     ? 1
+                   : form == SEARCH_CLUSTER ? kClusterBlocks
+                                            : std::min(g5::grid_for(per_sm), kMaxBlocks);
+        // an asynchronous search shares the GPU with those of other
+        // workspaces: two grids of half the blocks serve more queries than one
+        // that has every SM to itself (us per query of a full server, a grid of
+        // 304 or 152 exclusive blocks / this rule / the level graph before:
+        // scale 16 38 / 13 / 44, 20 84 / 43 / 69, 22 150 / 115 / 124, 24 380 /
+        // 328 / 337); below kGrid2Vertices half the SMs cost a lone query
+        // nothing that the server's polling shows, above they do (scale 24
+        // 757 us against 460)
+        b->aform = form;
+        b->agrid = b->sgrid;
+        if (form >= SEARCH_GRID1 &&
+            cudaFuncSetAttribute(search_kernel<Off>(SEARCH_GRID2), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)b->ssmem) == cudaSuccess) {
+            b->aform = SEARCH_GRID2;
+            b->agrid = std::min(b->sgrid, form == SEARCH_GRID1 ? (g5::num_sms() + 1) / 2 : g5::num_sms());
+        }
+        return true;
+    }
+    return false;
+}
+
+// The search's outcome as the host mirrors hold it; a search that gave up
+// waiting leaves the ring in the middle of a level, so it starts again clean.
+g5_status take_result(g5_bfs *b, const SearchState &r)
+{
+    b->h_st->level = r.level;
+    b->h_st->err = r.err;
+    b->h_st->nvisited = r.nvisited;
+    b->h_st->codec_acc[0] = b->h_st->codec_acc[1] = 0;
+    if (r.err & G5_DEVERR_WAIT) G5_CUDA(cudaMemset(b->sums, 0, sizeof(LevelSum) * (kRing + 1)));
+    return G5_OK;
+}
+
+// Status of a search without codec from its error bits.
+g5_status search_status(uint32_t err)
+{
+    if (err & (G5_DEVERR_LEVELS | G5_DEVERR_WAIT)) return G5_ERR_TIMEOUT;
+    return err ? G5_ERR_CAPACITY : G5_OK;
+}
+
 g5_status alloc_ws(g5_bfs *b)
 {
     g5_graph *g = b->g;
@@ -1521,30 +1530,49 @@ g5_status alloc_ws(g5_bfs *b)
     a.max_tiles = (uint64_t)g->nnz / a.tile + 2;
     a.max_levels = b->cfg.max_levels;
     G5_CUDA(cudaMalloc(&b->deg, sizeof(uint32_t) * (size_t)n));
-    G5_CUDA(cudaMalloc(&b->bitmaps, sizeof(uint32_t) * 3 * a.nwords));
+    G5_CUDA(cudaMalloc(&b->bitmaps, sizeof(uint32_t) * (b->one ? 4 * ((a.nwords + 3) & ~(uint64_t)3) : 3 * a.nwords)));
     G5_CUDA(cudaMalloc(&b->isolated, sizeof(uint32_t) * a.nwords));
     G5_CUDA(cudaMalloc(&b->heavy, sizeof(uint32_t) * a.nwords));
     // 32-bit offsets while every scan position (row end + one 32-entry step) fits
     if (g->nnz < ((int64_t)1 << 32) - 64) G5_CUDA(cudaMalloc(&b->ro32, sizeof(uint32_t) * (size_t)(n + 1)));
     G5_CUDA(cudaMalloc(&b->first, sizeof(uint32_t) * (size_t)n));
-    G5_CUDA(cudaMalloc(&b->multi, sizeof(uint32_t) * a.nwords));
-    G5_CUDA(cudaMalloc(&b->wdeg, sizeof(uint32_t) * a.nwords));
-    G5_CUDA(cudaMemset(b->wdeg, 0, sizeof(uint32_t) * a.nwords));
-    G5_CUDA(cudaMalloc(&b->ulist, sizeof(uint32_t) * (size_t)n + 16));
-    G5_CUDA(cudaMalloc(&b->done, sizeof(unsigned)));
-    G5_CUDA(cudaMemset(b->done, 0, sizeof(unsigned)));
-    G5_CUDA(cudaMemset(b->multi, 0, sizeof(uint32_t) * a.nwords));
     G5_CUDA(cudaMalloc(&b->pred, sizeof(int64_t) * (size_t)n));
     if (b->cfg.want_levels) G5_CUDA(cudaMalloc(&b->level, sizeof(int32_t) * (size_t)n));
-    G5_CUDA(cudaMalloc(&b->queue, sizeof(uint32_t) * (size_t)n + 16));
-    G5_CUDA(cudaMalloc(&b->qoff, sizeof(uint64_t) * (size_t)(n + 1)));
-    G5_CUDA(cudaMalloc(&b->qbase, sizeof(int64_t) * (size_t)n));
-    G5_CUDA(cudaMalloc(&b->tile_start, sizeof(uint32_t) * a.max_tiles));
-    G5_CUDA(cudaMalloc(&b->chunks, sizeof(uint64_t) * 3 * a.nchunks));
-    G5_CUDA(cudaMalloc(&b->slist, sizeof(uint32_t) * kSparseCap));
     G5_CUDA(cudaMalloc(&b->st, sizeof(BfsState)));
     G5_CUDA(cudaMalloc(&b->log, sizeof(LevelRec) * (size_t)b->cfg.max_levels));
-    G5_CUDA(cudaMalloc(&b->root_dev, sizeof(int64_t)));
+    if (b->one) {
+        // each vertex of a frontier has at most one item per whole tile of
+        // its row and one for the rest
+        SearchArgs &sa = b->sargs;
+        memset(&sa, 0, sizeof sa);
+        sa.tile_shift = std::max(a.tile_shift, kMinItemShift);
+        const uint64_t tiles = (uint64_t)g->nnz >> sa.tile_shift;
+        sa.claimed_cap = std::min<uint64_t>(std::min<uint64_t>(n, kClaimMax) + tiles + 1, kClaimedItems);
+        const size_t built = (size_t)n + tiles + 1;
+        G5_CUDA(cudaMalloc(&b->items, sizeof(Item) * (2 * sa.claimed_cap + built)));
+        sa.claimed[0] = b->items;
+        sa.claimed[1] = b->items + sa.claimed_cap;
+        sa.built = b->items + 2 * sa.claimed_cap;
+        G5_CUDA(cudaMalloc(&b->sums, sizeof(LevelSum) * (kRing + 1)));
+        G5_CUDA(cudaMemset(b->sums, 0, sizeof(LevelSum) * (kRing + 1)));
+        G5_CUDA(cudaMallocHost(&b->h_out, sizeof(SearchState)));
+        memset(b->h_out, 0, sizeof(SearchState));
+    } else {
+        G5_CUDA(cudaMalloc(&b->multi, sizeof(uint32_t) * a.nwords));
+        G5_CUDA(cudaMalloc(&b->wdeg, sizeof(uint32_t) * a.nwords));
+        G5_CUDA(cudaMemset(b->wdeg, 0, sizeof(uint32_t) * a.nwords));
+        G5_CUDA(cudaMalloc(&b->ulist, sizeof(uint32_t) * (size_t)n + 16));
+        G5_CUDA(cudaMalloc(&b->done, sizeof(unsigned)));
+        G5_CUDA(cudaMemset(b->done, 0, sizeof(unsigned)));
+        G5_CUDA(cudaMemset(b->multi, 0, sizeof(uint32_t) * a.nwords));
+        G5_CUDA(cudaMalloc(&b->queue, sizeof(uint32_t) * (size_t)n + 16));
+        G5_CUDA(cudaMalloc(&b->qoff, sizeof(uint64_t) * (size_t)(n + 1)));
+        G5_CUDA(cudaMalloc(&b->qbase, sizeof(int64_t) * (size_t)n));
+        G5_CUDA(cudaMalloc(&b->tile_start, sizeof(uint32_t) * a.max_tiles));
+        G5_CUDA(cudaMalloc(&b->chunks, sizeof(uint64_t) * 3 * a.nchunks));
+        G5_CUDA(cudaMalloc(&b->slist, sizeof(uint32_t) * kSparseCap));
+        G5_CUDA(cudaMalloc(&b->root_dev, sizeof(int64_t)));
+    }
     G5_CUDA(cudaMallocHost(&b->h_root, sizeof(int64_t)));
     G5_CUDA(cudaMallocHost(&b->h_st, sizeof(BfsState)));
     G5_CUDA(cudaMallocHost(&b->h_log, sizeof(LevelRec) * (size_t)b->cfg.max_levels));
@@ -1589,6 +1617,29 @@ g5_status alloc_ws(g5_bfs *b)
     a.codec_scal = b->cfg.codec ? b->cw.scal : nullptr;
     a.ccap = b->ccap;
     a.use_cond = 0;
+    if (b->one) {
+        SearchArgs &sa = b->sargs;
+        sa.row_off = g->row_off;
+        sa.ro32 = b->ro32;
+        sa.col = g->col;
+        sa.deg = b->deg;
+        sa.first = b->first;
+        sa.isolated = b->isolated;
+        sa.n = n;
+        sa.nnz = g->nnz;
+        sa.nwords = a.nwords;
+        sa.stride = (a.nwords + 3) & ~(uint64_t)3;
+        sa.per_warp = a.nwords / ((uint64_t)b->sgrid * kSW);
+        sa.bitmaps = b->bitmaps;
+        sa.level = b->level;
+        sa.log = b->h_log;
+        sa.sums = b->sums;
+        sa.ring = reinterpret_cast<unsigned *>(b->sums + kRing);
+        sa.bu_serial = a.bu_serial;
+        sa.max_levels = a.max_levels;
+        sa.alpha = a.alpha;
+        sa.beta = a.beta;
+    }
     return G5_OK;
 }
 
@@ -1650,6 +1701,10 @@ void free_ws(g5_bfs *b)
     cudaFree(b->tile_start);
     cudaFree(b->chunks);
     cudaFree(b->slist);
+    cudaFree(b->items);
+    cudaFree(b->sums);
+    cudaFreeHost(b->h_out);
+    cudaFreeHost(b->h_outs);
     cudaFree(b->st);
     cudaFree(b->log);
     cudaFree(b->root_dev);
@@ -1739,6 +1794,11 @@ g5_status g5_bfs_create(g5_graph *g, const g5_bfs_config *cfg, g5_bfs **out)
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(G5_ERR_CUDA);
     cudaEventCreate(&b->ev0);
     cudaEventCreate(&b->ev1);
+    // one launch per search, unless the search encodes its queues, finds its
+    // parents in a fix-up sweep or is driven from the host level by level
+    if (b->cfg.use_graph && !b->cfg.codec && b->cfg.parent_mode == 0) {
+        b->one = g->nnz < ((int64_t)1 << 32) - 64 ? plan_search<uint32_t>(b) : plan_search<int64_t>(b);
+    }
     if ((st = alloc_ws(b)) != G5_OK) return fail(st);
     k_degrees<<<g5::grid_for(8), kBlock, 0, b->stream>>>(g->row_off, g->col, g->n, b->deg, b->isolated,
                                                           b->heavy, b->ro32, b->first);
@@ -1751,9 +1811,9 @@ g5_status g5_bfs_create(g5_graph *g, const g5_bfs_config *cfg, g5_bfs **out)
             return fail(G5_ERR_CUDA);
         int64_t isolated = 0;
         for (uint32_t w : iso) isolated += __builtin_popcount(w);
-        b->with_edges = g->n - isolated;
+        b->with_edges = b->sargs.with_edges = g->n - isolated;
     }
-    if (b->cfg.use_graph && (st = build_graph(b, b->pred, &b->exec, &b->graph)) != G5_OK) return fail(st);
+    if (b->cfg.use_graph && !b->one && (st = build_graph(b, b->pred, &b->exec, &b->graph)) != G5_OK) return fail(st);
     b->cur_pred = b->pred;
     *out = b;
     return G5_OK;
@@ -1773,12 +1833,16 @@ g5_status g5_bfs_run(g5_bfs *b, int64_t root, int64_t *pred_out, int32_t *level_
     if (!b || root < 0 || root >= b->g->n) return G5_ERR_INVALID_ARG;
     if (level_out && !b->level) return G5_ERR_INVALID_ARG;
     cudaStream_t s = b->stream;
-    *b->h_root = root;
-    G5_CUDA(cudaMemcpyAsync(b->root_dev, b->h_root, sizeof(int64_t), cudaMemcpyHostToDevice, s));
-    G5_CUDA(cudaEventRecord(b->ev0, s));
-    b->prof.on = b->cfg.profile && !b->exec;
+    if (!b->one) {
+        *b->h_root = root;
+        G5_CUDA(cudaMemcpyAsync(b->root_dev, b->h_root, sizeof(int64_t), cudaMemcpyHostToDevice, s));
+    }
+    if (stats || !b->one) G5_CUDA(cudaEventRecord(b->ev0, s));
+    b->prof.on = b->cfg.profile && !b->exec && !b->one;
     b->prof.used = 0;
-    if (b->exec) {
+    if (b->one) {
+        G5_CUDA(launch_search(b, root, b->pred, b->h_out, s));
+    } else if (b->exec) {
         G5_CUDA(cudaGraphLaunch(b->exec, s));
     } else {
         b->prof.mark(KP_PRO, s);
@@ -1790,8 +1854,8 @@ g5_status g5_bfs_run(g5_bfs *b, int64_t root, int64_t *pred_out, int32_t *level_
             if (b->h_st->nf == 0 || b->h_st->err) break;
         }
     }
-    G5_CUDA(cudaEventRecord(b->ev1, s));
-    G5_CUDA(cudaMemcpyAsync(b->h_st, b->st, sizeof(BfsState), cudaMemcpyDeviceToHost, s));
+    if (stats || !b->one) G5_CUDA(cudaEventRecord(b->ev1, s));
+    if (!b->one) G5_CUDA(cudaMemcpyAsync(b->h_st, b->st, sizeof(BfsState), cudaMemcpyDeviceToHost, s));
     if (pred_out)
         G5_CUDA(cudaMemcpyAsync(pred_out, b->pred, sizeof(int64_t) * (size_t)b->g->n, cudaMemcpyDefault, s));
     if (level_out)
@@ -1803,16 +1867,17 @@ g5_status g5_bfs_run(g5_bfs *b, int64_t root, int64_t *pred_out, int32_t *level_
     b->ran = true;
     b->last_root = root;
     b->cur_pred = b->pred;
+    if (b->one) G5_TRY(take_result(b, *b->h_out));
     const BfsState &hs = *b->h_st;
     g5_status rc = G5_OK;
-    if (hs.err & G5_DEVERR_LEVELS) rc = G5_ERR_TIMEOUT;
-    else if (hs.err) rc = G5_ERR_CAPACITY;
+    if (hs.err) rc = search_status(hs.err);
     else if (b->cfg.codec && (cscal[g5::CS_ERR] & G5_DEVERR_WAIT)) rc = G5_ERR_TIMEOUT;
     else if (b->cfg.codec && (cscal[g5::CS_ERR] & G5_DEVERR_MISMATCH)) rc = G5_ERR_MISMATCH;
     else if (b->cfg.codec && cscal[g5::CS_ERR]) rc = G5_ERR_CORRUPT_STREAM;
     if (stats) {
         const int nlev = std::min(hs.level + 1, b->cfg.max_levels);
-        G5_CUDA(cudaMemcpy(b->h_log, b->log, sizeof(LevelRec) * (size_t)nlev, cudaMemcpyDeviceToHost));
+        if (!b->one)
+            G5_CUDA(cudaMemcpy(b->h_log, b->log, sizeof(LevelRec) * (size_t)nlev, cudaMemcpyDeviceToHost));
         memset(stats, 0, sizeof *stats);
         stats->levels = nlev;
         stats->visited = (int64_t)hs.nvisited;
@@ -1848,7 +1913,7 @@ g5_status g5_bfs_level_log(g5_bfs *b, int64_t *out, int max_rows, int *rows)
 {
     if (!b || !out || !rows || max_rows < 1 || !b->ran) return G5_ERR_INVALID_ARG;
     const int nlev = std::min(std::min(b->h_st->level + 1, b->cfg.max_levels), max_rows);
-    G5_CUDA(cudaMemcpy(b->h_log, b->log, sizeof(LevelRec) * (size_t)nlev, cudaMemcpyDeviceToHost));
+    if (!b->one) G5_CUDA(cudaMemcpy(b->h_log, b->log, sizeof(LevelRec) * (size_t)nlev, cudaMemcpyDeviceToHost));
     for (int L = 0; L < nlev; ++L) {
         out[4 * L + 0] = b->h_log[L].dir;
         out[4 * L + 1] = (int64_t)b->h_log[L].nf;
@@ -1877,8 +1942,17 @@ g5_status g5_bfs_launch(g5_bfs *b, int64_t root)
 {
     // asynchronous search on the workspace's stream (CUDA-graph workspaces
     // only): completion is polled with g5_bfs_poll
-    if (!b || root < 0 || root >= b->g->n || !b->exec) return G5_ERR_INVALID_ARG;
+    if (!b || root < 0 || root >= b->g->n || (!b->exec && !b->one)) return G5_ERR_INVALID_ARG;
     cudaStream_t s = b->stream;
+    if (b->one) {
+        G5_CUDA(cudaEventRecord(b->ev0, s));
+        G5_CUDA(launch_search(b, root, b->pred, b->h_out, s, true));
+        G5_CUDA(cudaEventRecord(b->ev1, s));
+        b->ran = true;
+        b->last_root = root;
+        b->cur_pred = b->pred;
+        return G5_OK;
+    }
     *b->h_root = root;
     G5_CUDA(cudaMemcpyAsync(b->root_dev, b->h_root, sizeof(int64_t), cudaMemcpyHostToDevice, s));
     G5_CUDA(cudaEventRecord(b->ev0, s));
@@ -1906,10 +1980,8 @@ g5_status g5_bfs_poll(g5_bfs *b, int *done, double *device_ms)
         cudaEventElapsedTime(&ms, b->ev0, b->ev1);
         *device_ms = ms;
     }
-    const BfsState &hs = *b->h_st;
-    if (hs.err & G5_DEVERR_LEVELS) return G5_ERR_TIMEOUT;
-    if (hs.err) return G5_ERR_CAPACITY;
-    return G5_OK;
+    if (b->one && b->ran) G5_TRY(take_result(b, *b->h_out));
+    return search_status(b->h_st->err);
 }
 
 g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const *pred_out, double *device_ms)
@@ -1917,7 +1989,7 @@ g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const
     if (!b || k < 0 || (k && !roots)) return G5_ERR_INVALID_ARG;
     for (int i = 0; i < k; ++i)
         if (roots[i] < 0 || roots[i] >= b->g->n) return G5_ERR_INVALID_ARG;
-    if (!b->exec) {
+    if (!b->exec && !b->one) {
         // host-driven workspaces: one search after the other
         for (int i = 0; i < k; ++i) {
             g5_bfs_stats st;
@@ -1928,24 +2000,28 @@ g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const
     }
     const int64_t n = b->g->n;
     cudaStream_t s = b->stream;
-    // first use: the second parent buffer, its graph, the copy stream, events
-    if (!b->exec2) {
-        G5_CUDA(cudaMalloc(&b->pred2, sizeof(int64_t) * (size_t)n));
-        G5_TRY(build_graph(b, b->pred2, &b->exec2, &b->graph2));
-        G5_CUDA(cudaStreamCreateWithFlags(&b->cstream, cudaStreamNonBlocking));
-        for (int i = 0; i < 2; ++i) {
-            G5_CUDA(cudaEventCreateWithFlags(&b->searched[i], cudaEventDisableTiming));
-            G5_CUDA(cudaEventCreateWithFlags(&b->copied[i], cudaEventDisableTiming));
-        }
+    // first use: the second parent buffer (and its graph), the copy stream, events
+    if (!b->pred2) G5_CUDA(cudaMalloc(&b->pred2, sizeof(int64_t) * (size_t)n));
+    if (!b->one && !b->exec2) G5_TRY(build_graph(b, b->pred2, &b->exec2, &b->graph2));
+    if (!b->cstream) G5_CUDA(cudaStreamCreateWithFlags(&b->cstream, cudaStreamNonBlocking));
+    for (int i = 0; i < 2; ++i) {
+        if (!b->searched[i]) G5_CUDA(cudaEventCreateWithFlags(&b->searched[i], cudaEventDisableTiming));
+        if (!b->copied[i]) G5_CUDA(cudaEventCreateWithFlags(&b->copied[i], cudaEventDisableTiming));
     }
     if (k > b->roots_cap) {
         cudaFreeHost(b->h_roots);
         cudaFreeHost(b->h_errs);
+        cudaFreeHost(b->h_outs);
         b->h_roots = nullptr;
         b->h_errs = nullptr;
+        b->h_outs = nullptr;
         b->roots_cap = 0;
-        G5_CUDA(cudaMallocHost(&b->h_roots, sizeof(int64_t) * (size_t)k));
-        G5_CUDA(cudaMallocHost(&b->h_errs, sizeof(uint32_t) * (size_t)k));
+        if (b->one) {
+            G5_CUDA(cudaMallocHost(&b->h_outs, sizeof(SearchState) * (size_t)k));
+        } else {
+            G5_CUDA(cudaMallocHost(&b->h_roots, sizeof(int64_t) * (size_t)k));
+            G5_CUDA(cudaMallocHost(&b->h_errs, sizeof(uint32_t) * (size_t)k));
+        }
         b->roots_cap = k;
     }
     while (device_ms && b->tev.size() < 2 * (size_t)k) {
@@ -1955,7 +2031,7 @@ g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const
     }
     int64_t *buf[2] = {b->pred, b->pred2};
     cudaGraphExec_t ex[2] = {b->exec, b->exec2};
-    for (int i = 0; i < k; ++i) {
+    for (int i = 0; i < k && !b->one; ++i) {
         b->h_roots[i] = roots[i];
         b->h_errs[i] = 0;
     }
@@ -1964,11 +2040,14 @@ g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const
     for (int i = 0; i < k; ++i) {
         const int slot = i & 1;
         if (i >= 2) G5_CUDA(cudaStreamWaitEvent(s, b->copied[slot], 0));
-        G5_CUDA(cudaMemcpyAsync(b->root_dev, b->h_roots + i, sizeof(int64_t), cudaMemcpyHostToDevice, s));
+        if (!b->one)
+            G5_CUDA(cudaMemcpyAsync(b->root_dev, b->h_roots + i, sizeof(int64_t), cudaMemcpyHostToDevice, s));
         if (device_ms) G5_CUDA(cudaEventRecord(b->tev[2 * i], s));
-        G5_CUDA(cudaGraphLaunch(ex[slot], s));
+        if (b->one) G5_CUDA(launch_search(b, roots[i], buf[slot], b->h_outs + i, s));
+        else G5_CUDA(cudaGraphLaunch(ex[slot], s));
         if (device_ms) G5_CUDA(cudaEventRecord(b->tev[2 * i + 1], s));
-        G5_CUDA(cudaMemcpyAsync(b->h_errs + i, &b->st->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        if (!b->one)
+            G5_CUDA(cudaMemcpyAsync(b->h_errs + i, &b->st->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         G5_CUDA(cudaEventRecord(b->searched[slot], s));
         G5_CUDA(cudaStreamWaitEvent(b->cstream, b->searched[slot], 0));
         if (pred_out && pred_out[i])
@@ -1982,7 +2061,7 @@ g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const
         b->ran = true;
         b->last_root = roots[k - 1];
         b->cur_pred = buf[(k - 1) & 1];
-        G5_CUDA(cudaMemcpy(b->h_st, b->st, sizeof(BfsState), cudaMemcpyDeviceToHost));
+        if (!b->one) G5_CUDA(cudaMemcpy(b->h_st, b->st, sizeof(BfsState), cudaMemcpyDeviceToHost));
     }
     g5_status rc = G5_OK;
     for (int i = 0; i < k; ++i) {
@@ -1991,7 +2070,8 @@ g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const
             cudaEventElapsedTime(&ms, b->tev[2 * i], b->tev[2 * i + 1]);
             device_ms[i] = ms;
         }
-        if (rc == G5_OK && b->h_errs[i]) rc = (b->h_errs[i] & G5_DEVERR_LEVELS) ? G5_ERR_TIMEOUT : G5_ERR_CAPACITY;
+        if (b->one) G5_TRY(take_result(b, b->h_outs[i]));
+        if (rc == G5_OK) rc = search_status(b->one ? b->h_outs[i].err : b->h_errs[i]);
     }
     return rc;
 }

@@ -136,8 +136,10 @@ typedef struct g5_bfs_config {
     double beta;         /* bottom-up -> top-down when n_f < n / beta           */
     int codec;           /* G5_CODEC_*: round-trip every level's sorted queue   */
     uint32_t codec_threshold; /* raw below or at this length (cpusimd.hh:27,44) */
-    int use_graph;       /* 1: level loop as one CUDA graph (conditional while
-                            node); 0: host-driven loop, one sync per level       */
+    int use_graph;       /* 1: the whole search on the device (one kernel, or with
+                            codec or parent_mode 1 and 2 one CUDA graph with a
+                            conditional while node); 0: host-driven loop, one sync
+                            per level                                            */
     int max_levels;      /* safety cap on levels (G5_ERR_TIMEOUT past it)       */
     int want_levels;     /* keep a per-vertex level array                        */
     int profile;         /* with use_graph = 0: time every launch with CUDA events
