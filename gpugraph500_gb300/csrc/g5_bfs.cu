@@ -1363,8 +1363,8 @@ void enqueue_level(g5_bfs *b, const BfsArgs &a, cudaStream_t s, Prof *pf = nullp
                                 b->cfg.codec_threshold, s);
         // the stream copy is launched only while a caller has a buffer set
         if (b->capture_on) k_codec_capture<<<g5::grid_for(1), kBlock, 0, s>>>(a.ccap, b->codec_stream, b->cw.scal, b->st);
-        g5::decode_launch_acc(b->cw, b->codec_stream, b->cw.scal + g5::CS_WORDS, b->dqueue, (size_t)a.n,
-                              a.codec, b->cfg.codec_threshold, &b->st->nf, b->queue, b->st->codec_acc, s);
+        g5::codec_decode_launch(b->cw, b->codec_stream, b->cw.scal + g5::CS_WORDS, 0, b->dqueue, (size_t)a.n, a.codec,
+                                b->cfg.codec_threshold, &b->st->nf, b->queue, b->st->codec_acc, s, nullptr, nullptr);
     }
     p.mark(KP_HOST, s);
 }

@@ -25,15 +25,13 @@
 // miniblock; a first launch stores every miniblock's bit width and the word
 // count of each block's range of groups, a second one places each range
 // after the ranges before it and packs (two launches, no device waits).
-// Decoding needs each group's position, which the
-// stream only gives as a chain (each header says how long its group is): a
-// first pass follows the chain inside chunks of the stream from every
-// possible entry and carries the real entries across chunks by look-back;
-// a second pass unpacks one group per block, with the running values
-// carried across groups by look-back (two launches).  The many-streams
-// calls (one launch set for k queues) resolve the chains by binary lifting
-// over all 16-byte positions (group starts are always 16-byte aligned) and
-// use separate scan passes.
+// Decoding needs each group's position, which the stream only gives as a
+// chain (each header says how long its group is), and the sums of all values
+// before it: one launch, a block per chunk of the stream, which finds its own
+// place in the chain and adds up what the chunks before it publish.  The
+// many-streams calls (one launch set for k queues) resolve the chains by
+// binary lifting over all 16-byte positions (group starts are always 16-byte
+// aligned) and use separate scan passes.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -259,150 +257,23 @@ __device__ __forceinline__ void mb_locate(const uint32_t *in, const uint32_t *gp
     off_vec = (uint64_t)p + 1 + s;
 }
 
-// ---- one-pass kernels: decoupled look-back -----------------------------------------------
+// ---- meetings of a launch's blocks -------------------------------------------------------
 //
-// The single-stream decoder's passes run over the stream's tiles (a group of
-// 16 miniblocks for unpacking, a range of stream vectors for locating
-// groups).  Blocks claim tiles in launch order
-// from a counter, so a tile only ever waits on tiles claimed before it, whose
-// blocks are already running.  Each tile publishes its own aggregate, then
-// its inclusive prefix once known; a tile combines the nearest inclusive
-// prefix before it with the aggregates in between.  Payloads are written
-// before their status word (with a fence between); a status word holds the
-// call's epoch, so what earlier calls left reads as "not published" and
-// nothing is cleared between calls.  The last block to finish resets the
-// counter and advances the epoch.  Every wait is bounded: past kSpinLimit
-// polls the kernel records G5_DEVERR_WAIT and goes on with what it has, so
-// no launch can spin forever.
+// Blocks claim chunks in launch order from a counter, so a chunk only ever
+// waits on chunks claimed before it, whose blocks are already running.  A
+// chunk's record holds the call's epoch, so what earlier calls left reads as
+// "not published" and nothing is cleared between calls.  The last block to finish
+// resets the counter and advances the epoch.  Every wait is bounded: past
+// kSpinLimit polls the kernel records G5_DEVERR_WAIT and goes on with what it
+// has, so no launch can spin forever.
 
-constexpr int kOB = 512;                 // one-pass blocks: 16 warps, one per miniblock of a group
 constexpr uint32_t kSpinLimit = 1u << 21;
-constexpr int kEntries = 513;            // a group spans at most 1 + 16 * 32 vectors
-constexpr uint32_t kDead = 0xFFFFu;
 enum : uint32_t { ST_NONE = 0, ST_AGG = 1, ST_INC = 2 };
 
-// scalar slots of the one-pass kernels (the scalar block holds kScalars)
-enum {
-    CS_L_CTR = 20, CS_L_DONE = 21,
-    CS_U_CTR = 25, CS_U_DONE = 26, CS_U_EPOCH = 27
-};
+// scalar slots of the decoder (the scalar block holds kScalars)
+enum { CS_U_CTR = 25, CS_U_DONE = 26, CS_U_EPOCH = 27, CS_U_ERR = 28, CS_U_N = 29 };
 
 __device__ __forceinline__ uint64_t vload64(const uint64_t *p) { return *reinterpret_cast<const volatile uint64_t *>(p); }
-__device__ __forceinline__ void vstore64(uint64_t *p, uint64_t v) { *reinterpret_cast<volatile uint64_t *>(p) = v; }
-
-__device__ __forceinline__ uint32_t status_flag(uint64_t s, uint64_t epoch)
-{
-    return (s >> 2) == epoch ? (uint32_t)(s & 3u) : ST_NONE;
-}
-
-// Running lane sums with resets (decoder: a raw miniblock restarts the sums).
-struct ResetAddV {
-    typedef VecFlag T;
-    __device__ static T id() { return ResetAdd::id(); }
-    __device__ static T op(T a, T b) { return ResetAdd::op(a, b); }
-    __device__ static T shfl_down(T v, int o)
-    {
-        T r;
-        r.v.x = __shfl_down_sync(0xFFFFFFFFu, v.v.x, o);
-        r.v.y = __shfl_down_sync(0xFFFFFFFFu, v.v.y, o);
-        r.v.z = __shfl_down_sync(0xFFFFFFFFu, v.v.z, o);
-        r.v.w = __shfl_down_sync(0xFFFFFFFFu, v.v.w, o);
-        r.f = __shfl_down_sync(0xFFFFFFFFu, v.f, o);
-        return r;
-    }
-    __device__ static T bcast0(const T &v)
-    {
-        T r;
-        r.v.x = __shfl_sync(0xFFFFFFFFu, v.v.x, 0);
-        r.v.y = __shfl_sync(0xFFFFFFFFu, v.v.y, 0);
-        r.v.z = __shfl_sync(0xFFFFFFFFu, v.v.z, 0);
-        r.v.w = __shfl_sync(0xFFFFFFFFu, v.v.w, 0);
-        r.f = __shfl_sync(0xFFFFFFFFu, v.f, 0);
-        return r;
-    }
-    __device__ static T load(const T *p)
-    {
-        const volatile uint32_t *q = reinterpret_cast<const volatile uint32_t *>(p);
-        T r;
-        r.v = make_uint4(q[0], q[1], q[2], q[3]);
-        r.f = q[4];
-        return r;
-    }
-    __device__ static void store(T *p, const T &v)
-    {
-        volatile uint32_t *q = reinterpret_cast<volatile uint32_t *>(p);
-        q[0] = v.v.x;
-        q[1] = v.v.y;
-        q[2] = v.v.z;
-        q[3] = v.v.w;
-        q[4] = v.f;
-    }
-};
-
-// Decoupled look-back of tile t, run by one whole warp: publishes `mine` as
-// the tile's aggregate (tile 0: as its inclusive prefix), combines the tiles
-// before it in order and publishes the inclusive prefix; returns the
-// exclusive prefix.  agg[t] / inc[t] hold the payloads, st[t] the status.
-template <class Op>
-__device__ typename Op::T lookback(uint64_t *st, typename Op::T *agg, typename Op::T *inc, uint64_t t,
-                                   uint64_t epoch, const typename Op::T &mine, uint64_t *err)
-{
-    typedef typename Op::T T;
-    const int lane = g5_lane();
-    if (t == 0) {
-        if (lane == 0) {
-            Op::store(inc, mine);
-            __threadfence();
-            vstore64(st, (epoch << 2) | ST_INC);
-        }
-        return Op::id();
-    }
-    if (lane == 0) {
-        Op::store(agg + t, mine);
-        __threadfence();
-        vstore64(st + t, (epoch << 2) | ST_AGG);
-    }
-    T acc = Op::id();  // combination of the tiles after the current window, in order
-    int64_t j = (int64_t)t - 1;
-    uint32_t spins = 0;
-    for (;;) {
-        const int64_t idx = j - lane;  // lane 0 is the nearest tile
-        const uint32_t flag = idx >= 0 ? status_flag(vload64(st + idx), epoch) : ST_INC;
-        const unsigned incm = __ballot_sync(0xFFFFFFFFu, flag == ST_INC);
-        const unsigned ready = __ballot_sync(0xFFFFFFFFu, flag != ST_NONE);
-        const int first = incm ? __ffs(incm) - 1 : 32;
-        const unsigned need = first == 32 ? 0xFFFFFFFFu : (2u << first) - 1u;
-        if ((ready & need) != need) {
-            if (++spins > kSpinLimit) {
-                if (lane == 0) atomicOr((unsigned long long *)err, (unsigned long long)G5_DEVERR_WAIT);
-                break;
-            }
-            __nanosleep(32);
-            continue;
-        }
-        __threadfence();
-        T v = Op::id();
-        if (lane <= first && idx >= 0) v = flag == ST_INC ? Op::load(inc + idx) : Op::load(agg + idx);
-        // in-order reduction: a higher lane is an earlier tile, so each step
-        // puts the value from the higher lane first; lane 0 ends with the
-        // window's tiles combined from the earliest to the latest
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const T y = Op::shfl_down(v, o);
-            if (lane + o < 32) v = Op::op(y, v);
-        }
-        acc = Op::op(Op::bcast0(v), acc);
-        if (first < 32) break;
-        j -= 32;
-    }
-    if (lane == 0) {
-        Op::store(inc + t, Op::op(acc, mine));
-        __threadfence();
-        vstore64(st + t, (epoch << 2) | ST_INC);
-    }
-    return acc;
-}
-
 // Claims the next tile for the whole block (thread 0 draws, all read).
 __device__ __forceinline__ uint64_t claim_tile(uint64_t *ctr, uint64_t *s_t)
 {
@@ -782,58 +653,136 @@ __global__ void __launch_bounds__(kEB, 2) k_enc_pack(const uint32_t *__restrict_
     if (g1 == e.ng && wid == 0) enc_tail_warp(in, e.n, e.n1, cbase, out, scal, words_out, s_bytes);
 }
 
-// ---- decoder: locate groups ----------------------------------------------------------
+// ---- decoder ---------------------------------------------------------------------------
 //
-// A group's position is only given by the chain of group headers before it
-// (each says how long its group is).  The stream's vectors are cut into
-// chunks of S (a power of two from kLocMin to kLocMax, chosen so that there
-// are at most kLocFit chunks); a chunk's first group starts somewhere in its
-// first kEntries vectors (a group spans at most that many).
-//   k_loc_tables  (one block per chunk) follows the chain inside the chunk
-//                 from every possible entry and writes, per entry, where the
-//                 chain leaves the chunk and how many groups it started (the
-//                 chunk's transfer table), and each vector's jump
-//   k_loc_walk    (one block) carries the real entry from chunk to chunk
-//                 through the tables, held in shared memory
-//   k_loc_pos     (one block per chunk) follows the chain from the chunk's
-//                 real entry and writes its groups' positions
-// Chains through vectors that cannot be headers (a width above 32, a group
-// running past the stream) are marked dead; a real chain that reaches one
-// before the last group makes the stream corrupt.
+// One launch.  A group's position is only given by the chain of group headers
+// before it (each says how long its group is), and its values need the sums of
+// all groups before it.  The stream's vectors are cut into chunks, a block per
+// chunk, its groups (the ones that start in it) decoded from shared memory:
+//
+//   entry   where the chain enters the chunk.  The group before the entry
+//           starts at most kSpan vectors before the chunk; the block tries every
+//           vector there that could be a header (16 bytes of at most 32: payload
+//           hardly ever is) and follows the chain from where it leads.  Where
+//           exactly one entry comes up whose chain reaches the next chunk, that
+//           is the one, known without any other chunk.  The first chunk's entry
+//           is given.  (Near the stream's end the chain may stop in the chunk:
+//           there every entry counts.)  Else the block waits for the chunk before
+//           to tell its exit.
+//   sums    the lane sums of every miniblock and, in order, of the chunk
+//           (a raw b = 32 miniblock restarts them)
+//   meet    the chunk publishes its entry, exit, groups and sums, and adds up
+//           those of all chunks before it: 512 of them are read at once, so on
+//           streams up to a wave there is one round trip and no chain.  Each
+//           chunk checks its entry against the exit before it; a chain that
+//           breaks before the last group makes the stream corrupt.
+//   values  the miniblocks are unpacked again, now with their base
+//
+// What bounds it: a chain of round trips whatever the size (ticket and stream
+// header 1.2 us, chunk 0.6, candidates 0.9, groups 0.6, sums 1.5-2.4, meeting
+// 1.2-3, the last block's exit 1) and, on large streams, the values (5 us for 20
+// MB: issue and the stores).  5 M values of 6 bits take 17 us, against 50 us for
+// the four launches this replaced (transfer tables from every entry, a
+// one-block walk through them, positions, an unpacker with a look-back chain
+// over its tiles); 3000 values 7 us against 12.  Unpacking twice is cheaper
+// than keeping a chunk's values (128 KB at 6 bits) in shared memory, which
+// would leave one block per SM.
+constexpr int kSpan = 513;         // a group spans at most 1 + 16 * 32 vectors
+constexpr uint32_t kDead = 0xFFFFu;
+constexpr int kDB = 512;           // threads per block
+constexpr int kDW = kDB / 32;
+constexpr uint32_t kMinChunk = 576, kMaxChunk = 1536;  // vectors per chunk (more than kSpan: every
+                                                       // chunk holds its entry)
+constexpr int kDG = 32;            // groups whose miniblocks are held together
+constexpr int kDM = 16 * kDG;
 
-// Header checks every block makes alike; false if the stream is raw or bad.
+// What a chunk tells the ones after it: the groups it starts and their sums
+// (ST_AGG), or those of all chunks up to it (ST_INC).  Each 16-byte part
+// carries the status and moves in one access, so a reader needs no fence and
+// no second round trip: three parts of one status are one record.
+struct ChunkRec {
+    uint4 v;
+    uint32_t f;       // the sums restart in the chunk
+    uint32_t exit;    // where the chain enters the next chunk (kDead: it does not)
+    uint32_t groups;
+};
+struct __align__(64) ChunkSlot {
+    unsigned long long part[3][2];
+    unsigned long long pad[2];
+};
+
+struct DecShared {
+    uint4 vec[kMaxChunk + kSpan + 1];  // the chunk, the rest of its last group, one more read by unpack4
+    uint16_t jump[kMaxChunk];             // where the group at a vector ends, if it is a header
+    uint16_t gpos[kMaxChunk];             // the chunk's groups
+    uint32_t mb[kDM];                     // miniblocks: payload vector | width << 16
+    uint4 v[kDM];                         // their sums, then the sums before them
+    uint8_t f[kDM];
+    uint32_t tail[kTailMaxBytes / 4];
+    uint4 wv[kDW];                        // warp totals of a scan
+    uint32_t wf[kDW];
+    uint64_t t;
+    uint32_t entry, exit, groups;
+    uint32_t stop;                        // the vector the chain stops at, if it is in the chunk
+    uint32_t first, last;                 // least and greatest entry that came up
+    uint4 cv;                             // the chunk's sums
+    uint32_t cf;
+    unsigned long long before;            // groups before the chunk
+    uint4 base;                           // sums before the chunk
+    int near_reset, near_inc;             // nearest record before that restarts the sums / holds them all
+};
+
+__device__ __forceinline__ uint4 add4(uint4 a, uint4 b)
+{
+    return make_uint4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+
+// Header checks every block makes alike.
 struct DecHead {
-    uint64_t words, nv, n1, nmb, ng;
+    uint64_t words, nv, n1, nmb, ng, nchunks;
+    uint32_t S;  // vectors per chunk
     bool raw, bad;
 };
 
-__device__ __forceinline__ DecHead dec_head(const uint32_t *in, const uint64_t *words_dev, uint64_t cap,
-                                            uint64_t raw_thr, const uint64_t *n_expect, uint64_t max_vec,
-                                            uint64_t max_mb)
+// Chunk size: one chunk per block where that leaves it between the limits.
+__device__ __forceinline__ void dec_chunks(DecHead &h, uint32_t blocks)
+{
+    const uint64_t per = (h.nv + blocks - 1) / blocks;
+    h.S = (uint32_t)min((uint64_t)kMaxChunk, max((uint64_t)kMinChunk, (per + 63) & ~(uint64_t)63));
+    h.nchunks = h.nv > 1 ? (h.nv - 1 + h.S - 1) / h.S : 0;
+}
+
+__device__ __forceinline__ DecHead dec_head(const uint32_t *in, uint64_t words, uint64_t cap, uint64_t raw_thr,
+                                            const uint64_t *n_expect, uint64_t max_vec, uint64_t max_mb,
+                                            uint32_t blocks)
 {
     DecHead h;
-    h.words = *words_dev;
-    h.nv = h.words / 4;
-    h.n1 = h.nmb = h.ng = 0;
+    h.words = words;
+    h.nv = words / 4;
+    h.n1 = h.nmb = h.ng = h.nchunks = 0;
+    h.S = kMinChunk;
     h.bad = false;
     // plugin semantics: raw when n <= thr or the stream is as long as n
     // (cpu_2d/compression/cpusimd.hh:169-173)
-    h.raw = raw_thr && n_expect && (*n_expect <= raw_thr || h.words == *n_expect);
+    h.raw = raw_thr && n_expect && (*n_expect <= raw_thr || words == *n_expect);
     if (h.raw) {
-        h.bad = h.words > cap;
+        h.bad = words > cap;
         return h;
     }
-    if (h.words < 4) {
+    if (words < 4) {
         h.bad = true;
     } else {
-        h.n1 = in[0];
-        if (in[1] != kCookie || in[2] != kCookie || in[3] != kCookie) h.bad = true;
+        const uint4 x = *reinterpret_cast<const uint4 *>(in);
+        h.n1 = x.x;
+        if (x.y != kCookie || x.z != kCookie || x.w != kCookie) h.bad = true;
         if (h.n1 % 128 || h.n1 > cap || h.n1 / 128 >= max_mb) h.bad = true;
     }
     if (h.nv > max_vec) h.bad = true;
     if (h.bad) h.n1 = 0;
     h.nmb = h.n1 / 128;
     h.ng = (h.nmb + 15) / 16;
+    if (!h.bad) dec_chunks(h, blocks);
+    if (h.ng == 0) h.nchunks = 0;
     return h;
 }
 
@@ -843,253 +792,23 @@ __device__ __forceinline__ uint32_t width_of(uint4 h, int i)
     return (w >> (24 - 8 * (i & 3))) & 0xFFu;
 }
 
-constexpr int kLocMin = 2048, kLocMax = 16384;  // chunk sizes in vectors
-constexpr int kLocBatch = 4;                    // candidate vectors a thread loads together
-// a chunk's candidates are read in whole rounds of kOB * kLocBatch, none past its end
-static_assert(kLocMin % (kOB * kLocBatch) == 0, "chunk sizes must be whole load rounds");
-constexpr int kLocFit = 96;                     // chunks whose tables the walk holds in shared memory
-constexpr int kWalkThreads = 1024;
-
-// Chunk size for a stream of nv vectors (the same in all three kernels).
-__device__ __forceinline__ uint32_t loc_chunk(uint64_t nv)
+// Sum of the 16 widths (bytes) of a vector taken as a group header, or kDead
+// if one is above 32.
+__device__ __forceinline__ uint32_t header_sum(uint4 x)
 {
-    uint32_t S = kLocMin;
-    while (S < kLocMax && (nv + S - 1) / S > (uint64_t)kLocFit) S <<= 1;
-    return S;
+    const uint32_t over = __vcmpgtu4(x.x, 0x20202020u) | __vcmpgtu4(x.y, 0x20202020u) |
+                          __vcmpgtu4(x.z, 0x20202020u) | __vcmpgtu4(x.w, 0x20202020u);
+    uint32_t sum = __dp4a(x.x, 0x01010101u, 0u);
+    sum = __dp4a(x.y, 0x01010101u, sum);
+    sum = __dp4a(x.z, 0x01010101u, sum);
+    sum = __dp4a(x.w, 0x01010101u, sum);
+    return over ? kDead : sum;
 }
 
-__global__ void __launch_bounds__(kOB) k_loc_tables(const uint32_t *__restrict__ in, const uint64_t *words_dev,
-                                                    uint64_t cap, uint64_t raw_thr, const uint64_t *n_expect,
-                                                    uint64_t *scal, uint64_t max_vec, uint64_t max_mb,
-                                                    uint32_t *ltab, uint16_t *ljump)
+// Sum of the first i widths of a group header (its leading, big-endian bytes).
+__device__ __forceinline__ uint32_t header_before(uint4 h, int i)
 {
-    __shared__ uint16_t s_j[kLocMax];
-    __shared__ uint64_t s_t;
-    g5_pdl_sync();
-    const DecHead h = dec_head(in, words_dev, cap, raw_thr, n_expect, max_vec, max_mb);
-    const uint32_t S = loc_chunk(h.nv);
-    const uint64_t nchunks = (h.raw || h.bad || h.ng == 0) ? 0 : (h.nv - 1 + S - 1) / S;
-    for (;;) {
-        const uint64_t c = claim_tile(&scal[CS_L_CTR], &s_t);
-        if (c >= nchunks) break;
-        const uint64_t a = 1 + c * S;  // first vector of the chunk
-        const uint4 *v = reinterpret_cast<const uint4 *>(in);
-        // kLocBatch of the thread's candidate vectors loaded together, then
-        // their jumps (S is a multiple of kOB * kLocBatch)
-        for (uint32_t p0 = threadIdx.x; p0 < S; p0 += kOB * kLocBatch) {
-            uint4 hv[kLocBatch];
-#pragma unroll
-            for (int i = 0; i < kLocBatch; ++i) {
-                const uint32_t p = p0 + i * kOB;
-                hv[i] = a + p < h.nv ? v[a + p] : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int i = 0; i < kLocBatch; ++i) {
-                const uint32_t p = p0 + i * kOB;
-                uint32_t r = kDead;
-                if (a + p < h.nv) {
-                    // the 16 widths (bytes) added four at a time; a byte
-                    // above 32 rules the vector out as a header
-                    const uint32_t x[4] = {hv[i].x, hv[i].y, hv[i].z, hv[i].w};
-                    uint32_t sum = 0, over = 0;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        sum = __dp4a(x[j], 0x01010101u, sum);
-                        over |= __vcmpgtu4(x[j], 0x20202020u);
-                    }
-                    if (!over && a + p + 1 + sum <= h.nv) r = p + 1 + sum;  // <= S + 512 < kDead
-                    ljump[a + p] = (uint16_t)r;
-                }
-                s_j[p] = (uint16_t)r;
-            }
-        }
-        __syncthreads();
-        // transfer table: entry e -> (exit offset in the next chunk, groups started)
-        for (uint32_t e = threadIdx.x; e < kEntries; e += kOB) {
-            uint32_t p = e, cnt = 0, exit = kDead;
-            if (a + e < h.nv) {
-                while (p < S) {
-                    const uint32_t r = s_j[p];
-                    ++cnt;  // a group starts at p
-                    if (r == kDead) break;
-                    p = r;
-                }
-                if (p >= S) exit = p - S;
-                else --cnt;  // the dead header starts no group
-            }
-            ltab[c * kEntries + e] = (exit << 16) | cnt;
-        }
-    }
-    if (last_block(&scal[CS_L_DONE])) {
-        scal[CS_L_CTR] = 0;
-        scal[CS_L_DONE] = 0;
-        __threadfence();
-    }
-}
-
-// One block: the real entry E_c and groups before it G_c of every chunk,
-// chained through the tables (in shared memory when they fit); writes
-// lent[c] = E_c | G_c << 32 and the stream's scalars.
-__global__ void __launch_bounds__(kWalkThreads) k_loc_walk(const uint32_t *__restrict__ in, const uint64_t *words_dev,
-                                                           uint64_t cap, uint64_t raw_thr, const uint64_t *n_expect,
-                                                           uint64_t *scal, uint64_t max_vec, uint64_t max_mb,
-                                                           const uint32_t *ltab, uint64_t *lent)
-{
-    extern __shared__ uint32_t s_tab[];
-    g5_pdl_sync();
-    const DecHead h = dec_head(in, words_dev, cap, raw_thr, n_expect, max_vec, max_mb);
-    const uint32_t S = loc_chunk(h.nv);
-    const uint64_t nchunks = (h.raw || h.bad || h.ng == 0) ? 0 : (h.nv - 1 + S - 1) / S;
-    const bool fit = nchunks <= (uint64_t)kLocFit;
-    if (fit) {
-        // eight loads per thread in flight at a time
-        const uint64_t tot = nchunks * kEntries;
-        for (uint64_t i0 = threadIdx.x; i0 < tot; i0 += 8ull * blockDim.x) {
-            uint32_t r[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const uint64_t i = i0 + (uint64_t)k * blockDim.x;
-                r[k] = i < tot ? ltab[i] : 0u;
-            }
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const uint64_t i = i0 + (uint64_t)k * blockDim.x;
-                if (i < tot) s_tab[i] = r[k];
-            }
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    uint64_t err = h.bad ? G5_DEVERR_CORRUPT : 0;
-    uint64_t E = 1, G = 0;
-    for (uint64_t c = 0; c < nchunks; ++c) {
-        const uint64_t a = 1 + c * S;
-        lent[c] = (E & 0xFFFFFFFFull) | (G << 32);
-        if (G >= h.ng) continue;  // the chain has ended: this chunk owns nothing
-        if (E < a || E - a >= kEntries) {
-            err |= G5_DEVERR_CORRUPT;
-            G = h.ng;
-            continue;
-        }
-        const uint32_t tv = fit ? s_tab[c * kEntries + (E - a)] : ltab[c * kEntries + (E - a)];
-        G += tv & 0xFFFFu;
-        if (G >= h.ng) {
-            G = h.ng;
-            continue;
-        }
-        if ((tv >> 16) == kDead) {  // the chain dies before the last group
-            err |= G5_DEVERR_CORRUPT;
-            G = h.ng;
-            continue;
-        }
-        E = a + S + (tv >> 16);
-    }
-    if (!h.raw && !h.bad && h.ng > 0 && G < h.ng) err |= G5_DEVERR_CORRUPT;
-    if (!h.raw && h.ng == 0) scal[CS_BLKEND] = 4;
-    scal[CS_ERR] = err;
-    scal[CS_WORDS] = h.words;
-    scal[CS_RAW] = h.raw ? 1 : 0;
-    scal[CS_N1] = h.n1;
-    scal[CS_NMB] = h.nmb;
-    scal[CS_NG] = h.ng;
-    scal[CS_N] = h.raw ? h.words : 0;
-}
-
-// One block per chunk: the positions of the chunk's own groups, from its
-// real entry along the jumps (staged in shared memory); the block with the
-// last group also checks it and sets the end of the block part.
-__global__ void __launch_bounds__(kOB) k_loc_pos(const uint32_t *__restrict__ in, uint64_t *scal,
-                                                 const uint16_t *ljump, const uint64_t *lent, uint32_t *gpos)
-{
-    __shared__ uint16_t s_j[kLocMax];
-    g5_pdl_sync();
-    if (scal[CS_RAW] || scal[CS_ERR]) return;
-    const uint64_t ng = scal[CS_NG], nmb = scal[CS_NMB];
-    const uint64_t nv = scal[CS_WORDS] / 4;
-    const uint32_t S = loc_chunk(nv);
-    const uint64_t nchunks = ng == 0 ? 0 : (nv - 1 + S - 1) / S;
-    const uint4 *v = reinterpret_cast<const uint4 *>(in);
-    for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        const uint64_t a = 1 + c * S;
-        const uint64_t en = lent[c];
-        const uint64_t g0 = en >> 32;
-        const uint64_t gnext = c + 1 < nchunks ? (lent[c + 1] >> 32) : ng;
-        if (g0 >= gnext) continue;  // uniform over the block
-        __syncthreads();            // the previous chunk's jumps are no longer read
-        for (uint32_t p0 = threadIdx.x; p0 < S; p0 += kOB * kLocBatch) {
-            uint16_t jv[kLocBatch];
-#pragma unroll
-            for (int i = 0; i < kLocBatch; ++i) {
-                const uint32_t p = p0 + i * kOB;
-                jv[i] = a + p < nv ? ljump[a + p] : (uint16_t)0;
-            }
-#pragma unroll
-            for (int i = 0; i < kLocBatch; ++i) {
-                const uint32_t p = p0 + i * kOB;
-                if (a + p < nv) s_j[p] = jv[i];
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x != 0) continue;
-        uint64_t p = en & 0xFFFFFFFFull;
-        for (uint64_t g = g0; g < gnext; ++g) {
-            gpos[g] = (uint32_t)p;
-            if (g == ng - 1) {
-                // the last group holds only the remaining miniblocks
-                const uint4 hv = v[p];
-                const uint64_t howmany = nmb - 16 * g;
-                uint64_t sum = 0;
-                bool ok = true;
-                for (uint64_t q = 0; q < howmany; ++q) {
-                    const uint32_t b = width_of(hv, (int)q);
-                    ok &= b <= 32;
-                    sum += b;
-                }
-                const uint64_t end = p + 1 + sum;
-                if (!ok || end > nv) atomicOr((unsigned long long *)&scal[CS_ERR], (unsigned long long)G5_DEVERR_CORRUPT);
-                else scal[CS_BLKEND] = 4 * end;
-                break;
-            }
-            if (g + 1 == gnext) break;  // the next group starts in the next chunk
-            const uint32_t r = s_j[p - a];
-            if (r == kDead) {  // the walk's tables rule this out; kept as a guard
-                atomicOr((unsigned long long *)&scal[CS_ERR], (unsigned long long)G5_DEVERR_CORRUPT);
-                break;
-            }
-            p = a + r;
-        }
-    }
-}
-
-// ---- decoder: unpack (one pass) --------------------------------------------------------
-//
-// Tiles of 4 or 8 groups (8 when tiles of 4 would need more than one wave
-// of the grid: fewer tiles make a shorter look-back chain), warp w taking
-// miniblocks w, w + 16, w + 32, ... of the tile, four at a time, at the
-// positions the locator found: one lane scan per miniblock gives its values
-// from the miniblock's start (staged in shared memory) and, in lane 31, its
-// aggregate (the lane sums, or for a raw b = 32 miniblock its last vector
-// with a reset flag); warp 0 scans the tile's aggregates, finds the tile's
-// prefix by look-back and each miniblock's base, which is added as the
-// values are written.  Block 0 first decodes the VariableByte tail, which
-// starts from 0 whatever the block part holds.  With `expect` every value
-// is compared with the expected one (the level loop's round-trip check);
-// `acc` accumulates words and values.
-constexpr int kTG = 8;          // groups per unpacker tile, at most (4 or 8, see k_dec_unpack)
-constexpr int kTM = 16 * kTG;   // miniblocks per tile, at most (each warp takes four at a time)
-// dynamic shared memory of the unpacker: each miniblock's values relative
-// to its start (kTM x 32 vectors), aggregates, in-tile prefixes, bases, raw flags
-constexpr size_t kUValBytes = sizeof(uint4) * kTM * 32;
-constexpr size_t kUSmem = kUValBytes + 2 * sizeof(VecFlag) * kTM + sizeof(uint4) * kTM + kTM;
-
-// Stream position (16-byte vectors) and width of miniblock i of the group
-// whose header is at vector p.
-__device__ __forceinline__ void mb_at(const uint32_t *in, uint32_t p, int i, uint64_t &off, uint32_t &b)
-{
-    const uint4 hv = reinterpret_cast<const uint4 *>(in)[p];
-    // the widths before i: the leading (big-endian) bytes of the header
-    // words, each word's bytes added by one dp4a
-    const uint32_t x[4] = {hv.x, hv.y, hv.z, hv.w};
+    const uint32_t x[4] = {h.x, h.y, h.z, h.w};
     uint32_t sum = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -1097,53 +816,274 @@ __device__ __forceinline__ void mb_at(const uint32_t *in, uint32_t p, int i, uin
         const uint32_t m = keep >= 4 ? 0xFFFFFFFFu : keep <= 0 ? 0u : ~(0xFFFFFFFFu >> (8 * keep));
         sum = __dp4a(x[j] & m, 0x01010101u, sum);
     }
-    off = (uint64_t)p + 1 + sum;
-    b = width_of(hv, i);
+    return sum;
 }
 
-// A miniblock's deltas (lane j: vector j) turned into its running sums from
-// the miniblock's start, in place, and the miniblock's aggregate in lane 31
-// (its lane sums, or for a raw b = 32 miniblock its last vector with a reset
-// flag).  d4 sums each lane component over the vectors; dm sums component 3
-// (every component of a vector is relative to component 3 of the vector
-// before), so components 0-2 keep their deltas.  One scan serves both the
-// aggregate and the values from the miniblock's start.
-__device__ __forceinline__ VecFlag mb_scan(uint4 &d, uint32_t b, int mode)
+// Values 4 q .. 4 q + 3 of component l of a miniblock (l = lane & 3, q = lane >> 2)
+// whose payload starts at word s and has width b.
+__device__ __forceinline__ void unpack4(const uint32_t *s, uint32_t b, uint32_t (&v)[4])
 {
-    const int lane = g5_lane();
-    VecFlag r;
+    const uint32_t l = g5_lane() & 3, q = g5_lane() >> 2;
     if (b == 32) {
-        r.v = d;
-        r.f = 1;
-        return r;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = s[16 * q + 4 * i + l];
+        return;
     }
-    if (mode == G5_CODEC_DM) {
-        uint32_t c = d.w;
+    const uint32_t mask = (1u << b) - 1u;
+    uint32_t bit = 4 * q * b;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, c, o);
-            if (lane >= o) c += y;
+    for (int i = 0; i < 4; ++i, bit += b) {
+        const uint32_t *p = s + 4 * (bit >> 5) + l;
+        v[i] = __funnelshift_r(p[0], p[4], bit) & mask;
+    }
+}
+
+// The sum of component l of a miniblock whose payload starts at word s, by one
+// thread: d4 adds each component; dm adds component 3 (every component of a
+// vector is relative to component 3 of the vector before); a raw miniblock
+// gives its last vector.  A thread walking its 32 values costs a third of the
+// issue slots of a warp unpacking them and adding them up by shuffles.
+__device__ __forceinline__ uint32_t mb_sum(const uint32_t *s, uint32_t b, uint32_t l)
+{
+    if (b == 32) return s[124 + l];
+    const uint32_t mask = (1u << b) - 1u;
+    uint32_t w0 = s[l], w1 = s[4 + l], bit = 0, sum = 0;
+    const uint32_t *p = s + 8 + l;
+#pragma unroll 8
+    for (int j = 0; j < 32; ++j) {
+        sum += __funnelshift_r(w0, w1, bit) & mask;
+        bit += b;
+        if (bit >= 32) {
+            bit -= 32;
+            w0 = w1;
+            w1 = *p;
+            p += 4;
         }
-        d.w = c;
-        r.v = make_uint4(c, c, c, c);
-    } else {
+    }
+    return sum;
+}
+
+// Lane j's vector j of a miniblock with the sums `base` before it.
+__device__ __forceinline__ uint4 mb_values(const uint32_t *s, uint32_t b, uint4 base, int mode)
+{
+    const int lane = g5_lane(), l = lane & 3;
+    if (b == 32) return reinterpret_cast<const uint4 *>(s)[lane];
+    uint32_t v[4];
+    unpack4(s, b, v);
+    // running sums of the lane's four values, then of the eight lanes of its
+    // component
+    uint32_t p[4];
+    p[0] = v[0];
+    p[1] = p[0] + v[1];
+    p[2] = p[1] + v[2];
+    p[3] = p[2] + v[3];
+    uint32_t inc = p[3];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t yx = __shfl_up_sync(0xFFFFFFFFu, d.x, o);
-            const uint32_t yy = __shfl_up_sync(0xFFFFFFFFu, d.y, o);
-            const uint32_t yz = __shfl_up_sync(0xFFFFFFFFu, d.z, o);
-            const uint32_t yw = __shfl_up_sync(0xFFFFFFFFu, d.w, o);
-            if (lane >= o) {
-                d.x += yx;
-                d.y += yy;
-                d.z += yz;
-                d.w += yw;
+    for (int o = 4; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    const uint32_t ex = inc - p[3];
+    if (mode == G5_CODEC_DM) {
+        // components 0..2 add component 3 of the vector before
+        const uint32_t c = base.w + ex;
+        const int w = lane | 3;
+        uint32_t before[4];
+        before[0] = __shfl_sync(0xFFFFFFFFu, c, w);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) before[i + 1] = __shfl_sync(0xFFFFFFFFu, c + p[i], w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = l == 3 ? c + p[i] : before[i] + v[i];
+    } else {
+        const uint32_t c = ex + (l == 0 ? base.x : l == 1 ? base.y : l == 2 ? base.z : base.w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = c + p[i];
+    }
+    // the four lanes of a q hold vectors 4 q .. 4 q + 3 by component: transposed,
+    // each holds one vector
+    uint32_t a = __shfl_xor_sync(0xFFFFFFFFu, l & 1 ? v[0] : v[1], 1), c = __shfl_xor_sync(0xFFFFFFFFu, l & 1 ? v[2] : v[3], 1);
+    if (l & 1) {
+        v[0] = a;
+        v[2] = c;
+    } else {
+        v[1] = a;
+        v[3] = c;
+    }
+    a = __shfl_xor_sync(0xFFFFFFFFu, l & 2 ? v[0] : v[2], 2);
+    c = __shfl_xor_sync(0xFFFFFFFFu, l & 2 ? v[1] : v[3], 2);
+    if (l & 2) {
+        v[0] = a;
+        v[1] = c;
+    } else {
+        v[2] = a;
+        v[3] = c;
+    }
+    return make_uint4(v[0], v[1], v[2], v[3]);
+}
+
+__device__ __forceinline__ void put_part(unsigned long long *p, unsigned long long value, unsigned long long status)
+{
+    const unsigned __int128 x = (unsigned __int128)status << 64 | value;
+    asm volatile("st.relaxed.gpu.global.b128 [%0], %1;\n" ::"l"(__cvta_generic_to_global(p)), "q"(x) : "memory");
+}
+
+__device__ __forceinline__ void get_part(const unsigned long long *p, unsigned long long &value,
+                                         unsigned long long &status)
+{
+    unsigned __int128 x;
+    asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];\n" : "=q"(x) : "l"(__cvta_generic_to_global(p)) : "memory");
+    value = (unsigned long long)x;
+    status = (unsigned long long)(x >> 64);
+}
+
+// Publishes a chunk's record (three threads of a warp, a part each).
+__device__ __forceinline__ void publish(ChunkSlot *p, const ChunkRec &r, uint64_t epoch, uint32_t flag)
+{
+    const int k = g5_lane();
+    if (k < 3)
+        put_part(p->part[k],
+                 k == 0   ? r.v.x | (unsigned long long)r.v.y << 32
+                 : k == 1 ? r.v.z | (unsigned long long)r.v.w << 32
+                          : r.groups | (unsigned long long)r.exit << 32 | (unsigned long long)r.f << 63,
+                 epoch << 2 | flag);
+}
+
+// Waits for a chunk's record; its flag, or ST_NONE past the limit.
+__device__ __forceinline__ uint32_t await_record(const ChunkSlot *p, uint64_t epoch, ChunkRec &r)
+{
+    for (uint32_t spins = 0; spins <= kSpinLimit; ++spins) {
+        unsigned long long x[3], t[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) get_part(p->part[k], x[k], t[k]);
+        if ((t[0] >> 2) == epoch && t[0] == t[1] && t[0] == t[2]) {
+            r.v = make_uint4((uint32_t)x[0], (uint32_t)(x[0] >> 32), (uint32_t)x[1], (uint32_t)(x[1] >> 32));
+            r.groups = (uint32_t)x[2];
+            r.exit = (uint32_t)(x[2] >> 32) & 0x7FFFFFFFu;
+            r.f = (uint32_t)(x[2] >> 63);
+            return (uint32_t)(t[0] & 3u);
+        }
+    }
+    return ST_NONE;
+}
+
+// The groups and sums of chunks 0 .. c - 1, by the whole block, into sh.before
+// and sh.base; sh.exit: where the chain leaves chunk c - 1.  The stream's
+// records start at slots.
+__device__ void dec_before(DecShared &sh, uint64_t c, uint64_t epoch, const ChunkSlot *slots, uint64_t *err)
+{
+    if (threadIdx.x == 0) {
+        sh.before = 0;
+        sh.base = make_uint4(0, 0, 0, 0);
+    }
+    bool sums = true;  // no restart met yet
+    for (int64_t hi = (int64_t)c - 1; hi >= 0; hi -= kDB) {
+        if (threadIdx.x == 0) sh.near_reset = sh.near_inc = kDB;
+        __syncthreads();
+        const int64_t j = hi - threadIdx.x;  // thread 0: the nearest
+        ChunkRec r;
+        r.v = make_uint4(0, 0, 0, 0);
+        r.f = r.groups = 0;
+        r.exit = kDead;
+        if (j >= 0) {
+            const uint32_t flag = await_record(slots + j, epoch, r);
+            if (flag == ST_NONE) atomicOr((unsigned long long *)err, (unsigned long long)G5_DEVERR_WAIT);
+            // (the first chunk's own sums are all there are up to it)
+            const bool all = flag == ST_INC || j == 0;
+            if (all) atomicMin(&sh.near_inc, (int)threadIdx.x);
+            if (all || r.f) atomicMin(&sh.near_reset, (int)threadIdx.x);
+            if (hi == (int64_t)c - 1 && threadIdx.x == 0) sh.exit = r.exit;
+        }
+        __syncthreads();
+        const int ni = sh.near_inc, nr = sh.near_reset;
+        uint32_t g = (int)threadIdx.x <= ni ? r.groups : 0u;
+        uint4 v = sums && (int)threadIdx.x <= nr ? r.v : make_uint4(0, 0, 0, 0);
+        if (__any_sync(0xFFFFFFFFu, j >= 0)) {
+            g = __reduce_add_sync(0xFFFFFFFFu, g);
+            v.x = __reduce_add_sync(0xFFFFFFFFu, v.x);
+            v.y = __reduce_add_sync(0xFFFFFFFFu, v.y);
+            v.z = __reduce_add_sync(0xFFFFFFFFu, v.z);
+            v.w = __reduce_add_sync(0xFFFFFFFFu, v.w);
+            if (g5_lane() == 0) {
+                atomicAdd(&sh.before, (unsigned long long)g);
+                atomicAdd(&sh.base.x, v.x);
+                atomicAdd(&sh.base.y, v.y);
+                atomicAdd(&sh.base.z, v.z);
+                atomicAdd(&sh.base.w, v.w);
             }
         }
-        r.v = d;
+        __syncthreads();
+        sums = sums && nr == kDB;
+        if (ni < kDB) break;
     }
-    r.f = 0;
-    return r;
+    __syncthreads();
+}
+
+// Groups g0 .. g0 + cnt - 1 of the chunk (cnt <= kDG): their miniblocks' places
+// and widths (the first `nmb` of them), sums, and the sums before each from
+// the first on, `carry` before that; the total comes back in carry.
+__device__ void dec_sums(DecShared &sh, uint32_t g0, uint32_t nmb, int mode, uint4 &carry, uint32_t &carry_f)
+{
+    const int lane = g5_lane(), wid = threadIdx.x >> 5;
+    const uint32_t m = threadIdx.x;
+    __syncthreads();
+    if (m < nmb) {
+        const uint32_t p = sh.gpos[g0 + m / 16];
+        const uint4 h = sh.vec[p];
+        sh.mb[m] = (p + 1 + header_before(h, m & 15)) | width_of(h, m & 15) << 16;
+    }
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < 4 * nmb; k += kDB) {
+        const uint32_t x = sh.mb[k / 4], b = x >> 16;
+        const bool dm = mode == G5_CODEC_DM && b != 32;
+        reinterpret_cast<uint32_t *>(sh.v)[k] =
+            mb_sum(reinterpret_cast<const uint32_t *>(sh.vec + (x & 0xFFFFu)), b, dm ? 3 : k & 3);
+        if ((k & 3) == 0) sh.f[k / 4] = b == 32;
+    }
+    __syncthreads();
+    // exclusive scan with restarts over the miniblocks, one per thread
+    VecFlag x = ResetAdd::id();
+    if (m < nmb) {
+        x.v = sh.v[m];
+        x.f = sh.f[m];
+    }
+    const uint32_t warps = (nmb + 31) / 32;
+    VecFlag inc = x;
+    if ((uint32_t)wid < warps) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const VecFlag y = ResetAdd::shfl_up(inc, o);
+            if (lane >= o) inc = ResetAdd::op(y, inc);
+        }
+        if (lane == 31) {
+            sh.wv[wid] = inc.v;
+            sh.wf[wid] = inc.f;
+        }
+    }
+    __syncthreads();
+    VecFlag pre;
+    pre.v = carry;
+    pre.f = carry_f;
+    VecFlag mine = pre;
+    for (uint32_t w = 0; w < warps; ++w) {
+        VecFlag t;
+        t.v = sh.wv[w];
+        t.f = sh.wf[w];
+        if (w == (uint32_t)wid) mine = pre;
+        pre = ResetAdd::op(pre, t);
+    }
+    carry = pre.v;
+    carry_f = pre.f;
+    if ((uint32_t)wid < warps) {
+        VecFlag ex = ResetAdd::shfl_up(inc, 1);
+        if (lane == 0) ex = ResetAdd::id();
+        ex = ResetAdd::op(mine, ex);
+        if (m < nmb) {
+            sh.v[m] = ex.v;
+            // bit 1: the miniblock's base does not include what is before the chunk
+            sh.f[m] = (uint8_t)(x.f | (ex.f ? 2u : 0u));
+        }
+    }
+    __syncthreads();
 }
 
 // VariableByte tail decoded by one warp (variablebyte.h:217-): nbytes bytes
@@ -1206,185 +1146,296 @@ __device__ void dec_tail_warp(const uint8_t *bb, uint32_t nbytes, uint64_t cap, 
     e |= __reduce_or_sync(0xFFFFFFFFu, (unsigned)(e & G5_DEVERR_MISMATCH)) ? G5_DEVERR_MISMATCH : 0;
 }
 
-__global__ void __launch_bounds__(kOB) k_dec_unpack(const uint32_t *__restrict__ in, uint64_t *scal,
-                                                    const uint32_t *__restrict__ gpos, uint32_t *__restrict__ out,
-                                                    uint64_t cap, const uint64_t *n_expect,
-                                                    const uint32_t *__restrict__ expect, uint64_t *acc,
-                                                    uint64_t *ust, VecFlag *uagg, VecFlag *uinc, uint64_t *n_out,
-                                                    int mode)
+// Lane j's vector j of miniblock k held in sh (dec_sums).
+__device__ __forceinline__ uint4 held_values(const DecShared &sh, uint32_t k, int mode)
 {
-    extern __shared__ __align__(16) unsigned char s_dyn_u[];
-    uint4 *s_val = reinterpret_cast<uint4 *>(s_dyn_u);                        // values from each miniblock's start
-    VecFlag *s_vf = reinterpret_cast<VecFlag *>(s_dyn_u + kUValBytes);        // miniblock aggregates
-    VecFlag *s_base = s_vf + kTM;                                              // prefixes from the tile's start
-    uint4 *s_full = reinterpret_cast<uint4 *>(s_base + kTM);                   // each miniblock's base
-    uint8_t *s_raw = reinterpret_cast<uint8_t *>(s_full + kTM);                // 1: a raw miniblock
-    __shared__ VecFlag s_ex;            // the tile's aggregate, then its exclusive prefix (look-back)
-    __shared__ uint64_t s_t;
-    __shared__ uint32_t s_b[kTailMaxBytes / 4];
-    const int lane = g5_lane(), wid = threadIdx.x >> 5;
-    g5_pdl_sync();
-    const uint64_t epoch = scal[CS_U_EPOCH];
-    const uint64_t err0 = scal[CS_ERR];
-    const uint64_t words = scal[CS_WORDS];
+    const uint32_t x = sh.mb[k];
+    uint4 base = sh.v[k];
+    if (!(sh.f[k] & 2)) base = add4(base, sh.base);
+    return mb_values(reinterpret_cast<const uint32_t *>(sh.vec + (x & 0xFFFFu)), x >> 16, base, mode);
+}
+
+// Writes them, to out (miniblock 0's values first); true if one differs from
+// `expect`.  ANY: out has no alignment.
+template <bool ANY>
+__device__ __forceinline__ bool put_values(uint4 v, uint32_t k, uint32_t *out, const uint32_t *expect)
+{
+    const uint64_t at = 32 * (uint64_t)k + g5_lane();
+    if (ANY) {
+        uint32_t *o = out + 4 * at;
+        o[0] = v.x;
+        o[1] = v.y;
+        o[2] = v.z;
+        o[3] = v.w;
+        return false;
+    }
+    reinterpret_cast<uint4 *>(out)[at] = v;
+    if (!expect) return false;
+    const uint4 e = reinterpret_cast<const uint4 *>(expect)[at];
+    return (e.x != v.x) | (e.y != v.y) | (e.z != v.z) | (e.w != v.w);
+}
+
+// The values of miniblocks 0 .. nmb - 1 held in sh, by warps 0 .. warps - 1 two
+// at a time (one miniblock's chain of shuffles leaves the issue slots half
+// empty).
+template <bool ANY>
+__device__ __forceinline__ bool dec_out(DecShared &sh, uint32_t nmb, uint32_t warps, uint32_t *out,
+                                        const uint32_t *expect, int mode)
+{
     bool bad = false;
-    // the value count: final here for a raw stream or one the locator
-    // rejected, else the tail's writer below sets it
-    if (n_out && blockIdx.x == 0 && threadIdx.x == 0 && (scal[CS_RAW] || err0)) *n_out = scal[CS_N];
-    if (scal[CS_RAW]) {
-        const uint64_t n = scal[CS_N];
-        if (!err0)
-            for (uint64_t i = (uint64_t)blockIdx.x * kOB + threadIdx.x; i < n; i += (uint64_t)gridDim.x * kOB) {
-                out[i] = in[i];
-                bad |= expect && expect[i] != in[i];
-            }
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            if (n_expect && n != *n_expect)
-                atomicOr((unsigned long long *)&scal[CS_ERR], (unsigned long long)G5_DEVERR_MISMATCH);
-            if (acc) {
-                acc[0] += words;
-                acc[1] += n;
+    uint32_t k = threadIdx.x >> 5;
+    if (k >= warps) return false;
+    for (; k + warps < nmb; k += 2 * warps) {
+        const uint4 v = held_values(sh, k, mode), u = held_values(sh, k + warps, mode);
+        bad |= put_values<ANY>(v, k, out, expect);
+        bad |= put_values<ANY>(u, k + warps, out, expect);
+    }
+    if (k < nmb) bad |= put_values<ANY>(held_values(sh, k, mode), k, out, expect);
+    return bad;
+}
+
+// The VariableByte tail of a stream (variablebyte.h:217-), words from blkend
+// on, by one warp: values to out[n1 ..], their end in n.  Returns error bits.
+__device__ __noinline__ uint32_t dec_tail(uint32_t *s_b, const uint32_t *in, uint64_t words, uint64_t blkend,
+                                          uint64_t n1, uint64_t cap, uint32_t *out, const uint32_t *expect, uint64_t &n)
+{
+    const uint64_t tw = words > blkend ? words - blkend : 0;
+    n = 0;
+    if (tw * 4 > kTailMaxBytes) return G5_DEVERR_CORRUPT;
+    for (uint64_t i = g5_lane(); i < tw; i += 32) s_b[i] = in[blkend + i];
+    __syncwarp();
+    uint64_t o = n1, e = 0;
+    dec_tail_warp(reinterpret_cast<const uint8_t *>(s_b), (uint32_t)(tw * 4), cap, out, expect, o, e);
+    n = o;
+    return (uint32_t)e;
+}
+
+// Chunk c of the stream `in`: decodes the groups that start in it.  Returns
+// error bits (of this thread).  The block whose chunk holds the last group also
+// decodes the tail (in its last warp, beside the values) and leaves the
+// stream's value count in *count.
+template <bool ANY>
+__device__ uint32_t dec_chunk(DecShared &sh, const DecHead &h, const uint32_t *in, uint64_t c, uint64_t epoch,
+                              ChunkSlot *slots, uint64_t *err, uint32_t *out, uint64_t cap, const uint32_t *expect,
+                              int mode, uint64_t *count)
+{
+    const uint32_t S = h.S;
+    const uint64_t a = 1 + c * S;  // the chunk's first vector
+    const uint32_t len = (uint32_t)min((uint64_t)S, h.nv - a), have = (uint32_t)min((uint64_t)S + kSpan, h.nv - a);
+    const uint4 *v = reinterpret_cast<const uint4 *>(in) + a, *before = v - kSpan;
+    __syncthreads();  // the chunk before is no longer read
+    for (uint32_t p = threadIdx.x; p < have; p += kDB) {
+        const unsigned sa = (unsigned)__cvta_generic_to_shared(sh.vec + p);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(__cvta_generic_to_global(v + p)) : "memory");
+    }
+    if (threadIdx.x == 0) {
+        sh.vec[have] = make_uint4(0, 0, 0, 0);
+        sh.first = kDead;
+        sh.last = 0;
+        sh.entry = c == 0 ? 0u : kDead;
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    for (uint32_t p = threadIdx.x; p < len; p += kDB) {
+        const uint32_t sum = header_sum(sh.vec[p]);
+        sh.jump[p] = (uint16_t)(sum != kDead && a + p + 1 + sum <= h.nv ? p + 1 + sum : kDead);
+    }
+    __syncthreads();
+    // far enough from the end that a block part ending in this chunk would
+    // leave more tail than any stream has (kTailMaxBytes)
+    const bool inner = a + S + kSpan + kTailMaxBytes / 16 + 1 <= h.nv;
+    if (c > 0) {
+        for (uint32_t k = threadIdx.x; k < kSpan; k += kDB) {
+            const uint32_t sum = header_sum(before[k]);  // kSpan - k vectors before the chunk
+            if (sum == kDead || k + 1 + sum < kSpan) continue;
+            const uint32_t e = k + 1 + sum - kSpan;
+            uint32_t p = e;
+            while (inner && p < S) p = sh.jump[p];  // (kDead is past S)
+            if (p != kDead) {
+                atomicMin(&sh.first, e);
+                atomicMax(&sh.last, e);
             }
         }
-    } else if (!err0) {
-        const uint64_t nmb = scal[CS_NMB], ng = scal[CS_NG], n1 = scal[CS_N1];
-        // tiles of 8 groups when tiles of 4 would not all fit in one wave of
-        // the grid (fewer tiles, so a shorter look-back chain), else of 4 (more
-        // blocks at work on mid-size streams); every block decides alike
-        const int R = (ng + 3) / 4 > (uint64_t)gridDim.x ? 2 : 1;  // rounds of four miniblocks per warp
-        const uint64_t tm = 64ull * R;                              // miniblocks per tile
-        const uint64_t ntiles = (nmb + tm - 1) / tm;
-        if (blockIdx.x == 0 && wid == 0) {
-            // VariableByte tail (variablebyte.h:217-): words after the block part
-            const uint64_t blkend = scal[CS_BLKEND];
-            const uint64_t tw = words > blkend ? words - blkend : 0;
-            if (tw * 4 > kTailMaxBytes) {
-                if (lane == 0) {
-                    atomicOr((unsigned long long *)&scal[CS_ERR], (unsigned long long)G5_DEVERR_CORRUPT);
-                    if (n_out) *n_out = 0;
-                }
-            } else {
-                for (uint64_t i = lane; i < tw; i += 32) s_b[i] = in[blkend + i];
-                __syncwarp();
-                uint64_t o = n1, e = 0;
-                dec_tail_warp(reinterpret_cast<const uint8_t *>(s_b), (uint32_t)(tw * 4), cap, out, expect, o, e);
-                if (lane == 0) {
-                    scal[CS_N] = o;
-                    if (n_out) *n_out = o;
-                    if (n_expect && o != *n_expect) e |= G5_DEVERR_MISMATCH;
-                    if (e) atomicOr((unsigned long long *)&scal[CS_ERR], (unsigned long long)e);
-                    if (acc) {
-                        acc[0] += words;
-                        acc[1] += o;
-                    }
-                }
-            }
+        __syncthreads();
+    }
+    const bool known = c == 0 || (sh.first != kDead && sh.first == sh.last);
+    if (!known || c == 0) {
+        dec_before(sh, c, epoch, slots, err);
+        if (c > 0 && threadIdx.x == 0) sh.entry = sh.exit;
+    } else if (threadIdx.x == 0) {
+        sh.entry = sh.first;
+    }
+    // the chunk's groups: down the chain to the chunk's end or to a vector that
+    // is no header (no vector of a tail is: each value ends in a byte above 127)
+    if (threadIdx.x == 0) {
+        uint32_t p = sh.entry, g = 0, nx = p;
+        while (p < len && (nx = sh.jump[p]) != kDead) {
+            sh.gpos[g++] = (uint16_t)p;
+            p = nx;
         }
-        for (;;) {
-            const uint64_t t = claim_tile(&scal[CS_U_CTR], &s_t);
-            if (t >= ntiles) break;
-            const uint64_t k0 = tm * t;
-            // each warp's miniblocks wid, wid + 16, ..., four at a time: the
-            // positions and loads first, then one lane scan per miniblock,
-            // whose running sums are the values from the miniblock's start
-            // (for dm, components 0-2 take the running component 3 of the
-            // vector before) and whose lane 31 holds the aggregate
-#pragma unroll 1
-            for (int r = 0; r < R; ++r) {
-                uint4 d[4];
-                uint32_t b[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint64_t k = k0 + wid + 16 * (4 * r + i);
-                    d[i] = make_uint4(0, 0, 0, 0);
-                    b[i] = 0;
-                    if (k < nmb) {
-                        uint64_t off;
-                        mb_at(in, gpos[k / 16], wid, off, b[i]);
-                        d[i] = unpack_vec(in, off, b[i]);
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int m = wid + 16 * (4 * r + i);
-                    if (k0 + m < nmb) {
-                        const VecFlag agg = mb_scan(d[i], b[i], mode);
-                        uint4 rel = d[i];
-                        if (b[i] != 32 && mode == G5_CODEC_DM) {
-                            uint32_t cp = __shfl_up_sync(0xFFFFFFFFu, d[i].w, 1);
-                            if (lane == 0) cp = 0;
-                            rel = make_uint4(d[i].x + cp, d[i].y + cp, d[i].z + cp, d[i].w);
-                        }
-                        s_val[m * 32 + lane] = rel;
-                        if (lane == 31) s_vf[m] = agg;
-                        if (lane == 0) s_raw[m] = b[i] == 32 ? 1 : 0;
-                    } else if (lane == 31) {
-                        s_vf[m] = ResetAdd::id();
-                    }
-                }
-            }
-            __syncthreads();
-            if (wid == 0) {
-                // prefixes from the tile's start, 2 R miniblocks per lane in
-                // order (a reset inside the tile makes the rest absolute)
-                const int kPer = 2 * R;
-                VecFlag c = s_vf[kPer * lane];
-                for (int j = 1; j < kPer; ++j) c = ResetAdd::op(c, s_vf[kPer * lane + j]);
-                VecFlag inc = c;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const VecFlag y = ResetAdd::shfl_up(inc, o);
-                    if (lane >= o) inc = ResetAdd::op(y, inc);
-                }
-                VecFlag ex = ResetAdd::shfl_up(inc, 1);
-                if (lane == 0) ex = ResetAdd::id();
-                for (int j = 0; j < kPer; ++j) {
-                    s_base[kPer * lane + j] = ex;
-                    ex = ResetAdd::op(ex, s_vf[kPer * lane + j]);
-                }
-                if (lane == 31) s_ex = inc;  // the tile's aggregate, until the look-back replaces it
-            }
-            __syncthreads();
-            // warp 0 finds the tile's prefix (look-back), then every
-            // miniblock's base: the tile's prefix combined with the
-            // miniblock's prefix inside the tile
-            if (wid == 0) {
-                const VecFlag pre = lookback<ResetAddV>(ust, uagg, uinc, t, epoch, s_ex, &scal[CS_ERR]);
-                for (int m = lane; m < (int)tm; m += 32) s_full[m] = ResetAdd::op(pre, s_base[m]).v;
-            }
-            __syncthreads();
-            {
-                const uint64_t kn = min(tm, nmb - k0);  // miniblocks in this tile
-                for (uint32_t q = threadIdx.x; q < kn * 32; q += kOB) {
-                    const uint32_t m = q >> 5;  // miniblock of this 16-byte vector
-                    uint4 x = s_val[q];
-                    if (!s_raw[m]) {
-                        const uint4 bm = s_full[m];
-                        if (mode == G5_CODEC_DM) {
-                            x.x += bm.w;
-                            x.y += bm.w;
-                            x.z += bm.w;
-                            x.w += bm.w;
-                        } else {
-                            x.x += bm.x;
-                            x.y += bm.y;
-                            x.z += bm.z;
-                            x.w += bm.w;
-                        }
-                    }
-                    reinterpret_cast<uint4 *>(out)[k0 * 32 + q] = x;
-                    if (expect) {
-                        const uint4 e = reinterpret_cast<const uint4 *>(expect)[k0 * 32 + q];
-                        bad |= (e.x != x.x) | (e.y != x.y) | (e.z != x.z) | (e.w != x.w);
-                    }
-                }
-            }
+        sh.groups = g;
+        sh.exit = nx == kDead || len < S ? kDead : p - S;
+        sh.stop = nx == kDead && p < len ? p : kDead;
+    }
+    __syncthreads();
+    uint32_t groups = sh.groups;
+    const uint32_t exit = sh.exit, entry = sh.entry;
+    if (!(known && c > 0) && sh.before + groups >= h.ng) groups = (uint32_t)(h.ng - min(h.ng, (uint64_t)sh.before));
+    // sums of the whole chunk (a last group that is not full has widths of 0
+    // where its miniblocks are missing: they add nothing)
+    uint4 cv = make_uint4(0, 0, 0, 0);
+    uint32_t cf = 0;
+    const uint32_t batches = (groups + kDG - 1) / kDG;
+    for (uint32_t i = 0; i < batches; ++i)
+        dec_sums(sh, i * kDG, min(16 * (groups - i * kDG), (uint32_t)kDM), mode, cv, cf);
+    // publish, and for an entry found alone the sums before
+    if (threadIdx.x < 32) {
+        ChunkRec r;
+        r.v = cv;
+        r.f = cf;
+        r.exit = exit;
+        r.groups = groups;
+        if (!known || c == 0) {
+            r.v = cf ? cv : add4(cv, sh.base);
+            r.f = 1;
+            r.groups = (uint32_t)(sh.before + groups);
+            publish(slots + c, r, epoch, ST_INC);
+        } else {
+            publish(slots + c, r, epoch, ST_AGG);
         }
     }
-    if (bad) atomicOr((unsigned long long *)&scal[CS_ERR], (unsigned long long)G5_DEVERR_MISMATCH);
+    if (known && c > 0) {
+        dec_before(sh, c, epoch, slots, err);
+        if (h.nchunks > (uint64_t)kDB && threadIdx.x < 32) {
+            // more chunks than one look reaches: everything up to this one
+            ChunkRec r;
+            r.v = cf ? cv : add4(cv, sh.base);
+            r.f = 1;
+            r.exit = exit;
+            r.groups = (uint32_t)(sh.before + groups);
+            publish(slots + c, r, epoch, ST_INC);
+        }
+        if (sh.before < h.ng && sh.exit != kDead && sh.exit != entry) return G5_DEVERR_CORRUPT;
+    }
+    // where the chain comes from: the chunk before's exit (the unknown entry's
+    // block has it as its entry)
+    const bool ended = c > 0 && (known ? sh.exit : entry) == kDead;
+    const uint64_t first = sh.before;
+    // the chain ended before this chunk (there it was checked to be complete)
+    if (first >= h.ng || ended) return 0;
+    const uint32_t rest = (uint32_t)(h.nmb - 16 * (h.ng - 1));  // miniblocks of the last group
+    bool again = batches > 1;  // the sums held are not the first batch's
+    if (first + groups < h.ng && sh.stop != kDead) {
+        // the chain stops before the last group, unless this is the last one,
+        // whose header need not be one past its `rest` widths
+        const uint32_t p = sh.stop;
+        const uint4 hv = sh.vec[p];
+        bool ok = first + groups + 1 == h.ng && a + p + 1 + header_before(hv, (int)rest) <= h.nv;
+        for (uint32_t q = 0; q < rest; ++q) ok &= width_of(hv, (int)q) <= 32;
+        if (!ok) return G5_DEVERR_CORRUPT;
+        if (threadIdx.x == 0) sh.gpos[groups] = (uint16_t)p;
+        ++groups;
+        again = true;  // (dec_sums begins with a barrier)
+    }
+    const uint32_t nmb = (uint32_t)min((uint64_t)16 * groups, h.nmb - 16 * first);
+    uint32_t bad = 0, warps = kDW;
+    if (first + groups >= h.ng) {
+        // the stream's last group, which may hold fewer miniblocks
+        if (again) __syncthreads();
+        --warps;
+        if (threadIdx.x >> 5 == warps) {
+            const uint32_t p = sh.gpos[h.ng - 1 - first];
+            uint64_t n;
+            bad = dec_tail(sh.tail, in, h.words, 4 * (a + p + 1 + header_before(sh.vec[p], (int)rest)), h.n1, cap, out,
+                           expect, n);
+            if (g5_lane() == 0) *count = n;
+        }
+    } else if (c + 1 == h.nchunks) {
+        return G5_DEVERR_CORRUPT;  // the stream ends before the last group
+    }
+    const uint64_t k0 = 16 * first;
+    bool diff = false;
+    uint4 rv = make_uint4(0, 0, 0, 0);
+    uint32_t rf = 0;
+    for (uint32_t i = 0; i * kDM < nmb; ++i) {
+        const uint32_t n = min(nmb - i * kDM, (uint32_t)kDM);
+        if (again) dec_sums(sh, i * kDG, n, mode, rv, rf);
+        const uint64_t at = 128 * (k0 + (uint64_t)i * kDM);
+        diff |= dec_out<ANY>(sh, n, warps, out + at, expect ? expect + at : nullptr, mode);
+    }
+    return bad | (diff ? (uint32_t)G5_DEVERR_MISMATCH : 0u);
+}
+
+// One stream.  With `expect` every value is compared with the expected one
+// (the level loop's round-trip check); `acc` accumulates words and values; the
+// count goes to n_out and, with the words and error bits, to `result` (pinned
+// host memory), each if given.  Blocks claim chunks in launch order, so a
+// chunk only ever waits on chunks whose blocks already run; records hold the
+// call's epoch, so what earlier calls left reads as "not published".
+__global__ void __launch_bounds__(kDB, 2) k_decode(const uint32_t *__restrict__ in, const uint64_t *words_dev,
+                                                   uint64_t words_val, uint32_t *__restrict__ out, uint64_t cap,
+                                                   uint64_t raw_thr, const uint64_t *n_expect,
+                                                   const uint32_t *__restrict__ expect, uint64_t *acc, uint64_t *scal,
+                                                   ChunkSlot *slots, uint64_t max_vec, uint64_t max_mb,
+                                                   uint64_t *n_out, uint64_t *result, int mode)
+{
+    extern __shared__ __align__(16) unsigned char s_dyn_d[];
+    DecShared &sh = *reinterpret_cast<DecShared *>(s_dyn_d);
+    g5_pdl_sync();
+    const uint64_t epoch = scal[CS_U_EPOCH];
+    const DecHead h = dec_head(in, words_dev ? *words_dev : words_val, cap, raw_thr, n_expect, max_vec, max_mb,
+                               gridDim.x);
+    uint32_t bad = 0;
+    if (h.raw) {
+        if (!h.bad)
+            for (uint64_t i = (uint64_t)blockIdx.x * kDB + threadIdx.x; i < h.words; i += (uint64_t)gridDim.x * kDB) {
+                const uint32_t x = in[i];
+                out[i] = x;
+                if (expect && expect[i] != x) bad |= G5_DEVERR_MISMATCH;
+            }
+    } else if (!h.bad) {
+        for (;;) {
+            const uint64_t c = claim_tile(&scal[CS_U_CTR], &sh.t);
+            if (c >= h.nchunks) break;
+            bad |= dec_chunk<false>(sh, h, in, c, epoch, slots, &scal[CS_U_ERR], out, cap, expect, mode, &scal[CS_U_N]);
+        }
+        if (h.ng == 0 && blockIdx.x == 0 && threadIdx.x < 32) {
+            uint64_t n;
+            bad |= dec_tail(sh.tail, in, h.words, 4, 0, cap, out, expect, n);
+            if (g5_lane() == 0) scal[CS_U_N] = n;
+        }
+    }
+    if (bad) atomicOr((unsigned long long *)&scal[CS_U_ERR], (unsigned long long)bad);
     if (last_block(&scal[CS_U_DONE])) {
+        __threadfence();
+        uint64_t e = vload64(&scal[CS_U_ERR]), n = vload64(&scal[CS_U_N]);
+        if (h.bad) e |= G5_DEVERR_CORRUPT;
+        if (h.raw) {
+            n = h.words;
+            if (n != *n_expect) e |= G5_DEVERR_MISMATCH;
+        } else if (e & ~(uint64_t)G5_DEVERR_MISMATCH) {
+            n = 0;
+        } else if (n_expect && n != *n_expect) {
+            e |= G5_DEVERR_MISMATCH;
+        }
+        scal[CS_ERR] = e;
+        scal[CS_N] = n;
+        scal[CS_WORDS] = h.words;
+        scal[CS_N1] = h.n1;
+        if (n_out) *n_out = n;
+        if (acc) {
+            acc[0] += h.words;
+            acc[1] += n;
+        }
+        if (result) {
+            result[0] = n;
+            result[1] = h.words;
+            result[2] = e;
+        }
         scal[CS_U_CTR] = 0;
         scal[CS_U_DONE] = 0;
+        scal[CS_U_ERR] = 0;
+        scal[CS_U_N] = 0;
         scal[CS_U_EPOCH] = epoch + 1;
         __threadfence();
     }
@@ -1827,7 +1878,12 @@ size_t codec_bound(size_t n)
 
 size_t codec_tiles(size_t max_n) { return (max_n / 128 + 1) / 16 + 2; }
 
-size_t codec_chunks(size_t max_n) { return (codec_bound(max_n) / 4 + 2) / kLocMin + 2; }
+// chunks of the longest stream: one per block, or as many of the largest size
+// as it takes
+size_t codec_chunks(size_t max_n)
+{
+    return std::max((size_t)codec_grid(), (codec_bound(max_n) / 4 + 2) / kMaxChunk) + 2;
+}
 
 int codec_grid() { return num_sms() * 2; }
 
@@ -1839,23 +1895,15 @@ g5_status codec_work_alloc(CodecWork &w, size_t max_n)
     w.grid = codec_grid();
     const size_t T = codec_tiles(max_n), C = codec_chunks(max_n);
     G5_CUDA(cudaMalloc(&w.scal, sizeof(uint64_t) * kScalars));
-    G5_CUDA(cudaMalloc(&w.gpos, sizeof(uint32_t) * T));
     w.enc_blocks = w.grid;
     G5_CUDA(cudaMalloc(&w.ewb, 16 * T));
     G5_CUDA(cudaMalloc(&w.etot, sizeof(uint64_t) * w.enc_blocks));
-    G5_CUDA(cudaMalloc(&w.ltab, sizeof(uint32_t) * kEntries * C));
-    G5_CUDA(cudaMalloc(&w.lent, sizeof(uint64_t) * C));
-    G5_CUDA(cudaMalloc(&w.ljump, sizeof(uint16_t) * (w.max_vec + 2)));
-    // the walk's table cache needs more than 48 KB of shared memory (set per device)
-    G5_CUDA(cudaFuncSetAttribute(k_loc_walk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(uint32_t) * kEntries * kLocFit)));
-    G5_CUDA(cudaFuncSetAttribute(k_dec_unpack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUSmem));
-    G5_CUDA(cudaMalloc(&w.ust, sizeof(uint64_t) * T));
-    G5_CUDA(cudaMalloc(&w.uagg, sizeof(VecFlag) * 2 * T));
-    w.uinc = w.uagg + T;
+    // the decoder's shared memory needs more than 48 KB (set per device)
+    G5_CUDA(cudaFuncSetAttribute(k_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecShared)));
+    G5_CUDA(cudaMalloc(&w.slots, sizeof(ChunkSlot) * C));
     // epochs start at 1, so zeroed status words read as "not published"
     G5_CUDA(cudaMemset(w.scal, 0, sizeof(uint64_t) * kScalars));
-    G5_CUDA(cudaMemset(w.ust, 0, sizeof(uint64_t) * T));
+    G5_CUDA(cudaMemset(w.slots, 0, sizeof(ChunkSlot) * C));
     const uint64_t one = 1;
     for (int e : {CS_U_EPOCH})
         G5_CUDA(cudaMemcpy(w.scal + e, &one, sizeof one, cudaMemcpyHostToDevice));
@@ -1865,14 +1913,9 @@ g5_status codec_work_alloc(CodecWork &w, size_t max_n)
 void codec_work_free(CodecWork &w)
 {
     cudaFree(w.scal);
-    cudaFree(w.gpos);
     cudaFree(w.ewb);
     cudaFree(w.etot);
-    cudaFree(w.ltab);
-    cudaFree(w.lent);
-    cudaFree(w.ljump);
-    cudaFree(w.ust);
-    cudaFree(w.uagg);
+    cudaFree(w.slots);
     w = CodecWork();
 }
 
@@ -1887,26 +1930,18 @@ void codec_encode_launch(CodecWork &w, const uint32_t *in, const uint64_t *n_dev
            (const uint8_t *)w.ewb, (const uint64_t *)w.etot, nb, words_out, mode);
 }
 
-void codec_decode_launch(CodecWork &w, const uint32_t *in, const uint64_t *words_dev, uint32_t *out, size_t cap,
-                         int mode, uint64_t raw_threshold, const uint64_t *n_expect_dev, const uint32_t *expect,
-                         cudaStream_t s, uint64_t *n_out)
+void codec_decode_launch(CodecWork &w, const uint32_t *in, const uint64_t *words_dev, uint64_t words, uint32_t *out,
+                         size_t cap, int mode, uint64_t raw_threshold, const uint64_t *n_expect_dev,
+                         const uint32_t *expect, uint64_t *acc, cudaStream_t s, uint64_t *n_out, uint64_t *result)
 {
-    decode_launch_acc(w, in, words_dev, out, cap, mode, raw_threshold, n_expect_dev, expect, nullptr, s, n_out);
-}
-
-void decode_launch_acc(CodecWork &w, const uint32_t *in, const uint64_t *words_dev, uint32_t *out, size_t cap,
-                       int mode, uint64_t raw_threshold, const uint64_t *n_expect_dev, const uint32_t *expect,
-                       uint64_t *acc, cudaStream_t s, uint64_t *n_out)
-{
-    // programmatic dependent launches: each kernel's first instruction waits
-    // for the kernel before it, so only the launch latency is overlapped
-    const uint64_t mv = w.max_vec, mm = w.max_mb, c = cap, rt = raw_threshold;
-    launch(true, k_loc_tables, w.grid, kOB, s, in, words_dev, c, rt, n_expect_dev, w.scal, mv, mm, w.ltab, w.ljump);
-    launch_dyn(true, k_loc_walk, 1, kWalkThreads, sizeof(uint32_t) * kEntries * kLocFit, s, in, words_dev, c, rt,
-               n_expect_dev, w.scal, mv, mm, (const uint32_t *)w.ltab, w.lent);
-    launch(true, k_loc_pos, w.grid, kOB, s, in, w.scal, (const uint16_t *)w.ljump, (const uint64_t *)w.lent, w.gpos);
-    launch_dyn(true, k_dec_unpack, w.grid, kOB, kUSmem, s, in, w.scal, (const uint32_t *)w.gpos, out, c,
-               n_expect_dev, expect, acc, w.ust, w.uagg, w.uinc, n_out, mode);
+    // a programmatic dependent launch: the kernel's first instruction waits
+    // for the kernel before it, so only the launch latency is overlapped.  A
+    // length known here needs no more blocks than it has chunks.
+    const uint64_t chunks = words_dev ? (uint64_t)w.grid : std::max<uint64_t>(1, (words / 4 + kMinChunk - 1) / kMinChunk);
+    const int grid = (int)std::min<uint64_t>(w.grid, chunks);
+    launch_dyn(true, k_decode, grid, kDB, sizeof(DecShared), s, in, words_dev, words, out, (uint64_t)cap,
+               raw_threshold, n_expect_dev, expect, acc, w.scal, static_cast<ChunkSlot *>(w.slots),
+               (uint64_t)w.max_vec, (uint64_t)w.max_mb, n_out, result, mode);
 }
 
 }  // namespace g5
@@ -2013,15 +2048,14 @@ g5_status g5_codec_decode(g5_codec *c, const uint32_t *in_dev, size_t words, uin
     if (((uintptr_t)in_dev | (uintptr_t)out_dev) & 15) return G5_ERR_INVALID_ARG;
     if (words / 4 > c->w.max_vec) return G5_ERR_CAPACITY;
     cudaStream_t s = (cudaStream_t)stream;
-    c->h_scal[15] = words;
-    G5_CUDA(cudaMemcpyAsync(c->n_dev + 1, &c->h_scal[15], sizeof(uint64_t), cudaMemcpyHostToDevice, s));
-    g5::codec_decode_launch(c->w, in_dev, c->n_dev + 1, out_dev, out_cap, mode, 0, nullptr, nullptr, s);
+    // the kernel leaves the count and status in pinned memory itself
+    g5::codec_decode_launch(c->w, in_dev, nullptr, words, out_dev, out_cap, mode, 0, nullptr, nullptr, nullptr, s,
+                            nullptr, c->h_scal);
     G5_CUDA(cudaGetLastError());
-    G5_CUDA(cudaMemcpyAsync(c->h_scal, c->w.scal, sizeof(uint64_t) * 8, cudaMemcpyDeviceToHost, s));
     G5_CUDA(cudaStreamSynchronize(s));
-    if (c->h_scal[g5::CS_ERR] & G5_DEVERR_WAIT) return G5_ERR_TIMEOUT;
-    if (c->h_scal[g5::CS_ERR]) return G5_ERR_CORRUPT_STREAM;
-    *out_n = (size_t)c->h_scal[g5::CS_N];
+    if (c->h_scal[2] & G5_DEVERR_WAIT) return G5_ERR_TIMEOUT;
+    if (c->h_scal[2]) return G5_ERR_CORRUPT_STREAM;
+    *out_n = (size_t)c->h_scal[0];
     return G5_OK;
 }
 
@@ -2044,7 +2078,8 @@ g5_status g5_codec_decode_async(g5_codec *c, const uint32_t *in_dev, const uint6
     if (mode != G5_CODEC_D4 && mode != G5_CODEC_DM) return G5_ERR_INVALID_ARG;
     if (((uintptr_t)in_dev | (uintptr_t)out_dev) & 15) return G5_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    g5::codec_decode_launch(c->w, in_dev, words_dev, out_dev, out_cap, mode, 0, nullptr, nullptr, s, out_n_dev);
+    g5::codec_decode_launch(c->w, in_dev, words_dev, 0, out_dev, out_cap, mode, 0, nullptr, nullptr, nullptr, s,
+                            out_n_dev, nullptr);
     G5_CUDA(cudaGetLastError());
     return G5_OK;
 }
