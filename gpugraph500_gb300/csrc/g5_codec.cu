@@ -668,7 +668,9 @@ __global__ void __launch_bounds__(kEB, 2) k_enc_pack(const uint32_t *__restrict_
 //           is the one, known without any other chunk.  The first chunk's entry
 //           is given.  (Near the stream's end the chain may stop in the chunk:
 //           there every entry counts.)  Else the block waits for the chunk before
-//           to tell its exit.
+//           to tell its exit, which that one mostly knows all the same: chains
+//           from several entries run together.  (Only miniblocks of a bit or
+//           two look like headers; no sorted queue of distinct ids has them.)
 //   sums    the lane sums of every miniblock and, in order, of the chunk
 //           (a raw b = 32 miniblock restarts them)
 //   meet    the chunk publishes its entry, exit, groups and sums, and adds up
@@ -691,8 +693,8 @@ constexpr int kSpan = 513;         // a group spans at most 1 + 16 * 32 vectors
 constexpr uint32_t kDead = 0xFFFFu;
 constexpr int kDB = 512;           // threads per block
 constexpr int kDW = kDB / 32;
-constexpr uint32_t kMinChunk = 576, kMaxChunk = 1536;  // vectors per chunk (more than kSpan: every
-                                                       // chunk holds its entry)
+constexpr uint32_t kMinChunk = 16, kMidChunk = 576, kMaxChunk = 1536;  // vectors per chunk
+constexpr uint64_t kChunkValues = 32768;  // values a chunk shorter than kMidChunk should have
 constexpr int kDG = 32;            // groups whose miniblocks are held together
 constexpr int kDM = 16 * kDG;
 
@@ -706,9 +708,10 @@ struct ChunkRec {
     uint32_t exit;    // where the chain enters the next chunk (kDead: it does not)
     uint32_t groups;
 };
+// The fourth part is the exit alone, published before the sums, so that a run
+// of chunks that wait for their entries waits for a walk each and no more.
 struct __align__(64) ChunkSlot {
-    unsigned long long part[3][2];
-    unsigned long long pad[2];
+    unsigned long long part[4][2];
 };
 
 struct DecShared {
@@ -725,6 +728,7 @@ struct DecShared {
     uint32_t entry, exit, groups;
     uint32_t stop;                        // the vector the chain stops at, if it is in the chunk
     uint32_t first, last;                 // least and greatest entry that came up
+    uint32_t xfirst, xlast;               // and exit their chains lead to
     uint4 cv;                             // the chunk's sums
     uint32_t cf;
     unsigned long long before;            // groups before the chunk
@@ -744,11 +748,15 @@ struct DecHead {
     bool raw, bad;
 };
 
-// Chunk size: one chunk per block where that leaves it between the limits.
+// Chunk size: one chunk per block, but none shorter than kMidChunk unless the
+// stream packs so many values into a vector that such chunks would hold far
+// more than kChunkValues.
 __device__ __forceinline__ void dec_chunks(DecHead &h, uint32_t blocks)
 {
     const uint64_t per = (h.nv + blocks - 1) / blocks;
-    h.S = (uint32_t)min((uint64_t)kMaxChunk, max((uint64_t)kMinChunk, (per + 63) & ~(uint64_t)63));
+    const uint64_t few = h.n1 > kChunkValues ? min((uint64_t)kMidChunk, kChunkValues * h.nv / h.n1) : kMidChunk;
+    h.S = (uint32_t)min((uint64_t)kMaxChunk, (max(per, few) + kMinChunk - 1) / kMinChunk * kMinChunk);
+    if (h.S < kMinChunk) h.S = kMinChunk;
     h.nchunks = h.nv > 1 ? (h.nv - 1 + h.S - 1) / h.S : 0;
 }
 
@@ -760,7 +768,7 @@ __device__ __forceinline__ DecHead dec_head(const uint32_t *in, uint64_t words, 
     h.words = words;
     h.nv = words / 4;
     h.n1 = h.nmb = h.ng = h.nchunks = 0;
-    h.S = kMinChunk;
+    h.S = kMidChunk;
     h.bad = false;
     // plugin semantics: raw when n <= thr or the stream is as long as n
     // (cpu_2d/compression/cpusimd.hh:169-173)
@@ -948,6 +956,18 @@ __device__ __forceinline__ void publish(ChunkSlot *p, const ChunkRec &r, uint64_
                  epoch << 2 | flag);
 }
 
+// Waits for a chunk's exit; kDead past the limit.
+__device__ __forceinline__ uint32_t await_exit(const ChunkSlot *p, uint64_t epoch, uint64_t *err)
+{
+    for (uint32_t spins = 0; spins <= kSpinLimit; ++spins) {
+        unsigned long long x, t;
+        get_part(p->part[3], x, t);
+        if ((t >> 2) == epoch) return (uint32_t)x;
+    }
+    atomicOr((unsigned long long *)err, (unsigned long long)G5_DEVERR_WAIT);
+    return kDead;
+}
+
 // Waits for a chunk's record; its flag, or ST_NONE past the limit.
 __device__ __forceinline__ uint32_t await_record(const ChunkSlot *p, uint64_t epoch, ChunkRec &r)
 {
@@ -987,8 +1007,7 @@ __device__ void dec_before(DecShared &sh, uint64_t c, uint64_t epoch, const Chun
         if (j >= 0) {
             const uint32_t flag = await_record(slots + j, epoch, r);
             if (flag == ST_NONE) atomicOr((unsigned long long *)err, (unsigned long long)G5_DEVERR_WAIT);
-            // (the first chunk's own sums are all there are up to it)
-            const bool all = flag == ST_INC || j == 0;
+            const bool all = flag == ST_INC;
             if (all) atomicMin(&sh.near_inc, (int)threadIdx.x);
             if (all || r.f) atomicMin(&sh.near_reset, (int)threadIdx.x);
             if (hi == (int64_t)c - 1 && threadIdx.x == 0) sh.exit = r.exit;
@@ -1230,8 +1249,8 @@ __device__ uint32_t dec_chunk(DecShared &sh, const DecHead &h, const uint32_t *i
     }
     if (threadIdx.x == 0) {
         sh.vec[have] = make_uint4(0, 0, 0, 0);
-        sh.first = kDead;
-        sh.last = 0;
+        sh.first = sh.xfirst = kDead;
+        sh.last = sh.xlast = 0;
         sh.entry = c == 0 ? 0u : kDead;
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -1246,6 +1265,7 @@ __device__ uint32_t dec_chunk(DecShared &sh, const DecHead &h, const uint32_t *i
     const bool inner = a + S + kSpan + kTailMaxBytes / 16 + 1 <= h.nv;
     if (c > 0) {
         for (uint32_t k = threadIdx.x; k < kSpan; k += kDB) {
+            if (a + k < kSpan + 1) continue;  // (before the first group)
             const uint32_t sum = header_sum(before[k]);  // kSpan - k vectors before the chunk
             if (sum == kDead || k + 1 + sum < kSpan) continue;
             const uint32_t e = k + 1 + sum - kSpan;
@@ -1254,20 +1274,23 @@ __device__ uint32_t dec_chunk(DecShared &sh, const DecHead &h, const uint32_t *i
             if (p != kDead) {
                 atomicMin(&sh.first, e);
                 atomicMax(&sh.last, e);
+                atomicMin(&sh.xfirst, p - S);
+                atomicMax(&sh.xlast, p - S);
             }
         }
         __syncthreads();
     }
-    const bool known = c == 0 || (sh.first != kDead && sh.first == sh.last);
-    if (!known || c == 0) {
-        dec_before(sh, c, epoch, slots, err);
-        if (c > 0 && threadIdx.x == 0) sh.entry = sh.exit;
-    } else if (threadIdx.x == 0) {
-        sh.entry = sh.first;
-    }
     // the chunk's groups: down the chain to the chunk's end or to a vector that
     // is no header (no vector of a tail is: each value ends in a byte above 127)
     if (threadIdx.x == 0) {
+        if (c > 0 && sh.first != kDead && sh.first == sh.last) {
+            sh.entry = sh.first;
+        } else if (c > 0) {
+            // (one of the entries that came up is the real one)
+            if (inner && sh.first != kDead && sh.xfirst == sh.xlast)
+                put_part(slots[c].part[3], sh.xfirst, epoch << 2 | ST_AGG);
+            sh.entry = await_exit(slots + c - 1, epoch, err);
+        }
         uint32_t p = sh.entry, g = 0, nx = p;
         while (p < len && (nx = sh.jump[p]) != kDead) {
             sh.gpos[g++] = (uint16_t)p;
@@ -1276,11 +1299,11 @@ __device__ uint32_t dec_chunk(DecShared &sh, const DecHead &h, const uint32_t *i
         sh.groups = g;
         sh.exit = nx == kDead || len < S ? kDead : p - S;
         sh.stop = nx == kDead && p < len ? p : kDead;
+        put_part(slots[c].part[3], sh.exit, epoch << 2 | ST_AGG);
     }
     __syncthreads();
     uint32_t groups = sh.groups;
     const uint32_t exit = sh.exit, entry = sh.entry;
-    if (!(known && c > 0) && sh.before + groups >= h.ng) groups = (uint32_t)(h.ng - min(h.ng, (uint64_t)sh.before));
     // sums of the whole chunk (a last group that is not full has widths of 0
     // where its miniblocks are missing: they add nothing)
     uint4 cv = make_uint4(0, 0, 0, 0);
@@ -1288,38 +1311,26 @@ __device__ uint32_t dec_chunk(DecShared &sh, const DecHead &h, const uint32_t *i
     const uint32_t batches = (groups + kDG - 1) / kDG;
     for (uint32_t i = 0; i < batches; ++i)
         dec_sums(sh, i * kDG, min(16 * (groups - i * kDG), (uint32_t)kDM), mode, cv, cf);
-    // publish, and for an entry found alone the sums before
-    if (threadIdx.x < 32) {
-        ChunkRec r;
-        r.v = cv;
-        r.f = cf;
-        r.exit = exit;
-        r.groups = groups;
-        if (!known || c == 0) {
-            r.v = cf ? cv : add4(cv, sh.base);
-            r.f = 1;
-            r.groups = (uint32_t)(sh.before + groups);
-            publish(slots + c, r, epoch, ST_INC);
-        } else {
-            publish(slots + c, r, epoch, ST_AGG);
-        }
-    }
-    if (known && c > 0) {
-        dec_before(sh, c, epoch, slots, err);
+    // publish, then add up what is before (the first chunk's own sums are all
+    // there are up to it)
+    ChunkRec r;
+    r.v = cv;
+    r.f = cf;
+    r.exit = exit;
+    r.groups = groups;
+    if (threadIdx.x < 32) publish(slots + c, r, epoch, c == 0 ? ST_INC : ST_AGG);
+    dec_before(sh, c, epoch, slots, err);
+    if (c > 0) {
         if (h.nchunks > (uint64_t)kDB && threadIdx.x < 32) {
             // more chunks than one look reaches: everything up to this one
-            ChunkRec r;
             r.v = cf ? cv : add4(cv, sh.base);
             r.f = 1;
-            r.exit = exit;
             r.groups = (uint32_t)(sh.before + groups);
             publish(slots + c, r, epoch, ST_INC);
         }
         if (sh.before < h.ng && sh.exit != kDead && sh.exit != entry) return G5_DEVERR_CORRUPT;
     }
-    // where the chain comes from: the chunk before's exit (the unknown entry's
-    // block has it as its entry)
-    const bool ended = c > 0 && (known ? sh.exit : entry) == kDead;
+    const bool ended = c > 0 && sh.exit == kDead;
     const uint64_t first = sh.before;
     // the chain ended before this chunk (there it was checked to be complete)
     if (first >= h.ng || ended) return 0;
