@@ -1359,8 +1359,8 @@ void enqueue_level(g5_bfs *b, const BfsArgs &a, cudaStream_t s, Prof *pf = nullp
     }
     p.mark(KP_CODEC, s);
     if (a.codec) {
-        g5::codec_encode_launch(b->cw, b->queue, &b->st->nf, b->codec_stream, a.codec,
-                                b->cfg.codec_threshold, s);
+        g5::codec_encode_launch(b->cw, b->queue, &b->st->nf, 0, b->codec_stream, a.codec, b->cfg.codec_threshold, s,
+                                nullptr, nullptr);
         // the stream copy is launched only while a caller has a buffer set
         if (b->capture_on) k_codec_capture<<<g5::grid_for(1), kBlock, 0, s>>>(a.ccap, b->codec_stream, b->cw.scal, b->st);
         g5::codec_decode_launch(b->cw, b->codec_stream, b->cw.scal + g5::CS_WORDS, 0, b->dqueue, (size_t)a.n, a.codec,

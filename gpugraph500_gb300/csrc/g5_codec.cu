@@ -21,10 +21,9 @@
 //   little-endian, high bit on the last byte, zero-padded to a word.
 //
 // GPU design, one stream per call: every miniblock is independent for
-// encoding (its deltas only need the input), so one warp packs one
-// miniblock; a first launch stores every miniblock's bit width and the word
-// count of each block's range of groups, a second one places each range
-// after the ranges before it and packs (two launches, no device waits).
+// encoding (its deltas only need the input), so one warp packs one miniblock,
+// and a chunk's place in the stream is the sum of the word counts that the
+// chunks before it publish.
 // Decoding needs each group's position, which the stream only gives as a
 // chain (each header says how long its group is), and the sums of all values
 // before it: one launch, a block per chunk of the stream, which finds its own
@@ -48,10 +47,6 @@ namespace {
 constexpr uint32_t kCookie = 123456u;
 constexpr int kB = 256;
 constexpr int kTailMaxBytes = 4096;  // largest VariableByte tail decoded
-
-// extra scalar slots (beyond CodecScalar)
-enum { CS_NMB = 5, CS_RAW = 6, CS_NG = 7 };
-// the scalar block holds CS_COUNT entries; decode uses a few more
 
 __device__ __forceinline__ uint32_t bits_of(uint32_t v) { return v ? 32u - __clz(v) : 0u; }
 
@@ -270,10 +265,34 @@ __device__ __forceinline__ void mb_locate(const uint32_t *in, const uint32_t *gp
 constexpr uint32_t kSpinLimit = 1u << 21;
 enum : uint32_t { ST_NONE = 0, ST_AGG = 1, ST_INC = 2 };
 
-// scalar slots of the decoder (the scalar block holds kScalars)
+// scalar slots of the two (the scalar block holds kScalars)
+enum { CS_E_CTR = 20, CS_E_DONE = 21, CS_E_EPOCH = 22, CS_E_ERR = 23, CS_E_WORDS = 24 };
 enum { CS_U_CTR = 25, CS_U_DONE = 26, CS_U_EPOCH = 27, CS_U_ERR = 28, CS_U_N = 29 };
 
 __device__ __forceinline__ uint64_t vload64(const uint64_t *p) { return *reinterpret_cast<const volatile uint64_t *>(p); }
+// A 16-byte part of a record and its status, in one access each way: a reader
+// needs no fence and no second round trip.
+__device__ __forceinline__ void put_part(unsigned long long *p, unsigned long long value, unsigned long long status)
+{
+    const unsigned __int128 x = (unsigned __int128)status << 64 | value;
+    asm volatile("st.relaxed.gpu.global.b128 [%0], %1;\n" ::"l"(__cvta_generic_to_global(p)), "q"(x) : "memory");
+}
+
+__device__ __forceinline__ void get_part(const unsigned long long *p, unsigned long long &value,
+                                         unsigned long long &status)
+{
+    unsigned __int128 x;
+    asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];\n" : "=q"(x) : "l"(__cvta_generic_to_global(p)) : "memory");
+    value = (unsigned long long)x;
+    status = (unsigned long long)(x >> 64);
+}
+
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
+{
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(__cvta_generic_to_global(gmem)) : "memory");
+}
+
 // Claims the next tile for the whole block (thread 0 draws, all read).
 __device__ __forceinline__ uint64_t claim_tile(uint64_t *ctr, uint64_t *s_t)
 {
@@ -294,14 +313,14 @@ __device__ __forceinline__ bool last_block(uint64_t *done)
 }
 
 // Stream header words and the VariableByte tail of n - n1 (< 128) values,
-// written by one warp; blkend = word after the block part.  Total words ->
-// scal[CS_WORDS] and, if given, *words_out.  (compositecodec.h:31-51,
-// variablebyte.h:100-161: each value's delta from the one before, 0 before
-// the first, in 7-bit groups from the low end, the high bit on the last
-// byte, zero-padded to a word.)  One lane per value: its byte count, their
-// exclusive prefix over the warp (its place), then its bytes.
-__device__ void enc_tail_warp(const uint32_t *in, uint64_t n, uint64_t n1, uint64_t blkend, uint32_t *out,
-                              uint64_t *scal, uint64_t *words_out, uint32_t *s_bytes)
+// written by one warp; blkend = word after the block part.  Returns the
+// stream's words.  (compositecodec.h:31-51, variablebyte.h:100-161: each
+// value's delta from the one before, 0 before the first, in 7-bit groups from
+// the low end, the high bit on the last byte, zero-padded to a word.)  One lane
+// per value: its byte count, their exclusive prefix over the warp (its place),
+// then its bytes.
+__device__ uint64_t enc_tail_warp(const uint32_t *in, uint64_t n, uint64_t n1, uint64_t blkend, uint32_t *out,
+                                  uint32_t *s_bytes)
 {
     const int lane = g5_lane();
     const uint32_t nt = (uint32_t)(n - n1);
@@ -336,163 +355,42 @@ __device__ void enc_tail_warp(const uint32_t *in, uint64_t n, uint64_t n1, uint6
         out[1] = kCookie;
         out[2] = kCookie;
         out[3] = kCookie;
-        scal[CS_WORDS] = blkend + tw;
-        if (words_out) *words_out = blkend + tw;
-        scal[CS_BLKEND] = blkend;
     }
     for (uint32_t i = lane; i < tw; i += 32) out[blkend + i] = s_bytes[i];
+    return blkend + tw;
 }
 
-// ---- encoder: two passes ----------------------------------------------------------------
+// ---- encoder ----------------------------------------------------------------------------
 //
-// A miniblock's bit width depends only on its own 128 values and the vector
-// before them, so the stream's layout is fixed once every width is known.
-// Block b of the B launched blocks takes the groups [b NG / B, (b + 1) NG / B)
-// in both passes (NG groups of 16 miniblocks):
-//   k_enc_widths  a warp per miniblock ORs the deltas and stores the width
-//                 (one byte per miniblock); the block stores its range's
-//                 word count (4 header words per group + 4 b per miniblock)
-//   k_enc_pack    the block adds up the counts of the blocks before it (its
-//                 range's place in the stream), scans its groups' sizes, and
-//                 a warp per miniblock packs the deltas at their place from a
-//                 second read of the input (mostly still in L2); the block
-//                 with the last group writes the stream header and the
-//                 VariableByte tail
-// No block waits on another: the launch boundary orders the passes.  n comes
-// from device memory, so both launches can sit in a CUDA graph with a fixed
-// grid.
-constexpr int kEB = 512;  // encoder threads per block: 16 warps
-constexpr int kEU = 4;    // miniblocks whose loads a warp has in flight together (widths)
-constexpr int kPU = 2;    // the same when packing (two blocks of 512 fit an SM at 64 registers)
-constexpr int kPC = 256;  // groups per packing chunk (each miniblock's place held in shared memory)
+// One launch.  A miniblock's bit width depends only on its own 128 values and
+// the vector before them, so the stream's layout is fixed once every width is
+// known.  A block takes a chunk of up to kEG groups (16 miniblocks each),
+// claimed in launch order:
+//   load    its values into shared memory
+//   widths  a warp per miniblock turns its values into deltas, in place, and
+//           ORs them
+//   meet    the chunk's word count is published (one 16-byte store that carries
+//           its own status) and those of up to 512 chunks before it are read
+//           at once: the chunk's place in the stream
+//   pack    a warp per miniblock gathers each word of the payload from the
+//           values that reach into it and stores it, coalesced
+// The block with the last group writes the stream header and the VariableByte
+// tail.  n may come from device memory: the launch can sit in a CUDA graph with
+// a fixed grid.
+//
+// What bounds it: a chain of round trips (start 1.1 us, load 0.4-0.8, widths and
+// their scan 0.8-2.5, meeting 0.7-1.6, the last block's exit 1.3), and on large
+// queues issue: widths 1.7 us and packing 3 us of the 13 that 5 M values take
+// (23.8 MB of traffic).  The values are read once; the two launches this replaced
+// (widths, then packing from a second read with shared-memory atomics) took 18
+// us for the same queue, and 5.7 against 3.9 for 3000 values.
+constexpr int kEB = 512;  // threads per block
+constexpr int kEW = kEB / 32;
+constexpr int kEG = 8;    // groups per chunk at most (64 KB of values: three blocks per SM)
+constexpr int kEM = 16 * kEG;
+constexpr uint32_t kSlot = 16;  // 64-bit words from one chunk's record to the next (a line each: all blocks read
+                                // all of them at once, and neighbours in one line queue up there)
 
-struct EncLen {
-    uint64_t n, n1, nmb, ng;
-    bool raw, too_long;
-};
-
-__device__ __forceinline__ EncLen enc_len(const uint64_t *n_dev, uint64_t max_n, uint64_t raw_thr)
-{
-    EncLen e;
-    const uint64_t n_in = *n_dev;
-    e.too_long = n_in > max_n;  // a device-side length past the workspace: nothing is written
-    e.n = e.too_long ? 0 : n_in;
-    e.n1 = e.n / 128 * 128;
-    e.nmb = e.n / 128;
-    e.ng = (e.nmb + 15) / 16;
-    e.raw = raw_thr && e.n <= raw_thr;
-    return e;
-}
-
-__device__ __forceinline__ void enc_range(uint64_t ng, uint32_t nb, uint64_t &g0, uint64_t &g1)
-{
-    g0 = ng * blockIdx.x / nb;
-    g1 = ng * (blockIdx.x + 1) / nb;
-}
-
-// Lane j's vector j of miniblock k; lane 0 also the vector before the
-// miniblock (zero before the first).  Loads only: prev_of() shuffles later.
-__device__ __forceinline__ void load_cur(const uint32_t *in, uint64_t k, uint4 &cur, uint4 &pl)
-{
-    const uint4 *v = reinterpret_cast<const uint4 *>(in) + k * 32;
-    cur = v[g5_lane()];
-    pl = (g5_lane() == 0 && k) ? v[-1] : make_uint4(0, 0, 0, 0);
-}
-
-__device__ __forceinline__ uint4 prev_of(const uint4 &cur, const uint4 &pl)
-{
-    uint4 p;
-    p.x = __shfl_up_sync(0xFFFFFFFFu, cur.x, 1);
-    p.y = __shfl_up_sync(0xFFFFFFFFu, cur.y, 1);
-    p.z = __shfl_up_sync(0xFFFFFFFFu, cur.z, 1);
-    p.w = __shfl_up_sync(0xFFFFFFFFu, cur.w, 1);
-    return g5_lane() == 0 ? pl : p;
-}
-
-// The widths of group g (16 bytes, byte q = miniblock 16 g + q) with the
-// bytes of miniblocks past nmb cleared (a partial last group's header
-// carries width 0 there, simdbinarypacking.h:200-214).
-__device__ __forceinline__ uint4 group_widths(const uint8_t *wb, uint64_t g, uint64_t nmb)
-{
-    uint4 w = *reinterpret_cast<const uint4 *>(wb + 16 * g);
-    const uint64_t c = nmb - 16 * g;  // miniblocks in the group
-    if (c < 16) {
-        uint32_t x[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int keep = (int)c - 4 * j;  // bytes of word j that stay
-            x[j] = keep >= 4 ? x[j] : keep <= 0 ? 0u : x[j] & ((1u << (8 * keep)) - 1u);
-        }
-        w = make_uint4(x[0], x[1], x[2], x[3]);
-    }
-    return w;
-}
-
-// Sum of the first i widths of a group (bytes 0 .. i-1 of w).
-__device__ __forceinline__ uint32_t widths_before(const uint4 &w, uint32_t i)
-{
-    const uint32_t x[4] = {w.x, w.y, w.z, w.w};
-    uint32_t s = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int keep = (int)i - 4 * j;
-        const uint32_t m = keep >= 4 ? 0xFFFFFFFFu : keep <= 0 ? 0u : (1u << (8 * keep)) - 1u;
-        s = __dp4a(x[j] & m, 0x01010101u, s);
-    }
-    return s;
-}
-
-__global__ void __launch_bounds__(kEB, 2) k_enc_widths(const uint32_t *__restrict__ in, const uint64_t *n_dev,
-                                                    uint64_t max_n, uint64_t raw_thr, uint8_t *__restrict__ wb,
-                                                    uint64_t *__restrict__ btot, uint32_t nb, int mode)
-{
-    __shared__ uint32_t s_sum;
-    g5_pdl_sync();
-    const EncLen e = enc_len(n_dev, max_n, raw_thr);
-    if (e.raw || e.too_long) return;
-    const int lane = g5_lane(), wid = threadIdx.x >> 5;
-    uint64_t g0, g1;
-    enc_range(e.ng, nb, g0, g1);
-    const uint64_t k1 = min(16 * g1, e.nmb);
-    if (threadIdx.x == 0) s_sum = 0;
-    __syncthreads();
-    uint32_t sum = 0;  // warp-uniform
-    for (uint64_t kb = 16 * g0 + wid; kb < k1; kb += 16 * kEU) {
-        uint4 cur[kEU], pl[kEU];
-#pragma unroll
-        for (int i = 0; i < kEU; ++i) {
-            cur[i] = pl[i] = make_uint4(0, 0, 0, 0);
-            if (kb + 16 * i < k1) load_cur(in, kb + 16 * i, cur[i], pl[i]);
-        }
-#pragma unroll
-        for (int i = 0; i < kEU; ++i) {
-            const uint64_t k = kb + 16 * i;
-            if (k >= k1) break;
-            const uint4 d = deltas(cur[i], prev_of(cur[i], pl[i]), mode);
-            const uint32_t b = bits_of(__reduce_or_sync(0xFFFFFFFFu, d.x | d.y | d.z | d.w));
-            if (lane == 0) wb[k] = (uint8_t)b;
-            sum += b;
-        }
-    }
-    if (lane == 0 && sum) atomicAdd(&s_sum, sum);
-    __syncthreads();
-    if (threadIdx.x == 0) btot[blockIdx.x] = 4 * (g1 - g0) + 4 * (uint64_t)s_sum;
-}
-
-// Sum over the block (kEB threads) of a 64-bit value, returned to all.
-__device__ __forceinline__ uint64_t block_sum_u64(uint64_t x, uint64_t *s_red)
-{
-    const int lane = g5_lane(), wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) x += __shfl_down_sync(0xFFFFFFFFu, x, o);
-    if (lane == 0) s_red[wid] = x;
-    __syncthreads();
-    uint64_t t = 0;
-#pragma unroll
-    for (int i = 0; i < kEB / 32; ++i) t += s_red[i];
-    __syncthreads();
-    return t;
-}
 
 // Exclusive scan over the block (kEB threads) of a 32-bit value; total -> tot.
 __device__ __forceinline__ uint32_t block_excl_u32(uint32_t x, uint32_t *s_w, uint32_t &tot)
@@ -524,133 +422,239 @@ __device__ __forceinline__ uint32_t block_excl_u32(uint32_t x, uint32_t *s_w, ui
     return r;
 }
 
-// Packs a miniblock's deltas (lane j holds vector j) with width b (1..31)
-// into shared memory at s: value j of lane l occupies bits j b .. of lane
-// l's bit stream, whose word w is s[4 w + l]
-// (ipackwithoutmask<b>, simdintegratedbitpacking.cpp:875).  Each lane ORs
-// its four values into place (a value that straddles two words into both)
-// after the words are cleared: no division, no loop over values.
-__device__ __forceinline__ void pack_mb_smem(const uint4 &d, uint32_t b, uint32_t *s)
+struct EncShared {
+    uint4 prev[kEM];               // the vector before each miniblock
+    uint4 vec[kEM * 32];           // the chunk's values, then their deltas
+    uint32_t off[kEM];             // words from the chunk's first header to each miniblock's payload
+    __align__(16) uint8_t b[kEM];  // widths
+    uint32_t w[kEB / 32 + 1];
+    uint64_t t;
+    unsigned long long before;     // words before the chunk
+    int near_inc;
+    uint32_t magic[32];            // 2^16 / b + 1: quotients by b of up to 1023
+    uint32_t bytes[(128 * 5 + 3) / 4 + 1];
+};
+
+struct EncLen {
+    uint64_t n, n1, nmb, ng, nchunks;
+    uint32_t gpc;  // groups per chunk
+    bool raw, too_long;
+};
+
+__device__ __forceinline__ EncLen enc_len(uint64_t n_in, uint64_t max_n, uint64_t raw_thr, uint32_t blocks)
 {
-    const int lane = g5_lane();
-    if (lane < (int)b) reinterpret_cast<uint4 *>(s)[lane] = make_uint4(0, 0, 0, 0);  // 4 b words
-    __syncwarp();
-    const uint32_t bit = (uint32_t)lane * b, w = bit >> 5, sh = bit & 31;
-    const bool spill = sh + b > 32;
-    uint32_t *p = s + 4 * w;
-    const uint32_t v[4] = {d.x, d.y, d.z, d.w};
+    EncLen e;
+    e.too_long = n_in > max_n;  // a device-side length past the workspace: nothing is written
+    e.n = e.too_long ? 0 : n_in;
+    e.nmb = e.n / 128;
+    e.n1 = e.nmb * 128;
+    e.ng = (e.nmb + 15) / 16;
+    e.gpc = (uint32_t)min((uint64_t)kEG, max((uint64_t)1, (e.ng + blocks - 1) / blocks));
+    e.nchunks = (e.ng + e.gpc - 1) / e.gpc;
+    e.raw = raw_thr && e.n <= raw_thr;
+    return e;
+}
+
+// Words of the chunks before chunk c, by the whole block, into sh.before.
+__device__ void enc_before(EncShared &sh, uint64_t c, uint64_t epoch, const unsigned long long *slots, uint32_t stride,
+                           uint64_t *err)
+{
+    if (threadIdx.x == 0) sh.before = 0;
+    for (int64_t hi = (int64_t)c - 1; hi >= 0; hi -= kEB) {
+        if (threadIdx.x == 0) sh.near_inc = kEB;
+        __syncthreads();
+        const int64_t j = hi - threadIdx.x;
+        unsigned long long x = 0, t = 0;
+        if (j >= 0) {
+            uint32_t spins = 0;
+            for (;;) {
+                get_part(slots + stride * j, x, t);
+                if ((t >> 2) == epoch && (t & 3)) break;
+                if (++spins > kSpinLimit) {
+                    atomicOr((unsigned long long *)err, (unsigned long long)G5_DEVERR_WAIT);
+                    x = 0;
+                    break;
+                }
+            }
+            if ((t & 3) == ST_INC) atomicMin(&sh.near_inc, (int)threadIdx.x);
+        }
+        __syncthreads();
+        const int ni = sh.near_inc;
+        if ((int)threadIdx.x > ni) x = 0;
+        if (__any_sync(0xFFFFFFFFu, x != 0)) {
 #pragma unroll
-    for (int l = 0; l < 4; ++l) {
-        atomicOr(p + l, v[l] << sh);
-        if (spill) atomicOr(p + 4 + l, v[l] >> (32 - sh));
+            for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xFFFFFFFFu, x, o);
+            if (g5_lane() == 0) atomicAdd(&sh.before, x);
+        }
+        __syncthreads();
+        if (ni < kEB) break;
+    }
+    __syncthreads();
+}
+
+// Word `idx` of a miniblock's payload (word w = idx / 4 of lane l = idx & 3's bit
+// stream, ipackwithoutmask<b>, simdintegratedbitpacking.cpp:875) from fields
+// of `b` bits at d (field j of lane l at d[4 j + l]): those whose bits j b .. j b
+// + b - 1 reach into bits 32 w .. 32 w + 31.
+__device__ __forceinline__ uint32_t pack_word(const uint32_t *d, uint32_t b, uint32_t magic, uint32_t idx)
+{
+    const uint32_t first = 8 * (idx & ~3u), l = idx & 3;  // bit 32 w
+    uint32_t j = (first * magic) >> 16;                   // floor(32 w / b)
+    int sh = (int)(j * b) - (int)first;                   // at most 0
+    uint32_t x = d[4 * j + l] >> -sh;
+    for (;;) {
+        sh += (int)b;
+        ++j;
+        if (sh >= 32) break;
+        x |= d[4 * j + l] << sh;
+    }
+    return x;
+}
+
+// The payload of a miniblock of width b (1..31) whose deltas are at d, by one
+// warp.  Up to 8 bits, a lane first joins four values of a component into one
+// field (in place: 32 of them), so that a word gathers at most 32 / 4 b + 2
+// fields instead of as many as 32 values.
+__device__ __forceinline__ void pack_mb(uint32_t *d, uint32_t b, const uint32_t *magic, uint32_t *dst)
+{
+    const uint32_t lane = g5_lane();
+    uint32_t f = b;
+    if (b < 8) {  // (fields of 32 bits would shift by 32)
+        const uint32_t *s = d + 16 * (lane >> 2) + (lane & 3);
+        const uint32_t x = s[0] | s[4] << b | s[8] << (2 * b) | s[12] << (3 * b);
+        __syncwarp();
+        d[lane] = x;
+        __syncwarp();
+        f = 4 * b;
+    }
+    for (uint32_t i = lane; i < 4 * b; i += 32) dst[i] = pack_word(d, f, magic[f], i);
+}
+
+// Chunk c of the queue: its groups to the stream at `out`.  The block with the
+// last group also writes the stream header and the tail (in its last warp,
+// beside the packing) and leaves the stream's words in *words.
+template <bool ANY>
+__device__ void enc_chunk(EncShared &sh, const EncLen &e, const uint32_t *in, uint64_t c, uint64_t epoch,
+                          unsigned long long *slots, uint32_t stride, uint64_t *err, uint32_t *out, int mode,
+                          uint64_t *words)
+{
+    const int lane = g5_lane(), wid = threadIdx.x >> 5;
+    const uint64_t k0 = 16 * c * e.gpc;  // the chunk's first miniblock
+    const uint32_t nmb = (uint32_t)min((uint64_t)16 * e.gpc, e.nmb - k0);
+    const uint32_t *x = in + 128 * k0;
+    // (claim_tile's barriers separate the chunks)
+    if (ANY) {
+        for (uint32_t p = threadIdx.x; p < 128 * nmb; p += kEB) reinterpret_cast<uint32_t *>(sh.vec)[p] = x[p];
+        if (threadIdx.x < 4) reinterpret_cast<uint32_t *>(sh.prev)[threadIdx.x] = k0 ? x[(int)threadIdx.x - 4] : 0u;
+    } else {
+        const uint4 *v = reinterpret_cast<const uint4 *>(x);
+        for (uint32_t p = threadIdx.x; p < 32 * nmb; p += kEB) cp_async16(sh.vec + p, v + p);
+        if (threadIdx.x == 0) {
+            if (k0) cp_async16(sh.prev, v - 1);
+            else sh.prev[0] = make_uint4(0, 0, 0, 0);
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+    }
+    __syncthreads();
+    for (uint32_t m = threadIdx.x + 1; m < nmb; m += kEB) sh.prev[m] = sh.vec[32 * m - 1];
+    __syncthreads();
+#pragma unroll 2
+    for (uint32_t m = wid; m < nmb; m += kEW) {
+        uint4 *v = sh.vec + 32 * m;
+        const uint4 d = deltas(v[lane], lane ? v[lane - 1] : sh.prev[m], mode);
+        const uint32_t b = bits_of(__reduce_or_sync(0xFFFFFFFFu, d.x | d.y | d.z | d.w));
+        if (b < 32) v[lane] = d;  // (a raw miniblock keeps its values; the reduction above orders the reads)
+        if (lane == 0) sh.b[m] = (uint8_t)b;
+    }
+    __syncthreads();
+    const uint32_t m = threadIdx.x, mb = m < nmb ? sh.b[m] : 0u, head = m < nmb && (m & 15) == 0 ? 4u : 0u;
+    uint32_t total;
+    const uint32_t at = block_excl_u32(head + 4 * mb, sh.w, total);
+    if (m < nmb) sh.off[m] = at + head;
+    if (threadIdx.x == 0) put_part(slots + stride * c, total, epoch << 2 | (c ? ST_AGG : ST_INC));
+    enc_before(sh, c, epoch, slots, stride, err);
+    const uint64_t base = 4 + sh.before;  // word of the chunk's first header
+    if (c && e.nchunks > (uint64_t)kEB && threadIdx.x == 0)
+        put_part(slots + stride * c, sh.before + total, epoch << 2 | ST_INC);
+    uint32_t *o = out + base;
+    // the 16 widths of each group, big-endian bytes in each word; 0 where a last
+    // group has no miniblock (simdbinarypacking.h:200-214)
+    const uint32_t groups = (nmb + 15) / 16;
+    if (threadIdx.x < 4 * groups) {
+        const uint32_t g = threadIdx.x / 4, k = threadIdx.x & 3;
+        uint32_t hw = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t i = 16 * g + 4 * k + q;
+            hw |= (i < nmb ? sh.b[i] : 0u) << (24 - 8 * q);
+        }
+        o[sh.off[16 * g] - 4 + k] = hw;
+    }
+    uint32_t warps = kEW;
+    if (c + 1 == e.nchunks) {
+        --warps;
+        if (wid == (int)warps) {
+            const uint64_t w = enc_tail_warp(in, e.n, e.n1, base + total, out, sh.bytes);
+            if (lane == 0) *words = w;
+            return;
+        }
+    }
+    for (uint32_t q = wid; q < nmb; q += warps) {
+        const uint32_t b = sh.b[q];
+        uint32_t *dst = o + sh.off[q];
+        if (b == 32) reinterpret_cast<uint4 *>(dst)[lane] = sh.vec[32 * q + lane];
+        else if (b) pack_mb(reinterpret_cast<uint32_t *>(sh.vec + 32 * q), b, sh.magic, dst);
     }
 }
 
-__global__ void __launch_bounds__(kEB, 2) k_enc_pack(const uint32_t *__restrict__ in, const uint64_t *n_dev,
-                                                  uint64_t max_n, uint64_t raw_thr, uint32_t *__restrict__ out,
-                                                  uint64_t *scal, const uint8_t *__restrict__ wb,
-                                                  const uint64_t *__restrict__ btot, uint32_t nb,
-                                                  uint64_t *words_out, int mode)
+__global__ void __launch_bounds__(kEB, 3) k_encode(const uint32_t *__restrict__ in, const uint64_t *n_dev, uint64_t n_val,
+                                                uint64_t max_n, uint64_t raw_thr, uint32_t *__restrict__ out,
+                                                uint64_t *scal, unsigned long long *slots, uint32_t stride,
+                                                uint64_t *words_out, uint64_t *result, int mode)
 {
-    __shared__ __align__(16) uint32_t s_stage[kEB / 32][128];  // one miniblock's payload per warp
-    __shared__ __align__(16) uint32_t s_moff[kPC * 16];  // words from the chunk's first header to each miniblock
-    __shared__ __align__(16) uint8_t s_mb[kPC * 16];     // each miniblock's width
-    __shared__ uint64_t s_red[kEB / 32];
-    __shared__ uint32_t s_w[kEB / 32 + 1];
-    __shared__ uint32_t s_bytes[(128 * 5 + 3) / 4 + 1];
+    extern __shared__ __align__(16) unsigned char s_dyn_e[];
+    EncShared &sh = *reinterpret_cast<EncShared *>(s_dyn_e);
+    if (threadIdx.x >= 1 && threadIdx.x < 32) sh.magic[threadIdx.x] = 65536u / threadIdx.x + 1u;
     g5_pdl_sync();
-    const EncLen e = enc_len(n_dev, max_n, raw_thr);
-    const int lane = g5_lane(), wid = threadIdx.x >> 5;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        scal[CS_N] = e.n;
-        scal[CS_N1] = e.n1;
-        scal[CS_NMB] = e.nmb;
-        scal[CS_RAW] = e.raw ? 1 : 0;
-        scal[CS_ERR] = e.too_long ? G5_DEVERR_CAPACITY : 0;
-    }
-    if (e.too_long) return;
+    const uint64_t epoch = scal[CS_E_EPOCH];
+    const EncLen e = enc_len(n_dev ? *n_dev : n_val, max_n, raw_thr, gridDim.x);
     if (e.raw) {
         for (uint64_t i = (uint64_t)blockIdx.x * kEB + threadIdx.x; i < e.n; i += (uint64_t)gridDim.x * kEB)
             out[i] = in[i];
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            scal[CS_WORDS] = e.n;
-            if (words_out) *words_out = e.n;
+    } else if (!e.too_long) {
+        for (;;) {
+            const uint64_t c = claim_tile(&scal[CS_E_CTR], &sh.t);
+            if (c >= e.nchunks) break;
+            enc_chunk<false>(sh, e, in, c, epoch, slots, stride, &scal[CS_E_ERR], out, mode, &scal[CS_E_WORDS]);
         }
-        return;
-    }
-    if (e.ng == 0) {
-        if (blockIdx.x == 0 && wid == 0) enc_tail_warp(in, e.n, e.n1, 4, out, scal, words_out, s_bytes);
-        return;
-    }
-    uint64_t g0, g1;
-    enc_range(e.ng, nb, g0, g1);
-    if (g0 == g1) return;
-    uint64_t x = 0;
-    for (uint32_t i = threadIdx.x; i < blockIdx.x; i += kEB) x += btot[i];
-    uint64_t cbase = 4 + block_sum_u64(x, s_red);  // word of the chunk's first group header
-    uint32_t *stage = s_stage[wid];
-    for (uint64_t c0 = g0; c0 < g1; c0 += kPC) {
-        // thread t < kPC takes group c0 + t: its size into the chunk's scan,
-        // then its header, and its miniblocks' places and widths into
-        // shared memory
-        const uint64_t g = c0 + threadIdx.x;
-        const bool mine = threadIdx.x < kPC && g < g1;
-        uint4 wv = make_uint4(0, 0, 0, 0);
-        if (mine) wv = group_widths(wb, g, e.nmb);
-        uint32_t ctot;
-        const uint32_t goff = block_excl_u32(mine ? 4 + 4 * widths_before(wv, 16) : 0u, s_w, ctot);
-        if (mine) {
-            // the 16 widths, big-endian bytes in each word (simdbinarypacking.h:200-214)
-            reinterpret_cast<uint4 *>(out + cbase + goff)[0] =
-                make_uint4(__byte_perm(wv.x, 0, 0x0123), __byte_perm(wv.y, 0, 0x0123),
-                           __byte_perm(wv.z, 0, 0x0123), __byte_perm(wv.w, 0, 0x0123));
-            reinterpret_cast<uint4 *>(s_mb)[threadIdx.x] = wv;
-            uint32_t o = goff + 4;
-            const uint32_t x[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                uint4 r;
-                r.x = o;
-                o += 4 * (x[j] & 0xFFu);
-                r.y = o;
-                o += 4 * ((x[j] >> 8) & 0xFFu);
-                r.z = o;
-                o += 4 * ((x[j] >> 16) & 0xFFu);
-                r.w = o;
-                o += 4 * (x[j] >> 24);
-                reinterpret_cast<uint4 *>(s_moff)[4 * threadIdx.x + j] = r;
-            }
+        if (e.ng == 0 && blockIdx.x == 0 && threadIdx.x < 32) {
+            const uint64_t w = enc_tail_warp(in, e.n, 0, 4, out, sh.bytes);
+            if (threadIdx.x == 0) scal[CS_E_WORDS] = w;
         }
-        __syncthreads();
-        const uint64_t kc = 16 * c0;  // the chunk's first miniblock
-        const uint32_t mk = (uint32_t)(min(16 * min(c0 + kPC, g1), e.nmb) - kc);  // its miniblocks
-        for (uint32_t mb = wid; mb < mk; mb += 16 * kPU) {
-            uint4 cur[kPU], pl[kPU];
-#pragma unroll
-            for (int i = 0; i < kPU; ++i) {
-                cur[i] = pl[i] = make_uint4(0, 0, 0, 0);
-                if (mb + 16 * i < mk) load_cur(in, kc + mb + 16 * i, cur[i], pl[i]);
-            }
-#pragma unroll
-            for (int i = 0; i < kPU; ++i) {
-                const uint32_t m = mb + 16 * i;
-                if (m >= mk) break;
-                const uint32_t b = s_mb[m];
-                uint4 *dst = reinterpret_cast<uint4 *>(out + cbase + s_moff[m]);
-                if (b == 32) {
-                    dst[lane] = cur[i];
-                } else if (b) {
-                    pack_mb_smem(deltas(cur[i], prev_of(cur[i], pl[i]), mode), b, stage);
-                    __syncwarp();
-                    if (lane < (int)b) dst[lane] = reinterpret_cast<const uint4 *>(stage)[lane];
-                    __syncwarp();
-                }
-            }
-        }
-        cbase += ctot;
-        __syncthreads();
     }
-    if (g1 == e.ng && wid == 0) enc_tail_warp(in, e.n, e.n1, cbase, out, scal, words_out, s_bytes);
+    if (last_block(&scal[CS_E_DONE])) {
+        __threadfence();
+        uint64_t err = vload64(&scal[CS_E_ERR]);
+        if (e.too_long) err |= G5_DEVERR_CAPACITY;
+        const uint64_t w = e.raw ? e.n : e.too_long ? 0 : vload64(&scal[CS_E_WORDS]);
+        scal[CS_N] = e.n;
+        scal[CS_N1] = e.n1;
+        scal[CS_ERR] = err;
+        if (!e.too_long) {
+            scal[CS_WORDS] = w;
+            if (words_out) *words_out = w;
+        }
+        if (result) {
+            result[0] = e.n;
+            result[1] = w;
+            result[2] = err;
+        }
+        scal[CS_E_CTR] = 0;
+        scal[CS_E_DONE] = 0;
+        scal[CS_E_ERR] = 0;
+        scal[CS_E_EPOCH] = epoch + 1;
+        __threadfence();
+    }
 }
 
 // ---- decoder ---------------------------------------------------------------------------
@@ -699,9 +703,7 @@ constexpr int kDG = 32;            // groups whose miniblocks are held together
 constexpr int kDM = 16 * kDG;
 
 // What a chunk tells the ones after it: the groups it starts and their sums
-// (ST_AGG), or those of all chunks up to it (ST_INC).  Each 16-byte part
-// carries the status and moves in one access, so a reader needs no fence and
-// no second round trip: three parts of one status are one record.
+// (ST_AGG), or those of all chunks up to it (ST_INC): three parts of one status.
 struct ChunkRec {
     uint4 v;
     uint32_t f;       // the sums restart in the chunk
@@ -710,7 +712,7 @@ struct ChunkRec {
 };
 // The fourth part is the exit alone, published before the sums, so that a run
 // of chunks that wait for their entries waits for a walk each and no more.
-struct __align__(64) ChunkSlot {
+struct __align__(128) ChunkSlot {  // (a line each: all blocks read all of them at once)
     unsigned long long part[4][2];
 };
 
@@ -927,21 +929,6 @@ __device__ __forceinline__ uint4 mb_values(const uint32_t *s, uint32_t b, uint4 
         v[3] = c;
     }
     return make_uint4(v[0], v[1], v[2], v[3]);
-}
-
-__device__ __forceinline__ void put_part(unsigned long long *p, unsigned long long value, unsigned long long status)
-{
-    const unsigned __int128 x = (unsigned __int128)status << 64 | value;
-    asm volatile("st.relaxed.gpu.global.b128 [%0], %1;\n" ::"l"(__cvta_generic_to_global(p)), "q"(x) : "memory");
-}
-
-__device__ __forceinline__ void get_part(const unsigned long long *p, unsigned long long &value,
-                                         unsigned long long &status)
-{
-    unsigned __int128 x;
-    asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];\n" : "=q"(x) : "l"(__cvta_generic_to_global(p)) : "memory");
-    value = (unsigned long long)x;
-    status = (unsigned long long)(x >> 64);
 }
 
 // Publishes a chunk's record (three threads of a warp, a part each).
@@ -1243,10 +1230,7 @@ __device__ uint32_t dec_chunk(DecShared &sh, const DecHead &h, const uint32_t *i
     const uint32_t len = (uint32_t)min((uint64_t)S, h.nv - a), have = (uint32_t)min((uint64_t)S + kSpan, h.nv - a);
     const uint4 *v = reinterpret_cast<const uint4 *>(in) + a, *before = v - kSpan;
     __syncthreads();  // the chunk before is no longer read
-    for (uint32_t p = threadIdx.x; p < have; p += kDB) {
-        const unsigned sa = (unsigned)__cvta_generic_to_shared(sh.vec + p);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(__cvta_generic_to_global(v + p)) : "memory");
-    }
+    for (uint32_t p = threadIdx.x; p < have; p += kDB) cp_async16(sh.vec + p, v + p);
     if (threadIdx.x == 0) {
         sh.vec[have] = make_uint4(0, 0, 0, 0);
         sh.first = sh.xfirst = kDead;
@@ -1887,7 +1871,12 @@ size_t codec_bound(size_t n)
     return 4 + 4 * (mb / 16 + 1) + mb * 128 + ((n % 128) * 5 + 3) / 4 + 8;
 }
 
-size_t codec_tiles(size_t max_n) { return (max_n / 128 + 1) / 16 + 2; }
+// chunks of the longest queue, likewise
+size_t codec_enc_chunks(size_t max_n)
+{
+    const size_t groups = (max_n / 128 + 15) / 16;
+    return std::min(groups, std::max((size_t)codec_enc_grid(), groups / kEG)) + 2;
+}
 
 // chunks of the longest stream: one per block, or as many of the largest size
 // as it takes
@@ -1897,6 +1886,14 @@ size_t codec_chunks(size_t max_n)
 }
 
 int codec_grid() { return num_sms() * 2; }
+int codec_enc_grid() { return num_sms() * 3; }
+
+g5_status codec_kernels()
+{
+    G5_CUDA(cudaFuncSetAttribute(k_encode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EncShared)));
+    G5_CUDA(cudaFuncSetAttribute(k_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecShared)));
+    return G5_OK;
+}
 
 g5_status codec_work_alloc(CodecWork &w, size_t max_n)
 {
@@ -1904,13 +1901,14 @@ g5_status codec_work_alloc(CodecWork &w, size_t max_n)
     w.max_mb = max_n / 128 + 1;
     w.max_vec = codec_bound(max_n) / 4 + 2;
     w.grid = codec_grid();
-    const size_t T = codec_tiles(max_n), C = codec_chunks(max_n);
+    w.egrid = codec_enc_grid();
+    const size_t C = codec_chunks(max_n), E = codec_enc_chunks(max_n);
     G5_CUDA(cudaMalloc(&w.scal, sizeof(uint64_t) * kScalars));
-    w.enc_blocks = w.grid;
-    G5_CUDA(cudaMalloc(&w.ewb, 16 * T));
-    G5_CUDA(cudaMalloc(&w.etot, sizeof(uint64_t) * w.enc_blocks));
-    // the decoder's shared memory needs more than 48 KB (set per device)
-    G5_CUDA(cudaFuncSetAttribute(k_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecShared)));
+    G5_CUDA(cudaMalloc(&w.eslots, 8 * kSlot * E));
+    G5_CUDA(cudaMemset(w.eslots, 0, 8 * kSlot * E));
+    w.estride = kSlot;
+    // more than 48 KB of shared memory each (set per device)
+    G5_TRY(codec_kernels());
     G5_CUDA(cudaMalloc(&w.slots, sizeof(ChunkSlot) * C));
     // epochs start at 1, so zeroed status words read as "not published"
     G5_CUDA(cudaMemset(w.scal, 0, sizeof(uint64_t) * kScalars));
@@ -1924,21 +1922,21 @@ g5_status codec_work_alloc(CodecWork &w, size_t max_n)
 void codec_work_free(CodecWork &w)
 {
     cudaFree(w.scal);
-    cudaFree(w.ewb);
-    cudaFree(w.etot);
+    cudaFree(w.eslots);
     cudaFree(w.slots);
     w = CodecWork();
 }
 
-void codec_encode_launch(CodecWork &w, const uint32_t *in, const uint64_t *n_dev, uint32_t *out, int mode,
-                         uint64_t raw_threshold, cudaStream_t s, uint64_t *words_out)
+void codec_encode_launch(CodecWork &w, const uint32_t *in, const uint64_t *n_dev, uint64_t n, uint32_t *out, int mode,
+                         uint64_t raw_threshold, cudaStream_t s, uint64_t *words_out, uint64_t *result)
 {
-    // programmatic dependent launches: each kernel's first instruction waits
-    // for the kernel before it, so only the launch latency is overlapped
-    const uint32_t nb = (uint32_t)std::min(w.grid, w.enc_blocks);
-    launch(true, k_enc_widths, nb, kEB, s, in, n_dev, (uint64_t)w.max_n, raw_threshold, w.ewb, w.etot, nb, mode);
-    launch(true, k_enc_pack, nb, kEB, s, in, n_dev, (uint64_t)w.max_n, raw_threshold, out, w.scal,
-           (const uint8_t *)w.ewb, (const uint64_t *)w.etot, nb, words_out, mode);
+    // a programmatic dependent launch: the kernel's first instruction waits
+    // for the kernel before it, so only the launch latency is overlapped.  A
+    // length known here needs no more blocks than it has groups.
+    const uint64_t groups = n_dev ? (uint64_t)w.egrid : std::max<uint64_t>(1, (n / 128 + 15) / 16);
+    const int grid = (int)std::min<uint64_t>(w.egrid, groups);
+    launch_dyn(true, k_encode, grid, kEB, sizeof(EncShared), s, in, n_dev, n, (uint64_t)w.max_n, raw_threshold, out,
+               w.scal, w.eslots, w.estride, words_out, result, mode);
 }
 
 void codec_decode_launch(CodecWork &w, const uint32_t *in, const uint64_t *words_dev, uint64_t words, uint32_t *out,
@@ -1989,7 +1987,6 @@ size_t round4(size_t w) { return (w + 3) & ~(size_t)3; }
 
 struct g5_codec {
     g5::CodecWork w;
-    uint64_t *n_dev = nullptr;
     uint64_t *h_scal = nullptr;  // pinned
     BatchWs bw;
 };
@@ -2009,11 +2006,9 @@ g5_status g5_codec_create(size_t max_n, g5_codec **out)
     }
     g5_codec *c = new g5_codec();
     g5_status s = g5::codec_work_alloc(c->w, max_n);
-    if (s == G5_OK && cudaMalloc(&c->n_dev, sizeof(uint64_t) * 2) != cudaSuccess) s = G5_ERR_OOM;
     if (s == G5_OK && cudaMallocHost(&c->h_scal, sizeof(uint64_t) * 16) != cudaSuccess) s = G5_ERR_OOM;
     if (s != G5_OK) {
         g5::codec_work_free(c->w);
-        cudaFree(c->n_dev);
         delete c;
         return s;
     }
@@ -2026,7 +2021,6 @@ g5_status g5_codec_destroy(g5_codec *c)
     if (!c) return G5_ERR_INVALID_ARG;
     cudaDeviceSynchronize();
     g5::codec_work_free(c->w);
-    cudaFree(c->n_dev);
     cudaFreeHost(c->h_scal);
     c->bw.release();
     delete c;
@@ -2040,14 +2034,13 @@ g5_status g5_codec_encode(g5_codec *c, const uint32_t *in_dev, size_t n, uint32_
     if (mode != G5_CODEC_D4 && mode != G5_CODEC_DM) return G5_ERR_INVALID_ARG;
     if (((uintptr_t)in_dev | (uintptr_t)out_dev) & 15) return G5_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    c->h_scal[15] = n;
-    G5_CUDA(cudaMemcpyAsync(c->n_dev, &c->h_scal[15], sizeof(uint64_t), cudaMemcpyHostToDevice, s));
-    g5::codec_encode_launch(c->w, in_dev, c->n_dev, out_dev, mode, 0, s);
+    // the kernel leaves the length and status in pinned memory itself
+    g5::codec_encode_launch(c->w, in_dev, nullptr, n, out_dev, mode, 0, s, nullptr, c->h_scal);
     G5_CUDA(cudaGetLastError());
-    G5_CUDA(cudaMemcpyAsync(c->h_scal, c->w.scal, sizeof(uint64_t) * 8, cudaMemcpyDeviceToHost, s));
     G5_CUDA(cudaStreamSynchronize(s));
-    if (c->h_scal[g5::CS_ERR]) return G5_ERR_CAPACITY;  // the encoder has no device waits
-    *out_words = (size_t)c->h_scal[g5::CS_WORDS];
+    if (c->h_scal[2] & G5_DEVERR_WAIT) return G5_ERR_TIMEOUT;
+    if (c->h_scal[2]) return G5_ERR_CAPACITY;
+    *out_words = (size_t)c->h_scal[1];
     return G5_OK;
 }
 
@@ -2077,7 +2070,7 @@ g5_status g5_codec_encode_async(g5_codec *c, const uint32_t *in_dev, const uint6
     if (mode != G5_CODEC_D4 && mode != G5_CODEC_DM) return G5_ERR_INVALID_ARG;
     if (((uintptr_t)in_dev | (uintptr_t)out_dev) & 15) return G5_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    g5::codec_encode_launch(c->w, in_dev, n_dev, out_dev, mode, 0, s, out_words_dev);
+    g5::codec_encode_launch(c->w, in_dev, n_dev, 0, out_dev, mode, 0, s, out_words_dev, nullptr);
     G5_CUDA(cudaGetLastError());
     return G5_OK;
 }
@@ -2278,12 +2271,11 @@ g5_status g5_codec_decode_batch(g5_codec *c, const uint32_t *in_dev, const uint6
 // that may not block on (or fragment) device memory between requests, or a
 // host process whose device memory is owned by another allocator (a
 // framework's caching pool) with no headroom for cudaMalloc.  The encoder's
-// scratch (its scalars, the length, the bit width of every miniblock and the
-// word count of every encoder block) lives in the file-scope array below
-// instead of a g5_codec workspace: 12,608 bytes (about 12 KiB,
+// scratch (its scalars and the record of every chunk) lives in the file-scope
+// array below instead of a g5_codec workspace: 8,480 bytes (about 8 KiB,
 // kNoAllocBytes) that every GPU which loads the library holds until the
-// process exits.  Nothing in it needs clearing between calls: each call
-// writes every width and count it reads.  The array's device address is looked up
+// process exits.  Nothing in it needs clearing between calls: records hold the
+// call's epoch.  The array's device address is looked up
 // once per device and cached for the life of the process, so the entry point
 // must not be used again on a device after cudaDeviceReset in the same
 // process (the reset frees the module that holds the array).
@@ -2291,12 +2283,10 @@ g5_status g5_codec_decode_batch(g5_codec *c, const uint32_t *in_dev, const uint6
 namespace {
 
 constexpr size_t kNoAllocMaxValues = (size_t)1 << 20;             // values per call
-constexpr size_t kNoAllocMb = kNoAllocMaxValues / 128 + 1;          // miniblocks
-constexpr size_t kNoAllocWb = (kNoAllocMb / 16 + 1) * 16;          // miniblock widths, whole groups
-constexpr size_t kNoAllocBlocks = 516;                              // encoder blocks at most
-constexpr size_t kNoAllocScal = sizeof(uint64_t) * g5::kScalars;    // scalars
-constexpr size_t kNoAllocBytes = kNoAllocScal + 16 + kNoAllocWb + sizeof(uint64_t) * kNoAllocBlocks;
-static_assert(kNoAllocBytes == 12608, "the documented size of the scratch array");
+constexpr size_t kNoAllocChunks = kNoAllocMaxValues / 2048 + 2;   // a chunk is one group at least
+constexpr size_t kNoAllocScal = sizeof(uint64_t) * g5::kScalars;  // scalars
+constexpr size_t kNoAllocBytes = kNoAllocScal + 16 * kNoAllocChunks;
+static_assert(kNoAllocBytes == 8480, "the documented size of the scratch array");
 
 // In host code this name is only a host-side stand-in for the device array;
 // kernels receive the device address fetched with cudaGetSymbolAddress.
@@ -2328,6 +2318,7 @@ extern "C" g5_status g5_codec_encode_noalloc(const uint32_t *in_dev, size_t n, u
         if (!g_noalloc_addr[dev]) {
             void *p = nullptr;
             G5_CUDA(cudaGetSymbolAddress(&p, g5_noalloc_scratch));
+            G5_TRY(g5::codec_kernels());
             g_noalloc_addr[dev] = p;
         }
         base = g_noalloc_addr[dev];
@@ -2335,22 +2326,18 @@ extern "C" g5_status g5_codec_encode_noalloc(const uint32_t *in_dev, size_t n, u
     unsigned char *b = static_cast<unsigned char *>(base);
     g5::CodecWork w;
     w.max_n = kNoAllocMaxValues;
-    w.max_mb = kNoAllocMb;
-    w.grid = g5::codec_grid();
+    w.egrid = g5::codec_enc_grid();
     w.scal = reinterpret_cast<uint64_t *>(b);
-    uint64_t *n_dev = reinterpret_cast<uint64_t *>(b + kNoAllocScal);
-    w.ewb = b + kNoAllocScal + 16;
-    w.etot = reinterpret_cast<uint64_t *>(b + kNoAllocScal + 16 + kNoAllocWb);
-    w.enc_blocks = (int)kNoAllocBlocks;
-    static_assert((kNoAllocScal + 16 + kNoAllocWb) % 16 == 0, "the widths are read as 16-byte vectors");
+    w.eslots = reinterpret_cast<unsigned long long *>(b + kNoAllocScal);
+    w.estride = 2;  // packed: the array is kept small
+    static_assert(kNoAllocScal % 16 == 0, "records are 16-byte vectors");
     cudaStream_t s = (cudaStream_t)stream;
-    uint64_t hn = n;
-    G5_CUDA(cudaMemcpyAsync(n_dev, &hn, sizeof hn, cudaMemcpyHostToDevice, s));
-    g5::codec_encode_launch(w, in_dev, n_dev, out_dev, mode, 0, s);
+    g5::codec_encode_launch(w, in_dev, nullptr, n, out_dev, mode, 0, s, nullptr, nullptr);
     G5_CUDA(cudaGetLastError());
     uint64_t sc[3] = {0, 0, 0};  // CS_N, CS_WORDS, CS_ERR
     G5_CUDA(cudaMemcpyAsync(sc, w.scal, sizeof sc, cudaMemcpyDeviceToHost, s));
     G5_CUDA(cudaStreamSynchronize(s));
+    if (sc[g5::CS_ERR] & G5_DEVERR_WAIT) return G5_ERR_TIMEOUT;
     if (sc[g5::CS_ERR]) return G5_ERR_CAPACITY;
     *out_words = (size_t)sc[g5::CS_WORDS];
     return G5_OK;

@@ -19,13 +19,10 @@ struct CodecWork {
     size_t max_n = 0;        // capacity in values
     size_t max_mb = 0;       // miniblocks
     size_t max_vec = 0;      // 16-byte vectors of the largest stream
-    int grid = 0;            // blocks of the fixed grid
+    int grid = 0, egrid = 0; // blocks of the decoder's and encoder's fixed grids
     uint64_t *scal = nullptr;  // device scalars (kScalars), see CodecScalar
-    // encoder: bit width of every miniblock (16-byte aligned, a group's 16
-    // widths one vector) and the word count of each encoder block's range
-    uint8_t *ewb = nullptr;
-    uint64_t *etot = nullptr;
-    int enc_blocks = 0;        // encoder blocks (entries of etot)
+    unsigned long long *eslots = nullptr;  // encoder: a record (16 bytes) per chunk,
+    uint32_t estride = 0;                  // this many 64-bit words apart
     void *slots = nullptr;     // decoder: a record per chunk
 };
 
@@ -34,27 +31,28 @@ enum CodecScalar {
     CS_WORDS = 1,   // encoded words
     CS_ERR = 2,     // error bits (G5_DEVERR_*)
     CS_N1 = 3,      // values in the block part
-    CS_BLKEND = 4,  // word index where the block part ends
     CS_COUNT = 8
 };
 
 constexpr int kScalars = 32;  // scalar slots of a CodecWork
 
-// Groups (with room to spare) and decoder chunks of a workspace for max_n
-// values, and the fixed grid of the codec kernels.
-size_t codec_tiles(size_t max_n);
-size_t codec_chunks(size_t max_n);
+// The fixed grids of the decoder and the encoder, and their attributes on the
+// current device.
 int codec_grid();
+int codec_enc_grid();
+g5_status codec_kernels();
 
 size_t codec_bound(size_t n);
 g5_status codec_work_alloc(CodecWork &w, size_t max_n);
 void codec_work_free(CodecWork &w);
 
-// Encode in[0 .. *n_dev) to out; words written -> w.scal[CS_WORDS] and, if
-// words_out is given, *words_out.  raw_threshold: if *n_dev <= raw_threshold,
-// a raw copy (plugin semantics); pass 0 for pure IntegerCODEC semantics.
-void codec_encode_launch(CodecWork &w, const uint32_t *in, const uint64_t *n_dev, uint32_t *out,
-                         int mode, uint64_t raw_threshold, cudaStream_t s, uint64_t *words_out = nullptr);
+// Encode in[0 .. *n_dev) (or [0 .. n) if n_dev is null) to out; words written
+// -> w.scal[CS_WORDS] and, if given, *words_out; result (pinned host memory, 3
+// entries) receives the length, the words and the error bits.  raw_threshold:
+// if the length is at most that, a raw copy (plugin semantics); pass 0 for pure
+// IntegerCODEC semantics.
+void codec_encode_launch(CodecWork &w, const uint32_t *in, const uint64_t *n_dev, uint64_t n, uint32_t *out, int mode,
+                         uint64_t raw_threshold, cudaStream_t s, uint64_t *words_out, uint64_t *result);
 
 // Decode in[0 .. *words_dev) (or [0 .. words) if words_dev is null) to out
 // (capacity cap); values -> w.scal[CS_N].  If expect != nullptr, each decoded

@@ -465,8 +465,8 @@ g5_status g5_codec_decode_batch(g5_codec *c, const uint32_t *in_dev, const uint6
  * memory: a serving loop that must never block on or fragment the CUDA
  * allocator between requests, or a process whose device memory belongs to
  * another allocator (a framework's caching pool) with nothing left for
- * cudaMalloc.  It needs no g5_codec: its scratch is a fixed array of 12,608
- * bytes (about 12 KiB) in the library's device image, held on every GPU that
+ * cudaMalloc.  It needs no g5_codec: its scratch is a fixed array of 8,480
+ * bytes (about 8 KiB) in the library's device image, held on every GPU that
  * loads the library until the process exits, and it calls no allocating
  * function.  At most 1,048,576 values per call (more gives
  * G5_ERR_CAPACITY).  The first call on a device looks up that device's copy

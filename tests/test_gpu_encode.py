@@ -1,0 +1,64 @@
+"""The one-launch encoder at the sizes where its chunks change: tails alone, a
+last group with missing miniblocks, one and several groups per chunk, more
+chunks than blocks; every width from 0 to 32.  Streams equal the oracle's."""
+import numpy as np
+import pytest
+
+import oracle as orc
+from test_gpu_decode import MODES, values
+
+pytestmark = pytest.mark.gpu
+
+g5 = pytest.importorskip("gpugraph500_gb300")
+torch = pytest.importorskip("torch")
+
+
+def check(codec, x):
+    n = len(x)
+    din = torch.from_numpy(x.view(np.int32)).cuda() if n else torch.zeros(4, dtype=torch.int32, device="cuda")
+    for mode, omode in MODES:
+        out = torch.full((g5.Codec.bound(n) + 8,), -1, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        for _ in range(2):  # records of the call before are not read
+            w = codec.encode(din, n, out, mode)
+            assert np.array_equal(out[:w].cpu().numpy().view(np.uint32), orc.encode(x, omode)), (n, mode)
+
+
+@pytest.mark.parametrize("kind", ["ids", "equal", "random", "jumps"])
+@pytest.mark.parametrize("n", [0, 1, 127, 128, 2047, 2048, 2049, 304 * 2048, 304 * 2048 + 129, 1_300_001, 8_000_003])
+def test_sizes(kind, n):
+    c = g5.Codec(max(n, 1))
+    check(c, values(kind, n, np.random.default_rng(n)))
+    c.close()
+
+
+def test_every_width():
+    rng = np.random.default_rng(2)
+    parts = []
+    for b in range(33):  # 17 miniblocks of each width: groups mix two widths
+        hi = (1 << b) - 1
+        parts.append(rng.integers(0, hi + 1, 128 * 17, dtype=np.uint64))
+    d = np.concatenate(parts)
+    x = d.copy()
+    for j in range(4, len(x)):  # d4: each lane runs on from four values before
+        x[j] = (x[j] + x[j - 4]) & 0xFFFFFFFF
+    c = g5.Codec(len(x))
+    check(c, x.astype(np.uint32))
+    c.close()
+
+
+def test_length_past_the_workspace_is_refused():
+    c = g5.Codec(1000)
+    din = torch.zeros(4096, dtype=torch.int32, device="cuda")
+    out = torch.full((8192,), -1, dtype=torch.int32, device="cuda")
+    n = torch.tensor([4096], dtype=torch.int64, device="cuda")
+    w = torch.full((1,), -5, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    c.encode_async(din, n, out, w)
+    assert c.status() == g5.G5_ERR_CAPACITY
+    assert int(w) == -5 and bool((out == -1).all())  # nothing is written
+    n.fill_(700)
+    torch.cuda.synchronize()
+    c.encode_async(din, n, out, w)
+    assert c.status() == 0 and int(w) > 0
+    c.close()
