@@ -28,9 +28,7 @@
 // chain (each header says how long its group is), and the sums of all values
 // before it: one launch, a block per chunk of the stream, which finds its own
 // place in the chain and adds up what the chunks before it publish.  The
-// many-streams calls (one launch set for k queues) resolve the chains by
-// binary lifting over all 16-byte positions (group starts are always 16-byte
-// aligned) and use separate scan passes.
+// many-streams calls run the chunks of all k queues in one launch each way.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -45,20 +43,11 @@ namespace g5 {
 namespace {
 
 constexpr uint32_t kCookie = 123456u;
-constexpr int kB = 256;
 constexpr int kTailMaxBytes = 4096;  // largest VariableByte tail decoded
 
 __device__ __forceinline__ uint32_t bits_of(uint32_t v) { return v ? 32u - __clz(v) : 0u; }
 
-// ---- generic device-count scans -------------------------------------------------
-
-struct AddU32 {
-    typedef uint32_t T;
-    __device__ static T id() { return 0u; }
-    __device__ static T op(T a, T b) { return a + b; }
-    __device__ static T shfl_up(T v, int o) { return __shfl_up_sync(0xFFFFFFFFu, v, o); }
-};
-
+// Running lane sums that a raw miniblock restarts.
 struct ResetAdd {
     typedef VecFlag T;
     __device__ static T id()
@@ -88,115 +77,6 @@ struct ResetAdd {
     }
 };
 
-// Inclusive block scan (blockDim.x == kB); returns inclusive value, total in *tot.
-template <class Op>
-__device__ typename Op::T block_scan_incl(typename Op::T x, typename Op::T *s_w, typename Op::T &tot)
-{
-    typedef typename Op::T T;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        T y = Op::shfl_up(x, o);
-        if (lane >= o) x = Op::op(y, x);
-    }
-    if (lane == 31) s_w[wid] = x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        T acc = Op::id();
-        for (int i = 0; i < kB / 32; ++i) {
-            T t = s_w[i];
-            s_w[i] = acc;
-            acc = Op::op(acc, t);
-        }
-        s_w[kB / 32] = acc;
-    }
-    __syncthreads();
-    T r = Op::op(s_w[wid], x);
-    tot = s_w[kB / 32];
-    __syncthreads();
-    return r;
-}
-
-__device__ __forceinline__ void range_of(uint64_t n, uint64_t &b0, uint64_t &b1)
-{
-    const uint64_t per = (n + gridDim.x - 1) / gridDim.x;
-    b0 = min(n, (uint64_t)blockIdx.x * per);
-    b1 = min(n, b0 + per);
-}
-
-template <class Op>
-__global__ void __launch_bounds__(kB) k_scan_red(const typename Op::T *in, const uint64_t *cnt,
-                                                 typename Op::T *part)
-{
-    typedef typename Op::T T;
-    __shared__ T s_w[kB / 32 + 1];
-    uint64_t b0, b1;
-    range_of(*cnt, b0, b1);
-    T carry = Op::id();
-    for (uint64_t t0 = b0; t0 < b1; t0 += kB) {
-        const uint64_t i = t0 + threadIdx.x;
-        T x = i < b1 ? in[i] : Op::id();
-        T tt;
-        block_scan_incl<Op>(x, s_w, tt);
-        carry = Op::op(carry, tt);
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = carry;
-}
-
-// Exclusive scan of the partials in place (single block); total -> *total.
-template <class Op>
-__global__ void __launch_bounds__(kB) k_scan_top(typename Op::T *part, int np, typename Op::T *total)
-{
-    typedef typename Op::T T;
-    __shared__ T s_w[kB / 32 + 1];
-    T carry = Op::id();
-    for (int t0 = 0; t0 < np; t0 += kB) {
-        const int i = t0 + threadIdx.x;
-        T x = i < np ? part[i] : Op::id();
-        T tt;
-        T inc = block_scan_incl<Op>(x, s_w, tt);
-        // exclusive = carry op (inclusive without x): recompute from shuffle
-        T exc_local = Op::shfl_up(inc, 1);
-        if ((threadIdx.x & 31) == 0) exc_local = Op::id();
-        __shared__ T s_prev[kB / 32];
-        if ((threadIdx.x & 31) == 31) s_prev[threadIdx.x >> 5] = inc;
-        __syncthreads();
-        T ex = ((threadIdx.x & 31) == 0) ? (threadIdx.x == 0 ? Op::id() : s_prev[(threadIdx.x >> 5) - 1])
-                                          : exc_local;
-        if (i < np) part[i] = Op::op(carry, ex);
-        __syncthreads();
-        carry = Op::op(carry, tt);
-    }
-    if (threadIdx.x == 0 && total) *total = carry;
-}
-
-// Exclusive scan of in[] into out[] (may alias) seeded by part[block].
-template <class Op>
-__global__ void __launch_bounds__(kB) k_scan_down(const typename Op::T *in, typename Op::T *out,
-                                                  const uint64_t *cnt, const typename Op::T *part)
-{
-    typedef typename Op::T T;
-    __shared__ T s_w[kB / 32 + 1];
-    __shared__ T s_prev[kB / 32];
-    uint64_t b0, b1;
-    range_of(*cnt, b0, b1);
-    T carry = part[blockIdx.x];
-    for (uint64_t t0 = b0; t0 < b1; t0 += kB) {
-        const uint64_t i = t0 + threadIdx.x;
-        T x = i < b1 ? in[i] : Op::id();
-        T tt;
-        T inc = block_scan_incl<Op>(x, s_w, tt);
-        T exc_local = Op::shfl_up(inc, 1);
-        if ((threadIdx.x & 31) == 31) s_prev[threadIdx.x >> 5] = inc;
-        __syncthreads();
-        T ex = ((threadIdx.x & 31) == 0) ? (threadIdx.x == 0 ? Op::id() : s_prev[(threadIdx.x >> 5) - 1])
-                                          : exc_local;
-        if (i < b1) out[i] = Op::op(carry, ex);
-        __syncthreads();
-        carry = Op::op(carry, tt);
-    }
-}
-
 // ---- encoder ---------------------------------------------------------------------------
 
 __device__ __forceinline__ uint4 deltas(uint4 cur, uint4 prev, int mode)
@@ -204,52 +84,6 @@ __device__ __forceinline__ uint4 deltas(uint4 cur, uint4 prev, int mode)
     if (mode == G5_CODEC_DM)
         return make_uint4(cur.x - prev.w, cur.y - prev.w, cur.z - prev.w, cur.w - prev.w);
     return make_uint4(cur.x - prev.x, cur.y - prev.y, cur.z - prev.z, cur.w - prev.w);
-}
-
-__device__ __forceinline__ uint32_t comp(const uint4 &v, int l)
-{
-    return l == 0 ? v.x : l == 1 ? v.y : l == 2 ? v.z : v.w;
-}
-
-// ---- decoder ---------------------------------------------------------------------------
-
-// Unpacks lane j's 4 deltas of miniblock k (b < 32) or raw values (b == 32).
-__device__ __forceinline__ uint4 unpack_vec(const uint32_t *in, uint64_t off_vec, uint32_t b)
-{
-    const int j = g5_lane();
-    const uint4 *v = reinterpret_cast<const uint4 *>(in) + off_vec;
-    if (b == 32) return v[j];
-    if (b == 0) return make_uint4(0, 0, 0, 0);
-    const uint32_t bit = (uint32_t)j * b, w = bit >> 5, s = bit & 31;
-    const uint4 a = v[w];
-    uint4 r;
-    const uint32_t mask = (b == 32) ? 0xFFFFFFFFu : ((1u << b) - 1u);
-    if (s + b > 32) {
-        const uint4 c = v[w + 1];
-        r.x = ((a.x >> s) | (c.x << (32 - s))) & mask;
-        r.y = ((a.y >> s) | (c.y << (32 - s))) & mask;
-        r.z = ((a.z >> s) | (c.z << (32 - s))) & mask;
-        r.w = ((a.w >> s) | (c.w << (32 - s))) & mask;
-    } else {
-        r.x = (a.x >> s) & mask;
-        r.y = (a.y >> s) & mask;
-        r.z = (a.z >> s) & mask;
-        r.w = (a.w >> s) & mask;
-    }
-    return r;
-}
-
-__device__ __forceinline__ void mb_locate(const uint32_t *in, const uint32_t *gpos, uint64_t k,
-                                          uint64_t &off_vec, uint32_t &b)
-{
-    const uint64_t g = k / 16, i = k % 16;
-    const uint32_t p = gpos[g];
-    const uint4 h = reinterpret_cast<const uint4 *>(in)[p];
-    const uint32_t hw[4] = {h.x, h.y, h.z, h.w};
-    uint64_t s = 0;
-    for (uint64_t q = 0; q < i; ++q) s += (hw[q / 4] >> (24 - 8 * (q % 4))) & 0xFF;
-    b = (hw[i / 4] >> (24 - 8 * (i % 4))) & 0xFF;
-    off_vec = (uint64_t)p + 1 + s;
 }
 
 // ---- meetings of a launch's blocks -------------------------------------------------------
@@ -750,16 +584,16 @@ struct DecHead {
     bool raw, bad;
 };
 
-// Chunk size: one chunk per block, but none shorter than kMidChunk unless the
+// Chunk size of a stream of nv vectors and n1 values in whole miniblocks, `per`
+// vectors a block's share: that, but no chunk shorter than kMidChunk unless the
 // stream packs so many values into a vector that such chunks would hold far
 // more than kChunkValues.
-__device__ __forceinline__ void dec_chunks(DecHead &h, uint32_t blocks)
+__host__ __device__ __forceinline__ uint32_t dec_chunk_size(uint64_t nv, uint64_t n1, uint64_t per)
 {
-    const uint64_t per = (h.nv + blocks - 1) / blocks;
-    const uint64_t few = h.n1 > kChunkValues ? min((uint64_t)kMidChunk, kChunkValues * h.nv / h.n1) : kMidChunk;
-    h.S = (uint32_t)min((uint64_t)kMaxChunk, (max(per, few) + kMinChunk - 1) / kMinChunk * kMinChunk);
-    if (h.S < kMinChunk) h.S = kMinChunk;
-    h.nchunks = h.nv > 1 ? (h.nv - 1 + h.S - 1) / h.S : 0;
+    uint64_t few = kMidChunk;
+    if (n1 > kChunkValues && kChunkValues * nv / n1 < few) few = kChunkValues * nv / n1;
+    const uint64_t s = ((per > few ? per : few) + kMinChunk - 1) / kMinChunk * kMinChunk;
+    return s < kMinChunk ? kMinChunk : s > kMaxChunk ? kMaxChunk : (uint32_t)s;
 }
 
 __device__ __forceinline__ DecHead dec_head(const uint32_t *in, uint64_t words, uint64_t cap, uint64_t raw_thr,
@@ -791,8 +625,8 @@ __device__ __forceinline__ DecHead dec_head(const uint32_t *in, uint64_t words, 
     if (h.bad) h.n1 = 0;
     h.nmb = h.n1 / 128;
     h.ng = (h.nmb + 15) / 16;
-    if (!h.bad) dec_chunks(h, blocks);
-    if (h.ng == 0) h.nchunks = 0;
+    if (!h.bad) h.S = dec_chunk_size(h.nv, h.n1, (h.nv + blocks - 1) / blocks);
+    h.nchunks = h.ng ? (h.nv - 1 + h.S - 1) / h.S : 0;
     return h;
 }
 
@@ -1436,430 +1270,146 @@ __global__ void __launch_bounds__(kDB, 2) k_decode(const uint32_t *__restrict__ 
     }
 }
 
-// ---- many streams in one launch set -------------------------------------------------------
+// ---- many streams in one launch -----------------------------------------------------------
 //
-// k queues (or k streams) are concatenated; each kernel below walks the global
-// index space of all streams' miniblocks, groups or vectors and finds the
-// stream of an index by a binary search over the per-stream first indices, so
-// the k streams cost one launch set instead of k.  Each stream's bytes are
-// exactly those of a single-stream call.
+// The chunks of k queues (or k streams) are numbered one after another and
+// claimed in that order; a chunk looks back only at those of its own stream.
+// Each stream's bytes are exactly those of a single-stream call.  A raw stream
+// is copied kRawChunk values per chunk; a stream without whole miniblocks has
+// one chunk, its tail.  Lengths and per-stream errors go straight to pinned
+// host memory.
+constexpr uint64_t kRawChunk = 8192;
 
-struct BStream {
-    uint64_t in_off;   // encode: first input value; decode: first stream word (multiple of 4)
-    uint64_t out_off;  // encode: first output word (multiple of 4); decode: first output value
-    uint64_t n;        // values
-    uint64_t words;    // decode: stream length; encode: written by k_benc_tail
-    uint64_t nmb;      // miniblocks of the block part (0 for a raw stream)
-    uint64_t nv;       // decode: whole 16-byte vectors of the stream
-    uint64_t blkend;   // decode: word after the block part
-    uint32_t raw;      // raw copy (plugin threshold semantics)
-    uint32_t err;      // G5_DEVERR_* bits
+struct EncStream {
+    uint64_t in_off, out_off, n;  // first input value, first output word (a multiple of 4), values
+    uint32_t t0;                  // its first chunk's number
+    uint32_t raw;                 // copied as it is (plugin threshold semantics)
 };
 
-// The last stream s < k with first[s] <= x (empty streams share a first
-// index with the next one, so x always lands in a stream that holds it).
-__device__ __forceinline__ int find_stream(const uint64_t *first, int k, uint64_t x)
+struct DecStream {
+    uint64_t in_off, out_off, n, words;  // first stream word (a multiple of 4), first output value
+    uint32_t t0, nchunks, S;
+    uint32_t raw;
+};
+
+__device__ __forceinline__ void raw_chunk(const uint32_t *in, uint32_t *out, uint64_t n, uint64_t c)
 {
-    int lo = 0, hi = k - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (first[mid] <= x) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
+    const uint64_t end = min(n, (c + 1) * kRawChunk);
+    for (uint64_t i = c * kRawChunk + threadIdx.x; i < end; i += blockDim.x) out[i] = in[i];
 }
 
-// load_vectors for an input of any alignment (queues start anywhere).
-__device__ __forceinline__ void load_vectors_any(const uint32_t *in, uint64_t k, uint4 &cur, uint4 &prev)
+__global__ void __launch_bounds__(kEB, 3) k_encode_batch(const uint32_t *__restrict__ in, const EncStream *streams,
+                                                      const uint32_t *stream_of, uint32_t chunks, uint32_t gpc,
+                                                      uint32_t *__restrict__ out, uint64_t *scal,
+                                                      unsigned long long *slots, uint32_t stride, uint64_t *words,
+                                                      uint64_t *result, int mode)
 {
-    const int lane = g5_lane();
-    const uint32_t *p = in + k * 128 + 4 * (uint64_t)lane;
-    cur = make_uint4(p[0], p[1], p[2], p[3]);
-    uint4 q;
-    q.x = __shfl_up_sync(0xFFFFFFFFu, cur.x, 1);
-    q.y = __shfl_up_sync(0xFFFFFFFFu, cur.y, 1);
-    q.z = __shfl_up_sync(0xFFFFFFFFu, cur.z, 1);
-    q.w = __shfl_up_sync(0xFFFFFFFFu, cur.w, 1);
-    if (lane == 0) q = k ? make_uint4(p[-4], p[-3], p[-2], p[-1]) : make_uint4(0, 0, 0, 0);
-    prev = q;
-}
-
-__global__ void __launch_bounds__(kB) k_benc_bits(const uint32_t *in, const BStream *bs, const uint64_t *mb0,
-                                                  int k, uint64_t total_mb, uint8_t *mb_bits, uint32_t *mb_len,
-                                                  int mode)
-{
-    const uint64_t gw = ((uint64_t)blockIdx.x * kB + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * kB) >> 5;
-    for (uint64_t kg = gw; kg < total_mb; kg += nw) {
-        const int s = find_stream(mb0, k, kg);
-        uint4 cur, prev;
-        load_vectors_any(in + bs[s].in_off, kg - mb0[s], cur, prev);
-        const uint4 d = deltas(cur, prev, mode);
-        uint32_t acc = d.x | d.y | d.z | d.w;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) acc |= __shfl_xor_sync(0xFFFFFFFFu, acc, o);
-        if (g5_lane() == 0) {
-            const uint32_t b = bits_of(acc);
-            mb_bits[kg] = (uint8_t)b;
-            mb_len[kg] = 4 * b;
-        }
-    }
-}
-
-// mb_off: exclusive prefix of the payload words over all miniblocks.
-__global__ void __launch_bounds__(kB) k_benc_pack(const uint32_t *in, const BStream *bs, const uint64_t *mb0,
-                                                  int k, uint64_t total_mb, const uint8_t *mb_bits,
-                                                  const uint32_t *mb_off, uint32_t *out, int mode)
-{
-    __shared__ uint4 s_d[kB / 32][32];
-    const int lane = g5_lane(), wib = threadIdx.x >> 5;
-    const uint64_t gw = ((uint64_t)blockIdx.x * kB + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * kB) >> 5;
-    for (uint64_t kg = gw; kg < total_mb; kg += nw) {
-        const int s = find_stream(mb0, k, kg);
-        const BStream &st = bs[s];
-        const uint64_t kl = kg - mb0[s];
-        const uint32_t base = mb_off[mb0[s]];
-        uint32_t *o = out + st.out_off;
-        const uint32_t b = mb_bits[kg];
-        const uint64_t off = 4 + 4 * (kl / 16 + 1) + (uint64_t)(mb_off[kg] - base);
-        if ((kl & 15) == 0 && lane < 4) {
-            uint32_t h = 0;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint64_t kk = kl + 4 * lane + q;
-                const uint32_t bb = kk < st.nmb ? mb_bits[mb0[s] + kk] : 0u;
-                h |= bb << (24 - 8 * q);
-            }
-            o[4 + 4 * (kl / 16) + (uint64_t)(mb_off[kg] - base) + lane] = h;
-        }
-        uint4 cur, prev;
-        load_vectors_any(in + st.in_off, kl, cur, prev);
-        if (b == 32) {
-            reinterpret_cast<uint4 *>(o + off)[lane] = cur;
-            continue;
-        }
-        if (b == 0) continue;
-        s_d[wib][lane] = deltas(cur, prev, mode);
-        __syncwarp();
-        for (uint32_t idx = lane; idx < 4 * b; idx += 32) {
-            const uint32_t w = idx >> 2, l = idx & 3;
-            const uint32_t bit0 = 32 * w;
-            const uint32_t j0 = bit0 / b, j1 = (bit0 + 31) / b;
-            uint32_t word = 0;
-            for (uint32_t j = j0; j <= j1 && j < 32; ++j) {
-                const uint32_t dd = comp(s_d[wib][j], l);
-                const int sh = (int)(j * b) - (int)bit0;
-                word |= sh >= 0 ? (dd << sh) : (dd >> (-sh));
-            }
-            o[off + idx] = word;
-        }
-        __syncwarp();
-    }
-}
-
-// One warp per stream: raw copies, header words and the VariableByte tail;
-// the stream's length -> bs[s].words.  payload_total: sum of all payloads.
-__global__ void k_benc_tail(const uint32_t *in, BStream *bs, const uint64_t *mb0, int k, uint64_t total_mb,
-                            const uint32_t *mb_off, const uint32_t *payload_total, uint32_t *out)
-{
-    __shared__ uint32_t s_val[128];
-    __shared__ uint32_t s_bytes[(128 * 5 + 3) / 4 + 1];
-    const int lane = threadIdx.x;
-    for (int s = blockIdx.x; s < k; s += gridDim.x) {
-        BStream &st = bs[s];
+    extern __shared__ __align__(16) unsigned char s_dyn_e[];
+    EncShared &sh = *reinterpret_cast<EncShared *>(s_dyn_e);
+    if (threadIdx.x >= 1 && threadIdx.x < 32) sh.magic[threadIdx.x] = 65536u / threadIdx.x + 1u;
+    g5_pdl_sync();
+    const uint64_t epoch = scal[CS_E_EPOCH];
+    for (;;) {
+        const uint64_t t = claim_tile(&scal[CS_E_CTR], &sh.t);
+        if (t >= chunks) break;
+        const uint32_t q = stream_of[t];
+        const EncStream st = streams[q];
+        const uint64_t c = t - st.t0;
         const uint32_t *x = in + st.in_off;
         uint32_t *o = out + st.out_off;
         if (st.raw) {
-            for (uint64_t i = lane; i < st.n; i += 32) o[i] = x[i];
-            if (lane == 0) st.words = st.n;
+            raw_chunk(x, o, st.n, c);
+            if (c == 0 && threadIdx.x == 0) words[q] = st.n;
             continue;
         }
-        const uint64_t nmb = st.nmb, n1 = nmb * 128, ngroups = (nmb + 15) / 16;
-        uint64_t payload = 0;
-        if (nmb) {
-            const uint64_t e = mb0[s] + nmb;
-            payload = (uint64_t)((e < total_mb ? mb_off[e] : *payload_total) - mb_off[mb0[s]]);
-        }
-        const uint64_t blkend = 4 + 4 * ngroups + payload;
-        const uint32_t nt = (uint32_t)(st.n - n1);
-        __syncwarp();
-        for (uint32_t i = lane; i < nt; i += 32) s_val[i] = x[n1 + i];
-        for (uint32_t i = lane; i < sizeof(s_bytes) / 4; i += 32) s_bytes[i] = 0;
-        __syncwarp();
-        if (lane == 0) {
-            o[0] = (uint32_t)n1;
-            o[1] = kCookie;
-            o[2] = kCookie;
-            o[3] = kCookie;
-            uint8_t *bb = reinterpret_cast<uint8_t *>(s_bytes);
-            uint32_t p = 0, prevv = 0;
-            for (uint32_t i = 0; i < nt; ++i) {
-                uint32_t v = s_val[i] - prevv;
-                prevv = s_val[i];
-                while (v >= 128u) {
-                    bb[p++] = (uint8_t)(v & 127u);
-                    v >>= 7;
-                }
-                bb[p++] = (uint8_t)(v | 128u);
+        EncLen e = enc_len(st.n, st.n, 0, 1);
+        e.gpc = gpc;
+        e.nchunks = (e.ng + gpc - 1) / gpc;
+        unsigned long long *sl = slots + (uint64_t)stride * st.t0;
+        if (e.ng == 0) {
+            if (threadIdx.x < 32) {
+                const uint64_t w = enc_tail_warp(x, e.n, 0, 4, o, sh.bytes);
+                if (threadIdx.x == 0) words[q] = w;
             }
-            const uint32_t tw = (p + 3) / 4;
-            s_val[0] = tw;
-            st.words = blkend + tw;
-        }
-        __syncwarp();
-        const uint32_t tw = s_val[0];
-        for (uint32_t i = lane; i < tw; i += 32) o[blkend + i] = s_bytes[i];
-    }
-}
-
-// Stream headers (one thread per stream): cookies and the block-part length.
-__global__ void k_bdec_prep(const uint32_t *in, BStream *bs, int k)
-{
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < k; s += gridDim.x * blockDim.x) {
-        BStream &st = bs[s];
-        st.err = 0;
-        st.blkend = 4;
-        if (st.raw) {
-            if (st.words != st.n) st.err |= G5_DEVERR_CORRUPT;
-            continue;
-        }
-        const uint32_t *x = in + st.in_off;
-        if (st.words < 4 || x[0] != st.nmb * 128 || x[1] != kCookie || x[2] != kCookie || x[3] != kCookie)
-            st.err |= G5_DEVERR_CORRUPT;
-    }
-}
-
-// jump[vg] = global vector after the group whose header is global vector vg,
-// or the sink (total_v) when that leaves the stream.
-__global__ void __launch_bounds__(kB) k_bdec_jump(const uint32_t *in, const BStream *bs, const uint64_t *v0,
-                                                  int k, uint64_t total_v, uint32_t *jump)
-{
-    for (uint64_t vg = (uint64_t)blockIdx.x * kB + threadIdx.x; vg <= total_v; vg += (uint64_t)gridDim.x * kB) {
-        uint32_t j = (uint32_t)total_v;
-        if (vg < total_v) {
-            const int s = find_stream(v0, k, vg);
-            const BStream &st = bs[s];
-            const uint64_t lv = vg - v0[s];
-            const uint4 h = reinterpret_cast<const uint4 *>(in + st.in_off)[lv];
-            const uint32_t hw[4] = {h.x, h.y, h.z, h.w};
-            uint32_t sum = 0;
-            bool ok = true;
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-#pragma unroll
-                for (int by = 0; by < 4; ++by) {
-                    const uint32_t b = (hw[q] >> (8 * by)) & 0xFF;
-                    ok &= b <= 32;
-                    sum += b;
-                }
-            if (ok && lv + 1 + sum < st.nv) j = (uint32_t)(vg + 1 + sum);
-        }
-        jump[vg] = j;
-    }
-}
-
-__global__ void __launch_bounds__(kB) k_bdec_lift(uint32_t *jump, uint64_t total_v, uint64_t stride, int r)
-{
-    const uint32_t *t = jump + stride * r;
-    uint32_t *t1 = jump + stride * (r + 1);
-    for (uint64_t i = (uint64_t)blockIdx.x * kB + threadIdx.x; i <= total_v; i += (uint64_t)gridDim.x * kB)
-        t1[i] = t[t[i]];
-}
-
-// Group positions (local vector index of each group header); the last group
-// of a stream gives the end of its block part.
-__global__ void __launch_bounds__(kB) k_bdec_pos(const uint32_t *in, BStream *bs, const uint64_t *g0,
-                                                 const uint64_t *v0, int k, uint64_t total_g, uint64_t total_v,
-                                                 const uint32_t *jump, uint64_t stride, int R, uint32_t *gpos)
-{
-    for (uint64_t gg = (uint64_t)blockIdx.x * kB + threadIdx.x; gg < total_g; gg += (uint64_t)gridDim.x * kB) {
-        const int s = find_stream(g0, k, gg);
-        BStream &st = bs[s];
-        const uint64_t g = gg - g0[s], ng = (st.nmb + 15) / 16;
-        uint64_t pos = v0[s] + 1;
-        for (int r = 0; r < R && pos < total_v; ++r)
-            if ((g >> r) & 1) pos = jump[stride * r + pos];
-        uint64_t lp = 0;
-        if (st.err || pos >= v0[s] + st.nv) {
-            atomicOr(&st.err, (uint32_t)G5_DEVERR_CORRUPT);
+        } else if ((uintptr_t)x & 15) {
+            enc_chunk<true>(sh, e, x, c, epoch, sl, stride, &scal[CS_E_ERR], o, mode, words + q);
         } else {
-            lp = pos - v0[s];
-            if (g == ng - 1) {
-                const uint64_t howmany = st.nmb - 16 * g;
-                const uint4 h = reinterpret_cast<const uint4 *>(in + st.in_off)[lp];
-                const uint32_t hw[4] = {h.x, h.y, h.z, h.w};
-                uint64_t sum = 0;
-                bool ok = true;
-                for (uint64_t i = 0; i < howmany; ++i) {
-                    const uint32_t b = (hw[i / 4] >> (24 - 8 * (i % 4))) & 0xFF;
-                    ok &= b <= 32;
-                    sum += b;
-                }
-                const uint64_t end = lp + 1 + sum;
-                if (!ok || end > st.nv) atomicOr(&st.err, (uint32_t)G5_DEVERR_CORRUPT);
-                else st.blkend = 4 * end;
-            }
+            enc_chunk<false>(sh, e, x, c, epoch, sl, stride, &scal[CS_E_ERR], o, mode, words + q);
         }
-        gpos[gg] = (uint32_t)lp;
+    }
+    if (last_block(&scal[CS_E_DONE])) {
+        __threadfence();
+        result[0] = vload64(&scal[CS_E_ERR]);
+        scal[CS_E_CTR] = 0;
+        scal[CS_E_DONE] = 0;
+        scal[CS_E_ERR] = 0;
+        scal[CS_E_EPOCH] = epoch + 1;
+        __threadfence();
     }
 }
 
-// Per miniblock lane sums (the first miniblock of a stream starts from zero,
-// so its sums are absolute and reset the scan).
-__global__ void __launch_bounds__(kB) k_bdec_sum(const uint32_t *in, const BStream *bs, const uint64_t *mb0,
-                                                 const uint64_t *g0, int k, uint64_t total_mb,
-                                                 const uint32_t *gpos, VecFlag *mb_sf, int mode)
+// err[q] becomes nonzero for a stream that does not decode to exactly its n
+// values (the host cleared it).
+__global__ void __launch_bounds__(kDB, 2) k_decode_batch(const uint32_t *__restrict__ in, const DecStream *streams,
+                                                      const uint32_t *stream_of, uint32_t chunks,
+                                                      uint32_t *__restrict__ out, uint64_t *scal, ChunkSlot *slots,
+                                                      uint32_t *err, uint64_t *result, int mode)
 {
-    const uint64_t gw = ((uint64_t)blockIdx.x * kB + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * kB) >> 5;
-    for (uint64_t kg = gw; kg < total_mb; kg += nw) {
-        const int s = find_stream(mb0, k, kg);
-        const BStream &st = bs[s];
-        const uint64_t kl = kg - mb0[s];
-        VecFlag r;
-        r.v = make_uint4(0, 0, 0, 0);
-        r.f = 1;
-        if (!st.err) {
-            const uint32_t *x = in + st.in_off;
-            uint64_t off;
-            uint32_t b;
-            mb_locate(x, gpos + g0[s], kl, off, b);
-            const uint4 d = unpack_vec(x, off, b);
-            if (b == 32) {
-                r.v.x = __shfl_sync(0xFFFFFFFFu, d.x, 31);
-                r.v.y = __shfl_sync(0xFFFFFFFFu, d.y, 31);
-                r.v.z = __shfl_sync(0xFFFFFFFFu, d.z, 31);
-                r.v.w = __shfl_sync(0xFFFFFFFFu, d.w, 31);
-            } else {
-                uint32_t sx = d.x, sy = d.y, sz = d.z, sw = d.w;
-#pragma unroll
-                for (int o = 16; o; o >>= 1) {
-                    sx += __shfl_xor_sync(0xFFFFFFFFu, sx, o);
-                    sy += __shfl_xor_sync(0xFFFFFFFFu, sy, o);
-                    sz += __shfl_xor_sync(0xFFFFFFFFu, sz, o);
-                    sw += __shfl_xor_sync(0xFFFFFFFFu, sw, o);
-                }
-                if (mode == G5_CODEC_DM) r.v = make_uint4(sw, sw, sw, sw);
-                else r.v = make_uint4(sx, sy, sz, sw);
-                r.f = kl == 0 ? 1u : 0u;
-            }
-        }
-        if (g5_lane() == 0) mb_sf[kg] = r;
-    }
-}
-
-__global__ void __launch_bounds__(kB) k_bdec_out(const uint32_t *in, const BStream *bs, const uint64_t *mb0,
-                                                 const uint64_t *g0, int k, uint64_t total_mb,
-                                                 const uint32_t *gpos, const VecFlag *mb_base, uint32_t *out,
-                                                 int mode)
-{
-    const int lane = g5_lane();
-    const uint64_t gw = ((uint64_t)blockIdx.x * kB + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * kB) >> 5;
-    for (uint64_t kg = gw; kg < total_mb; kg += nw) {
-        const int s = find_stream(mb0, k, kg);
-        const BStream &st = bs[s];
-        if (st.err) continue;
-        const uint64_t kl = kg - mb0[s];
-        const uint32_t *x = in + st.in_off;
-        uint64_t off;
-        uint32_t b;
-        mb_locate(x, gpos + g0[s], kl, off, b);
-        const uint4 d = unpack_vec(x, off, b);
-        const uint4 base = kl == 0 ? make_uint4(0, 0, 0, 0) : mb_base[kg].v;
-        uint4 v;
-        if (b == 32) {
-            v = d;
-        } else if (mode == G5_CODEC_DM) {
-            uint32_t c = d.w;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, c, o);
-                if (lane >= o) c += y;
-            }
-            c += base.w;
-            uint32_t pc = __shfl_up_sync(0xFFFFFFFFu, c, 1);
-            if (lane == 0) pc = base.w;
-            v = make_uint4(d.x + pc, d.y + pc, d.z + pc, c);
-        } else {
-            uint32_t cx = d.x, cy = d.y, cz = d.z, cw = d.w;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t yx = __shfl_up_sync(0xFFFFFFFFu, cx, o);
-                const uint32_t yy = __shfl_up_sync(0xFFFFFFFFu, cy, o);
-                const uint32_t yz = __shfl_up_sync(0xFFFFFFFFu, cz, o);
-                const uint32_t yw = __shfl_up_sync(0xFFFFFFFFu, cw, o);
-                if (lane >= o) {
-                    cx += yx;
-                    cy += yy;
-                    cz += yz;
-                    cw += yw;
-                }
-            }
-            v = make_uint4(cx + base.x, cy + base.y, cz + base.z, cw + base.w);
-        }
-        uint32_t *o = out + st.out_off + kl * 128 + 4 * (uint64_t)lane;  // any alignment
-        o[0] = v.x;
-        o[1] = v.y;
-        o[2] = v.z;
-        o[3] = v.w;
-    }
-}
-
-// One warp per stream: raw copies and the VariableByte tail; every stream
-// must decode to exactly its n values.
-__global__ void k_bdec_tail(const uint32_t *in, BStream *bs, int k, uint32_t *out)
-{
-    __shared__ uint32_t s_b[kTailMaxBytes / 4];
-    const int lane = threadIdx.x;
-    for (int s = blockIdx.x; s < k; s += gridDim.x) {
-        BStream &st = bs[s];
+    extern __shared__ __align__(16) unsigned char s_dyn_d[];
+    DecShared &sh = *reinterpret_cast<DecShared *>(s_dyn_d);
+    g5_pdl_sync();
+    const uint64_t epoch = scal[CS_U_EPOCH];
+    for (;;) {
+        const uint64_t t = claim_tile(&scal[CS_U_CTR], &sh.t);
+        if (t >= chunks) break;
+        const uint32_t q = stream_of[t];
+        const DecStream st = streams[q];
+        const uint64_t c = t - st.t0;
         const uint32_t *x = in + st.in_off;
         uint32_t *o = out + st.out_off;
-        if (st.err) continue;
         if (st.raw) {
-            for (uint64_t i = lane; i < st.n; i += 32) o[i] = x[i];
+            if (st.words == st.n) raw_chunk(x, o, st.n, c);
+            else err[q] = 1;
             continue;
         }
-        const uint64_t n1 = st.nmb * 128;
-        const uint64_t tw = st.words > st.blkend ? st.words - st.blkend : 0;
-        if (tw * 4 > kTailMaxBytes) {
-            if (lane == 0) st.err |= G5_DEVERR_CORRUPT;
+        DecHead h;
+        h.words = st.words;
+        h.nv = st.words / 4;
+        h.nmb = st.n / 128;
+        h.n1 = h.nmb * 128;
+        h.ng = (h.nmb + 15) / 16;
+        h.S = st.S;
+        h.nchunks = st.nchunks;
+        h.raw = false;
+        h.bad = st.words < 4;
+        if (!h.bad) {
+            const uint4 w = *reinterpret_cast<const uint4 *>(x);
+            h.bad = w.x != h.n1 || w.y != kCookie || w.z != kCookie || w.w != kCookie;
+        }
+        // (a stream with groups but no vector for them has no chunk to find it)
+        if (h.bad || (h.ng && h.nv < 2)) {
+            err[q] = 1;
             continue;
         }
-        __syncwarp();
-        for (uint64_t i = lane; i < tw; i += 32) s_b[i] = x[st.blkend + i];
-        __syncwarp();
-        if (lane == 0) {
-            const uint8_t *bb = reinterpret_cast<const uint8_t *>(s_b);
-            uint64_t c = n1;
-            uint32_t prevv = 0, v = 0;
-            int shift = 0;
-            uint32_t err = 0;
-            for (uint64_t p = 0; p < tw * 4; ++p) {
-                const uint32_t ch = bb[p];
-                v |= (ch & 127u) << shift;
-                if (ch & 128u) {
-                    if (c >= st.n) {
-                        err |= G5_DEVERR_CORRUPT;
-                        break;
-                    }
-                    prevv += v;
-                    o[c++] = prevv;
-                    v = 0;
-                    shift = 0;
-                } else {
-                    shift += 7;
-                    if (shift > 28) {
-                        err |= G5_DEVERR_CORRUPT;
-                        break;
-                    }
-                }
-            }
-            if (c != st.n) err |= G5_DEVERR_CORRUPT;
-            st.err |= err;
+        uint32_t bad = 0;
+        uint64_t n = ~0ull;  // the value count, in the lane that decoded the tail
+        if (h.ng == 0) {
+            if (threadIdx.x < 32) bad = dec_tail(sh.tail, x, h.words, 4, 0, st.n, o, nullptr, n);
+        } else if ((uintptr_t)o & 15) {
+            bad = dec_chunk<true>(sh, h, x, c, epoch, slots + st.t0, &scal[CS_U_ERR], o, st.n, nullptr, mode, &n);
+        } else {
+            bad = dec_chunk<false>(sh, h, x, c, epoch, slots + st.t0, &scal[CS_U_ERR], o, st.n, nullptr, mode, &n);
         }
+        if (bad || (n != ~0ull && n != st.n)) err[q] = 1;
+    }
+    if (last_block(&scal[CS_U_DONE])) {
+        __threadfence();
+        result[0] = vload64(&scal[CS_U_ERR]);
+        scal[CS_U_CTR] = 0;
+        scal[CS_U_DONE] = 0;
+        scal[CS_U_ERR] = 0;
+        scal[CS_U_EPOCH] = epoch + 1;
+        __threadfence();
     }
 }
 
@@ -1892,6 +1442,8 @@ g5_status codec_kernels()
 {
     G5_CUDA(cudaFuncSetAttribute(k_encode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EncShared)));
     G5_CUDA(cudaFuncSetAttribute(k_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecShared)));
+    G5_CUDA(cudaFuncSetAttribute(k_encode_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EncShared)));
+    G5_CUDA(cudaFuncSetAttribute(k_decode_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecShared)));
     return G5_OK;
 }
 
@@ -1959,24 +1511,46 @@ void codec_decode_launch(CodecWork &w, const uint32_t *in, const uint64_t *words
 
 namespace {
 
-// Device buffers of the batched calls, grown on demand (contents not kept).
+// Buffers of the batched calls, grown on demand (contents not kept).
 struct BatchWs {
-    void *p[10] = {nullptr};
-    size_t cap[10] = {0};
-    enum { BS, IDX, BITS, LEN, JUMP, GPOS, SF, BASE, PART, CNT };
-    g5_status grow(int i, size_t bytes)
+    void *desc = nullptr, *slots = nullptr;  // device: streams and chunk numbers; records
+    void *h_desc = nullptr, *h_res = nullptr;  // pinned: what goes to desc; what the kernel leaves
+    size_t desc_cap = 0, slots_cap = 0, res_cap = 0;
+    g5_status grow(size_t desc_bytes, size_t slot_bytes, size_t res_bytes)
     {
-        if (p[i] && cap[i] >= bytes) return G5_OK;
-        cudaFree(p[i]);
-        p[i] = nullptr;
-        cap[i] = 0;
-        if (cudaMalloc(&p[i], bytes ? bytes : 16) != cudaSuccess) return G5_ERR_OOM;
-        cap[i] = bytes;
+        if (desc_bytes > desc_cap) {
+            cudaFree(desc);
+            cudaFreeHost(h_desc);
+            desc = h_desc = nullptr;
+            desc_cap = 0;
+            if (cudaMalloc(&desc, desc_bytes) != cudaSuccess || cudaMallocHost(&h_desc, desc_bytes) != cudaSuccess)
+                return G5_ERR_OOM;
+            desc_cap = desc_bytes;
+        }
+        if (slot_bytes > slots_cap) {
+            cudaFree(slots);
+            slots = nullptr;
+            slots_cap = 0;
+            if (cudaMalloc(&slots, slot_bytes) != cudaSuccess) return G5_ERR_OOM;
+            // (zeroed records read as not published)
+            if (cudaMemset(slots, 0, slot_bytes) != cudaSuccess) return G5_ERR_CUDA;
+            slots_cap = slot_bytes;
+        }
+        if (res_bytes > res_cap) {
+            cudaFreeHost(h_res);
+            h_res = nullptr;
+            res_cap = 0;
+            if (cudaMallocHost(&h_res, res_bytes) != cudaSuccess) return G5_ERR_OOM;
+            res_cap = res_bytes;
+        }
         return G5_OK;
     }
     void release()
     {
-        for (int i = 0; i < 10; ++i) cudaFree(p[i]);
+        cudaFree(desc);
+        cudaFree(slots);
+        cudaFreeHost(h_desc);
+        cudaFreeHost(h_res);
         *this = BatchWs();
     }
 };
@@ -1988,7 +1562,7 @@ size_t round4(size_t w) { return (w + 3) & ~(size_t)3; }
 struct g5_codec {
     g5::CodecWork w;
     uint64_t *h_scal = nullptr;  // pinned
-    BatchWs bw;
+    BatchWs be, bd;  // encode, decode
 };
 
 extern "C" {
@@ -2022,7 +1596,8 @@ g5_status g5_codec_destroy(g5_codec *c)
     cudaDeviceSynchronize();
     g5::codec_work_free(c->w);
     cudaFreeHost(c->h_scal);
-    c->bw.release();
+    c->be.release();
+    c->bd.release();
     delete c;
     return G5_OK;
 }
@@ -2120,51 +1695,52 @@ g5_status g5_codec_encode_batch(g5_codec *c, const uint32_t *in_dev, const uint6
     for (int q = 0; q < k; ++q)
         if (in_off[q + 1] < in_off[q]) return G5_ERR_INVALID_ARG;
     if (in_off[k] > ((uint64_t)1 << 31)) return G5_ERR_CAPACITY;  // payload offsets are 32-bit
-    std::vector<g5::BStream> hb((size_t)k);
-    std::vector<uint64_t> mb0((size_t)k + 1);
-    uint64_t total_mb = 0;
+    // groups per chunk: one chunk per block if that fits, the same for all queues
+    uint64_t groups = 0;
     for (int q = 0; q < k; ++q) {
-        g5::BStream &b = hb[q];
-        memset(&b, 0, sizeof b);
+        const uint64_t n = in_off[q + 1] - in_off[q];
+        out_off[q + 1] = out_off[q] + round4(g5::codec_bound((size_t)n));
+        if (!(raw_threshold && n <= raw_threshold)) groups += (n / 128 + 15) / 16;
+    }
+    const uint64_t blocks = (uint64_t)c->w.egrid;
+    const uint32_t gpc = (uint32_t)std::min<uint64_t>(g5::kEG, std::max<uint64_t>(1, (groups + blocks - 1) / blocks));
+    auto chunks_of = [&](uint64_t n, bool raw) -> uint64_t {
+        if (raw) return std::max<uint64_t>(1, (n + g5::kRawChunk - 1) / g5::kRawChunk);
+        return std::max<uint64_t>(1, ((n / 128 + 15) / 16 + gpc - 1) / gpc);
+    };
+    uint64_t chunks = 0;
+    for (int q = 0; q < k; ++q) {
+        const uint64_t n = in_off[q + 1] - in_off[q];
+        chunks += chunks_of(n, raw_threshold && n <= raw_threshold);
+    }
+    if (chunks >= ((uint64_t)1 << 32)) return G5_ERR_CAPACITY;
+    BatchWs &w = c->be;
+    const size_t sb = sizeof(g5::EncStream) * (size_t)k, db = sb + sizeof(uint32_t) * (size_t)chunks;
+    const uint32_t stride = chunks > 16384 ? 2 : g5::kSlot;  // (very many: packed)
+    G5_TRY(w.grow(db, sizeof(uint64_t) * stride * (size_t)chunks, sizeof(uint64_t) * ((size_t)k + 1)));
+    g5::EncStream *hs = static_cast<g5::EncStream *>(w.h_desc);
+    uint32_t *ho = reinterpret_cast<uint32_t *>(static_cast<char *>(w.h_desc) + sb);
+    uint32_t t = 0;
+    for (int q = 0; q < k; ++q) {
+        g5::EncStream &b = hs[q];
         b.in_off = in_off[q];
         b.out_off = out_off[q];
         b.n = in_off[q + 1] - in_off[q];
         b.raw = raw_threshold && b.n <= raw_threshold;
-        b.nmb = b.raw ? 0 : b.n / 128;
-        out_off[q + 1] = out_off[q] + round4(g5::codec_bound((size_t)b.n));
-        mb0[q] = total_mb;
-        total_mb += b.nmb;
+        b.t0 = t;
+        for (uint64_t e = t + chunks_of(b.n, b.raw != 0); t < e; ++t) ho[t] = (uint32_t)q;
     }
-    mb0[k] = total_mb;
-    BatchWs &w = c->bw;
-    const int grid = g5::num_sms() * 4;
-    G5_TRY(w.grow(BatchWs::BS, sizeof(g5::BStream) * (size_t)k));
-    G5_TRY(w.grow(BatchWs::IDX, sizeof(uint64_t) * ((size_t)k + 1)));
-    G5_TRY(w.grow(BatchWs::BITS, total_mb + 1));
-    G5_TRY(w.grow(BatchWs::LEN, sizeof(uint32_t) * (total_mb + 1)));
-    G5_TRY(w.grow(BatchWs::PART, sizeof(uint32_t) * ((size_t)grid + 1)));
-    G5_TRY(w.grow(BatchWs::CNT, sizeof(uint64_t)));
-    g5::BStream *bs = (g5::BStream *)w.p[BatchWs::BS];
-    uint64_t *idx = (uint64_t *)w.p[BatchWs::IDX], *cnt = (uint64_t *)w.p[BatchWs::CNT];
-    uint8_t *bits = (uint8_t *)w.p[BatchWs::BITS];
-    uint32_t *len = (uint32_t *)w.p[BatchWs::LEN], *part = (uint32_t *)w.p[BatchWs::PART];
     cudaStream_t s = (cudaStream_t)stream;
-    G5_CUDA(cudaMemcpyAsync(bs, hb.data(), sizeof(g5::BStream) * (size_t)k, cudaMemcpyHostToDevice, s));
-    G5_CUDA(cudaMemcpyAsync(idx, mb0.data(), sizeof(uint64_t) * ((size_t)k + 1), cudaMemcpyHostToDevice, s));
-    G5_CUDA(cudaMemcpyAsync(cnt, &mb0[k], sizeof(uint64_t), cudaMemcpyHostToDevice, s));
-    G5_CUDA(cudaMemsetAsync(part + grid, 0, sizeof(uint32_t), s));
-    if (total_mb) {
-        g5::k_benc_bits<<<grid, g5::kB, 0, s>>>(in_dev, bs, idx, k, total_mb, bits, len, mode);
-        g5::k_scan_red<g5::AddU32><<<grid, g5::kB, 0, s>>>(len, cnt, part);
-        g5::k_scan_top<g5::AddU32><<<1, g5::kB, 0, s>>>(part, grid, part + grid);
-        g5::k_scan_down<g5::AddU32><<<grid, g5::kB, 0, s>>>(len, len, cnt, part);
-        g5::k_benc_pack<<<grid, g5::kB, 0, s>>>(in_dev, bs, idx, k, total_mb, bits, len, out_dev, mode);
-    }
-    g5::k_benc_tail<<<std::min(k, 65535), 32, 0, s>>>(in_dev, bs, idx, k, total_mb, len, part + grid, out_dev);
+    G5_CUDA(cudaMemcpyAsync(w.desc, w.h_desc, db, cudaMemcpyHostToDevice, s));
+    uint64_t *hw = static_cast<uint64_t *>(w.h_res);
+    const g5::EncStream *ds = static_cast<const g5::EncStream *>(w.desc);
+    g5::launch_dyn(true, g5::k_encode_batch, (int)std::min(chunks, blocks), g5::kEB, sizeof(g5::EncShared), s, in_dev, ds,
+                   reinterpret_cast<const uint32_t *>(static_cast<const char *>(w.desc) + sb), (uint32_t)chunks, gpc,
+                   out_dev, c->w.scal, static_cast<unsigned long long *>(w.slots), stride, hw, hw + k, mode);
     G5_CUDA(cudaGetLastError());
-    G5_CUDA(cudaMemcpyAsync(hb.data(), bs, sizeof(g5::BStream) * (size_t)k, cudaMemcpyDeviceToHost, s));
     G5_CUDA(cudaStreamSynchronize(s));
-    for (int q = 0; q < k; ++q) out_words[q] = hb[q].words;
+    if (hw[k]) return G5_ERR_TIMEOUT;
+    for (int q = 0; q < k; ++q) out_words[q] = hw[q];
     return G5_OK;
 }
 
@@ -2178,89 +1754,63 @@ g5_status g5_codec_decode_batch(g5_codec *c, const uint32_t *in_dev, const uint6
     out_off[0] = 0;
     if (k == 0) return G5_OK;
     if (!in_dev || !out_dev || ((uintptr_t)in_dev & 15)) return G5_ERR_INVALID_ARG;
-    std::vector<g5::BStream> hb((size_t)k);
-    std::vector<uint64_t> mb0((size_t)k + 1), g0((size_t)k + 1), v0((size_t)k + 1);
-    uint64_t total_mb = 0, total_g = 0, total_v = 0;
-    int max_ng = 0;
+    uint64_t total_v = 0;
     for (int q = 0; q < k; ++q) {
         if (in_off[q] % 4) return G5_ERR_INVALID_ARG;  // streams start 16-byte aligned
-        g5::BStream &b = hb[q];
-        memset(&b, 0, sizeof b);
+        // plugin semantics: raw when n <= thr or the stream is as long as n
+        const bool raw = raw_threshold && (n[q] <= raw_threshold || words[q] == n[q]);
+        out_off[q + 1] = out_off[q] + n[q];
+        if (!raw) total_v += words[q] / 4;
+    }
+    if (total_v >= ((uint64_t)1 << 32) - 2 || out_off[k] > ((uint64_t)1 << 40)) return G5_ERR_CAPACITY;
+    const uint64_t blocks = (uint64_t)c->w.grid, per = (total_v + blocks - 1) / blocks;
+    auto plan = [&](int q, g5::DecStream &b) -> uint64_t {
         b.in_off = in_off[q];
         b.out_off = out_off[q];
         b.n = n[q];
         b.words = words[q];
-        // plugin semantics: raw when n <= thr or the stream is as long as n
         b.raw = raw_threshold && (b.n <= raw_threshold || b.words == b.n);
-        b.nmb = b.raw ? 0 : b.n / 128;
-        b.nv = b.raw ? 0 : b.words / 4;
-        out_off[q + 1] = out_off[q] + b.n;
-        mb0[q] = total_mb;
-        g0[q] = total_g;
-        v0[q] = total_v;
-        const uint64_t ng = (b.nmb + 15) / 16;
-        total_mb += b.nmb;
-        total_g += ng;
-        total_v += b.nv;
-        max_ng = std::max<int>(max_ng, (int)std::min<uint64_t>(ng, 1u << 30));
-    }
-    mb0[k] = total_mb;
-    g0[k] = total_g;
-    v0[k] = total_v;
-    if (total_v >= ((uint64_t)1 << 32) - 2 || out_off[k] > ((uint64_t)1 << 40)) return G5_ERR_CAPACITY;
-    int R = 1;
-    while (((uint64_t)1 << R) < (uint64_t)max_ng + 1) ++R;
-    const uint64_t stride = total_v + 1;
-    BatchWs &w = c->bw;
-    const int grid = g5::num_sms() * 4;
-    G5_TRY(w.grow(BatchWs::BS, sizeof(g5::BStream) * (size_t)k));
-    G5_TRY(w.grow(BatchWs::IDX, sizeof(uint64_t) * 3 * ((size_t)k + 1)));
-    G5_TRY(w.grow(BatchWs::JUMP, sizeof(uint32_t) * stride * (size_t)R));
-    G5_TRY(w.grow(BatchWs::GPOS, sizeof(uint32_t) * (total_g + 1)));
-    G5_TRY(w.grow(BatchWs::SF, sizeof(g5::VecFlag) * (total_mb + 1)));
-    G5_TRY(w.grow(BatchWs::BASE, sizeof(g5::VecFlag) * (total_mb + 1)));
-    G5_TRY(w.grow(BatchWs::PART, sizeof(g5::VecFlag) * ((size_t)grid + 1)));
-    G5_TRY(w.grow(BatchWs::CNT, sizeof(uint64_t)));
-    g5::BStream *bs = (g5::BStream *)w.p[BatchWs::BS];
-    uint64_t *idx = (uint64_t *)w.p[BatchWs::IDX], *cnt = (uint64_t *)w.p[BatchWs::CNT];
-    uint64_t *dmb0 = idx, *dg0 = idx + (k + 1), *dv0 = idx + 2 * (k + 1);
-    uint32_t *jump = (uint32_t *)w.p[BatchWs::JUMP], *gpos = (uint32_t *)w.p[BatchWs::GPOS];
-    g5::VecFlag *sf = (g5::VecFlag *)w.p[BatchWs::SF], *base = (g5::VecFlag *)w.p[BatchWs::BASE];
-    g5::VecFlag *part = (g5::VecFlag *)w.p[BatchWs::PART];
-    cudaStream_t s = (cudaStream_t)stream;
-    std::vector<uint64_t> allidx;
-    allidx.reserve(3 * ((size_t)k + 1));
-    allidx.insert(allidx.end(), mb0.begin(), mb0.end());
-    allidx.insert(allidx.end(), g0.begin(), g0.end());
-    allidx.insert(allidx.end(), v0.begin(), v0.end());
-    G5_CUDA(cudaMemcpyAsync(bs, hb.data(), sizeof(g5::BStream) * (size_t)k, cudaMemcpyHostToDevice, s));
-    G5_CUDA(cudaMemcpyAsync(idx, allidx.data(), sizeof(uint64_t) * allidx.size(), cudaMemcpyHostToDevice, s));
-    G5_CUDA(cudaMemcpyAsync(cnt, &mb0[k], sizeof(uint64_t), cudaMemcpyHostToDevice, s));
-    const int pgrid = std::max(1, std::min(grid, (k + g5::kB - 1) / g5::kB));
-    g5::k_bdec_prep<<<pgrid, g5::kB, 0, s>>>(in_dev, bs, k);
-    if (total_g) {
-        g5::k_bdec_jump<<<grid, g5::kB, 0, s>>>(in_dev, bs, dv0, k, total_v, jump);
-        for (int r = 0; r + 1 < R; ++r) g5::k_bdec_lift<<<grid, g5::kB, 0, s>>>(jump, total_v, stride, r);
-        g5::k_bdec_pos<<<grid, g5::kB, 0, s>>>(in_dev, bs, dg0, dv0, k, total_g, total_v, jump, stride, R, gpos);
-    }
-    if (total_mb) {
-        g5::k_bdec_sum<<<grid, g5::kB, 0, s>>>(in_dev, bs, dmb0, dg0, k, total_mb, gpos, sf, mode);
-        g5::k_scan_red<g5::ResetAdd><<<grid, g5::kB, 0, s>>>(sf, cnt, part);
-        g5::k_scan_top<g5::ResetAdd><<<1, g5::kB, 0, s>>>(part, grid, nullptr);
-        g5::k_scan_down<g5::ResetAdd><<<grid, g5::kB, 0, s>>>(sf, base, cnt, part);
-        g5::k_bdec_out<<<grid, g5::kB, 0, s>>>(in_dev, bs, dmb0, dg0, k, total_mb, gpos, base, out_dev, mode);
-    }
-    g5::k_bdec_tail<<<std::min(k, 65535), 32, 0, s>>>(in_dev, bs, k, out_dev);
-    G5_CUDA(cudaGetLastError());
-    G5_CUDA(cudaMemcpyAsync(hb.data(), bs, sizeof(g5::BStream) * (size_t)k, cudaMemcpyDeviceToHost, s));
-    G5_CUDA(cudaStreamSynchronize(s));
-    bool all = true;
+        const uint64_t nv = b.words / 4, n1 = b.n / 128 * 128;
+        b.S = g5::dec_chunk_size(nv, n1, per);
+        const uint64_t nc = b.raw ? (b.n + g5::kRawChunk - 1) / g5::kRawChunk : n1 && nv > 1 ? (nv - 1 + b.S - 1) / b.S : 1;
+        b.nchunks = (uint32_t)std::max<uint64_t>(1, nc);
+        return b.nchunks;
+    };
+    uint64_t chunks = 0;
     for (int q = 0; q < k; ++q) {
-        const bool ok = hb[q].err == 0;
+        g5::DecStream b;
+        chunks += plan(q, b);
+    }
+    if (chunks >= ((uint64_t)1 << 32)) return G5_ERR_CAPACITY;
+    BatchWs &w = c->bd;
+    const size_t sb = sizeof(g5::DecStream) * (size_t)k, db = sb + sizeof(uint32_t) * (size_t)chunks;
+    G5_TRY(w.grow(db, sizeof(g5::ChunkSlot) * (size_t)chunks, sizeof(uint64_t) + sizeof(uint32_t) * (size_t)k));
+    g5::DecStream *hs = static_cast<g5::DecStream *>(w.h_desc);
+    uint32_t *ho = reinterpret_cast<uint32_t *>(static_cast<char *>(w.h_desc) + sb);
+    uint32_t t = 0;
+    for (int q = 0; q < k; ++q) {
+        const uint64_t nc = plan(q, hs[q]);
+        hs[q].t0 = t;
+        for (uint64_t e = t + nc; t < e; ++t) ho[t] = (uint32_t)q;
+    }
+    uint64_t *hr = static_cast<uint64_t *>(w.h_res);
+    uint32_t *herr = reinterpret_cast<uint32_t *>(hr + 1);
+    memset(w.h_res, 0, sizeof(uint64_t) + sizeof(uint32_t) * (size_t)k);
+    cudaStream_t s = (cudaStream_t)stream;
+    G5_CUDA(cudaMemcpyAsync(w.desc, w.h_desc, db, cudaMemcpyHostToDevice, s));
+    const g5::DecStream *ds = static_cast<const g5::DecStream *>(w.desc);
+    g5::launch_dyn(true, g5::k_decode_batch, (int)std::min(chunks, blocks), g5::kDB, sizeof(g5::DecShared), s, in_dev, ds,
+                   reinterpret_cast<const uint32_t *>(static_cast<const char *>(w.desc) + sb), (uint32_t)chunks, out_dev,
+                   c->w.scal, static_cast<g5::ChunkSlot *>(w.slots), herr, hr, mode);
+    G5_CUDA(cudaGetLastError());
+    G5_CUDA(cudaStreamSynchronize(s));
+    bool all = hr[0] == 0;
+    for (int q = 0; q < k; ++q) {
+        const bool ok = herr[q] == 0;
         if (stream_ok) stream_ok[q] = ok ? 1 : 0;
         all &= ok;
     }
-    return all ? G5_OK : G5_ERR_CORRUPT_STREAM;
+    return all ? G5_OK : (hr[0] & G5_DEVERR_WAIT) ? G5_ERR_TIMEOUT : G5_ERR_CORRUPT_STREAM;
 }
 
 }  // extern "C"

@@ -116,3 +116,20 @@ def test_one_corrupt_stream_is_flagged(codec):
     with pytest.raises(g5.G5Error) as e:
         codec.decode_batch(dout, out_off[:-1], words, n, back)
     assert e.value.stream_ok.tolist() == [1, 1, 0]
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+def test_large_and_small_queues_at_any_alignment(codec, shift):
+    """Queues of several chunks each way beside tails alone, starting at any
+    word of the input and output (shift moves every queue after the first)."""
+    rng = np.random.default_rng(40 + shift)
+    sizes = [shift, 900_001, 0, 1, 2_000_003, 127, 128 * 16, 128 * 16 * 9 + 1, 64, 400_002] + [3] * 40
+    queues = [np.cumsum(rng.integers(1, 9, n), dtype=np.uint64).astype(np.uint32) for n in sizes]
+    queues.append(rng.integers(0, 1 << 32, 30_000, dtype=np.uint64).astype(np.uint32))  # raw miniblocks
+    for mode, omode in ((g5.CODEC_D4, orc.D4), (g5.CODEC_DM, orc.DM)):
+        streams = batch_round_trip(codec, queues, mode)
+        for q, s in zip(queues, streams):
+            assert np.array_equal(s, orc.encode(q, omode)), len(q)
+        streams = batch_round_trip(codec, queues, mode, thr=30_000)  # raw copies of several chunks
+        for q, s in zip(queues, streams):
+            assert np.array_equal(s, q if len(q) <= 30_000 else orc.encode(q, omode)), len(q)
