@@ -68,6 +68,17 @@ class BfsStats(C.Structure):
 
 
 _lib_handle = None
+_free = None  # the C library's free, for the plugin's buffers
+
+
+def _c_free(p) -> None:
+    global _free
+    if _free is None:
+        _free = C.CDLL(None).free
+        _free.argtypes = [C.c_void_p]
+        _free.restype = None
+    _free(p)
+
 
 # name -> (restype, argtypes); every symbol of include/g5bfs.h
 _P, _I64, _U64, _SZ, _I, _U32 = C.c_void_p, C.c_int64, C.c_uint64, C.c_size_t, C.c_int, C.c_uint32
@@ -509,7 +520,7 @@ class GpuSimd:
                                         self.threshold, self.mode), "g5_plugin_compress")
         arr = np.ctypeslib.as_array(C.cast(out, C.POINTER(C.c_uint32)), shape=(max(cs.value, 1),))
         res = arr[: cs.value].copy()
-        C.CDLL(None).free(out)
+        _c_free(out)
         return res, cs.value
 
     def decompress(self, compressed: np.ndarray, size: int, uncompressedsize: int) -> np.ndarray:
@@ -520,7 +531,7 @@ class GpuSimd:
                                           self.threshold, self.mode), "g5_plugin_decompress")
         arr = np.ctypeslib.as_array(C.cast(out, C.POINTER(C.c_int64)), shape=(max(us.value, 1),))
         res = arr[: us.value].copy()
-        C.CDLL(None).free(out)
+        _c_free(out)
         return res
 
 

@@ -62,3 +62,19 @@ def test_length_past_the_workspace_is_refused():
     c.encode_async(din, n, out, w)
     assert c.status() == 0 and int(w) > 0
     c.close()
+
+
+@pytest.mark.parametrize("n", [10, 5000, 300_000])
+def test_plugin_refuses_ids_past_32_bits(n):
+    """One id below 0 or above 2^32 - 1 anywhere: refused; the queue without it
+    goes through unchanged afterwards."""
+    p = g5.GpuSimd()
+    x = np.arange(n, dtype=np.int64) * 7
+    for bad in (-1, 1 << 32, -(1 << 40)):
+        for at in (0, n // 2, n - 1):
+            y = x.copy()
+            y[at] = bad
+            with pytest.raises(g5.G5Error):
+                p.compress(y)
+    c, size = p.compress(x)
+    assert np.array_equal(p.decompress(c, size, n), x)
