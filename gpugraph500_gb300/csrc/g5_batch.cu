@@ -118,12 +118,7 @@ struct BArgs {
     int serving;            // continuous batching: no level cap, fixed m_u
 };
 
-__device__ __forceinline__ uint64_t wsum(uint64_t v)
-{
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    return v;
-}
+__device__ __forceinline__ uint64_t wsum(uint64_t v) { return warp_sum_u64(v); }
 
 __device__ __forceinline__ int graph_of(const BArgs &a, uint64_t v) { return a.chunk_graph[v / kChunk]; }
 
@@ -239,24 +234,53 @@ __device__ void bexp_td(const BArgs &a, uint64_t &examined)
 // the lanes) are written at once.  The serial hits are written last, lane r
 // taking root r of each vertex: each vertex's parents are one contiguous run
 // of nroots words, so those stores are contiguous.
-__global__ void __launch_bounds__(kB, 4) k_bbu(BArgs a)
+struct BuScratch {  // one warp's serial hits
+    uint64_t evm[kSerial][32];
+    uint32_t evu[kSerial][32];
+};
+
+// A row of which more than kLongRow entries are left after its warp has
+// scanned kLongRow goes to `longs` in pieces of that many (SPLIT; bexp_long
+// scans them afterwards): a hub's row of a million entries held its warp as
+// long as all the others together needed for the level.  The owner's share keeps
+// the early end of rows whose roots are soon found: with none of it, scale 24
+// took 10958 us a batch instead of 8160, and without pieces 9593 (eight mixed
+// graphs 1324, 1252 and 1432).  Pieces of 128, 256, 512, 1024 and 2048 entries:
+// 8598, 8266, 8154, 8152, 8222 (mixed 1325, 1280, 1257, 1235, 1306; scale 16 211,
+// 220, 242, 244, 244).
+constexpr uint32_t kLongRow = 512;
+
+// Entries [start, start + cnt) of global vertex u's row, and the roots it is
+// still to be searched for.
+struct __align__(32) LongItem {
+    int64_t start;  // in the graph's col
+    uint64_t need;
+    uint32_t u;
+    uint32_t cnt;   // | graph << 16
+    uint64_t pad;
+};
+
+struct LongRows {
+    LongItem *items;
+    unsigned long long *alloc;
+};
+
+// vps_shift: log2 of the vertices per warp step (32, less on graphs with fewer
+// steps of 32 than there are warps: scale 8 took 84 us at 32 and takes 76).
+template <bool SPLIT>
+__device__ __forceinline__ void bexp_bu(const BArgs &a, const GraphDesc *gd, BuScratch &ws, uint64_t gw, uint64_t nw,
+                                        int vps_shift, LongRows longs, uint64_t &examined)
 {
-    __shared__ uint64_t s_evm[kW][kSerial][32];
-    __shared__ uint32_t s_evu[kW][kSerial][32];
-    // no graph expands bottom-up this level
-    if (a.st->err || a.st->level < 0 || a.st->active == 0 || !(a.st->dirs & 2u)) return;
-    const int lane = g5_lane(), wib = threadIdx.x >> 5;
-    const uint64_t gw = ((uint64_t)blockIdx.x * kB + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * kB) >> 5;
-    uint64_t examined = 0;
-    for (uint64_t w = gw; w < a.nsteps; w += nw) {
+    const int lane = g5_lane();
+    for (uint64_t w = gw; w < (a.nsteps << (5 - vps_shift)); w += nw) {
         // the graph's vertices with edges in original-id order, 32 per warp
         // step (vertices without edges are never reached, and half the
         // vertices of a Kronecker graph have none): high-degree vertices,
         // which have the lowest new ids, spread over the warps
-        const GraphDesc &d = a.gd[a.step_graph[w]];
+        const int gi = a.step_graph[w >> (5 - vps_shift)];
+        const GraphDesc &d = gd[gi];
         if (d.dir != BU || d.nf == 0) continue;
-        const uint64_t li = (w - d.step0) * 32 + lane;
+        const uint64_t li = lane < 1 << vps_shift ? ((w - (d.step0 << (5 - vps_shift))) << vps_shift) + lane : d.nblist;
         const uint64_t ol = li < d.nblist ? __ldg(d.blist + li) : 0u;
         const uint32_t R = (uint32_t)d.nroots;
         // new id and row bounds, indexed by original id: three loads issued
@@ -284,10 +308,10 @@ __global__ void __launch_bounds__(kB, 4) k_bbu(BArgs a)
 #pragma unroll
         for (int k = 0; k < kSerial; ++k) {
             const uint64_t hit = f[k] & need;
-            s_evm[wib][k][lane] = hit;
+            ws.evm[k][lane] = hit;
             // the parent's original id lands in shared memory while the
             // rest of the row is scanned (read at the write-out below)
-            if (hit) cp_async4(&s_evu[wib][k][lane], d.orig + u[k]);
+            if (hit) cp_async4(&ws.evu[k][lane], d.orig + u[k]);
             need &= ~hit;
             sfound |= hit;
             if (u[k] != 0xFFFFFFFFu && (need | hit)) j = s + k + 1;
@@ -392,13 +416,16 @@ __global__ void __launch_bounds__(kB, 4) k_bbu(BArgs a)
             uint32_t *pv = a.pred + d.pred_base + (uint64_t)__shfl_sync(0xFFFFFFFFu, vo, l) * R;
             const int64_t st = jj;
             uint64_t fnd = 0;
-            while (jj < ee && nd) {
+            // what is left of a long row after its first entries goes to
+            // `longs`, with the roots it is still to be searched for
+            const int64_t own = SPLIT && ee - jj > 2 * kLongRow ? jj + kLongRow : ee;
+            while (jj < own && nd) {
                 uint32_t uw[4];
                 uint64_t hw[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const int64_t i = jj + 32 * q + lane;
-                    uw[q] = i < ee ? __ldg(d.col + i) : 0xFFFFFFFFu;
+                    uw[q] = i < own ? __ldg(d.col + i) : 0xFFFFFFFFu;
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q) hw[q] = uw[q] != 0xFFFFFFFFu ? a.front[d.vbase + uw[q]] : 0ull;
@@ -444,7 +471,22 @@ __global__ void __launch_bounds__(kB, 4) k_bbu(BArgs a)
                     jj += nd ? 32 : __ffs(cov);
                 }
             }
-            jj = min(jj, ee);
+            jj = min(jj, own);
+            if (SPLIT && nd && own < ee) {
+                const uint32_t pieces = (uint32_t)((ee - own + kLongRow - 1) / kLongRow);
+                unsigned long long base = 0;
+                if (lane == 0) base = atomicAdd(longs.alloc, (unsigned long long)pieces);
+                base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                const uint32_t vv = __shfl_sync(0xFFFFFFFFu, (uint32_t)v, l);
+                for (uint32_t k = lane; k < pieces; k += 32) {
+                    LongItem it;
+                    it.start = own + (int64_t)k * kLongRow;
+                    it.u = vv;
+                    it.cnt = (uint32_t)min(ee - it.start, (int64_t)kLongRow) | (uint32_t)gi << 16;
+                    it.need = nd;
+                    longs.items[base + k] = it;
+                }
+            }
             if (lane == l) {
                 found |= fnd;
                 need = nd;
@@ -459,12 +501,12 @@ __global__ void __launch_bounds__(kB, 4) k_bbu(BArgs a)
         // once.
 #pragma unroll
         for (int k = 0; k < kSerial; ++k) {
-            unsigned em = __ballot_sync(0xFFFFFFFFu, s_evm[wib][k][lane] != 0ull);
+            unsigned em = __ballot_sync(0xFFFFFFFFu, ws.evm[k][lane] != 0ull);
             while (em) {
                 const int vi = __ffs(em) - 1;
                 em &= em - 1;
-                const uint64_t m = s_evm[wib][k][vi];
-                const uint32_t u = s_evu[wib][k][vi];
+                const uint64_t m = ws.evm[k][vi];
+                const uint32_t u = ws.evu[k][vi];
                 uint32_t *pv = a.pred + d.pred_base + (uint64_t)__shfl_sync(0xFFFFFFFFu, vo, vi) * R;
                 if ((m >> lane) & 1ull) pv[lane] = u;
                 if ((m >> (lane + 32)) & 1ull) pv[lane + 32] = u;
@@ -474,8 +516,78 @@ __global__ void __launch_bounds__(kB, 4) k_bbu(BArgs a)
         if (found) a.next[v] |= found;  // only this lane writes v in a bottom-up level
         examined += ex;
     }
+}
+
+// The pieces of long rows, a warp each: as the long rows of bexp_bu, but each
+// root's first hit in the piece takes its parent slot by atomicMin (rows are in
+// original-id order, so the first hit of the whole row is the smallest id).
+__device__ __forceinline__ void bexp_long(const BArgs &a, const GraphDesc *gd, const LongItem *items, uint64_t nitems,
+                                          uint64_t gw, uint64_t nw)
+{
+    const int lane = g5_lane();
+    for (uint64_t t = gw; t < nitems; t += nw) {
+        const ulonglong2 x0 = __ldcg(reinterpret_cast<const ulonglong2 *>(items + t));
+        const ulonglong2 x1 = __ldcg(reinterpret_cast<const ulonglong2 *>(items + t) + 1);
+        const uint64_t v = (uint32_t)x1.x;
+        const uint32_t cnt = (uint32_t)(x1.x >> 32);
+        const GraphDesc &d = gd[cnt >> 16];
+        int64_t jj = (int64_t)x0.x;
+        const int64_t ee = jj + (cnt & 0xFFFFu);
+        uint64_t nd = x0.y;
+        uint32_t *pv = a.pred + d.pred_base + (uint64_t)__ldg(d.orig + (v - d.vbase)) * (uint32_t)d.nroots;
+        uint64_t fnd = 0;
+        while (jj < ee && nd) {
+            uint32_t uw[4];
+            uint64_t hw[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int64_t i = jj + 32 * q + lane;
+                uw[q] = i < ee ? __ldg(d.col + i) : 0xFFFFFFFFu;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) hw[q] = uw[q] != 0xFFFFFFFFu ? a.front[d.vbase + uw[q]] & nd : 0ull;
+            const uint64_t any = hw[0] | hw[1] | hw[2] | hw[3];
+            const uint32_t lo = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)any), hi = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)(any >> 32));
+            jj += 128;
+            uint64_t left = (uint64_t)hi << 32 | lo;
+            if (!left) continue;
+            fnd |= left;
+            nd &= ~left;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint64_t hit = hw[q] & left;
+                if (!__any_sync(0xFFFFFFFFu, hit != 0)) continue;
+                const uint32_t uo = hit ? __ldg(d.orig + uw[q]) : 0u;
+                uint64_t incl = hit;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint64_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                    if (lane >= o) incl |= y;
+                }
+                uint64_t excl = __shfl_up_sync(0xFFFFFFFFu, incl, 1);
+                if (lane == 0) excl = 0;
+                for (uint64_t x = hit & ~excl; x; x &= x - 1) {
+                    uint32_t *slot = pv + (__ffsll((long long)x) - 1);
+                    if (*slot > uo) atomicMin(slot, uo);
+                }
+                left &= ~__shfl_sync(0xFFFFFFFFu, incl, 31);
+            }
+        }
+        if (lane == 0 && (fnd & ~a.next[v])) atomicOr((unsigned long long *)&a.next[v], (unsigned long long)fnd);
+    }
+}
+
+__global__ void __launch_bounds__(kB, 4) k_bbu(BArgs a)
+{
+    __shared__ BuScratch s_ws[kW];
+    // no graph expands bottom-up this level
+    if (a.st->err || a.st->level < 0 || a.st->active == 0 || !(a.st->dirs & 2u)) return;
+    const uint64_t gw = ((uint64_t)blockIdx.x * kB + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * kB) >> 5;
+    uint64_t examined = 0;
+    bexp_bu<false>(a, a.gd, s_ws[threadIdx.x >> 5], gw, nw, 5, LongRows(), examined);
     examined = wsum(examined);
-    if (lane == 0 && examined) atomicAdd((unsigned long long *)&a.st->examined, (unsigned long long)examined);
+    if (g5_lane() == 0 && examined) atomicAdd((unsigned long long *)&a.st->examined, (unsigned long long)examined);
 }
 
 // Top-down part of a level (graphs expanding top-down).
@@ -748,6 +860,465 @@ __global__ void __launch_bounds__(kB, 4) k_bwrite(BArgs a)
     }
 }
 
+// ---- the whole batch as one launch -----------------------------------------------------
+//
+// g5_batch_run's form (the asynchronous and serving forms keep the level graph
+// below, whose kernels other work on the GPU runs between): one cooperative
+// grid of a block per SM, whose blocks meet twice a level.
+//   expand  top-down graphs by work items of up to kItemEntries entries,
+//           bottom-up ones as in k_bbu
+//   commit  visited |= next, next -> front, the next frontier's sums per graph
+//   decide  every block computes each graph's direction from the sums
+// A top-down level of at most kClaimMax entries appends the rows it reaches
+// first to the items of the next level; otherwise, and for graphs that come back
+// from bottom-up, the items are built from the frontier words.
+//
+// Five launches and a while node a level cost about 35 us whatever the level
+// held; a level now costs its work and 6-8 us.  Device us per batch of Kronecker
+// graphs, 16 edges a vertex, before and after: scale 8, 4 roots, 230 and 76;
+// scale 13, 64 roots, 410 and 135; scale 16 479 and 242; scale 20 1281 and 758;
+// scale 24 10267 and 8160; eight graphs of scales 14 to 20, 16 roots each, 1820
+// and 1252.
+constexpr int kSB = 1024;
+constexpr int kSW = kSB / 32;
+constexpr uint32_t kItemEntries = 256;
+constexpr uint64_t kClaimMax = 1u << 18;
+constexpr uint64_t kClaimedItems = 1u << 19;
+constexpr int kRing = 4;  // levels of sums held
+
+// A work item: entries [start, start + cnt) of the row of global vertex u.
+struct __align__(16) BItem {
+    uint32_t u;
+    uint32_t cnt;    // | graph << 16
+    int64_t start;   // in the graph's col
+};
+
+struct GraphSum {
+    unsigned long long nf, mf, amask, pad;
+};
+
+struct LevelMeet {
+    unsigned long long arrive[5];  // meetings of a level
+    unsigned long long alloc;      // claimed items of its frontier
+    unsigned long long built;      // items built for it
+    unsigned long long longs;      // pieces of long rows
+};
+
+struct PArgs {
+    BArgs b;
+    const GraphDesc *gd;    // the host's descriptors of this run
+    uint64_t npred;         // parents in pred_out
+    BItem *claimed[2];      // by level parity
+    uint64_t claimed_cap;
+    BItem *built;
+    LongItem *longs;        // pieces of long rows (bottom-up)
+    int vps_shift;          // log2 of the vertices per bottom-up warp step
+    GraphSum *sums;         // kRing x ngraphs
+    LevelMeet *meets;       // kRing; kRing levels are cleared at the start of a run
+    unsigned *abort;
+    uint32_t unit;          // vertices per warp step of the passes over the words (32, 64, ... 256)
+    uint8_t *live;          // per unit: its frontier is not empty
+    BState *out;            // pinned host
+};
+
+struct TdScratch {
+    uint32_t end[32];
+    uint32_t u[32];
+    int64_t base[32];
+    uint64_t front[32];
+    uint8_t g[32];
+};
+
+union BWarpScratch {
+    BuScratch bu;
+    TdScratch td;
+};
+
+struct PShared {
+    GraphDesc gd[kMaxGraphs];
+    unsigned long long nf[kMaxGraphs], mf[kMaxGraphs], am[kMaxGraphs];  // the block's share of the next frontier
+    BWarpScratch w[kSW];
+    unsigned long long active, td_entries;
+    uint32_t dirs;   // bit 0: a graph expands top-down, bit 1: bottom-up
+    uint32_t build;  // some graph's items are to be built
+    uint8_t build_g[kMaxGraphs];
+    uint32_t stop;
+};
+
+__device__ __forceinline__ void pmeet(const PArgs &a, PShared &sh, unsigned long long *word)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(word, 1ull << kArrive);
+        unsigned long long x;
+        if (!await<1>(word, a.abort, &x)) sh.stop = 1;
+        __threadfence();
+    }
+    __syncthreads();
+}
+
+// Appends the rows of the warp's vertices (lanes with nseg > 0) to the items;
+// long rows are laid out by the whole warp.
+__device__ __forceinline__ void put_rows(BItem *items, uint64_t cap, uint64_t base, uint32_t excl, uint32_t ug, int g,
+                                         int64_t s, uint32_t d, uint32_t nseg)
+{
+    if (base + excl + nseg > cap) nseg = 0;  // no room: the caller sees it from the total
+    BItem *p = items + base + excl;
+    if (nseg <= 8)
+        for (uint32_t k = 0; k < nseg; ++k) {
+            BItem it;
+            it.u = ug;
+            it.cnt = min(d - k * kItemEntries, kItemEntries) | (uint32_t)g << 16;
+            it.start = s + (int64_t)k * kItemEntries;
+            p[k] = it;
+        }
+    unsigned big = __ballot_sync(0xFFFFFFFFu, nseg > 8);
+    while (big) {
+        const int l = __ffs(big) - 1;
+        big &= big - 1;
+        const uint32_t uu = __shfl_sync(0xFFFFFFFFu, ug, l), c = __shfl_sync(0xFFFFFFFFu, nseg, l);
+        const uint32_t x = __shfl_sync(0xFFFFFFFFu, excl, l), dd = __shfl_sync(0xFFFFFFFFu, d, l);
+        const int64_t ss = __shfl_sync(0xFFFFFFFFu, s, l);
+        const int gg = __shfl_sync(0xFFFFFFFFu, g, l);
+        for (uint32_t k = g5_lane(); k < c; k += 32) {
+            BItem it;
+            it.u = uu;
+            it.cnt = min(dd - k * kItemEntries, kItemEntries) | (uint32_t)gg << 16;
+            it.start = ss + (int64_t)k * kItemEntries;
+            items[base + x + k] = it;
+        }
+    }
+}
+
+// Top-down over a list of items (those of graphs that have turned bottom-up are
+// passed over): 32 items per warp step, one, or a part of one, as many as it
+// takes to give every warp some.
+template <bool CLAIM>
+__device__ __forceinline__ void bexp_items(const PArgs &a, PShared &sh, const BItem *items, uint64_t nitems, BItem *out,
+                                           unsigned long long *alloc)
+{
+    const int lane = g5_lane();
+    TdScratch &ws = sh.w[threadIdx.x >> 5].td;
+    const uint64_t gw = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, nw = (uint64_t)gridDim.x * kSW;
+    uint32_t ipw_shift = 0, split_shift = 0;
+    while (ipw_shift < 5 && nitems > (nw << ipw_shift)) ++ipw_shift;
+    while (split_shift < 3 && (nitems << (split_shift + 1)) <= nw) ++split_shift;
+    const uint64_t units = ((nitems << split_shift) + (1u << ipw_shift) - 1) >> ipw_shift;
+    for (uint64_t t = gw; t < units; t += nw) {
+        const uint64_t i = ((t << ipw_shift) >> split_shift) + lane;
+        uint32_t cnt = 0, u = 0;
+        int g = 0;
+        int64_t s = 0;
+        uint64_t f = 0;
+        if ((uint32_t)lane < (1u << ipw_shift) && i < nitems) {
+            const uint4 raw = __ldcg(reinterpret_cast<const uint4 *>(items + i));
+            u = raw.x;
+            g = (int)(raw.y >> 16);
+            cnt = raw.y & 0xFFFFu;
+            s = (int64_t)(raw.z | (uint64_t)raw.w << 32);
+            const uint32_t part = kItemEntries >> split_shift;
+            const uint32_t at = (uint32_t)(t & ((1u << split_shift) - 1)) * part;
+            s += at;
+            cnt = cnt > at ? min(cnt - at, part) : 0u;
+            if (sh.gd[g].dir != TD) cnt = 0;
+            else if (cnt) f = a.b.front[u];
+        }
+        uint32_t total;
+        const uint32_t excl = warp_excl_u32(cnt, total);
+        __syncwarp();
+        ws.end[lane] = excl + cnt;
+        // the parent's original id, which is what the parents hold
+        ws.u[lane] = cnt ? __ldg(sh.gd[g].orig + (u - sh.gd[g].vbase)) : 0u;
+        ws.base[lane] = s - (int64_t)excl;
+        ws.front[lane] = f;
+        ws.g[lane] = (uint8_t)g;
+        __syncwarp();
+        for (uint32_t e0 = 0; e0 < total; e0 += 32) {
+            const uint32_t x = e0 + lane;
+            bool claimed = false;
+            uint32_t vl = 0, dv = 0;
+            int64_t vs = 0;
+            int gv = 0;
+            if (x < total) {
+                int lo = 0;
+                if (ipw_shift) {
+                    int hi = 31;
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if (ws.end[mid] <= x) lo = mid + 1;
+                        else hi = mid;
+                    }
+                }
+                gv = ws.g[lo];
+                const GraphDesc &d = sh.gd[gv];
+                vl = __ldg(d.col + (ws.base[lo] + (int64_t)x));
+                const uint64_t vg = d.vbase + vl;
+                const uint64_t seen = a.b.vis[vg];
+                const uint32_t vo = __ldg(d.orig + vl);
+                if (CLAIM) {
+                    vs = __ldg(d.row_off + vl);
+                    dv = __ldg(a.b.deg + vg);
+                }
+                const uint64_t nb = ws.front[lo] & ~seen;
+                if (nb) {
+                    const uint32_t ul = ws.u[lo];
+                    uint32_t *pv = a.b.pred + d.pred_base + (uint64_t)vo * d.nroots;
+                    for (uint64_t y = nb; y; y &= y - 1) {
+                        uint32_t *slot = pv + (__ffsll((long long)y) - 1);
+                        if (CLAIM || *slot > ul) atomicMin(slot, ul);
+                    }
+                    if (CLAIM) claimed = atomicOr((unsigned long long *)&a.b.next[vg], (unsigned long long)nb) == 0;
+                    else if (nb & ~a.b.next[vg]) atomicOr((unsigned long long *)&a.b.next[vg], (unsigned long long)nb);
+                }
+            }
+            if (CLAIM && __any_sync(0xFFFFFFFFu, claimed)) {
+                const uint32_t nseg = claimed ? (dv + kItemEntries - 1) / kItemEntries : 0u;
+                uint32_t tot;
+                const uint32_t at = warp_excl_u32(nseg, tot);
+                unsigned long long base = 0;
+                if (lane == 0) base = atomicAdd(alloc, (unsigned long long)tot);
+                base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                put_rows(out, a.claimed_cap, base, at, (uint32_t)(sh.gd[gv].vbase + vl), gv, vs, dv, nseg);
+            }
+        }
+    }
+}
+
+// visited |= next, next -> front, and the sums of the next frontier per graph.
+// A unit idle this level and the last is passed over.
+__device__ __forceinline__ void bcommit(const PArgs &a, PShared &sh, GraphSum *sums)
+{
+    constexpr int kK = 8;
+    const int lane = g5_lane();
+    const uint32_t rounds = a.unit / 32;
+    const uint64_t units = a.b.ntot / a.unit, nw = (uint64_t)gridDim.x * kSW;
+    int cur = -1;
+    uint32_t nf = 0;
+    uint64_t mf = 0, am = 0;
+    auto flush = [&]() {
+        if (cur >= 0 && __any_sync(0xFFFFFFFFu, nf != 0)) {
+            nf = __reduce_add_sync(0xFFFFFFFFu, nf);
+            mf = warp_add_u51(mf);
+            const uint32_t lo = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)am), hi = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)(am >> 32));
+            if (lane == 0) {
+                atomicAdd(&sh.nf[cur], (unsigned long long)nf);
+                atomicAdd(&sh.mf[cur], (unsigned long long)mf);
+                atomicOr(&sh.am[cur], (unsigned long long)hi << 32 | lo);
+            }
+        }
+        nf = 0;
+        mf = am = 0;
+    };
+    for (uint64_t t = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; t < units; t += nw) {
+        const uint64_t v0 = t * a.unit;
+        const int g = a.b.chunk_graph[v0 / kChunk];
+        if (g != cur) {
+            flush();
+            cur = g;
+        }
+        const bool was = a.live[t] != 0;
+        uint64_t nx[kK], all = 0;
+#pragma unroll
+        for (int k = 0; k < kK; ++k) {
+            nx[k] = k < (int)rounds ? a.b.next[v0 + 32 * k + lane] : 0ull;
+            all |= nx[k];
+        }
+        const bool now = __any_sync(0xFFFFFFFFu, all != 0);
+        if (!now && !was) continue;
+        if (lane == 0 && now != was) a.live[t] = now;
+        uint64_t vs[kK];
+        uint32_t dg[kK];
+#pragma unroll
+        for (int k = 0; k < kK; ++k) {
+            vs[k] = nx[k] ? a.b.vis[v0 + 32 * k + lane] : 0ull;
+            dg[k] = nx[k] ? __ldg(a.b.deg + v0 + 32 * k + lane) : 0u;
+        }
+        am |= all;
+#pragma unroll
+        for (int k = 0; k < kK; ++k) {
+            if (k < (int)rounds) a.b.front[v0 + 32 * k + lane] = nx[k];
+            if (nx[k]) {
+                a.b.vis[v0 + 32 * k + lane] = vs[k] | nx[k];
+                a.b.next[v0 + 32 * k + lane] = 0;
+                ++nf;
+                mf += dg[k];
+            }
+        }
+    }
+    flush();
+    __syncthreads();
+    for (int g = threadIdx.x; g < a.b.ngraphs; g += kSB) {
+        if (sh.nf[g]) {
+            atomicAdd(&sums[g].nf, sh.nf[g]);
+            atomicAdd(&sums[g].mf, sh.mf[g]);
+            atomicOr(&sums[g].amask, sh.am[g]);
+        }
+        sh.nf[g] = sh.mf[g] = sh.am[g] = 0;
+    }
+    // (pmeet's barrier and fence follow)
+}
+
+// The items of the frontiers of the graphs marked in build_g.
+__device__ __forceinline__ void bbuild(const PArgs &a, PShared &sh, unsigned long long *alloc)
+{
+    const int lane = g5_lane();
+    const uint64_t units = a.b.ntot / a.unit, nw = (uint64_t)gridDim.x * kSW;
+    for (uint64_t t = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; t < units; t += nw) {
+        if (!a.live[t]) continue;
+        const uint64_t v0 = t * a.unit;
+        const int g = a.b.chunk_graph[v0 / kChunk];
+        if (!sh.build_g[g]) continue;
+        for (uint32_t k = 0; k < a.unit; k += 32) {
+            const uint64_t vg = v0 + k + lane;
+            const bool on = a.b.front[vg] != 0;
+            if (!__any_sync(0xFFFFFFFFu, on)) continue;
+            const uint32_t d = on ? __ldg(a.b.deg + vg) : 0u, nseg = (d + kItemEntries - 1) / kItemEntries;
+            const int64_t s = on ? __ldg(sh.gd[g].row_off + (vg - sh.gd[g].vbase)) : 0;
+            uint32_t tot;
+            const uint32_t at = warp_excl_u32(nseg, tot);
+            unsigned long long base = 0;
+            if (lane == 0) base = atomicAdd(alloc, (unsigned long long)tot);
+            base = __shfl_sync(0xFFFFFFFFu, base, 0);
+            put_rows(a.built, ~0ull, base, at, (uint32_t)vg, g, s, d, nseg);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kSB, 1) k_bsearch(const __grid_constant__ PArgs a)
+{
+    extern __shared__ __align__(16) unsigned char s_batch[];
+    PShared &sh = *reinterpret_cast<PShared *>(s_batch);
+    const uint64_t tid = (uint64_t)blockIdx.x * kSB + threadIdx.x, nthr = (uint64_t)gridDim.x * kSB;
+    const int ng = a.b.ngraphs;
+    // prologue: empty words, no parents, the graphs' descriptors
+    for (uint64_t i = tid; i < 3 * a.b.ntot / 2; i += nthr)
+        reinterpret_cast<ulonglong2 *>(a.b.vis)[i] = make_ulonglong2(0, 0);
+    for (uint64_t i = tid; i < a.b.ntot / a.unit; i += nthr) a.live[i] = 0;
+    const uint64_t head = min(a.npred, (uint64_t)((16 - ((uintptr_t)a.b.pred & 15)) & 15) / 4);
+    const uint64_t vecs = (a.npred - head) / 4;
+    for (uint64_t i = tid; i < vecs; i += nthr)
+        reinterpret_cast<uint4 *>(a.b.pred + head)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    if (tid < head) a.b.pred[tid] = ~0u;
+    if (tid < a.npred - head - 4 * vecs) a.b.pred[head + 4 * vecs + tid] = ~0u;
+    for (uint32_t i = threadIdx.x; i < ng * sizeof(GraphDesc) / 8; i += kSB)
+        reinterpret_cast<uint64_t *>(sh.gd)[i] = __ldcg(reinterpret_cast<const unsigned long long *>(a.gd) + i);
+    for (int g = threadIdx.x; g < ng; g += kSB) sh.nf[g] = sh.mf[g] = sh.am[g] = 0;
+    if (threadIdx.x == 0) sh.stop = 0;
+    pmeet(a, sh, &a.meets[0].arrive[0]);
+    // the roots: into next, their own parents
+    for (int g = blockIdx.x; g < ng; g += gridDim.x) {
+        const GraphDesc &d = sh.gd[g];
+        for (int r = threadIdx.x; r < d.nroots; r += kSB) {
+            const int64_t root = a.b.roots[a.b.root_off[g] + r];
+            atomicOr((unsigned long long *)&a.b.next[d.vbase + d.perm[root]], 1ull << r);
+            a.b.pred[d.pred_base + (uint64_t)root * d.nroots + r] = (uint32_t)root;
+        }
+    }
+    for (int g = threadIdx.x; g < ng; g += kSB) {
+        sh.gd[g].dir = TD;
+        sh.gd[g].mu = (uint64_t)sh.gd[g].nnz;
+    }
+    pmeet(a, sh, &a.meets[0].arrive[1]);
+    uint32_t err = 0;
+    bool claim = false;  // the level before claimed: its items are those of the top-down graphs
+    int32_t L = -1;
+    for (;; ++L) {
+        // level L: expand its frontier (none before level 0), then commit
+        LevelMeet *cur = a.meets + (L + kRing) % kRing, *nxt = a.meets + (L + 1) % kRing;
+        GraphSum *sums = a.sums + (uint64_t)((L + 1) % kRing) * ng;
+        if (L >= 0) {
+            // (the records of the level after next)
+            if (tid < sizeof(LevelMeet) / 8)
+                reinterpret_cast<unsigned long long *>(a.meets + (L + 2) % kRing)[tid] = 0;
+            for (uint64_t i = tid; i < (uint64_t)ng * sizeof(GraphSum) / 8; i += nthr)
+                reinterpret_cast<unsigned long long *>(a.sums + (uint64_t)((L + 2) % kRing) * ng)[i] = 0;
+            const uint64_t nclaimed = claim ? __ldcg(&cur->alloc) : 0;
+            if (sh.build) {
+                bbuild(a, sh, &cur->built);
+                pmeet(a, sh, &cur->arrive[2]);
+                if (sh.stop) break;
+            }
+            const uint64_t nbuilt = sh.build ? __ldcg(&cur->built) : 0;
+            const bool now = sh.td_entries <= kClaimMax;
+            if (sh.dirs & 1u) {
+                BItem *out = a.claimed[(L + 1) & 1];
+                if (now) {
+                    bexp_items<true>(a, sh, a.claimed[L & 1], nclaimed, out, &nxt->alloc);
+                    bexp_items<true>(a, sh, a.built, nbuilt, out, &nxt->alloc);
+                } else {
+                    bexp_items<false>(a, sh, a.claimed[L & 1], nclaimed, nullptr, nullptr);
+                    bexp_items<false>(a, sh, a.built, nbuilt, nullptr, nullptr);
+                }
+            }
+            if (sh.dirs & 2u) {
+                uint64_t ex = 0;
+                const uint64_t gw = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, nw = (uint64_t)gridDim.x * kSW;
+                __syncwarp();
+                bexp_bu<true>(a.b, sh.gd, sh.w[threadIdx.x >> 5].bu, gw, nw, a.vps_shift, LongRows{a.longs, &cur->longs}, ex);
+                pmeet(a, sh, &cur->arrive[4]);
+                if (sh.stop) break;
+                bexp_long(a.b, sh.gd, a.longs, __ldcg(&cur->longs), gw, nw);
+            }
+            claim = now;
+            pmeet(a, sh, &nxt->arrive[0]);
+            if (sh.stop) break;
+        }
+        bcommit(a, sh, sums);
+        pmeet(a, sh, L < 0 ? &a.meets[0].arrive[3] : &nxt->arrive[1]);
+        if (sh.stop) break;
+        // decide, alike in every block: Beamer's switch on the union frontier of
+        // the graph's roots
+        if (threadIdx.x == 0) {
+            sh.active = sh.td_entries = 0;
+            sh.dirs = sh.build = 0;
+        }
+        __syncthreads();
+        const bool fits = claim && L >= 0 && __ldcg(&nxt->alloc) <= a.claimed_cap;
+        for (int g = threadIdx.x; g < ng; g += kSB) {
+            GraphDesc &d = sh.gd[g];
+            const uint64_t tn = __ldcg(&sums[g].nf), tm = __ldcg(&sums[g].mf);
+            const uint64_t mu = d.mu >= tm ? d.mu - tm : 0;
+            const int was = d.dir;
+            int nd = was;
+            if (L >= 0) {
+                if (was == TD) {
+                    // a frontier large enough, too, to pay for a sweep over all
+                    // of the graph's vertices
+                    if (above_quotient(tm, mu, a.b.alpha) && tm > (uint64_t)d.n / kBuMinFrac) nd = BU;
+                } else if (tn < d.nf && below_quotient(tn, (uint64_t)d.n, a.b.beta)) {
+                    nd = TD;
+                }
+            }
+            d.mu = mu;
+            d.dir = nd;
+            d.nf = tn;
+            d.mf = tm;
+            d.amask = __ldcg(&sums[g].amask) & d.mask;
+            const bool build = nd == TD && tn && !(fits && was == TD);
+            sh.build_g[g] = build;
+            if (tn) {
+                atomicAdd(&sh.active, (unsigned long long)tn);
+                atomicOr(&sh.dirs, nd == TD ? 1u : 2u);
+                if (nd == TD) atomicAdd(&sh.td_entries, (unsigned long long)tm);
+                if (build) atomicOr(&sh.build, 1u);
+            }
+        }
+        __syncthreads();
+        claim = fits;
+        if (sh.active == 0) break;
+        if (L + 2 >= kMaxLevels) {
+            err = 8u;
+            break;
+        }
+    }
+    if (tid == 0) {
+        a.out->level = L + 1;
+        a.out->err = err | (sh.stop ? 16u : 0u);
+        a.out->active = sh.active;
+    }
+}
+
 // Continuous batching: roots admitted into free slots (bit r of their
 // graph) join the next level as its frontier; retired roots' visited bits are
 // cleared so the slot can be reused.
@@ -893,6 +1464,15 @@ struct g5_batch {
     cudaGraph_t graph = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<void *> owned;        // degree-ordered graph copies
+    // the one-launch form (g5_batch_run; made on its first call)
+    void *scratch = nullptr;          // queue arrays of the level graph, or built items
+    int pgrid = 0;                    // its blocks (0: not made yet, -1: the device cannot hold it)
+    PArgs pargs;
+    BItem *claimed = nullptr;
+    uint8_t *live = nullptr;
+    LongItem *longs = nullptr;
+    char *stage = nullptr, *h_stage = nullptr;  // descriptors, roots and cleared records of a run
+    size_t stage_bytes = 0, roots_at = 0, off_at = 0, zero_at = 0;
 };
 
 namespace {
@@ -973,10 +1553,12 @@ void free_batch(g5_batch *b)
     cudaFree(b->deg);
     cudaFree(b->iso);
     cudaFree(b->words);
-    cudaFree(b->queue);
-    cudaFree(b->qoff);
-    cudaFree(b->qbase);
-    cudaFree(b->tile_start);
+    cudaFree(b->scratch);
+    cudaFree(b->claimed);
+    cudaFree(b->live);
+    cudaFree(b->longs);
+    cudaFree(b->stage);
+    cudaFreeHost(b->h_stage);
     cudaFree(b->chunks);
     cudaFree(b->step_graph);
     cudaFree(b->st);
@@ -1064,11 +1646,62 @@ g5_status build_relabel(g5_batch *b, const g5_graph *g, GraphDesc &d)
 
 }  // namespace
 
-extern "C" {
-
-}  // extern "C"
-
 namespace {
+
+// Sets up the one-launch form: its buffers, grid and arguments; pgrid = -1 if
+// the device cannot hold a block per SM of it.
+g5_status plan_one_launch(g5_batch *b)
+{
+    const int ng = (int)b->graphs.size();
+    const uint64_t vb = b->args.ntot;
+    uint64_t nnz = 0;
+    for (const g5_graph *g : b->graphs) nnz += (uint64_t)g->nnz;
+    int per_sm = 0;
+    if (cudaFuncSetAttribute(k_bsearch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PShared)) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bsearch, kSB, sizeof(PShared)) != cudaSuccess ||
+        per_sm < 1) {
+        cudaGetLastError();
+        b->pgrid = -1;
+        return G5_OK;
+    }
+    PArgs &a = b->pargs;
+    memset(&a, 0, sizeof a);
+    a.claimed_cap = std::min<uint64_t>(std::min<uint64_t>(vb, kClaimMax) + nnz / kItemEntries + 1, kClaimedItems);
+    auto align16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
+    b->roots_at = align16(sizeof(GraphDesc) * ng);
+    b->off_at = align16(b->roots_at + sizeof(int64_t) * 64 * ng);
+    b->zero_at = align16(b->off_at + sizeof(int32_t) * (ng + 1));
+    const size_t sums_at = b->zero_at + sizeof(LevelMeet) * kRing, abort_at = sums_at + sizeof(GraphSum) * kRing * ng;
+    b->stage_bytes = abort_at + 16;
+    // (a failed call can leave some made: the next one goes on from there)
+    if (!b->claimed) G5_CUDA(cudaMalloc(&b->claimed, sizeof(BItem) * 2 * a.claimed_cap));
+    if (!b->live) G5_CUDA(cudaMalloc(&b->live, vb / 32));
+    // (a row has a piece per kLongRow entries and one for the rest, and more
+    // than kLongRow entries to have any)
+    if (!b->longs) G5_CUDA(cudaMalloc(&b->longs, sizeof(LongItem) * (2 * (nnz / kLongRow) + 1)));
+    if (!b->stage) G5_CUDA(cudaMalloc(&b->stage, b->stage_bytes));
+    if (!b->h_stage) G5_CUDA(cudaMallocHost(&b->h_stage, b->stage_bytes));
+    memset(b->h_stage, 0, b->stage_bytes);
+    a.gd = reinterpret_cast<const GraphDesc *>(b->stage);
+    a.claimed[0] = b->claimed;
+    a.claimed[1] = b->claimed + a.claimed_cap;
+    a.built = static_cast<BItem *>(b->scratch);
+    a.meets = reinterpret_cast<LevelMeet *>(b->stage + b->zero_at);
+    a.sums = reinterpret_cast<GraphSum *>(b->stage + sums_at);
+    a.abort = reinterpret_cast<unsigned *>(b->stage + abort_at);
+    a.live = b->live;
+    a.longs = b->longs;
+    a.out = b->h_st;
+    // a block per SM, fewer where their warps would have no words or entries
+    const uint64_t warps = std::max<uint64_t>(vb / 32, nnz / 64);
+    b->pgrid = (int)std::min<uint64_t>((uint64_t)std::min(g5::num_sms(), kMaxBlocks), (warps + kSW - 1) / kSW);
+    a.unit = 256;
+    while (a.unit > 32 && vb / a.unit < (uint64_t)b->pgrid * kSW) a.unit /= 2;
+    a.vps_shift = 5;
+    while (a.vps_shift > 2 && (b->args.nsteps << (5 - a.vps_shift)) < (uint64_t)b->pgrid * kSW) --a.vps_shift;
+    return G5_OK;
+}
+
 
 // A batch workspace over `graphs`; with `share` (a workspace over the same
 // graphs), its degree-ordered graph copies are borrowed instead of built, so
@@ -1148,10 +1781,15 @@ g5_status batch_create_impl(g5_graph *const *graphs, int ngraphs, const g5_batch
     B_ALLOC(b->deg, sizeof(uint32_t) * vb);
     B_ALLOC(b->iso, sizeof(uint32_t) * (vb / 32));
     B_ALLOC(b->words, sizeof(uint64_t) * 3 * vb);
-    B_ALLOC(b->queue, sizeof(uint32_t) * vb);
-    B_ALLOC(b->qoff, sizeof(uint64_t) * (vb + 1));
-    B_ALLOC(b->qbase, sizeof(int64_t) * vb);
-    B_ALLOC(b->tile_start, sizeof(uint32_t) * a.max_tiles);
+    // the queue arrays of the level graph; the one-launch form holds its built
+    // items in the same memory
+    const size_t queue_bytes = sizeof(uint64_t) * (2 * vb + 2) + sizeof(uint32_t) * (vb + a.max_tiles);
+    const size_t item_bytes = sizeof(BItem) * (vb + nnz_max / kItemEntries + 1);
+    B_ALLOC(b->scratch, std::max(queue_bytes, item_bytes));
+    b->qoff = static_cast<uint64_t *>(b->scratch);
+    b->qbase = reinterpret_cast<int64_t *>(b->qoff + vb + 2);
+    b->queue = reinterpret_cast<uint32_t *>(b->qbase + vb);
+    b->tile_start = b->queue + vb;
     B_ALLOC(b->chunks, sizeof(uint64_t) * 2 * a.nchunks + a.nchunks);
     B_ALLOC(b->st, sizeof(BState));
     B_ALLOC(b->roots, sizeof(int64_t) * 64 * ngraphs);
@@ -1401,9 +2039,10 @@ g5_status g5_batch_destroy(g5_batch *b)
     return G5_OK;
 }
 
-g5_status g5_batch_launch(g5_batch *b, const int64_t *roots_host, const int *nroots, uint32_t *pred_out_dev)
+// Checks the roots of a run and lays them out: the graphs' descriptors, h_roots
+// and h_root_off; *npred = parents in the output, *count = roots.
+static g5_status bind_roots(g5_batch *b, const int64_t *roots_host, const int *nroots, uint64_t *npred, int *count)
 {
-    if (!b || !roots_host || !nroots || !pred_out_dev) return G5_ERR_INVALID_ARG;
     const int ng = (int)b->graphs.size();
     uint64_t pb = 0;
     int off = 0;
@@ -1423,6 +2062,18 @@ g5_status g5_batch_launch(g5_batch *b, const int64_t *roots_host, const int *nro
         off += nroots[i];
     }
     b->h_root_off[ng] = off;
+    *npred = pb;
+    *count = off;
+    return G5_OK;
+}
+
+g5_status g5_batch_launch(g5_batch *b, const int64_t *roots_host, const int *nroots, uint32_t *pred_out_dev)
+{
+    if (!b || !roots_host || !nroots || !pred_out_dev) return G5_ERR_INVALID_ARG;
+    const int ng = (int)b->graphs.size();
+    uint64_t pb = 0;
+    int off = 0;
+    G5_TRY(bind_roots(b, roots_host, nroots, &pb, &off));
     cudaStream_t s = b->stream;
     b->args.pred = pred_out_dev;
     b->args.serving = 0;
@@ -1460,7 +2111,7 @@ g5_status g5_batch_poll(g5_batch *b, int wait, int *done, double *device_ms)
         cudaEventElapsedTime(&ms, b->ev0, b->ev1);
         *device_ms = ms;
     }
-    if (b->h_st->err & 8u) return G5_ERR_TIMEOUT;
+    if (b->h_st->err & 24u) return G5_ERR_TIMEOUT;  // the level cap, or a wait
     if (b->h_st->err) return G5_ERR_CAPACITY;
     return G5_OK;
 }
@@ -1468,7 +2119,42 @@ g5_status g5_batch_poll(g5_batch *b, int wait, int *done, double *device_ms)
 g5_status g5_batch_run(g5_batch *b, const int64_t *roots_host, const int *nroots, uint32_t *pred_out_dev,
                        double *device_ms)
 {
-    G5_TRY(g5_batch_launch(b, roots_host, nroots, pred_out_dev));
+    if (!b || !roots_host || !nroots || !pred_out_dev) return G5_ERR_INVALID_ARG;
+    if (!b->pgrid) G5_TRY(plan_one_launch(b));
+    if (b->pgrid < 0) {
+        G5_TRY(g5_batch_launch(b, roots_host, nroots, pred_out_dev));
+        int done = 0;
+        return g5_batch_poll(b, 1, &done, device_ms);
+    }
+    const int ng = (int)b->graphs.size();
+    uint64_t pb = 0;
+    int off = 0;
+    G5_TRY(bind_roots(b, roots_host, nroots, &pb, &off));
+    cudaStream_t s = b->stream;
+    b->args.serving = 0;
+    memcpy(b->h_stage, b->hgd.data(), sizeof(GraphDesc) * ng);
+    memcpy(b->h_stage + b->roots_at, b->h_roots, sizeof(int64_t) * off);
+    memcpy(b->h_stage + b->off_at, b->h_root_off, sizeof(int32_t) * (ng + 1));
+    G5_CUDA(cudaMemcpyAsync(b->stage, b->h_stage, b->stage_bytes, cudaMemcpyHostToDevice, s));
+    PArgs a = b->pargs;
+    a.b = b->args;
+    a.b.pred = pred_out_dev;
+    a.b.roots = reinterpret_cast<const int64_t *>(b->stage + b->roots_at);
+    a.b.root_off = reinterpret_cast<const int32_t *>(b->stage + b->off_at);
+    a.npred = pb;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(b->pgrid);
+    cfg.blockDim = dim3(kSB);
+    cfg.dynamicSmemBytes = sizeof(PShared);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    G5_CUDA(cudaEventRecord(b->ev0, s));
+    G5_CUDA(cudaLaunchKernelEx(&cfg, k_bsearch, a));
+    G5_CUDA(cudaEventRecord(b->ev1, s));
     int done = 0;
     return g5_batch_poll(b, 1, &done, device_ms);
 }

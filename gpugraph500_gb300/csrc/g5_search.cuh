@@ -49,13 +49,6 @@ struct LevelRec {
     uint64_t examined;  // adjacency entries read while expanding
 };
 
-__device__ __forceinline__ uint64_t warp_sum_u64(uint64_t v)
-{
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    return v;
-}
-
 // A frontier probe: through the read-only path where the bitmap does not
 // change while the kernel runs, else an ordinary load.
 template <bool RO>
@@ -155,8 +148,6 @@ constexpr uint64_t kThin = 8;            // candidates per bitmap word below whi
 constexpr uint64_t kClaimedItems = 1u << 19;  // items a claimed frontier may have (else it is built from its bitmap)
 constexpr int kMinItemShift = 8;         // an item holds 256 entries at least (the tile size if that is larger)
 constexpr int kClusterBlocks = 16;       // blocks of the cluster form
-constexpr int kMaxBlocks = 4000;         // blocks of a grid form at most (their count takes 12 bits)
-constexpr unsigned long long kMeetNs = 10ull * 1000 * 1000 * 1000;
 
 // Where the blocks of a search meet: one block whose bitmaps and sums live in
 // shared memory, one cluster, or a cooperative grid of one block per SM (64
@@ -197,8 +188,6 @@ struct __align__(32) LevelSum {
     unsigned long long built;           // work items built from its bitmap so far
 };
 constexpr int kRing = 8;
-constexpr int kArrive = 52;
-constexpr unsigned long long kValueMask = (1ull << kArrive) - 1;
 
 // A work item: entries [start, start + cnt) of vertex u's row.
 struct __align__(16) Item {
@@ -280,27 +269,6 @@ __device__ __forceinline__ void offsets_of(const SearchArgs &a, uint64_t v, int6
     e = __ldg(a.row_off + v + 1);
 }
 
-__device__ __forceinline__ uint32_t warp_excl_u32(uint32_t x, uint32_t &total)
-{
-    const int lane = g5_lane();
-    uint32_t inc = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    total = __shfl_sync(0xFFFFFFFFu, inc, 31);
-    return inc - x;
-}
-
-// Sum over the warp of values below 2^51, in two warp reductions.
-__device__ __forceinline__ uint64_t warp_add_u51(uint64_t x)
-{
-    const uint64_t lo = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)(x & 0xFFFFFFu));
-    const uint64_t hi = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)(x >> 24));
-    return lo + (hi << 24);
-}
-
 // The warp's new vertices and their entries, into the block's share.
 __device__ __forceinline__ void add_sums(SearchShared &sh, uint32_t nf, uint64_t mf)
 {
@@ -310,36 +278,6 @@ __device__ __forceinline__ void add_sums(SearchShared &sh, uint32_t nf, uint64_t
     if (g5_lane() == 0) {
         atomicAdd(&sh.nf, (unsigned long long)nf);
         atomicAdd(&sh.mf, (unsigned long long)mf);
-    }
-}
-
-// Polls until each of the K words at p holds the arrivals of every block (grid
-// form), their loads issued together; false if a block gave up.  Every wait
-// ends: past kMeetNs the block gives up itself.
-template <int K>
-__device__ __forceinline__ bool await(const unsigned long long *p, unsigned *abort, unsigned long long *value)
-{
-    const unsigned long long all = gridDim.x;
-    unsigned long long t0 = 0;
-    uint32_t polls = 0;
-    for (;;) {
-        unsigned long long x[K];
-#pragma unroll
-        for (int k = 0; k < K; ++k) x[k] = *(const volatile unsigned long long *)(p + k);
-        bool done = true;
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            done = done && (x[k] >> kArrive) == all;
-            value[k] = x[k] & kValueMask;
-        }
-        if (done) return true;
-        if ((++polls & 255u) == 0) {
-            unsigned long long t;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (!t0) t0 = t;
-            if (t - t0 > kMeetNs) *(volatile unsigned *)abort = 1;
-            if (*(volatile unsigned *)abort) return false;
-        }
     }
 }
 
@@ -363,26 +301,6 @@ __device__ __forceinline__ void meet(const SearchArgs &a, SearchShared &sh, unsi
         __threadfence();
     }
     __syncthreads();
-}
-
-// a > b / c as double arithmetic gives it.  The FP64 units are few and slow
-// here, so single precision decides unless the two sides are within its
-// rounding (three roundings of 2^-24, far inside the margin).
-__device__ __forceinline__ bool above_quotient(uint64_t x, uint64_t y, double c)
-{
-    const float l = (float)x * (float)c, r = (float)y;
-    if (l > r * 1.00001f) return true;
-    if (l < r * 0.99999f) return false;
-    return (double)x > (double)y / c;
-}
-
-// a < b / c, likewise.
-__device__ __forceinline__ bool below_quotient(uint64_t x, uint64_t y, double c)
-{
-    const float l = (float)x * (float)c, r = (float)y;
-    if (l < r * 0.99999f) return true;
-    if (l > r * 1.00001f) return false;
-    return (double)x < (double)y / c;
 }
 
 // The end of a level: the blocks' shares of the next level's sums come
