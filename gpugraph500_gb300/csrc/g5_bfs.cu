@@ -131,6 +131,7 @@ struct BfsArgs {
     uint64_t *chunk_u;     // per chunk: unvisited vertices after the level
     uint32_t *slist;       // vertices a sparse top-down level discovered (unordered)
     int parent_mode;       // 0 atomicMin, 1 heavy atomicMin + fix-up, 2 first writer + fix-up
+    const uint32_t *isolated;  // one bit per vertex of degree 0
     const uint32_t *first; // first (smallest) neighbour of each vertex, 0 for isolated ones
     uint64_t tile;         // frontier edges per top-down warp tile (a power of two >= 32)
     int tile_shift;        // log2(tile)
@@ -169,63 +170,68 @@ __device__ __forceinline__ int32_t sparse_next_list(const BfsArgs &a, uint64_t u
 
 // ---- init -----------------------------------------------------------------
 
-__global__ void k_init(BfsArgs a)
+// The level loop's prologue as one launch: bound by its fills (8 N bytes of
+// parents, four bitmaps), 11 us at scale 22 where five memory nodes and a
+// one-block kernel took 29-35.
+__global__ void __launch_bounds__(kBlock) k_init(BfsArgs a)
 {
-    __shared__ int64_t s_root, s_deg, s_base;
-    __shared__ int s_ok;
-    if (threadIdx.x == 0) {
-        int64_t r = *a.root_dev;
-        s_ok = (r >= 0 && r < a.n);
-        s_root = s_ok ? r : 0;
-        s_base = s_ok ? a.row_off[r] : 0;
-        s_deg = s_ok ? a.row_off[r + 1] - s_base : 0;
-        BfsState *st = a.st;
-        st->level = 0;
-        st->dir = DIR_TD;
-        st->nf = s_ok ? 1 : 0;
-        st->mf = (uint64_t)s_deg;
-        st->mu = (uint64_t)(a.nnz - s_deg);
-        st->nvisited = s_ok ? 1 : 0;
-        st->examined = 0;
-        st->err = s_ok ? 0u : G5_DEVERR_CAPACITY;
-        st->want_queue = 1;
-        st->bu_levels = 0;
-        st->codec_acc[0] = st->codec_acc[1] = 0;
-        st->list_mode = 0;
-        st->ulen = 0;
-        st->slen = 0;
-        st->stm = 0;
-        st->sparse = s_ok ? sparse_next(a, (uint64_t)s_deg) : 0;
-        st->sdone = 0;
-        a.log[0].dir = DIR_TD;
-        a.log[0].nf = st->nf;
-        a.log[0].mf = st->mf;
-        a.log[0].examined = 0;
-        if (a.ccap) {
-            a.ccap->count = 0;
-            a.ccap->off = 0;
-            a.ccap->overflow = 0;
-        }
-        if (s_ok) {
-            const int64_t r = s_root;
-            a.pred[r] = r;
-            a.visited[r >> 5] |= 1u << (r & 31);
-            a.front[r >> 5] |= 1u << (r & 31);
-            if (a.level) a.level[r] = 0;
-            a.queue[0] = (uint32_t)r;
-            if (a.qsrc != a.queue) const_cast<uint32_t *>(a.qsrc)[0] = (uint32_t)r;
-            a.qoff[0] = 0;
-            a.qoff[1] = (uint64_t)s_deg;
-            a.qbase[0] = s_base;
-        }
-        // vertices past n in the last word count as visited
-        const int tail = (int)(a.n & 31);
-        if (tail) a.visited[a.nwords - 1] |= ~((1u << tail) - 1u);
+    const uint64_t tid = (uint64_t)blockIdx.x * kBlock + threadIdx.x, nthr = (uint64_t)gridDim.x * kBlock;
+    const int64_t r = *a.root_dev;
+    const bool ok = r >= 0 && r < a.n;
+    const int64_t base = ok ? a.row_off[r] : 0, deg = ok ? a.row_off[r + 1] - base : 0;
+    // vertices without edges can never be reached: they start out visited, so
+    // bottom-up sweeps skip them, as do the ones past n in the last word
+    for (uint64_t w = tid; w < a.nwords; w += nthr) {
+        const uint32_t mine = ok && w == (uint64_t)(r >> 5) ? 1u << (r & 31) : 0u;
+        uint32_t vis = a.isolated[w] | mine;
+        if (w == a.nwords - 1 && (a.n & 31)) vis |= ~((1u << (a.n & 31)) - 1u);
+        a.visited[w] = vis;
+        a.front[w] = mine;
+        a.next[w] = 0;
+        a.wdeg[w] = 0;  // (a search stopped by an error can leave some behind)
     }
-    __syncthreads();
-    if (!s_ok) return;
-    const uint64_t tiles = ((uint64_t)s_deg + a.tile - 1) >> a.tile_shift;
-    for (uint64_t t = threadIdx.x; t < tiles; t += blockDim.x) a.tile_start[t] = 0;
+    for (uint64_t v = tid; v < (uint64_t)a.n; v += nthr) {
+        const bool root = ok && v == (uint64_t)r;
+        a.pred[v] = root ? r : -1;
+        if (a.level) a.level[v] = root ? 0 : -1;
+    }
+    const uint64_t tiles = ((uint64_t)deg + a.tile - 1) >> a.tile_shift;
+    for (uint64_t t = tid; t < tiles && t < a.max_tiles; t += nthr) a.tile_start[t] = 0;
+    if (tid != 0) return;
+    BfsState *st = a.st;
+    st->level = 0;
+    st->dir = DIR_TD;
+    st->nf = ok ? 1 : 0;
+    st->mf = (uint64_t)deg;
+    st->mu = (uint64_t)(a.nnz - deg);
+    st->nvisited = ok ? 1 : 0;
+    st->examined = 0;
+    st->err = ok ? 0u : G5_DEVERR_CAPACITY;
+    st->want_queue = 1;
+    st->bu_levels = 0;
+    st->codec_acc[0] = st->codec_acc[1] = 0;
+    st->list_mode = 0;
+    st->ulen = 0;
+    st->slen = 0;
+    st->stm = 0;
+    st->sparse = ok ? sparse_next(a, (uint64_t)deg) : 0;
+    st->sdone = 0;
+    a.log[0].dir = DIR_TD;
+    a.log[0].nf = st->nf;
+    a.log[0].mf = st->mf;
+    a.log[0].examined = 0;
+    if (a.ccap) {
+        a.ccap->count = 0;
+        a.ccap->off = 0;
+        a.ccap->overflow = 0;
+    }
+    if (ok) {
+        a.queue[0] = (uint32_t)r;
+        if (a.qsrc != a.queue) const_cast<uint32_t *>(a.qsrc)[0] = (uint32_t)r;
+        a.qoff[0] = 0;
+        a.qoff[1] = (uint64_t)deg;
+        a.qbase[0] = base;
+    }
 }
 
 // ---- expansion ----------------------------------------------------------------
@@ -618,7 +624,23 @@ __global__ void __launch_bounds__(kBlock) k_fixup(BfsArgs a)
 // A compaction chunk is CW bitmap words; each of the 8 warps of a
 // block owns 256 consecutive words and walks them 32 at a time: lane l loads
 // word l (coalesced), then for every non-empty word the lanes read the
-// degrees of its set vertices in one coalesced 128-byte load.
+// degrees of its set vertices in one coalesced 128-byte load, kBatchWords words
+// at a time so that their loads are in flight together.
+constexpr int kBatchWords = 4;
+
+// The next kBatchWords of the warp's words x (lane l holds word l) with a bit in
+// act, as the bits themselves: w[k], of word j[k] (0 if there is none left).
+__device__ __forceinline__ void take_words(uint32_t x, unsigned &act, uint32_t (&w)[kBatchWords], int (&j)[kBatchWords])
+{
+#pragma unroll
+    for (int k = 0; k < kBatchWords; ++k) {
+        j[k] = act ? __ffs(act) - 1 : 0;
+        const uint32_t y = __shfl_sync(0xFFFFFFFFu, x, j[k]);
+        w[k] = act ? y : 0u;
+        act &= act - 1;
+    }
+}
+
 template <int CW>
 __device__ __forceinline__ void warp_chunk_counts(const BfsArgs &a, uint64_t wbeg, const uint32_t (&xs)[CW / kWarps / 32],
                                                   uint64_t &cn, uint64_t &cm)
@@ -632,10 +654,14 @@ __device__ __forceinline__ void warp_chunk_counts(const BfsArgs &a, uint64_t wbe
         cn += __popc(x);
         unsigned act = __ballot_sync(0xFFFFFFFFu, x != 0u);
         while (act) {
-            const int j = __ffs(act) - 1;
-            act &= act - 1;
-            const uint32_t wj = __shfl_sync(0xFFFFFFFFu, x, j);
-            if ((wj >> lane) & 1u) cm += __ldg(a.deg + (wbeg + i * 32 + j) * 32 + lane);
+            uint32_t w[kBatchWords], d[kBatchWords];
+            int j[kBatchWords];
+            take_words(x, act, w, j);
+#pragma unroll
+            for (int k = 0; k < kBatchWords; ++k)
+                d[k] = (w[k] >> lane) & 1u ? __ldg(a.deg + (wbeg + i * 32 + j[k]) * 32 + lane) : 0u;
+#pragma unroll
+            for (int k = 0; k < kBatchWords; ++k) cm += d[k];
         }
     }
     cn = warp_sum_u64(cn);
@@ -943,10 +969,15 @@ __device__ void sparse_finish(const BfsArgs &a)
     }
 }
 
-// (at most 48 registers: the sparse finish must not cost the full pass its
-// fifth block per SM)
+// The next level's queue (sorted) and, for a top-down level, its edge offsets
+// and tiles, or the list of unvisited vertices; the bitmaps move on.  Bound by
+// its chain: a warp walks its words one after another.  So the degrees and row
+// offsets of four words are in flight together (64 registers: at 48, one more
+// block per SM, they spill), and a queue that only the codec reads is written
+// without them: a scale-22 level of 1.9 M vertices takes 16 us instead of 72,
+// the codec search 1284 us per two roots before this and k_init, 934 after.
 template <int CW>
-__global__ void __launch_bounds__(kBlock, 5) k_write(BfsArgs a)
+__global__ void __launch_bounds__(kBlock, 4) k_write(BfsArgs a)
 {
     constexpr int kWordsPerWarp = CW / kWarps;
     constexpr int kWordIters = kWordsPerWarp / 32;  // words per lane
@@ -959,6 +990,9 @@ __global__ void __launch_bounds__(kBlock, 5) k_write(BfsArgs a)
     const uint64_t wbeg = (uint64_t)c * CW + (uint64_t)wid * kWordsPerWarp;
     const int32_t L = a.st->level;  // index of the new frontier
     const bool want_q = a.st->want_queue != 0;
+    // edge offsets and tiles are what a top-down level reads; a queue that only
+    // the codec wants is the ids alone
+    const bool want_off = want_q && a.st->dir == DIR_TD;
     const bool want_u = a.st->list_mode != 0;  // next level is bottom-up
     uint64_t pos = a.chunk_n[c], mpos = a.chunk_m[c], upos = a.chunk_u[c];
     // every word of the warp's range up front (one load per lane and word,
@@ -973,7 +1007,13 @@ __global__ void __launch_bounds__(kBlock, 5) k_write(BfsArgs a)
     }
     // per-warp totals, then the warp's offsets inside the chunk
     uint64_t cn = 0, cm = 0, cu = 0;
-    if (want_q || a.level) warp_chunk_counts<CW>(a, wbeg, xs, cn, cm);
+    if (want_off) {
+        warp_chunk_counts<CW>(a, wbeg, xs, cn, cm);
+    } else if (want_q) {
+#pragma unroll
+        for (int i = 0; i < kWordIters; ++i) cn += __popc(xs[i]);
+        cn = warp_sum_u64(cn);
+    }
     if (want_u) {
 #pragma unroll
         for (int i = 0; i < kWordIters; ++i) cu += __popc(~(vs[i] | xs[i]));
@@ -1020,35 +1060,54 @@ __global__ void __launch_bounds__(kBlock, 5) k_write(BfsArgs a)
         }
         if (!want_q && !a.level) continue;
         unsigned act = __ballot_sync(0xFFFFFFFFu, x != 0u);
-        while (act) {
+        while (!want_off && act) {
             const int j = __ffs(act) - 1;
             act &= act - 1;
             const uint32_t wj = __shfl_sync(0xFFFFFFFFu, x, j);
-            const bool mine = (wj >> lane) & 1u;
-            const uint64_t v = (wbeg + i * 32 + j) * 32 + lane;
-            uint64_t d = mine ? (uint64_t)__ldg(a.deg + v) : 0;
-            // inclusive scan of the degrees of this word's vertices
-            uint64_t incl = d;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint64_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            if (mine) {
-                const uint64_t p = pos + __popc(wj & g5_lanemask_lt());
-                const uint64_t mp = mpos + incl - d;
+            if ((wj >> lane) & 1u) {
+                const uint64_t v = (wbeg + i * 32 + j) * 32 + lane;
                 if (a.level) a.level[v] = L;
-                if (want_q) {
+                if (want_q) a.queue[pos + __popc(wj & g5_lanemask_lt())] = (uint32_t)v;
+            }
+            pos += __popc(wj);
+        }
+        while (act) {
+            uint32_t w[kBatchWords], dg[kBatchWords];
+            int64_t rs[kBatchWords];
+            int j[kBatchWords];
+            take_words(x, act, w, j);
+#pragma unroll
+            for (int k = 0; k < kBatchWords; ++k) {
+                const bool mine = (w[k] >> lane) & 1u;
+                const uint64_t v = (wbeg + i * 32 + j[k]) * 32 + lane;
+                dg[k] = mine ? __ldg(a.deg + v) : 0u;
+                rs[k] = mine ? __ldg(a.row_off + v) : 0;
+            }
+#pragma unroll
+            for (int k = 0; k < kBatchWords; ++k) {
+                // inclusive scan of the degrees of this word's vertices
+                const uint64_t d = dg[k];
+                uint64_t incl = d;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint64_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                if ((w[k] >> lane) & 1u) {
+                    const uint64_t v = (wbeg + i * 32 + j[k]) * 32 + lane;
+                    const uint64_t p = pos + __popc(w[k] & g5_lanemask_lt());
+                    const uint64_t mp = mpos + incl - d;
+                    if (a.level) a.level[v] = L;
                     a.queue[p] = (uint32_t)v;
                     a.qoff[p] = mp;
-                    a.qbase[p] = a.row_off[v] - (int64_t)mp;
+                    a.qbase[p] = rs[k] - (int64_t)mp;
                     uint64_t t = (mp + a.tile - 1) >> a.tile_shift;
                     const uint64_t tend = (mp + d + a.tile - 1) >> a.tile_shift;
                     for (; t < tend && t < a.max_tiles; ++t) a.tile_start[t] = (uint32_t)p;
                 }
+                pos += __popc(w[k]);
+                mpos += __shfl_sync(0xFFFFFFFFu, incl, 31);
             }
-            pos += __popc(wj);
-            mpos += __shfl_sync(0xFFFFFFFFu, incl, 31);
         }
     }
 }
@@ -1319,16 +1378,7 @@ namespace {
 
 void enqueue_prologue(g5_bfs *b, const BfsArgs &a, cudaStream_t s)
 {
-    // vertices without edges can never be reached: they start out visited, so
-    // bottom-up sweeps skip them (the root is set again by k_init)
-    cudaMemcpyAsync(b->bitmaps, b->isolated, sizeof(uint32_t) * a.nwords, cudaMemcpyDeviceToDevice, s);
-    cudaMemsetAsync(b->bitmaps + a.nwords, 0, sizeof(uint32_t) * 2 * a.nwords, s);
-    // per-word degree sums start at zero (a search stopped by an error can
-    // leave some behind)
-    cudaMemsetAsync(b->wdeg, 0, sizeof(uint32_t) * a.nwords, s);
-    cudaMemsetAsync(a.pred, 0xFF, sizeof(int64_t) * (size_t)a.n, s);
-    if (b->level) cudaMemsetAsync(b->level, 0xFF, sizeof(int32_t) * (size_t)a.n, s);
-    k_init<<<1, kBlock, 0, s>>>(a);
+    k_init<<<g5::grid_for(4), kBlock, 0, s>>>(a);
 }
 
 void enqueue_level(g5_bfs *b, const BfsArgs &a, cudaStream_t s, Prof *pf = nullptr)
@@ -1586,6 +1636,7 @@ g5_status alloc_ws(g5_bfs *b)
     a.row_off = g->row_off;
     a.col = g->col;
     a.deg = b->deg;
+    a.isolated = b->isolated;
     a.visited = b->bitmaps;
     a.front = b->bitmaps + a.nwords;
     a.next = b->bitmaps + 2 * a.nwords;
