@@ -250,10 +250,27 @@ __device__ void expand_td(const BfsArgs &a, uint64_t &examined)
         if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(&a.st->err, G5_DEVERR_CAPACITY);
         return;
     }
-    for (uint64_t t = gw; t < ntiles; t += nw) {
-        const uint64_t e0 = t << a.tile_shift;
-        const uint64_t e1 = min(e0 + a.tile, mf);
+    // few tiles: a tile's entries are split over several warps, down to 32 each
+    // (a chain of steps of 4 us otherwise: a level of 2255 entries took 34 us)
+    uint32_t split = 0;
+    while (5 + (int)split < a.tile_shift && (ntiles << (split + 1)) <= nw) ++split;
+    for (uint64_t p = gw; p < ntiles << split; p += nw) {
+        const uint64_t t = p >> split;
+        const uint64_t e0 = p << (a.tile_shift - split);
+        const uint64_t e1 = min(e0 + (a.tile >> split), mf);
+        if (e0 >= e1) continue;
         uint64_t cur = a.tile_start[t];
+        if (e0 & (a.tile - 1)) {
+            // the last vertex that starts at or before e0, 32 probes at a time
+            uint64_t len = (t + 1 < ntiles ? (uint64_t)a.tile_start[t + 1] : nf - 1) - cur + 1;
+            while (len > 1) {
+                const uint64_t step = (len + 31) / 32, at = lane * step;
+                const unsigned m = __ballot_sync(0xFFFFFFFFu, at < len && a.qoff[cur + at] <= e0);
+                const uint64_t k = (uint64_t)(31 - __clz(m)) * step;  // (lane 0's always is)
+                cur += k;
+                len = min(step, len - k);
+            }
+        }
         for (uint64_t gb = e0; gb < e1; gb += 32) {
             const uint64_t idx = cur + 1 + lane;
             s_q[wib][lane] = idx <= nf ? a.qoff[idx] : ~0ull;
