@@ -599,6 +599,7 @@ __device__ __forceinline__ void add_examined(const BfsArgs &a, uint64_t examined
 // Top-down expansion of the level (no-op when the level is bottom-up).
 __global__ void __launch_bounds__(kBlock, 8) k_td(BfsArgs a)
 {
+    g5_pdl_sync();
     if (a.st->err || a.st->dir != DIR_TD) return;
     uint64_t examined = 0;
     expand_td(a, examined);
@@ -611,6 +612,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_td(BfsArgs a)
 template <typename Off>
 __global__ void __launch_bounds__(kBlock, 8) k_bu(BfsArgs a)
 {
+    g5_pdl_sync();
     if (a.st->err || a.st->dir != DIR_BU) return;
     uint64_t examined = 0;
     if (a.st->list_mode) bottom_up_list<Off>(a, examined);
@@ -621,6 +623,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_bu(BfsArgs a)
 // Parents of the vertices a top-down level discovered (no-op after bottom-up).
 __global__ void __launch_bounds__(kBlock) k_fixup(BfsArgs a)
 {
+    g5_pdl_sync();
     if (a.st->err || a.st->dir != DIR_TD || a.parent_mode == 0) return;
     uint64_t examined = 0;
     if (a.ro32) sweep<true, uint32_t>(a, examined);
@@ -699,6 +702,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_count(BfsArgs a)
     // a level the sparse path takes needs no counts: block 0 of k_write
     // builds its queue from the list
     __shared__ int s_take;
+    g5_pdl_sync();
     if (threadIdx.x == 0) {
         s_take = sparse_take(a) ? 1 : 0;
         if (blockIdx.x == 0) a.st->sdone = s_take;
@@ -998,6 +1002,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_write(BfsArgs a)
 {
     constexpr int kWordsPerWarp = CW / kWarps;
     constexpr int kWordIters = kWordsPerWarp / 32;  // words per lane
+    g5_pdl_sync();
     if (a.st->sdone) {  // the sparse path took the level
         if (blockIdx.x == 0) sparse_finish(a);
         return;
@@ -1402,27 +1407,28 @@ void enqueue_level(g5_bfs *b, const BfsArgs &a, cudaStream_t s, Prof *pf = nullp
 {
     Prof dummy;
     Prof &p = pf ? *pf : dummy;
-    // (programmatic dependent launches here measured no faster: 605 against
-    // 603 GTEPS at scale 26, 508 against 516 at scale 24)
+    // programmatic dependent launches, so that a kernel sets up while the one
+    // before it drains: 2.5 to 3 % of a scale-22 search with the codec (875 and
+    // 854 us per two roots).  Not under the per-kernel timer.
+    const bool pdl = !pf;
     p.mark(KP_EXPAND, s);
-    k_td<<<g5::grid_for(8), kBlock, 0, s>>>(a);
-    if (a.ro32) k_bu<uint32_t><<<g5::grid_for(8), kBlock, 0, s>>>(a);
-    else k_bu<int64_t><<<g5::grid_for(8), kBlock, 0, s>>>(a);
+    g5::launch(false, k_td, g5::grid_for(8), kBlock, s, a);
+    g5::launch(pdl, a.ro32 ? k_bu<uint32_t> : k_bu<int64_t>, g5::grid_for(8), kBlock, s, a);
     p.mark(KP_FIXUP, s);
-    if (a.parent_mode != 0) k_fixup<<<g5::grid_for(8), kBlock, 0, s>>>(a);
+    if (a.parent_mode != 0) g5::launch(pdl, k_fixup, g5::grid_for(8), kBlock, s, a);
     p.mark(KP_COUNT, s);
     switch (a.chunk_words) {
-    case 256: k_count<256><<<a.nchunks, kBlock, 0, s>>>(a); break;
-    case 512: k_count<512><<<a.nchunks, kBlock, 0, s>>>(a); break;
-    case 1024: k_count<1024><<<a.nchunks, kBlock, 0, s>>>(a); break;
-    default: k_count<2048><<<a.nchunks, kBlock, 0, s>>>(a); break;
+    case 256: g5::launch(pdl, k_count<256>, a.nchunks, kBlock, s, a); break;
+    case 512: g5::launch(pdl, k_count<512>, a.nchunks, kBlock, s, a); break;
+    case 1024: g5::launch(pdl, k_count<1024>, a.nchunks, kBlock, s, a); break;
+    default: g5::launch(pdl, k_count<2048>, a.nchunks, kBlock, s, a); break;
     }
     p.mark(KP_WRITE, s);
     switch (a.chunk_words) {
-    case 256: k_write<256><<<a.nchunks, kBlock, 0, s>>>(a); break;
-    case 512: k_write<512><<<a.nchunks, kBlock, 0, s>>>(a); break;
-    case 1024: k_write<1024><<<a.nchunks, kBlock, 0, s>>>(a); break;
-    default: k_write<2048><<<a.nchunks, kBlock, 0, s>>>(a); break;
+    case 256: g5::launch(pdl, k_write<256>, a.nchunks, kBlock, s, a); break;
+    case 512: g5::launch(pdl, k_write<512>, a.nchunks, kBlock, s, a); break;
+    case 1024: g5::launch(pdl, k_write<1024>, a.nchunks, kBlock, s, a); break;
+    default: g5::launch(pdl, k_write<2048>, a.nchunks, kBlock, s, a); break;
     }
     p.mark(KP_CODEC, s);
     if (a.codec) {
