@@ -263,6 +263,7 @@ struct __align__(32) LongItem {
 struct LongRows {
     LongItem *items;
     unsigned long long *alloc;
+    unsigned long long *steps;  // steps claimed so far
 };
 
 // vps_shift: log2 of the vertices per warp step (32, less on graphs with fewer
@@ -272,15 +273,28 @@ __device__ __forceinline__ void bexp_bu(const BArgs &a, const GraphDesc *gd, BuS
                                         int vps_shift, LongRows longs, uint64_t &examined)
 {
     const int lane = g5_lane();
-    for (uint64_t w = gw; w < (a.nsteps << (5 - vps_shift)); w += nw) {
+    const uint64_t steps = a.nsteps << (5 - vps_shift);
+    uint64_t w = gw;
+    while (w < steps) {
         // the graph's vertices with edges in original-id order, 32 per warp
         // step (vertices without edges are never reached, and half the
         // vertices of a Kronecker graph have none): high-degree vertices,
         // which have the lowest new ids, spread over the warps
         const int gi = a.step_graph[w >> (5 - vps_shift)];
         const GraphDesc &d = gd[gi];
-        if (d.dir != BU || d.nf == 0) continue;
         const uint64_t li = lane < 1 << vps_shift ? ((w - (d.step0 << (5 - vps_shift))) << vps_shift) + lane : d.nblist;
+        if (SPLIT && steps > 2 * nw) {
+            // the next step goes to the warp that is free first (scale 24 8220
+            // -> 7920 us, 20 757 -> 733, the eight mixed graphs 1255 -> 1198);
+            // fewer steps a warp do not pay for the claims (scale 16 248 and
+            // 264, 13 141 and 147)
+            unsigned long long x = 0;
+            if (lane == 0) x = atomicAdd(longs.steps, 1ull);
+            w = nw + __shfl_sync(0xFFFFFFFFu, x, 0);
+        } else {
+            w += nw;
+        }
+        if (d.dir != BU || d.nf == 0) continue;
         const uint64_t ol = li < d.nblist ? __ldg(d.blist + li) : 0u;
         const uint32_t R = (uint32_t)d.nroots;
         // new id and row bounds, indexed by original id: three loads issued
@@ -902,6 +916,7 @@ struct LevelMeet {
     unsigned long long alloc;      // claimed items of its frontier
     unsigned long long built;      // items built for it
     unsigned long long longs;      // pieces of long rows
+    unsigned long long steps;      // bottom-up steps claimed
 };
 
 struct PArgs {
@@ -1255,7 +1270,7 @@ __global__ void __launch_bounds__(kSB, 1) k_bsearch(const __grid_constant__ PArg
                 uint64_t ex = 0;
                 const uint64_t gw = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, nw = (uint64_t)gridDim.x * kSW;
                 __syncwarp();
-                bexp_bu<true>(a.b, sh.gd, sh.w[threadIdx.x >> 5].bu, gw, nw, a.vps_shift, LongRows{a.longs, &cur->longs}, ex);
+                bexp_bu<true>(a.b, sh.gd, sh.w[threadIdx.x >> 5].bu, gw, nw, a.vps_shift, LongRows{a.longs, &cur->longs, &cur->steps}, ex);
                 pmeet(a, sh, &cur->arrive[4]);
                 if (sh.stop) break;
                 bexp_long(a.b, sh.gd, a.longs, __ldcg(&cur->longs), gw, nw);
