@@ -224,6 +224,12 @@ __device__ void bexp_td(const BArgs &a, uint64_t &examined)
     }
 }
 
+__device__ __forceinline__ uint64_t warp_or_u64(uint64_t x)
+{
+    const uint32_t lo = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)x), hi = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)(x >> 32));
+    return lo | (uint64_t)hi << 32;
+}
+
 // Bottom-up: the candidates of v are the roots that have not visited it;
 // the first frontier hit of each root along v's ascending adjacency is its
 // parent.  A warp takes 32 consecutive vertices (never two graphs: graphs
@@ -446,8 +452,7 @@ __device__ __forceinline__ void bexp_bu(const BArgs &a, const GraphDesc *gd, BuS
                 // one OR over the four windows; the first hits are located
                 // only when the step holds a root not found before
                 uint64_t lo = (hw[0] | hw[1] | hw[2] | hw[3]) & nd;
-#pragma unroll
-                for (int o = 16; o; o >>= 1) lo |= __shfl_xor_sync(0xFFFFFFFFu, lo, o);
+                lo = warp_or_u64(lo);
                 if (!lo) {
                     jj += 128;
                     continue;
@@ -517,13 +522,19 @@ __device__ __forceinline__ void bexp_bu(const BArgs &a, const GraphDesc *gd, BuS
         for (int k = 0; k < kSerial; ++k) {
             unsigned em = __ballot_sync(0xFFFFFFFFu, ws.evm[k][lane] != 0ull);
             while (em) {
-                const int vi = __ffs(em) - 1;
+                // two events together: their loads overlap
+                const int v0 = __ffs(em) - 1;
                 em &= em - 1;
-                const uint64_t m = ws.evm[k][vi];
-                const uint32_t u = ws.evu[k][vi];
-                uint32_t *pv = a.pred + d.pred_base + (uint64_t)__shfl_sync(0xFFFFFFFFu, vo, vi) * R;
-                if ((m >> lane) & 1ull) pv[lane] = u;
-                if ((m >> (lane + 32)) & 1ull) pv[lane + 32] = u;
+                const int v1 = em ? __ffs(em) - 1 : v0;
+                const uint64_t m0 = ws.evm[k][v0], m1 = em ? ws.evm[k][v1] : 0ull;
+                const uint32_t u0 = ws.evu[k][v0], u1 = ws.evu[k][v1];
+                uint32_t *p0 = a.pred + d.pred_base + (uint64_t)__shfl_sync(0xFFFFFFFFu, vo, v0) * R;
+                uint32_t *p1 = a.pred + d.pred_base + (uint64_t)__shfl_sync(0xFFFFFFFFu, vo, v1) * R;
+                em &= em - 1;
+                if ((m0 >> lane) & 1ull) p0[lane] = u0;
+                if ((m0 >> (lane + 32)) & 1ull) p0[lane + 32] = u0;
+                if ((m1 >> lane) & 1ull) p1[lane] = u1;
+                if ((m1 >> (lane + 32)) & 1ull) p1[lane + 32] = u1;
             }
         }
         __syncwarp();
