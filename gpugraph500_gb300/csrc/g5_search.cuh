@@ -664,18 +664,20 @@ __device__ __forceinline__ void search_count(const SearchArgs &a, SearchShared &
 }
 
 // The work items of a frontier of nf vertices held as a bitmap.  Few vertices
-// per word: a warp looks through 32 words and allocates for each that holds
-// any.  Many: a lane takes four words, and one allocation serves a block step;
-// so also from kBuildWarp vertices on, where the warps' allocations queue up at
-// their one counter (43,541 vertices in 2 M words: 40 us of 52 for the level,
-// now 18; mean search at scale 24 417 -> 400 us, 26 1456 -> 1393).
+// per word, or no more than two per warp: a warp looks through 32 words and
+// allocates for each that holds any.  Many: a lane takes four words, and one
+// allocation serves a block step; so also from kBuildWarp vertices on, where the
+// warps' allocations queue up at their one counter (43,541 vertices in 2 M words:
+// 40 us of 52 for the level, now 18; mean search at scale 24 417 -> 400 us, 26
+// 1456 -> 1393).  (Two per warp: 1038 vertices in 2048 words took one block 9.5
+// us; mean search at scale 16 49 -> 44 us, 14 36 -> 32, 18 52 -> 49.)
 template <typename Off>
 __device__ __forceinline__ void search_build(const SearchArgs &a, SearchShared &sh, const uint32_t *front, uint64_t nf, Item *items,
                              unsigned long long *alloc)
 {
     const int lane = g5_lane(), wid = threadIdx.x >> 5;
     const uint32_t round = (1u << a.tile_shift) - 1;
-    if (4 * nf <= a.nwords && nf <= kBuildWarp) {
+    if (nf <= kBuildWarp && (4 * nf <= a.nwords || nf <= 2 * gridDim.x * kSW)) {
         const uint64_t gw = (uint64_t)wid * gridDim.x + blockIdx.x;
         // (small graphs: fewer words per warp, so that every warp has some)
         uint32_t wpw = 32;
