@@ -1499,6 +1499,9 @@ cudaError_t launch_search(g5_bfs *b, int64_t root, int64_t *pred, SearchState *o
     a.root = root;
     a.pred = pred;
     a.out = out;
+    const uint64_t warps = (uint64_t)grid * kSW;
+    a.per_warp = a.nwords / warps;
+    a.wps = bu_step_words(a.nwords, warps);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kSB);
@@ -1703,7 +1706,6 @@ g5_status alloc_ws(g5_bfs *b)
         sa.nnz = g->nnz;
         sa.nwords = a.nwords;
         sa.stride = (a.nwords + 3) & ~(uint64_t)3;
-        sa.per_warp = a.nwords / ((uint64_t)b->sgrid * kSW);
         sa.bitmaps = b->bitmaps;
         sa.level = b->level;
         sa.log = b->h_log;

@@ -176,6 +176,20 @@ inline int search_form(int64_t n, int64_t nnz)
     return n < kGrid2Vertices ? SEARCH_GRID1 : SEARCH_GRID2;
 }
 
+// Bitmap words per warp step of a bottom-up level: the fewest steps of at most
+// 32 words, all warps alike.  A step is a chain (words, list, offsets, probes)
+// that pipelines over its own rounds only, and a last round of steps that half
+// of the warps take costs the other half the same.  us per search, against
+// powers of two of which each warp took about eight steps: scale 19 66 -> 60,
+// 20 79 -> 71, 21 96 -> 89, 22 159 -> 149, 24 399 -> 393, 26 1435 -> 1385; two
+// or three times as many steps: scale 20 75 and 78, 22 154 and 156, 26 1405 and
+// 1409.
+inline uint32_t bu_step_words(uint64_t nwords, uint64_t warps)
+{
+    const uint64_t per = (nwords + warps - 1) / warps, steps = (per + 31) / 32;
+    return (uint32_t)((per + steps - 1) / steps);
+}
+
 // One level's sums, in a ring (a level adds to the next one's nf, mf and
 // nitems and to its own examined, and clears the two after that, so the ring
 // goes on from search to search without being cleared by the host).  In the
@@ -220,6 +234,7 @@ struct SearchArgs {
     LevelRec *log;             // pinned host: its level records
     int64_t root;
     uint64_t per_warp;         // bitmap words per warp of the grid
+    uint32_t wps;              // bitmap words per step of a bottom-up level
     int tile_shift;
     int bu_serial;
     int max_levels;
@@ -821,16 +836,12 @@ __global__ void __launch_bounds__(kSB, MODE == SEARCH_GRID2 ? 2 : 1) k_search(co
                 search_count(a, sh, next, L);
             }
         } else {
-            // words per warp step: few candidates, one step per warp and up to
-            // 4 words per lane (short chains); many, a few steps per warp
             const uint64_t unv = (uint64_t)a.with_edges - visited;
             const bool thin = unv < a.nwords * kThin;
             if (thin && a.per_warp > 32) {
                 search_bu<Off, true>(a, sh, V, front, next, spare, 0, L);
             } else {
-                uint32_t wps = 1;
-                while (wps < 32 && (uint64_t)wps * (thin ? 1 : 8) <= a.per_warp) wps *= 2;
-                search_bu<Off, false>(a, sh, V, front, next, spare, wps, L);
+                search_bu<Off, false>(a, sh, V, front, next, spare, a.wps, L);
             }
         }
         finish_level<MODE>(a, sh, cur, nxt, L, dir, cnf, mu);
