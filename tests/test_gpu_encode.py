@@ -78,3 +78,28 @@ def test_plugin_refuses_ids_past_32_bits(n):
                 p.compress(y)
     c, size = p.compress(x)
     assert np.array_equal(p.decompress(c, size, n), x)
+
+
+@pytest.mark.parametrize("kind", ["ids", "random"])
+@pytest.mark.parametrize("n", [1, 127, 128, 2049, 4095, 4096, 4097, 4223, 4224, 9000])
+def test_queues_of_one_block(n, kind):
+    """Around two groups, up to which one block does a queue alone; async calls of
+    changing lengths on one codec (a lone block leaves the counters as the whole
+    grid does)."""
+    x = values(kind, n, np.random.default_rng(n))
+    c = g5.Codec(50_000)
+    check(c, x)
+    long = values(kind, 50_000, np.random.default_rng(1))
+    for q in (x, long, x):
+        din = torch.from_numpy(q.view(np.int32)).cuda()
+        out = torch.empty(g5.Codec.bound(len(q)) + 8, dtype=torch.int32, device="cuda")
+        back = torch.full((len(q) + 128,), -1, dtype=torch.int32, device="cuda")
+        cnt = torch.tensor([len(q)], dtype=torch.int64, device="cuda")
+        words, n_back = torch.zeros_like(cnt), torch.zeros_like(cnt)
+        torch.cuda.synchronize()
+        c.encode_async(din, cnt, out, words)
+        c.decode_async(out, words, back, len(q) + 128, n_back)
+        assert c.status() == 0 and int(n_back) == len(q)
+        assert np.array_equal(out[:int(words)].cpu().numpy().view(np.uint32), orc.encode(q, MODES[0][1]))
+        assert np.array_equal(back[:len(q)].cpu().numpy().view(np.uint32), q)
+    c.close()

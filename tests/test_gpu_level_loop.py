@@ -1,6 +1,6 @@
 """The level loop (searches with the codec, with fix-up parents, without the
 graph) where its passes change: tiles split over warps, queues with and without
-edge offsets, levels and no levels; parents and levels equal the oracle's."""
+edge offsets, raw copies by one block and by all, levels and no levels; parents and levels equal the oracle's."""
 import numpy as np
 import pytest
 
@@ -41,7 +41,8 @@ def test_level_loop(name, tile):
     g = g5.Graph.from_csr(ro, col)
     # (mostly bottom-up, top-down only, the default switch)
     for alpha, beta in ((1e9, 1e9), (1e-9, 1e-9), (14.0, 24.0)):
-        for kw in (dict(codec=g5.CODEC_D4), dict(codec=g5.CODEC_DM, want_levels=True), dict(parent_mode=1),
+        for kw in (dict(codec=g5.CODEC_D4), dict(codec=g5.CODEC_DM, want_levels=True),
+                   dict(codec=g5.CODEC_D4, codec_threshold=20_000), dict(parent_mode=1),
                    dict(parent_mode=2, want_levels=True), dict(use_graph=False, want_levels=True)):
             s = g5.CudaBFS(g, alpha=alpha, beta=beta, tile_edges=tile, **kw)
             for r in roots + roots[:1]:
