@@ -269,7 +269,7 @@ struct __align__(32) LongItem {
 struct LongRows {
     LongItem *items;
     unsigned long long *alloc;
-    unsigned long long *steps;  // steps claimed so far
+    uint32_t *steps;  // shared: steps the block has given out
 };
 
 // vps_shift: log2 of the vertices per warp step (32, less on graphs with fewer
@@ -289,14 +289,14 @@ __device__ __forceinline__ void bexp_bu(const BArgs &a, const GraphDesc *gd, BuS
         const int gi = a.step_graph[w >> (5 - vps_shift)];
         const GraphDesc &d = gd[gi];
         const uint64_t li = lane < 1 << vps_shift ? ((w - (d.step0 << (5 - vps_shift))) << vps_shift) + lane : d.nblist;
-        if (SPLIT && steps > 2 * nw) {
-            // the next step goes to the warp that is free first (scale 24 8220
-            // -> 7920 us, 20 757 -> 733, the eight mixed graphs 1255 -> 1198);
-            // fewer steps a warp do not pay for the claims (scale 16 248 and
-            // 264, 13 141 and 147)
-            unsigned long long x = 0;
-            if (lane == 0) x = atomicAdd(longs.steps, 1ull);
-            w = nw + __shfl_sync(0xFFFFFFFFu, x, 0);
+        if (SPLIT) {
+            // the block's next step goes to its first free warp (fixed shares
+            // left a sixth of the warps' time to waiting; steps claimed over the
+            // whole grid, 2 ns each at one counter, cost the light levels of
+            // scale 24 twice their time)
+            uint32_t x = 0;
+            if (lane == 0) x = atomicAdd(longs.steps, 1u);
+            w = (uint64_t)__shfl_sync(0xFFFFFFFFu, x, 0) * gridDim.x + blockIdx.x;
         } else {
             w += nw;
         }
@@ -927,7 +927,6 @@ struct LevelMeet {
     unsigned long long alloc;      // claimed items of its frontier
     unsigned long long built;      // items built for it
     unsigned long long longs;      // pieces of long rows
-    unsigned long long steps;      // bottom-up steps claimed
 };
 
 struct PArgs {
@@ -967,6 +966,7 @@ struct PShared {
     unsigned long long active, td_entries;
     uint32_t dirs;   // bit 0: a graph expands top-down, bit 1: bottom-up
     uint32_t build;  // some graph's items are to be built
+    uint32_t steps;  // bottom-up steps given out
     uint8_t build_g[kMaxGraphs];
     uint32_t stop;
 };
@@ -1281,7 +1281,7 @@ __global__ void __launch_bounds__(kSB, 1) k_bsearch(const __grid_constant__ PArg
                 uint64_t ex = 0;
                 const uint64_t gw = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, nw = (uint64_t)gridDim.x * kSW;
                 __syncwarp();
-                bexp_bu<true>(a.b, sh.gd, sh.w[threadIdx.x >> 5].bu, gw, nw, a.vps_shift, LongRows{a.longs, &cur->longs, &cur->steps}, ex);
+                bexp_bu<true>(a.b, sh.gd, sh.w[threadIdx.x >> 5].bu, gw, nw, a.vps_shift, LongRows{a.longs, &cur->longs, &sh.steps}, ex);
                 pmeet(a, sh, &cur->arrive[4]);
                 if (sh.stop) break;
                 bexp_long(a.b, sh.gd, a.longs, __ldcg(&cur->longs), gw, nw);
@@ -1298,6 +1298,7 @@ __global__ void __launch_bounds__(kSB, 1) k_bsearch(const __grid_constant__ PArg
         if (threadIdx.x == 0) {
             sh.active = sh.td_entries = 0;
             sh.dirs = sh.build = 0;
+            sh.steps = kSW;
         }
         __syncthreads();
         const bool fits = claim && L >= 0 && __ldcg(&nxt->alloc) <= a.claimed_cap;
