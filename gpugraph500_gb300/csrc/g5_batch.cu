@@ -251,7 +251,7 @@ struct BuScratch {  // one warp's serial hits
 // long as all the others together needed for the level.  The owner's share keeps
 // the early end of rows whose roots are soon found: with none of it, scale 24
 // took 10958 us a batch instead of 8160, and without pieces 9593 (eight mixed
-// graphs 1324, 1252 and 1432).  Pieces of 128, 256, 512, 1024 and 2048 entries:
+// graphs 1324, 1252 and 1432; before the roots that lag were split off).  Pieces of 128, 256, 512, 1024 and 2048 entries:
 // 8598, 8266, 8154, 8152, 8222 (mixed 1325, 1280, 1257, 1235, 1306; scale 16 211,
 // 220, 242, 244, 244).
 constexpr uint32_t kLongRow = 512;
@@ -300,7 +300,7 @@ __device__ __forceinline__ void bexp_bu(const BArgs &a, const GraphDesc *gd, BuS
         } else {
             w += nw;
         }
-        if (d.dir != BU || d.nf == 0) continue;
+        if (d.dir != BU || d.nf == 0 || d.amask == 0) continue;
         const uint64_t ol = li < d.nblist ? __ldg(d.blist + li) : 0u;
         const uint32_t R = (uint32_t)d.nroots;
         // new id and row bounds, indexed by original id: three loads issued
@@ -538,7 +538,11 @@ __device__ __forceinline__ void bexp_bu(const BArgs &a, const GraphDesc *gd, BuS
             }
         }
         __syncwarp();
-        if (found) a.next[v] |= found;  // only this lane writes v in a bottom-up level
+        // (only this lane writes v in a bottom-up level, unless some roots go top-down)
+        if (found) {
+            if (SPLIT) atomicOr((unsigned long long *)&a.next[v], (unsigned long long)found);
+            else a.next[v] |= found;
+        }
         examined += ex;
     }
 }
@@ -893,23 +897,41 @@ __global__ void __launch_bounds__(kB, 4) k_bwrite(BArgs a)
 //   expand  top-down graphs by work items of up to kItemEntries entries,
 //           bottom-up ones as in k_bbu
 //   commit  visited |= next, next -> front, the next frontier's sums per graph
-//   decide  every block computes each graph's direction from the sums
+//   decide  every block computes each graph's direction from the sums, and
+//           which roots go top-down in its first bottom-up level all the same
 // A top-down level of at most kClaimMax entries appends the rows it reaches
 // first to the items of the next level; otherwise, and for graphs that come back
 // from bottom-up, the items are built from the frontier words.
 //
 // Five launches and a while node a level cost about 35 us whatever the level
 // held; a level now costs its work and 6-8 us.  Device us per batch of Kronecker
-// graphs, 16 edges a vertex, before and after: scale 8, 4 roots, 230 and 76;
-// scale 13, 64 roots, 410 and 135; scale 16 479 and 242; scale 20 1281 and 758;
-// scale 24 10267 and 8160; eight graphs of scales 14 to 20, 16 roots each, 1820
-// and 1252.
+// graphs, 16 edges a vertex, before and after: scale 8, 4 roots, 230 and 70;
+// scale 13, 64 roots, 410 and 134; scale 16 479 and 226; scale 20 1281 and 662;
+// scale 24 10267 and 6667; eight graphs of scales 14 to 20, 16 roots each, 1820
+// and 1070.  What bounds it: the bottom-up sweeps, half by instructions and half
+// by the latency of their gathers (39 % of the issue slots, 39 % of the memory
+// bandwidth at 64 registers, which two windows of loads and 64-bit roots need;
+// 48 registers and a quarter more warps measured slower).
 constexpr int kSB = 1024;
 constexpr int kSW = kSB / 32;
 constexpr uint32_t kItemEntries = 256;
 constexpr uint64_t kClaimMax = 1u << 18;
 constexpr uint64_t kClaimedItems = 1u << 19;
 constexpr int kRing = 4;  // levels of sums held
+// Roots whose frontier has less than 1/kFewShare of the graph's entries, and all
+// together at most 1/kFewTotal, expand top-down in the graph's first bottom-up
+// level.  A root that lags behind (its few frontier vertices are nobody's
+// neighbours) keeps every row of that level from being left early: with all 64
+// roots of a scale-22 batch the level examines 102.7 M of 128 M entries, without
+// the four that lag most 42 M, without eight 33 M.  Top-down an entry costs more
+// (atomics all over the parents), so only few.  us per batch, shares of 32, 64,
+// 128, 256 and none: scale 24 6676, 6661, 6667, 6891, 7659; scale 20 672, 668,
+// 671, 672, 715; the eight mixed graphs 1082, 1089, 1078, 1082, 1116 (with a
+// total of 1/4 instead, scale 24 11300).  Graphs of fewer than kSplitEntries
+// entries are not worth the counting (scale 8 70 and 76).
+constexpr uint64_t kFewShare = 128, kFewTotal = 32;
+constexpr int64_t kSplitEntries = 1 << 16;
+constexpr uint32_t kRootEntries = 16;  // the unit of the per-root sums (so that a block's fit 32 bits)
 
 // A work item: entries [start, start + cnt) of the row of global vertex u.
 struct __align__(16) BItem {
@@ -939,6 +961,7 @@ struct PArgs {
     LongItem *longs;        // pieces of long rows (bottom-up)
     int vps_shift;          // log2 of the vertices per bottom-up warp step
     GraphSum *sums;         // kRing x ngraphs
+    unsigned long long *rsums;  // kRing x ngraphs x 64: entries of each root's frontier, in kRootEntries
     LevelMeet *meets;       // kRing; kRing levels are cleared at the start of a run
     unsigned *abort;
     uint32_t unit;          // vertices per warp step of the passes over the words (32, 64, ... 256)
@@ -962,12 +985,16 @@ union BWarpScratch {
 struct PShared {
     GraphDesc gd[kMaxGraphs];
     unsigned long long nf[kMaxGraphs], mf[kMaxGraphs], am[kMaxGraphs];  // the block's share of the next frontier
+    uint32_t rs[kMaxGraphs][64];                                        // and of each root's
+    uint64_t td_mask[kMaxGraphs];  // roots that expand top-down
     BWarpScratch w[kSW];
     unsigned long long active, td_entries;
     uint32_t dirs;   // bit 0: a graph expands top-down, bit 1: bottom-up
     uint32_t build;  // some graph's items are to be built
     uint32_t steps;  // bottom-up steps given out
+    uint32_t splits;  // some graph's roots may split
     uint8_t build_g[kMaxGraphs];
+    uint8_t split[kMaxGraphs];  // the graph turns bottom-up with this level
     uint32_t stop;
 };
 
@@ -1017,7 +1044,7 @@ __device__ __forceinline__ void put_rows(BItem *items, uint64_t cap, uint64_t ba
     }
 }
 
-// Top-down over a list of items (those of graphs that have turned bottom-up are
+// Top-down over a list of items (vertices in no top-down root's frontier are
 // passed over): 32 items per warp step, one, or a part of one, as many as it
 // takes to give every warp some.
 template <bool CLAIM>
@@ -1047,8 +1074,9 @@ __device__ __forceinline__ void bexp_items(const PArgs &a, PShared &sh, const BI
             const uint32_t at = (uint32_t)(t & ((1u << split_shift) - 1)) * part;
             s += at;
             cnt = cnt > at ? min(cnt - at, part) : 0u;
-            if (sh.gd[g].dir != TD) cnt = 0;
-            else if (cnt) f = a.b.front[u];
+            if (!sh.td_mask[g]) cnt = 0;
+            if (cnt) f = a.b.front[u] & sh.td_mask[g];
+            if (!f) cnt = 0;
         }
         uint32_t total;
         const uint32_t excl = warp_excl_u32(cnt, total);
@@ -1113,7 +1141,7 @@ __device__ __forceinline__ void bexp_items(const PArgs &a, PShared &sh, const BI
 
 // visited |= next, next -> front, and the sums of the next frontier per graph.
 // A unit idle this level and the last is passed over.
-__device__ __forceinline__ void bcommit(const PArgs &a, PShared &sh, GraphSum *sums)
+__device__ __forceinline__ void bcommit(const PArgs &a, PShared &sh, GraphSum *sums, unsigned long long *rsums)
 {
     constexpr int kK = 8;
     const int lane = g5_lane();
@@ -1121,8 +1149,12 @@ __device__ __forceinline__ void bcommit(const PArgs &a, PShared &sh, GraphSum *s
     const uint64_t units = a.b.ntot / a.unit, nw = (uint64_t)gridDim.x * kSW;
     int cur = -1;
     uint32_t nf = 0;
-    uint64_t mf = 0, am = 0;
+    uint64_t mf = 0, am = 0, r0 = 0, r1 = 0;
     auto flush = [&]() {
+        // (lane l has summed up roots l and l + 32)
+        if (r0) atomicAdd(&sh.rs[cur][lane], (uint32_t)((r0 + kRootEntries - 1) / kRootEntries));
+        if (r1) atomicAdd(&sh.rs[cur][lane + 32], (uint32_t)((r1 + kRootEntries - 1) / kRootEntries));
+        r0 = r1 = 0;
         if (cur >= 0 && __any_sync(0xFFFFFFFFu, nf != 0)) {
             nf = __reduce_add_sync(0xFFFFFFFFu, nf);
             mf = warp_add_u51(mf);
@@ -1171,6 +1203,18 @@ __device__ __forceinline__ void bcommit(const PArgs &a, PShared &sh, GraphSum *s
                 mf += dg[k];
             }
         }
+        if (sh.gd[g].dir != TD || sh.gd[g].nnz < kSplitEntries) continue;
+        // each root's entries, for the split of a first bottom-up level
+#pragma unroll
+        for (int k = 0; k < kK; ++k) {
+            for (unsigned on = __ballot_sync(0xFFFFFFFFu, nx[k] != 0); on; on &= on - 1) {
+                const int l = __ffs(on) - 1;
+                const uint64_t x = __shfl_sync(0xFFFFFFFFu, nx[k], l);
+                const uint32_t d = __shfl_sync(0xFFFFFFFFu, dg[k], l);
+                if ((x >> lane) & 1u) r0 += d;
+                if ((x >> (lane + 32)) & 1u) r1 += d;
+            }
+        }
     }
     flush();
     __syncthreads();
@@ -1181,6 +1225,11 @@ __device__ __forceinline__ void bcommit(const PArgs &a, PShared &sh, GraphSum *s
             atomicOr(&sums[g].amask, sh.am[g]);
         }
         sh.nf[g] = sh.mf[g] = sh.am[g] = 0;
+    }
+    for (int i = threadIdx.x; i < 64 * a.b.ngraphs; i += kSB) {
+        const uint32_t x = (&sh.rs[0][0])[i];
+        if (x) atomicAdd(&rsums[i], (unsigned long long)x);
+        (&sh.rs[0][0])[i] = 0;
     }
     // (pmeet's barrier and fence follow)
 }
@@ -1197,7 +1246,7 @@ __device__ __forceinline__ void bbuild(const PArgs &a, PShared &sh, unsigned lon
         if (!sh.build_g[g]) continue;
         for (uint32_t k = 0; k < a.unit; k += 32) {
             const uint64_t vg = v0 + k + lane;
-            const bool on = a.b.front[vg] != 0;
+            const bool on = (a.b.front[vg] & sh.td_mask[g]) != 0;
             if (!__any_sync(0xFFFFFFFFu, on)) continue;
             const uint32_t d = on ? __ldg(a.b.deg + vg) : 0u, nseg = (d + kItemEntries - 1) / kItemEntries;
             const int64_t s = on ? __ldg(sh.gd[g].row_off + (vg - sh.gd[g].vbase)) : 0;
@@ -1216,7 +1265,7 @@ __global__ void __launch_bounds__(kSB, 1) k_bsearch(const __grid_constant__ PArg
     extern __shared__ __align__(16) unsigned char s_batch[];
     PShared &sh = *reinterpret_cast<PShared *>(s_batch);
     const uint64_t tid = (uint64_t)blockIdx.x * kSB + threadIdx.x, nthr = (uint64_t)gridDim.x * kSB;
-    const int ng = a.b.ngraphs;
+    const int ng = a.b.ngraphs, lane = g5_lane();
     // prologue: empty words, no parents, the graphs' descriptors
     for (uint64_t i = tid; i < 3 * a.b.ntot / 2; i += nthr)
         reinterpret_cast<ulonglong2 *>(a.b.vis)[i] = make_ulonglong2(0, 0);
@@ -1230,6 +1279,8 @@ __global__ void __launch_bounds__(kSB, 1) k_bsearch(const __grid_constant__ PArg
     for (uint32_t i = threadIdx.x; i < ng * sizeof(GraphDesc) / 8; i += kSB)
         reinterpret_cast<uint64_t *>(sh.gd)[i] = __ldcg(reinterpret_cast<const unsigned long long *>(a.gd) + i);
     for (int g = threadIdx.x; g < ng; g += kSB) sh.nf[g] = sh.mf[g] = sh.am[g] = 0;
+    for (int i = threadIdx.x; i < 64 * ng; i += kSB) (&sh.rs[0][0])[i] = 0;
+    for (uint64_t i = tid; i < (uint64_t)kRing * 64 * ng; i += nthr) a.rsums[i] = 0;
     if (threadIdx.x == 0) sh.stop = 0;
     pmeet(a, sh, &a.meets[0].arrive[0]);
     // the roots: into next, their own parents
@@ -1253,12 +1304,15 @@ __global__ void __launch_bounds__(kSB, 1) k_bsearch(const __grid_constant__ PArg
         // level L: expand its frontier (none before level 0), then commit
         LevelMeet *cur = a.meets + (L + kRing) % kRing, *nxt = a.meets + (L + 1) % kRing;
         GraphSum *sums = a.sums + (uint64_t)((L + 1) % kRing) * ng;
+        unsigned long long *rsums = a.rsums + (uint64_t)((L + 1) % kRing) * ng * 64;
         if (L >= 0) {
             // (the records of the level after next)
             if (tid < sizeof(LevelMeet) / 8)
                 reinterpret_cast<unsigned long long *>(a.meets + (L + 2) % kRing)[tid] = 0;
             for (uint64_t i = tid; i < (uint64_t)ng * sizeof(GraphSum) / 8; i += nthr)
                 reinterpret_cast<unsigned long long *>(a.sums + (uint64_t)((L + 2) % kRing) * ng)[i] = 0;
+            for (uint64_t i = tid; i < (uint64_t)ng * 64; i += nthr)
+                a.rsums[(uint64_t)((L + 2) % kRing) * ng * 64 + i] = 0;
             const uint64_t nclaimed = claim ? __ldcg(&cur->alloc) : 0;
             if (sh.build) {
                 bbuild(a, sh, &cur->built);
@@ -1290,14 +1344,14 @@ __global__ void __launch_bounds__(kSB, 1) k_bsearch(const __grid_constant__ PArg
             pmeet(a, sh, &nxt->arrive[0]);
             if (sh.stop) break;
         }
-        bcommit(a, sh, sums);
+        bcommit(a, sh, sums, rsums);
         pmeet(a, sh, L < 0 ? &a.meets[0].arrive[3] : &nxt->arrive[1]);
         if (sh.stop) break;
         // decide, alike in every block: Beamer's switch on the union frontier of
         // the graph's roots
         if (threadIdx.x == 0) {
             sh.active = sh.td_entries = 0;
-            sh.dirs = sh.build = 0;
+            sh.dirs = sh.build = sh.splits = 0;
             sh.steps = kSW;
         }
         __syncthreads();
@@ -1322,6 +1376,9 @@ __global__ void __launch_bounds__(kSB, 1) k_bsearch(const __grid_constant__ PArg
             d.nf = tn;
             d.mf = tm;
             d.amask = __ldcg(&sums[g].amask) & d.mask;
+            sh.td_mask[g] = nd == TD ? ~0ull : 0ull;
+            sh.split[g] = nd == BU && was == TD && d.nnz >= kSplitEntries;
+            if (sh.split[g]) sh.splits = 1;
             const bool build = nd == TD && tn && !(fits && was == TD);
             sh.build_g[g] = build;
             if (tn) {
@@ -1332,6 +1389,29 @@ __global__ void __launch_bounds__(kSB, 1) k_bsearch(const __grid_constant__ PArg
             }
         }
         __syncthreads();
+        for (int g = threadIdx.x >> 5; sh.splits && g < ng; g += kSW) {
+            if (!sh.split[g]) continue;
+            const uint64_t r0 = __ldcg(rsums + 64 * g + lane), r1 = __ldcg(rsums + 64 * g + 32 + lane);
+            const uint64_t all = (uint64_t)sh.gd[g].nnz / kRootEntries;
+            uint64_t most = all / kFewShare, few;
+            for (;; most /= 2) {
+                few = warp_sum_u64((r0 < most ? r0 : 0) + (r1 < most ? r1 : 0));
+                if (few <= all / kFewTotal) break;
+            }
+            const uint64_t mask = __ballot_sync(0xFFFFFFFFu, r0 && r0 < most) |
+                                  (uint64_t)__ballot_sync(0xFFFFFFFFu, r1 && r1 < most) << 32;
+            if (lane == 0 && mask) {
+                sh.td_mask[g] = mask;
+                sh.gd[g].amask &= ~mask;
+                atomicAdd(&sh.td_entries, (unsigned long long)few * kRootEntries);
+                atomicOr(&sh.dirs, 1u);
+                if (!fits) {
+                    sh.build_g[g] = 1;
+                    atomicOr(&sh.build, 1u);
+                }
+            }
+        }
+        if (sh.splits) __syncthreads();
         claim = fits;
         if (sh.active == 0) break;
         if (L + 2 >= kMaxLevels) {
@@ -1497,6 +1577,7 @@ struct g5_batch {
     PArgs pargs;
     BItem *claimed = nullptr;
     uint8_t *live = nullptr;
+    unsigned long long *rsums = nullptr;
     LongItem *longs = nullptr;
     char *stage = nullptr, *h_stage = nullptr;  // descriptors, roots and cleared records of a run
     size_t stage_bytes = 0, roots_at = 0, off_at = 0, zero_at = 0;
@@ -1583,6 +1664,7 @@ void free_batch(g5_batch *b)
     cudaFree(b->scratch);
     cudaFree(b->claimed);
     cudaFree(b->live);
+    cudaFree(b->rsums);
     cudaFree(b->longs);
     cudaFree(b->stage);
     cudaFreeHost(b->h_stage);
@@ -1703,6 +1785,7 @@ g5_status plan_one_launch(g5_batch *b)
     // (a failed call can leave some made: the next one goes on from there)
     if (!b->claimed) G5_CUDA(cudaMalloc(&b->claimed, sizeof(BItem) * 2 * a.claimed_cap));
     if (!b->live) G5_CUDA(cudaMalloc(&b->live, vb / 32));
+    if (!b->rsums) G5_CUDA(cudaMalloc(&b->rsums, sizeof(uint64_t) * kRing * 64 * ng));
     // (a row has a piece per kLongRow entries and one for the rest, and more
     // than kLongRow entries to have any)
     if (!b->longs) G5_CUDA(cudaMalloc(&b->longs, sizeof(LongItem) * (2 * (nnz / kLongRow) + 1)));
@@ -1717,6 +1800,7 @@ g5_status plan_one_launch(g5_batch *b)
     a.sums = reinterpret_cast<GraphSum *>(b->stage + sums_at);
     a.abort = reinterpret_cast<unsigned *>(b->stage + abort_at);
     a.live = b->live;
+    a.rsums = b->rsums;
     a.longs = b->longs;
     a.out = b->h_st;
     // a block per SM, fewer where their warps would have no words or entries

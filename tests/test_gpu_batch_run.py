@@ -96,6 +96,27 @@ def test_long_rows_bottom_up(d):
     check([csr], [roots], directions=((1e12, 1e12), (14.0, 24.0)))
 
 
+@pytest.mark.parametrize("scale,chains", [(12, 3), (13, 40), (14, 62)])
+def test_roots_that_lag(scale, chains):
+    """Roots at the ends of chains hung on a Kronecker graph are levels behind the
+    others when it turns bottom-up, so that they expand top-down in that level;
+    beside it a graph below the least size for that, and one of only such roots."""
+    rng = np.random.default_rng(scale)
+    n, edges, ends = 1 << scale, [orc.kronecker(scale)], []
+    for c in range(chains):
+        length = 1 + c % 5
+        ids = np.concatenate([[rng.integers(0, 1 << scale)], n + np.arange(length)])
+        edges.append(np.stack([ids[:-1], ids[1:]], 1))
+        n += length
+        ends.append(n - 1)
+    csr = orc.build_csr(n, np.concatenate(edges))
+    heads = orc.select_roots(csr[0], 64 - chains)
+    roots = rng.permutation(np.concatenate([heads, ends]))
+    small = random_csr(3000, 20_000, 5)
+    check([csr, small, csr], [roots, rng.integers(0, 3000, 9), ends[:9]],
+          directions=((14.0, 24.0), (200.0, 24.0), (1.0, 1e6)))
+
+
 def test_many_uneven_graphs():
     """64 graphs, some without edges, whose directions change at different levels."""
     rng = np.random.default_rng(4)
