@@ -235,7 +235,8 @@ __device__ __forceinline__ uint64_t warp_or_u64(uint64_t x)
 // parent.  A warp takes 32 consecutive vertices (never two graphs: graphs
 // are chunk aligned).  Each lane first probes v's first kSerial entries with
 // independent loads and keeps the hits as (parent, roots) events in shared
-// memory; vertices still missing roots are then scanned by the whole warp,
+// memory (in the one-launch form again and again while many lanes are short of
+// roots); vertices still missing roots are then scanned by the whole warp,
 // 64 entries per step, whose first hits per root (an exclusive prefix OR over
 // the lanes) are written at once.  The serial hits are written last, lane r
 // taking root r of each vertex: each vertex's parents are one contiguous run
@@ -256,6 +257,13 @@ struct BuScratch {  // one warp's serial hits
 // 220, 242, 244, 244).
 constexpr uint32_t kLongRow = 512;
 
+// While this many lanes are still short of roots they go on by themselves for
+// another kSerial entries: a window of 64 entries takes the warp as long as a
+// round of the lanes, 4 entries each.  us per batch, from 6, 10, 16, 24 and never:
+// scale 24 6511, 6482, 6597, 6713, 6670; scale 20 660, 650, 649, 664, 666; the
+// eight mixed graphs 1125, 1078, 1071, 1078, 1078.
+constexpr int kMany = 12;
+
 // Entries [start, start + cnt) of global vertex u's row, and the roots it is
 // still to be searched for.
 struct __align__(32) LongItem {
@@ -271,6 +279,37 @@ struct LongRows {
     unsigned long long *alloc;
     uint32_t *steps;  // shared: steps the block has given out
 };
+
+// Writes the warp's serial hits: the parents of (vertex, roots) events, two at a
+// time over the warp: lane k writes roots k and k + 32.  Empty events cost
+// nothing, and the events' root sets are disjoint, so each parent is written once.
+__device__ __forceinline__ void put_events(const BArgs &a, const GraphDesc &d, BuScratch &ws, uint32_t vo)
+{
+    const int lane = g5_lane();
+    const uint32_t R = (uint32_t)d.nroots;
+    cp_async_wait_all();
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < kSerial; ++k) {
+        unsigned em = __ballot_sync(0xFFFFFFFFu, ws.evm[k][lane] != 0ull);
+        while (em) {
+            // two events together: their loads overlap
+            const int v0 = __ffs(em) - 1;
+            em &= em - 1;
+            const int v1 = em ? __ffs(em) - 1 : v0;
+            const uint64_t m0 = ws.evm[k][v0], m1 = em ? ws.evm[k][v1] : 0ull;
+            const uint32_t u0 = ws.evu[k][v0], u1 = ws.evu[k][v1];
+            uint32_t *p0 = a.pred + d.pred_base + (uint64_t)__shfl_sync(0xFFFFFFFFu, vo, v0) * R;
+            uint32_t *p1 = a.pred + d.pred_base + (uint64_t)__shfl_sync(0xFFFFFFFFu, vo, v1) * R;
+            em &= em - 1;
+            if ((m0 >> lane) & 1ull) p0[lane] = u0;
+            if ((m0 >> (lane + 32)) & 1ull) p0[lane + 32] = u0;
+            if ((m1 >> lane) & 1ull) p1[lane] = u1;
+            if ((m1 >> (lane + 32)) & 1ull) p1[lane + 32] = u1;
+        }
+    }
+    __syncwarp();
+}
 
 // vps_shift: log2 of the vertices per warp step (32, less on graphs with fewer
 // steps of 32 than there are warps: scale 8 took 84 us at 32 and takes 76).
@@ -316,29 +355,35 @@ __device__ __forceinline__ void bexp_bu(const BArgs &a, const GraphDesc *gd, BuS
         const uint64_t v = d.vbase + vl;
         // roots with an empty frontier cannot reach v
         uint64_t need = dg ? (~a.vis[v] & d.amask) : 0;
-        // serial probes: all loads first, then the hits in adjacency order
-        uint32_t u[kSerial];
-        uint64_t f[kSerial];
-#pragma unroll
-        for (int k = 0; k < kSerial; ++k) u[k] = (need && s + k < e) ? __ldg(d.col + s + k) : 0xFFFFFFFFu;
-#pragma unroll
-        for (int k = 0; k < kSerial; ++k) f[k] = u[k] != 0xFFFFFFFFu ? a.front[d.vbase + u[k]] : 0ull;
-        uint64_t found = 0, sfound = 0;
+        uint64_t found = 0;
         int64_t j = s;
-#pragma unroll
-        for (int k = 0; k < kSerial; ++k) {
-            const uint64_t hit = f[k] & need;
-            ws.evm[k][lane] = hit;
-            // the parent's original id lands in shared memory while the
-            // rest of the row is scanned (read at the write-out below)
-            if (hit) cp_async4(&ws.evu[k][lane], d.orig + u[k]);
-            need &= ~hit;
-            sfound |= hit;
-            if (u[k] != 0xFFFFFFFFu && (need | hit)) j = s + k + 1;
-        }
-        found = sfound;
         const uint32_t vo = (uint32_t)ol;  // original id of v: its parents' row
-        uint64_t ex = (uint64_t)(j - s);
+        uint64_t ex = 0;
+        for (;;) {
+            // serial probes: all loads first, then the hits in adjacency order
+            uint32_t u[kSerial];
+            uint64_t f[kSerial];
+#pragma unroll
+            for (int k = 0; k < kSerial; ++k) u[k] = (need && j + k < e) ? __ldg(d.col + j + k) : 0xFFFFFFFFu;
+#pragma unroll
+            for (int k = 0; k < kSerial; ++k) f[k] = u[k] != 0xFFFFFFFFu ? a.front[d.vbase + u[k]] : 0ull;
+            uint32_t n = 0;  // entries examined
+#pragma unroll
+            for (int k = 0; k < kSerial; ++k) {
+                const uint64_t hit = f[k] & need;
+                ws.evm[k][lane] = hit;
+                // the parent's original id lands in shared memory while the
+                // rest of the row is scanned (read at the write-out below)
+                if (hit) cp_async4(&ws.evu[k][lane], d.orig + u[k]);
+                need &= ~hit;
+                found |= hit;
+                if (u[k] != 0xFFFFFFFFu && (need | hit)) n = k + 1;
+            }
+            j += n;
+            ex += n;
+            if (!SPLIT || __popc(__ballot_sync(0xFFFFFFFFu, need && j < e)) < kMany) break;
+            put_events(a, d, ws, vo);
+        }
         // short rows: pending vertices with at most 64 entries left are
         // packed whole, in lane order, into windows of 64 slots (slots lane
         // and lane + 32); each root's first hit in a row is found with a
@@ -512,32 +557,7 @@ __device__ __forceinline__ void bexp_bu(const BArgs &a, const GraphDesc *gd, BuS
                 ex += (uint64_t)(jj - st);
             }
         }
-        cp_async_wait_all();
-        __syncwarp();
-        // serial hits, one (vertex, parent, roots) event at a time over the
-        // warp: lane k writes roots k and k + 32.  Empty events cost nothing,
-        // and the events' root sets are disjoint, so each parent is written
-        // once.
-#pragma unroll
-        for (int k = 0; k < kSerial; ++k) {
-            unsigned em = __ballot_sync(0xFFFFFFFFu, ws.evm[k][lane] != 0ull);
-            while (em) {
-                // two events together: their loads overlap
-                const int v0 = __ffs(em) - 1;
-                em &= em - 1;
-                const int v1 = em ? __ffs(em) - 1 : v0;
-                const uint64_t m0 = ws.evm[k][v0], m1 = em ? ws.evm[k][v1] : 0ull;
-                const uint32_t u0 = ws.evu[k][v0], u1 = ws.evu[k][v1];
-                uint32_t *p0 = a.pred + d.pred_base + (uint64_t)__shfl_sync(0xFFFFFFFFu, vo, v0) * R;
-                uint32_t *p1 = a.pred + d.pred_base + (uint64_t)__shfl_sync(0xFFFFFFFFu, vo, v1) * R;
-                em &= em - 1;
-                if ((m0 >> lane) & 1ull) p0[lane] = u0;
-                if ((m0 >> (lane + 32)) & 1ull) p0[lane + 32] = u0;
-                if ((m1 >> lane) & 1ull) p1[lane] = u1;
-                if ((m1 >> (lane + 32)) & 1ull) p1[lane + 32] = u1;
-            }
-        }
-        __syncwarp();
+        put_events(a, d, ws, vo);
         // (only this lane writes v in a bottom-up level, unless some roots go top-down)
         if (found) {
             if (SPLIT) atomicOr((unsigned long long *)&a.next[v], (unsigned long long)found);
