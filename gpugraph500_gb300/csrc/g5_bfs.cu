@@ -1329,6 +1329,20 @@ struct Prof {
 
 // ---- workspace --------------------------------------------------------------------
 
+// Searches at a time of a g5_bfs_run_many call of k.  A search leaves most of the
+// GPU's time to its chains of loads, so several on a share of the SMs each finish
+// sooner than one after the other: us per call, one at a time / two / four:
+// 8 roots, 30001 vertices of degree 12, 405 / - / 150; scale 18 - / 252 / 154;
+// 1 M vertices 920 / 832 / 634; scale 20 563 / 385 / 267; 3 M - / 1900 / 1693;
+// scale 22 - / 844 / 845; scale 24 3145 / 2914 / -.  With few long searches the
+// copies of the parents to the host have nothing left to hide behind (4 M
+// vertices, 4 roots 1400 / 1385 / 1431; 8 roots - / 2503 / 2330).
+constexpr int kLanes = 4;
+inline int run_lanes(int64_t n, int k)
+{
+    return std::min(k, n < kGrid2Vertices / 2 || (n < kGrid2Vertices && k >= 2 * kLanes) ? kLanes : 2);
+}
+
 struct g5_bfs {
     g5_graph *g = nullptr;
     g5_bfs_config cfg;
@@ -1372,7 +1386,16 @@ struct g5_bfs {
     cudaGraphExec_t exec2 = nullptr;
     cudaGraph_t graph2 = nullptr;
     cudaStream_t cstream = nullptr;
-    cudaEvent_t searched[2] = {nullptr, nullptr}, copied[2] = {nullptr, nullptr};
+    cudaEvent_t searched[kLanes] = {}, copied[kLanes] = {};
+    // further lanes of g5_bfs_run_many (lane 0 is the workspace itself): what a
+    // search writes, in one allocation, and a stream
+    struct Lane {
+        void *mem = nullptr;
+        int64_t *pred = nullptr;
+        LevelSum *sums = nullptr;
+        cudaStream_t stream = nullptr;
+        SearchArgs args;
+    } lanes[kLanes - 1];
     std::vector<cudaEvent_t> tev;   // start/end of each search of a run_many call
     int64_t *h_roots = nullptr;     // pinned roots of a run_many call
     uint32_t *h_errs = nullptr;     // pinned error flags, one per search
@@ -1490,12 +1513,15 @@ void (*search_kernel(int form))(const SearchArgs)
                                     : k_search<Off, SEARCH_GRID2>;
 }
 
-// Launches the search of `root` on s as one kernel: parents to `pred`, its
-// result to `out` (pinned).
-cudaError_t launch_search(g5_bfs *b, int64_t root, int64_t *pred, SearchState *out, cudaStream_t s, bool async = false)
+// Launches the search of `root` on s as one kernel over the buffers of `args`:
+// parents to `pred`, its result to `out` (pinned).  share: blocks of the grid
+// forms where other searches run beside it (0: it has the GPU to itself).
+cudaError_t launch_search(g5_bfs *b, const SearchArgs &args, int64_t root, int64_t *pred, SearchState *out,
+                          cudaStream_t s, int share = 0)
 {
-    const int form = async ? b->aform : b->sform, grid = async ? b->agrid : b->sgrid;
-    SearchArgs a = b->sargs;
+    const int form = share ? b->aform : b->sform;
+    const int grid = share && form >= SEARCH_GRID1 ? std::min(share, b->sgrid) : b->sgrid;
+    SearchArgs a = args;
     a.root = root;
     a.pred = pred;
     a.out = out;
@@ -1566,14 +1592,48 @@ bool plan_search(g5_bfs *b)
 
 // The search's outcome as the host mirrors hold it; a search that gave up
 // waiting leaves the ring in the middle of a level, so it starts again clean.
-g5_status take_result(g5_bfs *b, const SearchState &r)
+g5_status take_result(g5_bfs *b, const SearchState &r, LevelSum *sums)
 {
     b->h_st->level = r.level;
     b->h_st->err = r.err;
     b->h_st->nvisited = r.nvisited;
     b->h_st->codec_acc[0] = b->h_st->codec_acc[1] = 0;
-    if (r.err & G5_DEVERR_WAIT) G5_CUDA(cudaMemset(b->sums, 0, sizeof(LevelSum) * (kRing + 1)));
+    if (r.err & G5_DEVERR_WAIT) G5_CUDA(cudaMemset(sums, 0, sizeof(LevelSum) * (kRing + 1)));
     return G5_OK;
+}
+
+// Makes lane i of g5_bfs_run_many; false if there is no memory for it.
+bool open_lane(g5_bfs *b, int i)
+{
+    g5_bfs::Lane &l = b->lanes[i];
+    if (l.stream) return true;
+    const SearchArgs &sa = b->sargs;
+    auto align = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const size_t pred = align(sizeof(int64_t) * (size_t)sa.n), bitmaps = align(sizeof(uint32_t) * 4 * sa.stride),
+                 items = align(sizeof(Item) * (2 * sa.claimed_cap + sa.built_cap)),
+                 sums = align(sizeof(LevelSum) * (kRing + 1)), log = sizeof(LevelRec) * (size_t)sa.max_levels;
+    if (!l.mem && cudaMalloc(&l.mem, pred + bitmaps + items + sums + log) != cudaSuccess) {
+        cudaGetLastError();
+        l.mem = nullptr;
+        return false;
+    }
+    char *p = static_cast<char *>(l.mem);
+    l.args = sa;
+    l.pred = reinterpret_cast<int64_t *>(p);
+    l.args.bitmaps = reinterpret_cast<uint32_t *>(p += pred);
+    l.args.claimed[0] = reinterpret_cast<Item *>(p += bitmaps);
+    l.args.claimed[1] = l.args.claimed[0] + sa.claimed_cap;
+    l.args.built = l.args.claimed[1] + sa.claimed_cap;
+    l.args.sums = l.sums = reinterpret_cast<LevelSum *>(p += items);
+    l.args.ring = reinterpret_cast<unsigned *>(l.sums + kRing);
+    l.args.log = reinterpret_cast<LevelRec *>(p += sums);
+    if (cudaMemset(l.sums, 0, sizeof(LevelSum) * (kRing + 1)) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking) != cudaSuccess) {
+        cudaGetLastError();
+        l.stream = nullptr;
+        return false;
+    }
+    return true;
 }
 
 // Status of a search without codec from its error bits.
@@ -1624,8 +1684,8 @@ g5_status alloc_ws(g5_bfs *b)
         sa.tile_shift = std::max(a.tile_shift, kMinItemShift);
         const uint64_t tiles = (uint64_t)g->nnz >> sa.tile_shift;
         sa.claimed_cap = std::min<uint64_t>(std::min<uint64_t>(n, kClaimMax) + tiles + 1, kClaimedItems);
-        const size_t built = (size_t)n + tiles + 1;
-        G5_CUDA(cudaMalloc(&b->items, sizeof(Item) * (2 * sa.claimed_cap + built)));
+        sa.built_cap = (uint64_t)n + tiles + 1;
+        G5_CUDA(cudaMalloc(&b->items, sizeof(Item) * (2 * sa.claimed_cap + sa.built_cap)));
         sa.claimed[0] = b->items;
         sa.claimed[1] = b->items + sa.claimed_cap;
         sa.built = b->items + 2 * sa.claimed_cap;
@@ -1751,7 +1811,11 @@ void free_ws(g5_bfs *b)
     if (b->graph2) cudaGraphDestroy(b->graph2);
     cudaFree(b->pred2);
     if (b->cstream) cudaStreamDestroy(b->cstream);
-    for (int i = 0; i < 2; ++i) {
+    for (g5_bfs::Lane &l : b->lanes) {
+        if (l.stream) cudaStreamDestroy(l.stream);
+        cudaFree(l.mem);
+    }
+    for (int i = 0; i < kLanes; ++i) {
         if (b->searched[i]) cudaEventDestroy(b->searched[i]);
         if (b->copied[i]) cudaEventDestroy(b->copied[i]);
     }
@@ -1917,7 +1981,7 @@ g5_status g5_bfs_run(g5_bfs *b, int64_t root, int64_t *pred_out, int32_t *level_
     b->prof.on = b->cfg.profile && !b->exec && !b->one;
     b->prof.used = 0;
     if (b->one) {
-        G5_CUDA(launch_search(b, root, b->pred, b->h_out, s));
+        G5_CUDA(launch_search(b, b->sargs, root, b->pred, b->h_out, s));
     } else if (b->exec) {
         G5_CUDA(cudaGraphLaunch(b->exec, s));
     } else {
@@ -1943,7 +2007,7 @@ g5_status g5_bfs_run(g5_bfs *b, int64_t root, int64_t *pred_out, int32_t *level_
     b->ran = true;
     b->last_root = root;
     b->cur_pred = b->pred;
-    if (b->one) G5_TRY(take_result(b, *b->h_out));
+    if (b->one) G5_TRY(take_result(b, *b->h_out, b->sums));
     const BfsState &hs = *b->h_st;
     g5_status rc = G5_OK;
     if (hs.err) rc = search_status(hs.err);
@@ -2022,7 +2086,7 @@ g5_status g5_bfs_launch(g5_bfs *b, int64_t root)
     cudaStream_t s = b->stream;
     if (b->one) {
         G5_CUDA(cudaEventRecord(b->ev0, s));
-        G5_CUDA(launch_search(b, root, b->pred, b->h_out, s, true));
+        G5_CUDA(launch_search(b, b->sargs, root, b->pred, b->h_out, s, b->agrid));
         G5_CUDA(cudaEventRecord(b->ev1, s));
         b->ran = true;
         b->last_root = root;
@@ -2056,7 +2120,7 @@ g5_status g5_bfs_poll(g5_bfs *b, int *done, double *device_ms)
         cudaEventElapsedTime(&ms, b->ev0, b->ev1);
         *device_ms = ms;
     }
-    if (b->one && b->ran) G5_TRY(take_result(b, *b->h_out));
+    if (b->one && b->ran) G5_TRY(take_result(b, *b->h_out, b->sums));
     return search_status(b->h_st->err);
 }
 
@@ -2076,11 +2140,14 @@ g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const
     }
     const int64_t n = b->g->n;
     cudaStream_t s = b->stream;
+    int lanes = 1;
+    if (b->one && !b->level)
+        while (lanes < run_lanes(n, k) && open_lane(b, lanes - 1)) ++lanes;
     // first use: the second parent buffer (and its graph), the copy stream, events
-    if (!b->pred2) G5_CUDA(cudaMalloc(&b->pred2, sizeof(int64_t) * (size_t)n));
+    if (lanes == 1 && !b->pred2) G5_CUDA(cudaMalloc(&b->pred2, sizeof(int64_t) * (size_t)n));
     if (!b->one && !b->exec2) G5_TRY(build_graph(b, b->pred2, &b->exec2, &b->graph2));
     if (!b->cstream) G5_CUDA(cudaStreamCreateWithFlags(&b->cstream, cudaStreamNonBlocking));
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < kLanes; ++i) {
         if (!b->searched[i]) G5_CUDA(cudaEventCreateWithFlags(&b->searched[i], cudaEventDisableTiming));
         if (!b->copied[i]) G5_CUDA(cudaEventCreateWithFlags(&b->copied[i], cudaEventDisableTiming));
     }
@@ -2111,15 +2178,46 @@ g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const
         b->h_roots[i] = roots[i];
         b->h_errs[i] = 0;
     }
+    if (lanes > 1) {
+        const int share = std::max(1, 2 * g5::num_sms() / lanes);
+        // the last search in lane 0, whose parents and level log are the
+        // workspace's; the others' copies follow `lanes` launches behind, as
+        // one to pageable memory holds up this thread
+        auto lane_of = [&](int i) { return (k - 1 - i) % lanes; };
+        auto search = [&](int i) -> g5_status {
+            const int l = lane_of(i);
+            const cudaStream_t ls = l ? b->lanes[l - 1].stream : s;
+            if (device_ms) G5_CUDA(cudaEventRecord(b->tev[2 * i], ls));
+            G5_CUDA(launch_search(b, l ? b->lanes[l - 1].args : b->sargs, roots[i], l ? b->lanes[l - 1].pred : b->pred,
+                                  b->h_outs + i, ls, share));
+            if (device_ms) G5_CUDA(cudaEventRecord(b->tev[2 * i + 1], ls));
+            G5_CUDA(cudaEventRecord(b->searched[l], ls));
+            return G5_OK;
+        };
+        G5_CUDA(cudaEventRecord(b->copied[0], s));
+        for (int l = 1; l < lanes; ++l) G5_CUDA(cudaStreamWaitEvent(b->lanes[l - 1].stream, b->copied[0], 0));
+        for (int i = 0; i < lanes; ++i) G5_TRY(search(i));
+        for (int i = 0; i < k; ++i) {
+            const int l = lane_of(i);
+            G5_CUDA(cudaStreamWaitEvent(b->cstream, b->searched[l], 0));
+            if (pred_out && pred_out[i])
+                G5_CUDA(cudaMemcpyAsync(pred_out[i], l ? b->lanes[l - 1].pred : b->pred, sizeof(int64_t) * (size_t)n,
+                                        cudaMemcpyDefault, b->cstream));
+            if (i + lanes >= k) continue;
+            G5_CUDA(cudaEventRecord(b->copied[l], b->cstream));
+            G5_CUDA(cudaStreamWaitEvent(l ? b->lanes[l - 1].stream : s, b->copied[l], 0));
+            G5_TRY(search(i + lanes));
+        }
+    }
     // search i writes buffer i % 2 on the search stream while the copy stream
     // moves search i - 1's parents out; search i + 2 waits for that copy
-    for (int i = 0; i < k; ++i) {
+    for (int i = 0; i < k && lanes == 1; ++i) {
         const int slot = i & 1;
         if (i >= 2) G5_CUDA(cudaStreamWaitEvent(s, b->copied[slot], 0));
         if (!b->one)
             G5_CUDA(cudaMemcpyAsync(b->root_dev, b->h_roots + i, sizeof(int64_t), cudaMemcpyHostToDevice, s));
         if (device_ms) G5_CUDA(cudaEventRecord(b->tev[2 * i], s));
-        if (b->one) G5_CUDA(launch_search(b, roots[i], buf[slot], b->h_outs + i, s));
+        if (b->one) G5_CUDA(launch_search(b, b->sargs, roots[i], buf[slot], b->h_outs + i, s));
         else G5_CUDA(cudaGraphLaunch(ex[slot], s));
         if (device_ms) G5_CUDA(cudaEventRecord(b->tev[2 * i + 1], s));
         if (!b->one)
@@ -2136,7 +2234,7 @@ g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const
     if (k) {
         b->ran = true;
         b->last_root = roots[k - 1];
-        b->cur_pred = buf[(k - 1) & 1];
+        b->cur_pred = lanes > 1 ? b->pred : buf[(k - 1) & 1];
         if (!b->one) G5_CUDA(cudaMemcpy(b->h_st, b->st, sizeof(BfsState), cudaMemcpyDeviceToHost));
     }
     g5_status rc = G5_OK;
@@ -2146,7 +2244,8 @@ g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const
             cudaEventElapsedTime(&ms, b->tev[2 * i], b->tev[2 * i + 1]);
             device_ms[i] = ms;
         }
-        if (b->one) G5_TRY(take_result(b, b->h_outs[i]));
+        const int l = lanes > 1 ? (k - 1 - i) % lanes : 0;
+        if (b->one) G5_TRY(take_result(b, b->h_outs[i], l ? b->lanes[l - 1].sums : b->sums));
         if (rc == G5_OK) rc = search_status(b->one ? b->h_outs[i].err : b->h_errs[i]);
     }
     return rc;

@@ -228,6 +228,7 @@ struct SearchArgs {
     Item *claimed[2];          // work items of claimed frontiers, by level parity
     uint64_t claimed_cap;
     Item *built;               // work items of a frontier built from its bitmap (room for any)
+    uint64_t built_cap;
     LevelSum *sums;            // the ring
     unsigned *ring;            // [0] its place of the next search's level 0, [1] set by a block that gave up waiting
     struct SearchState *out;   // pinned host: the search's result

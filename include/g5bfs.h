@@ -216,8 +216,11 @@ g5_status g5_bfs_poll(g5_bfs *b, int *done, double *device_ms);
  * give the same results.  device_ms (nullable, k entries) receives each
  * search's device time.  Same parents as g5_bfs_run root by root; afterwards
  * g5_bfs_device_pred, g5_bfs_teps_edges and g5_bfs_validate refer to the
- * last root.  The first call allocates the second parent buffer (8n bytes)
- * and builds its CUDA graph. */
+ * last root.  Where a search is one launch and needs no levels, two to four run
+ * at a time (a search's device time is then its share of the GPU's); the first
+ * call allocates what each writes (25n bytes and a sixteenth of the edges), or
+ * searches one at a time if there is no memory for it.  Else it allocates the
+ * second parent buffer (8n bytes) and builds its CUDA graph. */
 g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const *pred_out, double *device_ms);
 
 /* Per-level record of the last search, 4 int64 per level: direction
