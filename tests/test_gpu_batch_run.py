@@ -150,3 +150,33 @@ def test_level_cap():
     assert np.array_equal(out.cpu().numpy().view(np.uint32), oracle_u32(*csr, 600))
     bt.close()
     g.close()
+
+
+def test_degree_past_24_bits():
+    """A star of 2^24 + 2 leaves: the hub's record holds no degree."""
+    leaves = (1 << 24) + 2
+    n = leaves + 1
+    ro = np.concatenate([[0], leaves + np.arange(n)]).astype(np.int64)
+    col = np.concatenate([np.arange(1, n), np.zeros(leaves)]).astype(np.uint32)
+    g = g5.Graph.from_csr(ro, col)
+    bt = g5.Batch([g])
+    roots = np.array([0, 1, leaves], np.int64)
+    out = torch.empty(3 * n, dtype=torch.int32, device="cuda")
+    for alpha in (1e12, 14.0):
+        bt.set_direction(alpha, 1e12 if alpha > 100 else 24.0)
+        for graph_loop in (False, True):
+            out.fill_(7)
+            torch.cuda.synchronize()
+            if graph_loop:
+                bt.launch(roots, [3], out)
+                assert bt.poll(wait=True)[0]
+            else:
+                assert bt.run(roots, [3], out) > 0
+            got = out.view(n, 3)
+            for j, r in enumerate(roots):
+                want = torch.zeros(n, dtype=torch.int32, device="cuda")
+                want[int(r)] = int(r)
+                want[0] = int(r)
+                assert torch.equal(got[:, j], want), (alpha, graph_loop, j)
+    bt.close()
+    g.close()
