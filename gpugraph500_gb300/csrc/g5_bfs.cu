@@ -1336,10 +1336,14 @@ struct Prof {
 // 1 M vertices 920 / 832 / 634; scale 20 563 / 385 / 267; 3 M - / 1900 / 1693;
 // scale 22 - / 844 / 845; scale 24 3145 / 2914 / -.  With few long searches the
 // copies of the parents to the host have nothing left to hide behind (4 M
-// vertices, 4 roots 1400 / 1385 / 1431; 8 roots - / 2503 / 2330).
+// vertices, 4 roots 1400 / 1385 / 1431; 8 roots - / 2503 / 2330); on the largest
+// graphs they take longer than the searches, whose pairs only start them later
+// (scale 26, 16 roots, 2856 / 2883 us a search).
 constexpr int kLanes = 4;
-inline int run_lanes(int64_t n, int k)
+constexpr int64_t kCopyBound = 1 << 24;
+inline int run_lanes(int64_t n, int k, bool to_host)
 {
+    if (to_host && n >= kCopyBound) return 1;
     return std::min(k, n < kGrid2Vertices / 2 || (n < kGrid2Vertices && k >= 2 * kLanes) ? kLanes : 2);
 }
 
@@ -2141,8 +2145,12 @@ g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const
     const int64_t n = b->g->n;
     cudaStream_t s = b->stream;
     int lanes = 1;
-    if (b->one && !b->level)
-        while (lanes < run_lanes(n, k) && open_lane(b, lanes - 1)) ++lanes;
+    if (b->one && !b->level) {
+        bool to_host = false;
+        for (int i = 0; i < k && pred_out && n >= kCopyBound; ++i)
+            to_host = to_host || (pred_out[i] && !g5::is_device_ptr(pred_out[i]));
+        while (lanes < run_lanes(n, k, to_host) && open_lane(b, lanes - 1)) ++lanes;
+    }
     // first use: the second parent buffer (and its graph), the copy stream, events
     if (lanes == 1 && !b->pred2) G5_CUDA(cudaMalloc(&b->pred2, sizeof(int64_t) * (size_t)n));
     if (!b->one && !b->exec2) G5_TRY(build_graph(b, b->pred2, &b->exec2, &b->graph2));
