@@ -538,8 +538,8 @@ def main():
             # p99 and GTEPS of every mode at every offered rate
             line["p99_query_ms_by_rate"] = {m: {str(int(r["rate_qps"])): {"p99_ms": r["p99_ms"], "gteps": r["gteps"]}
                                                 for r in serve[m]["rates"]} for m in modes}
-        # per search: k_init + (k_td, k_bu, k_count, k_write) per level
-        line["gpu_launches"] = sum(1 + 4 * rec[3] for rec in recs)
+        # a search is one launch (k_search); host-driven, k_init and k_td, k_bu, k_count, k_write per level
+        line["gpu_launches"] = sum(1 + 4 * rec[3] if args.host_loop else 1 for rec in recs)
         print(json.dumps(line))
     bfs.close()
     g.close()

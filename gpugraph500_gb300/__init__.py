@@ -439,7 +439,7 @@ class Codec:
 
     def encode_batch(self, in_dev, in_off: np.ndarray, out_dev, raw_threshold: int = 0, mode: int = CODEC_D4,
                      stream=None) -> tuple[np.ndarray, np.ndarray]:
-        """Encodes k concatenated queues in one launch set; returns (out_off, out_words)."""
+        """Encodes k concatenated queues in one launch; returns (out_off, out_words)."""
         in_off = np.ascontiguousarray(in_off, dtype=np.uint64)
         k = len(in_off) - 1
         out_off = np.zeros(k + 1, np.uint64)
@@ -450,7 +450,7 @@ class Codec:
 
     def decode_batch(self, in_dev, in_off: np.ndarray, words: np.ndarray, n: np.ndarray, out_dev,
                      raw_threshold: int = 0, mode: int = CODEC_D4, stream=None) -> tuple[np.ndarray, np.ndarray]:
-        """Decodes k streams in one launch set; returns (out_off, per-stream ok flags).
+        """Decodes k streams in one launch; returns (out_off, per-stream ok flags).
         Raises G5Error if a stream is malformed (the flags say which)."""
         in_off = np.ascontiguousarray(in_off, dtype=np.uint64)
         words = np.ascontiguousarray(words, dtype=np.uint64)

@@ -1,5 +1,6 @@
 // g5_batch.cu -- batched BFS: up to 64 roots per graph, any number of graphs
-// of uneven scale, all in one device-resident level loop.
+// of uneven scale, all together: g5_batch_run as one launch (k_bsearch), the
+// asynchronous and serving forms in a device-resident level loop.
 //
 // Each vertex carries three 64-bit words (one bit per root of its graph):
 // visited, frontier and next-frontier.  One read of a vertex's adjacency
@@ -32,7 +33,7 @@
 //
 // Vertex ranges of the graphs are padded to whole compaction chunks so every
 // chunk belongs to one graph; the level loop is one CUDA graph (conditional
-// while node) like the plain search.
+// while node).
 #include <cub/cub.cuh>
 
 #include <algorithm>

@@ -1577,8 +1577,8 @@ bool plan_search(g5_bfs *b)
         // workspaces: two grids of half the blocks serve more queries than one
         // that has every SM to itself (us per query of a full server, a grid of
         // 304 or 152 exclusive blocks / this rule / the level graph before:
-        // scale 16 38 / 13 / 44, 20 84 / 43 / 69, 22 150 / 115 / 124, 24 380 /
-        // 328 / 337); below kGrid2Vertices half the SMs cost a lone query
+        // scale 16 38 / 13 / 44, 20 84 / 32 / 69, 22 150 / 99 / 124, 24 380 /
+        // 309 / 337); below kGrid2Vertices half the SMs cost a lone query
         // nothing that the server's polling shows, above they do (scale 24
         // 757 us against 460)
         b->aform = form;

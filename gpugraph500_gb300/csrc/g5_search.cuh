@@ -7,8 +7,8 @@
 // 2000 entries take none of that).  What a level costs now is its chain of
 // dependent loads and one meeting: 1-3 us in a block, 2-5 in a cluster, 3-8
 // over the grid.  Device time per search, before and after (thresholds at
-// their defaults, scale 26 with the tuned ones): scale 10 108 -> 24 us,
-// 16 164 -> 49, 20 193 -> 79, 22 280 -> 160, 24 619 -> 422, 26 1451 -> 1244.
+// their defaults): scale 10 108 -> 22 us, 16 164 -> 44, 20 193 -> 70, 22 280 ->
+// 147, 24 619 -> 392, 26 (tuned) 1451 -> 1187.
 // Four forms (enum below), by the graph's size: see search_form().
 //
 // The level's result is accounted while it is produced, so no counting or
@@ -157,14 +157,14 @@ enum { SEARCH_BLOCK, SEARCH_CLUSTER, SEARCH_GRID1, SEARCH_GRID2 };
 
 // The form for a graph, and where each pays (us per search, mean of 8 roots):
 //             block  cluster  grid1  grid2
-//   scale 10   23.9    27.8    33.4   43.2    few vertices: no latency beyond
-//   scale 11   26.8    30.2    34.9   45.1    the block's own shared memory
-//   scale 12   36.3    31.0    40.9   52.7    16 SMs, the hardware barrier
-//   scale 15   93.4    40.6    42.4   55.2
-//   scale 16  178.9    52.6    48.5   62.8    the whole GPU's loads in flight
-//   scale 21                   96.9  112.9
-//   scale 22                  165.2  159.5    the sweeps outweigh the meetings
-//   scale 24                  507.6  421.6
+//   scale 10   22.3    27.5    32.4   42.2    few vertices: no latency beyond
+//   scale 11   25.8    28.9    33.9   44.2    the block's own shared memory
+//   scale 12   33.6    28.9    36.7   50.4    16 SMs, the hardware barrier
+//   scale 15           38.1    38.7   52.4
+//   scale 16           47.5    43.6   58.2    the whole GPU's loads in flight
+//   scale 21                   88.4  100.6
+//   scale 22                  156.3  146.8    the sweeps outweigh the meetings
+//   scale 24                  482.6  391.5
 constexpr int64_t kBlockVertices = 1 << 12, kBlockEntries = 1 << 16;
 constexpr int64_t kClusterVertices = 1 << 15, kClusterEntries = 1 << 20;
 constexpr int64_t kGrid2Vertices = 1 << 22;

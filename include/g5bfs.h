@@ -435,7 +435,7 @@ g5_status g5_codec_decode_async(g5_codec *c, const uint32_t *in_dev, const uint6
                                 size_t out_cap, uint64_t *out_n_dev, int mode, void *stream);
 g5_status g5_codec_status(g5_codec *c);
 
-/* Many queues per call, one launch set for all of them (the reference's
+/* Many queues per call, one launch for all of them (the reference's
  * compress/decompress run once per queue, vreduce.hpp:192-528,
  * globalbfs.hh:853-938; a level's queues or a microbench's queue set go
  * through the GPU together).  The streams are byte for byte those of
