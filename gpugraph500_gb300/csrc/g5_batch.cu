@@ -923,10 +923,10 @@ __global__ void __launch_bounds__(kB, 4) k_bwrite(BArgs a)
 //
 // Five launches and a while node a level cost about 35 us whatever the level
 // held; a level now costs its work and 6-8 us.  Device us per batch of Kronecker
-// graphs, 16 edges a vertex, before and after: scale 8, 4 roots, 230 and 70;
-// scale 13, 64 roots, 410 and 134; scale 16 479 and 226; scale 20 1281 and 662;
-// scale 24 10267 and 6667; eight graphs of scales 14 to 20, 16 roots each, 1820
-// and 1070.  What bounds it: the bottom-up sweeps, half by instructions and half
+// graphs, 16 edges a vertex, before and after: scale 8, 4 roots, 230 and 71;
+// scale 13, 64 roots, 410 and 138; scale 16 479 and 230; scale 20 1281 and 627;
+// scale 24 10267 and 6140; eight graphs of scales 14 to 20, 16 roots each, 1820
+// and 890.  What bounds it: the bottom-up sweeps, half by instructions and half
 // by the latency of their gathers (39 % of the issue slots, 39 % of the memory
 // bandwidth at 64 registers, which two windows of loads and 64-bit roots need;
 // 48 registers and a quarter more warps measured slower).
@@ -1072,17 +1072,20 @@ __device__ __forceinline__ void bexp_items(const PArgs &a, PShared &sh, const BI
     const int lane = g5_lane();
     TdScratch &ws = sh.w[threadIdx.x >> 5].td;
     const uint64_t gw = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, nw = (uint64_t)gridDim.x * kSW;
-    uint32_t ipw_shift = 0, split_shift = 0;
-    while (ipw_shift < 5 && nitems > (nw << ipw_shift)) ++ipw_shift;
+    const uint32_t ipw = items_per_step(nitems, (uint32_t)nw);
+    uint32_t split_shift = 0;
     while (split_shift < 3 && (nitems << (split_shift + 1)) <= nw) ++split_shift;
-    const uint64_t units = ((nitems << split_shift) + (1u << ipw_shift) - 1) >> ipw_shift;
+    const uint64_t units = ipw == 1 ? nitems << split_shift : item_steps(nitems, ipw);
     for (uint64_t t = gw; t < units; t += nw) {
-        const uint64_t i = ((t << ipw_shift) >> split_shift) + lane;
+        // a step's items lie apart, so that each has its share of the hubs',
+        // which come first (taken in order, 32 a step: scale 22 1892 us a batch
+        // and 1760 so, the eight mixed graphs 1059 and 890)
+        const uint64_t i = ipw == 1 ? (t >> split_shift) + lane : t + lane * units;
         uint32_t cnt = 0, u = 0;
         int g = 0;
         int64_t s = 0;
         uint64_t f = 0;
-        if ((uint32_t)lane < (1u << ipw_shift) && i < nitems) {
+        if ((uint32_t)lane < ipw && i < nitems) {
             const uint4 raw = __ldcg(reinterpret_cast<const uint4 *>(items + i));
             u = raw.x;
             g = (int)(raw.y >> 16);
@@ -1114,7 +1117,7 @@ __device__ __forceinline__ void bexp_items(const PArgs &a, PShared &sh, const BI
             int gv = 0;
             if (x < total) {
                 int lo = 0;
-                if (ipw_shift) {
+                if (ipw > 1) {
                     int hi = 31;
                     while (lo < hi) {
                         const int mid = (lo + hi) >> 1;

@@ -216,3 +216,20 @@ __device__ __forceinline__ bool below_quotient(uint64_t x, uint64_t y, double c)
     if (l > r * 1.00001f) return false;
     return (double)x < (double)y / c;
 }
+
+// Work items per warp step of a list of nitems over nw warps: the fewest steps of
+// at most 32 items, all warps alike.  (Lists of 2^32 items and more, which no
+// graph in 280 GB has, are cut as if they were shorter; 64-bit divisions are a
+// call.)
+__device__ __forceinline__ uint32_t items_per_step(uint64_t nitems, uint32_t nw)
+{
+    if (nitems <= nw) return 1u;
+    const uint32_t per = (uint32_t)min(nitems, (uint64_t)0xFFFFFFFFu) / nw + 1, steps = (per + 31) / 32;
+    return (per + steps - 1) / steps;
+}
+
+// Steps of ipw items that a list of nitems makes.
+__device__ __forceinline__ uint64_t item_steps(uint64_t nitems, uint32_t ipw)
+{
+    return nitems >> 32 ? nitems : ((uint32_t)nitems - 1) / ipw + 1;
+}

@@ -427,15 +427,15 @@ __device__ __forceinline__ void search_td(const SearchArgs &a, SearchShared &sh,
     // neighbouring warps of the work order sit in different blocks
     const uint64_t gw = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
     const uint64_t nw = (uint64_t)gridDim.x * kSW;
-    uint32_t ipw_shift = 0, split_shift = 0;
-    while (ipw_shift < 5 && nitems > (nw << ipw_shift)) ++ipw_shift;
+    const uint32_t ipw = items_per_step(nitems, (uint32_t)nw);
+    uint32_t split_shift = 0;
     while ((5 + (int)split_shift) < a.tile_shift && (nitems << (split_shift + 1)) <= nw) ++split_shift;
-    const uint32_t ipw = 1u << ipw_shift;
     uint32_t nf = 0;
     uint64_t mf = 0;
-    const uint64_t units = ((nitems << split_shift) + ipw - 1) >> ipw_shift;
+    const uint64_t units = ipw == 1 ? nitems << split_shift : item_steps(nitems, ipw);
     for (uint64_t t = gw; t < units; t += nw) {
-        const uint64_t i = ((t << ipw_shift) >> split_shift) + lane;
+        // (a step's items lie apart, so that each has its share of the hubs')
+        const uint64_t i = ipw == 1 ? (t >> split_shift) + lane : t + lane * units;
         uint32_t cnt = 0, u = 0;
         int64_t s = 0;
         if ((uint32_t)lane < ipw && i < nitems) {
