@@ -1139,9 +1139,25 @@ __device__ __forceinline__ void bexp_items(const PArgs &a, PShared &sh, const BI
                 if (nb) {
                     const uint32_t ul = ws.u[lo];
                     uint32_t *pv = a.b.pred + d.pred_base + (uint64_t)vo * d.nroots;
-                    for (uint64_t y = nb; y; y &= y - 1) {
-                        uint32_t *slot = pv + (__ffsll((long long)y) - 1);
-                        if (CLAIM || *slot > ul) atomicMin(slot, ul);
+                    if (CLAIM) {
+                        for (uint64_t y = nb; y; y &= y - 1) atomicMin(pv + (__ffsll((long long)y) - 1), ul);
+                    } else {
+                        // the slots are read first: most hold a smaller parent
+                        // already; four at a time (scale 20 630 -> 619 us a
+                        // batch, 22 1744 -> 1725, against one after another)
+                        for (uint64_t y = nb; y;) {
+                            uint32_t r[4], x[4];
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                r[q] = y ? (uint32_t)(__ffsll((long long)y) - 1) : 64u;
+                                y &= y - 1;
+                            }
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) x[q] = r[q] < 64 ? pv[r[q]] : 0u;
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                                if (x[q] > ul) atomicMin(pv + r[q], ul);
+                        }
                     }
                     if (CLAIM) claimed = atomicOr((unsigned long long *)&a.b.next[vg], (unsigned long long)nb) == 0;
                     else if (nb & ~a.b.next[vg]) atomicOr((unsigned long long *)&a.b.next[vg], (unsigned long long)nb);
