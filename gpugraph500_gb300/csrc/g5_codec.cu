@@ -630,6 +630,9 @@ __device__ __forceinline__ DecHead dec_head(const uint32_t *in, uint64_t words, 
         h.n1 = x.x;
         if (x.y != kCookie || x.z != kCookie || x.w != kCookie) h.bad = true;
         if (h.n1 % 128 || h.n1 > cap || h.n1 / 128 >= max_mb) h.bad = true;
+        // groups but no vector that could hold one's header: there is no chunk
+        // that would find the chain broken
+        if (h.n1 && h.nv < 2) h.bad = true;
     }
     if (h.nv > max_vec) h.bad = true;
     if (h.bad) h.n1 = 0;
