@@ -1595,14 +1595,15 @@ bool plan_search(g5_bfs *b)
 }
 
 // The search's outcome as the host mirrors hold it; a search that gave up
-// waiting leaves the ring in the middle of a level, so it starts again clean.
-g5_status take_result(g5_bfs *b, const SearchState &r, LevelSum *sums)
+// waiting leaves the ring in the middle of a level, so it starts again clean
+// (cleared on `s`, the stream its next search runs on).
+g5_status take_result(g5_bfs *b, const SearchState &r, LevelSum *sums, cudaStream_t s)
 {
     b->h_st->level = r.level;
     b->h_st->err = r.err;
     b->h_st->nvisited = r.nvisited;
     b->h_st->codec_acc[0] = b->h_st->codec_acc[1] = 0;
-    if (r.err & G5_DEVERR_WAIT) G5_CUDA(cudaMemset(sums, 0, sizeof(LevelSum) * (kRing + 1)));
+    if (r.err & G5_DEVERR_WAIT) G5_CUDA(cudaMemsetAsync(sums, 0, sizeof(LevelSum) * (kRing + 1), s));
     return G5_OK;
 }
 
@@ -1631,12 +1632,15 @@ bool open_lane(g5_bfs *b, int i)
     l.args.sums = l.sums = reinterpret_cast<LevelSum *>(p += items);
     l.args.ring = reinterpret_cast<unsigned *>(l.sums + kRing);
     l.args.log = reinterpret_cast<LevelRec *>(p += sums);
-    if (cudaMemset(l.sums, 0, sizeof(LevelSum) * (kRing + 1)) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking) != cudaSuccess) {
+    // (cleared on the lane's own stream: no search waits for the default one)
+    cudaStream_t s = nullptr;
+    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaMemsetAsync(l.sums, 0, sizeof(LevelSum) * (kRing + 1), s) != cudaSuccess) {
         cudaGetLastError();
-        l.stream = nullptr;
+        if (s) cudaStreamDestroy(s);
         return false;
     }
+    l.stream = s;
     return true;
 }
 
@@ -2011,7 +2015,7 @@ g5_status g5_bfs_run(g5_bfs *b, int64_t root, int64_t *pred_out, int32_t *level_
     b->ran = true;
     b->last_root = root;
     b->cur_pred = b->pred;
-    if (b->one) G5_TRY(take_result(b, *b->h_out, b->sums));
+    if (b->one) G5_TRY(take_result(b, *b->h_out, b->sums, s));
     const BfsState &hs = *b->h_st;
     g5_status rc = G5_OK;
     if (hs.err) rc = search_status(hs.err);
@@ -2124,7 +2128,7 @@ g5_status g5_bfs_poll(g5_bfs *b, int *done, double *device_ms)
         cudaEventElapsedTime(&ms, b->ev0, b->ev1);
         *device_ms = ms;
     }
-    if (b->one && b->ran) G5_TRY(take_result(b, *b->h_out, b->sums));
+    if (b->one && b->ran) G5_TRY(take_result(b, *b->h_out, b->sums, b->stream));
     return search_status(b->h_st->err);
 }
 
@@ -2253,7 +2257,8 @@ g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const
             device_ms[i] = ms;
         }
         const int l = lanes > 1 ? (k - 1 - i) % lanes : 0;
-        if (b->one) G5_TRY(take_result(b, b->h_outs[i], l ? b->lanes[l - 1].sums : b->sums));
+        if (b->one)
+            G5_TRY(take_result(b, b->h_outs[i], l ? b->lanes[l - 1].sums : b->sums, l ? b->lanes[l - 1].stream : s));
         if (rc == G5_OK) rc = search_status(b->one ? b->h_outs[i].err : b->h_errs[i]);
     }
     return rc;
