@@ -1481,12 +1481,14 @@ g5_status codec_work_alloc(CodecWork &w, size_t max_n)
     // more than 48 KB of shared memory each (set per device)
     G5_TRY(codec_kernels());
     G5_CUDA(cudaMalloc(&w.slots, sizeof(ChunkSlot) * C));
-    // epochs start at 1, so zeroed status words read as "not published"
+    // the decoder's epochs start at 1, so zeroed status words read as "not
+    // published" (the encoder's records say so in their low bits)
     G5_CUDA(cudaMemset(w.scal, 0, sizeof(uint64_t) * kScalars));
     G5_CUDA(cudaMemset(w.slots, 0, sizeof(ChunkSlot) * C));
     const uint64_t one = 1;
-    for (int e : {CS_U_EPOCH})
-        G5_CUDA(cudaMemcpy(w.scal + e, &one, sizeof one, cudaMemcpyHostToDevice));
+    G5_CUDA(cudaMemcpy(w.scal + CS_U_EPOCH, &one, sizeof one, cudaMemcpyHostToDevice));
+    // a call may be made on a stream that does not wait for the default one
+    G5_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     return G5_OK;
 }
 
@@ -1535,7 +1537,8 @@ struct BatchWs {
     void *desc = nullptr, *slots = nullptr;  // device: streams and chunk numbers; records
     void *h_desc = nullptr, *h_res = nullptr;  // pinned: what goes to desc; what the kernel leaves
     size_t desc_cap = 0, slots_cap = 0, res_cap = 0;
-    g5_status grow(size_t desc_bytes, size_t slot_bytes, size_t res_bytes)
+    // s: the stream of the launch that will read the records
+    g5_status grow(size_t desc_bytes, size_t slot_bytes, size_t res_bytes, cudaStream_t s)
     {
         if (desc_bytes > desc_cap) {
             cudaFree(desc);
@@ -1551,8 +1554,9 @@ struct BatchWs {
             slots = nullptr;
             slots_cap = 0;
             if (cudaMalloc(&slots, slot_bytes) != cudaSuccess) return G5_ERR_OOM;
-            // (zeroed records read as not published)
-            if (cudaMemset(slots, 0, slot_bytes) != cudaSuccess) return G5_ERR_CUDA;
+            // (zeroed records read as not published; on the launch's own stream,
+            // which may not wait for the default one)
+            if (cudaMemsetAsync(slots, 0, slot_bytes, s) != cudaSuccess) return G5_ERR_CUDA;
             slots_cap = slot_bytes;
         }
         if (res_bytes > res_cap) {
@@ -1736,7 +1740,8 @@ g5_status g5_codec_encode_batch(g5_codec *c, const uint32_t *in_dev, const uint6
     BatchWs &w = c->be;
     const size_t sb = sizeof(g5::EncStream) * (size_t)k, db = sb + sizeof(uint32_t) * (size_t)chunks;
     const uint32_t stride = chunks > 16384 ? 2 : g5::kSlot;  // (very many: packed)
-    G5_TRY(w.grow(db, sizeof(uint64_t) * stride * (size_t)chunks, sizeof(uint64_t) * ((size_t)k + 1)));
+    G5_TRY(w.grow(db, sizeof(uint64_t) * stride * (size_t)chunks, sizeof(uint64_t) * ((size_t)k + 1),
+                  (cudaStream_t)stream));
     g5::EncStream *hs = static_cast<g5::EncStream *>(w.h_desc);
     uint32_t *ho = reinterpret_cast<uint32_t *>(static_cast<char *>(w.h_desc) + sb);
     uint32_t t = 0;
@@ -1803,7 +1808,8 @@ g5_status g5_codec_decode_batch(g5_codec *c, const uint32_t *in_dev, const uint6
     if (chunks >= ((uint64_t)1 << 32)) return G5_ERR_CAPACITY;
     BatchWs &w = c->bd;
     const size_t sb = sizeof(g5::DecStream) * (size_t)k, db = sb + sizeof(uint32_t) * (size_t)chunks;
-    G5_TRY(w.grow(db, sizeof(g5::ChunkSlot) * (size_t)chunks, sizeof(uint64_t) + sizeof(uint32_t) * (size_t)k));
+    G5_TRY(w.grow(db, sizeof(g5::ChunkSlot) * (size_t)chunks, sizeof(uint64_t) + sizeof(uint32_t) * (size_t)k,
+                  (cudaStream_t)stream));
     g5::DecStream *hs = static_cast<g5::DecStream *>(w.h_desc);
     uint32_t *ho = reinterpret_cast<uint32_t *>(static_cast<char *>(w.h_desc) + sb);
     uint32_t t = 0;

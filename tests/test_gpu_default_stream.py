@@ -36,3 +36,28 @@ def test_first_call_of_many_roots(n, m):
             assert np.array_equal(o.numpy(), w)
         b.close()
     g.close()
+
+
+def test_first_batch_of_queues():
+    """g5_codec_encode_batch and g5_codec_decode_batch clear the chunks' records
+    where these are new or have grown."""
+    rng = np.random.default_rng(7)
+    stream = torch.cuda.Stream()  # (non-blocking)
+    c = g5.Codec(1 << 20)
+    for sizes in ([3000, 40_000], [200_000, 1, 300_001, 70_000], [900_001] * 4):
+        queues = [np.cumsum(rng.integers(1, 9, n), dtype=np.uint64).astype(np.uint32) for n in sizes]
+        off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.uint64)
+        values = torch.from_numpy(np.concatenate(queues).view(np.int32)).cuda()
+        out = torch.zeros(g5.Codec.batch_bound(off), dtype=torch.int32, device="cuda")
+        back = torch.zeros_like(values)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(CYCLES)
+        at, words = c.encode_batch(values, off, out, stream=stream.cuda_stream)
+        _, ok = c.decode_batch(out, at[:-1], words, np.diff(off), back, stream=stream.cuda_stream)
+        assert ok.all()
+        torch.cuda.synchronize()
+        got = out.cpu().numpy().view(np.uint32)
+        for q, o, w in zip(queues, at[:-1], words):
+            assert np.array_equal(got[int(o):int(o) + int(w)], orc.encode(q, orc.D4))
+        assert torch.equal(back, values)
+    c.close()
