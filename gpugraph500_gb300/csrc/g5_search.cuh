@@ -797,7 +797,9 @@ __global__ void __launch_bounds__(kSB, MODE == SEARCH_GRID2 ? 2 : 1) k_search(co
         put_item<Off>(a.claimed[0] + k, (uint32_t)root, rs, re, (uint32_t)k, a.tile_shift);
     if (threadIdx.x == 0) {
         sh.nf = sh.mf = sh.nitems = sh.ex = 0;
-        sh.stop = 0;
+        // (a search queued behind one that gave up waiting, whose ring the host
+        // has not cleared yet, gives up as well)
+        sh.stop = MODE >= SEARCH_GRID1 ? __ldcg(a.ring + 1) : 0;
     }
     if (MODE == SEARCH_BLOCK)
         for (uint32_t i = threadIdx.x; i < kRing * sizeof(LevelSum) / 8; i += kSB)
