@@ -1420,6 +1420,8 @@ struct g5_bfs {
     SearchState *h_outs = nullptr;  // pinned: one per search of a run_many call
     int64_t with_edges = 0;  // vertices of degree > 0
     bool ran = false;
+    bool pending = false;  // a g5_bfs_launch whose result no poll has taken
+    bool timed = true;     // ev0 and ev1 are those of the last run or launch
     int64_t last_root = -1;
 };
 
@@ -1985,7 +1987,8 @@ g5_status g5_bfs_run(g5_bfs *b, int64_t root, int64_t *pred_out, int32_t *level_
         *b->h_root = root;
         G5_CUDA(cudaMemcpyAsync(b->root_dev, b->h_root, sizeof(int64_t), cudaMemcpyHostToDevice, s));
     }
-    if (stats || !b->one) G5_CUDA(cudaEventRecord(b->ev0, s));
+    b->timed = stats || !b->one;
+    if (b->timed) G5_CUDA(cudaEventRecord(b->ev0, s));
     b->prof.on = b->cfg.profile && !b->exec && !b->one;
     b->prof.used = 0;
     if (b->one) {
@@ -2002,7 +2005,7 @@ g5_status g5_bfs_run(g5_bfs *b, int64_t root, int64_t *pred_out, int32_t *level_
             if (b->h_st->nf == 0 || b->h_st->err) break;
         }
     }
-    if (stats || !b->one) G5_CUDA(cudaEventRecord(b->ev1, s));
+    if (b->timed) G5_CUDA(cudaEventRecord(b->ev1, s));
     if (!b->one) G5_CUDA(cudaMemcpyAsync(b->h_st, b->st, sizeof(BfsState), cudaMemcpyDeviceToHost, s));
     if (pred_out)
         G5_CUDA(cudaMemcpyAsync(pred_out, b->pred, sizeof(int64_t) * (size_t)b->g->n, cudaMemcpyDefault, s));
@@ -2013,6 +2016,7 @@ g5_status g5_bfs_run(g5_bfs *b, int64_t root, int64_t *pred_out, int32_t *level_
         G5_CUDA(cudaMemcpyAsync(cscal, b->cw.scal, sizeof cscal, cudaMemcpyDeviceToHost, s));
     G5_CUDA(cudaStreamSynchronize(s));
     b->ran = true;
+    b->pending = false;
     b->last_root = root;
     b->cur_pred = b->pred;
     if (b->one) G5_TRY(take_result(b, *b->h_out, b->sums, s));
@@ -2096,7 +2100,7 @@ g5_status g5_bfs_launch(g5_bfs *b, int64_t root)
         G5_CUDA(cudaEventRecord(b->ev0, s));
         G5_CUDA(launch_search(b, b->sargs, root, b->pred, b->h_out, s, b->agrid));
         G5_CUDA(cudaEventRecord(b->ev1, s));
-        b->ran = true;
+        b->ran = b->pending = b->timed = true;
         b->last_root = root;
         b->cur_pred = b->pred;
         return G5_OK;
@@ -2124,11 +2128,15 @@ g5_status g5_bfs_poll(g5_bfs *b, int *done, double *device_ms)
     G5_CUDA(e);
     *done = 1;
     if (device_ms) {
+        // (a run without stats records no events)
         float ms = 0;
-        cudaEventElapsedTime(&ms, b->ev0, b->ev1);
+        if (!b->timed) ms = (float)b->h_out->ns * 1e-6f;
+        else if (cudaEventElapsedTime(&ms, b->ev0, b->ev1) != cudaSuccess) cudaGetLastError();
         *device_ms = ms;
     }
-    if (b->one && b->ran) G5_TRY(take_result(b, *b->h_out, b->sums, b->stream));
+    // (once: the mirrors may since hold what another call left)
+    if (b->pending) G5_TRY(take_result(b, *b->h_out, b->sums, b->stream));
+    b->pending = false;
     return search_status(b->h_st->err);
 }
 
@@ -2245,6 +2253,7 @@ g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const
     G5_CUDA(cudaStreamSynchronize(b->cstream));
     if (k) {
         b->ran = true;
+        b->pending = false;
         b->last_root = roots[k - 1];
         b->cur_pred = lanes > 1 ? b->pred : buf[(k - 1) & 1];
         if (!b->one) G5_CUDA(cudaMemcpy(b->h_st, b->st, sizeof(BfsState), cudaMemcpyDeviceToHost));

@@ -247,6 +247,7 @@ struct SearchState {
     int32_t level;       // index of the last (empty) level's frontier
     uint32_t err;
     uint64_t nvisited;
+    uint64_t ns;         // the kernel's own time
 };
 
 // Per-warp scratch: the items of a top-down step or the words and candidates
@@ -273,7 +274,15 @@ struct SearchShared {
     uint32_t stop;
     uint32_t warp_items[kSW];
     unsigned long long item_base;
+    uint64_t t0;                          // start of the search (block 0)
 };
+
+__device__ __forceinline__ uint64_t now_ns()
+{
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
 
 __device__ __forceinline__ void offsets_of(const SearchArgs &a, uint64_t v, uint32_t &s, uint32_t &e)
 {
@@ -767,6 +776,7 @@ __global__ void __launch_bounds__(kSB, MODE == SEARCH_GRID2 ? 2 : 1) k_search(co
     uint32_t *V = MODE == SEARCH_BLOCK ? reinterpret_cast<uint32_t *>(s_search + sizeof(SearchShared)) : a.bitmaps;
     uint32_t *N = V + a.stride;
     LevelSum *sums = MODE == SEARCH_BLOCK ? sh.sums : a.sums;
+    if (blockIdx.x == 0 && threadIdx.x == kSB - 1) sh.t0 = now_ns();
     // prologue: vertices without edges count as visited (they are never
     // reached), as do the ones past n
     const uint64_t root = (uint64_t)a.root;
@@ -887,6 +897,7 @@ __global__ void __launch_bounds__(kSB, MODE == SEARCH_GRID2 ? 2 : 1) k_search(co
         a.out->level = L;
         a.out->err = err | (sh.stop ? (uint32_t)G5_DEVERR_WAIT : 0u);
         a.out->nvisited = visited;
+        a.out->ns = now_ns() - sh.t0;
         // levels L and L + 1 of this search are the last records used, and
         // level L - 1 cleared the two after its next one
         if (MODE != SEARCH_BLOCK) a.ring[0] = (place + L + 1) % kRing;
