@@ -456,8 +456,9 @@ __global__ void __launch_bounds__(kEB, 3) k_encode(const uint32_t *__restrict__ 
     const EncLen e = enc_len(n_dev ? *n_dev : n_val, max_n, raw_thr, gridDim.x);
     // a queue of one chunk is block 0's alone: no claim and no counting out
     // (3000 ids there and back through the plugin 55.2 -> 52.7 us, a scale-22
-    // search with the codec 436 -> 428)
-    const bool lone = e.raw ? e.n <= kLoneRaw : e.nchunks <= 1;
+    // search with the codec 436 -> 428).  Not where the words go to the place of
+    // the length: a block that starts late would read them as one
+    const bool lone = (!n_dev || n_dev != words_out) && (e.raw ? e.n <= kLoneRaw : e.nchunks <= 1);
     if (lone && blockIdx.x) return;
     if (e.raw) {
         const uint64_t step = lone ? kEB : (uint64_t)gridDim.x * kEB;
@@ -470,7 +471,7 @@ __global__ void __launch_bounds__(kEB, 3) k_encode(const uint32_t *__restrict__ 
             // every block has drawn one: none is left (5 M values 26.4 -> 25.5 us a call)
             if (e.nchunks <= gridDim.x) break;
         }
-        if (e.ng == 0 && threadIdx.x < 32) {
+        if (e.ng == 0 && blockIdx.x == 0 && threadIdx.x < 32) {
             const uint64_t w = enc_tail_warp(in, e.n, 0, 4, out, sh.bytes);
             if (threadIdx.x == 0) scal[CS_E_WORDS] = w;
         }
@@ -1229,7 +1230,8 @@ __global__ void __launch_bounds__(kDB, 2) k_decode(const uint32_t *__restrict__ 
                                gridDim.x);
     uint32_t bad = 0;
     // (as in k_encode)
-    const bool lone = h.bad || (h.raw ? h.words <= kLoneRaw : h.nchunks <= 1);
+    const bool lone =
+        (!words_dev || words_dev != n_out) && (h.bad || (h.raw ? h.words <= kLoneRaw : h.nchunks <= 1));
     if (lone && blockIdx.x) return;
     if (h.raw) {
         const uint64_t step = lone ? kDB : (uint64_t)gridDim.x * kDB;
@@ -1246,7 +1248,7 @@ __global__ void __launch_bounds__(kDB, 2) k_decode(const uint32_t *__restrict__ 
             bad |= dec_chunk<false>(sh, h, in, c, epoch, slots, &scal[CS_U_ERR], out, cap, expect, mode, &scal[CS_U_N]);
             if (h.nchunks <= gridDim.x) break;  // (as in k_encode)
         }
-        if (h.ng == 0 && threadIdx.x < 32) {
+        if (h.ng == 0 && blockIdx.x == 0 && threadIdx.x < 32) {
             uint64_t n;
             bad |= dec_tail(sh.tail, in, h.words, 4, 0, cap, out, expect, n);
             if (g5_lane() == 0) scal[CS_U_N] = n;
