@@ -1567,7 +1567,8 @@ bool plan_search(g5_bfs *b)
         if ((form == SEARCH_CLUSTER &&
              cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->ssmem) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSB, b->ssmem) != cudaSuccess || per_sm < 1) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSB, b->ssmem) != cudaSuccess || per_sm < 1 ||
+            (form == SEARCH_CLUSTER && !cluster_fits((const void *)kern, kClusterBlocks, b->ssmem))) {
             cudaGetLastError();
             continue;
         }

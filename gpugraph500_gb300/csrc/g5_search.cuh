@@ -176,6 +176,27 @@ inline int search_form(int64_t n, int64_t nnz)
     return n < kGrid2Vertices ? SEARCH_GRID1 : SEARCH_GRID2;
 }
 
+// Whether the device can hold a cluster of `blocks` blocks of the cluster form.
+// Sixteen is more than every device or share of one must have in one place, and
+// neither the attribute that allows it nor the blocks per SM tell.
+inline bool cluster_fits(const void *kern, int blocks, size_t smem)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = blocks;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kSB);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess) return n > 0;
+    cudaGetLastError();
+    return false;
+}
+
 // Bitmap words per warp step of a bottom-up level: the fewest steps of at most
 // 32 words, all warps alike.  A step is a chain (words, list, offsets, probes)
 // that pipelines over its own rounds only, and a last round of steps that half

@@ -5,6 +5,8 @@
 //   search_forms waits GRAPH OUT ROOT        a search whose blocks wait for arrivals
 //       that never come, one queued behind it, and one after the ring is cleared:
 //       the error bits and parents of each, per grid form, to OUT
+//   search_forms clusters GRAPH OUT N...     1 or 0 (int64) to OUT for each N: whether
+//       the device can hold a cluster of N blocks of the cluster form
 // GRAPH: int64 n, int64 nnz, int64 row offsets, uint32 columns.  Built with a
 // short G5_MEET_NS.
 #include <cstdio>
@@ -160,6 +162,15 @@ int main(int argc, char **argv)
                     put(lev.data(), 4 * lev.size());
                 }
             }
+    } else if (!std::strcmp(argv[1], "clusters")) {
+        auto kern = k_search<uint32_t, SEARCH_CLUSTER>;
+        CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SearchShared)));
+        CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        for (int i = 4; i < argc; ++i) {
+            const int64_t fits = cluster_fits((const void *)kern, std::atoi(argv[i]), sizeof(SearchShared));
+            CHECK(cudaGetLastError());  // (none left behind)
+            put(&fits, 8);
+        }
     } else {
         for (int form = SEARCH_GRID1; form <= SEARCH_GRID2; ++form) {
             // arrivals of blocks that are not there: the meeting after the prologue

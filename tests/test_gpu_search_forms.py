@@ -69,6 +69,14 @@ def test_every_form_and_offset_width(exe, tmp_path, which):
                 at += 12 * n
 
 
+def test_clusters_that_do_not_fit(exe, tmp_path):
+    """No device holds a cluster of 32 blocks; the answer leaves no error behind."""
+    ro, col = orc.build_csr(4, np.array([(0, 1)], np.int64))
+    out = tmp_path / "out"
+    run(exe, "clusters", graph_file(tmp_path / "g", ro, col), out, 32, 1, 8, 64)
+    assert np.fromfile(out, np.int64).tolist() == [0, 1, 1, 0]
+
+
 def test_waits_that_run_out(exe, tmp_path):
     n = 20_000
     ro, col = orc.build_csr(n, np.random.default_rng(1).integers(0, n, (90_000, 2)))
