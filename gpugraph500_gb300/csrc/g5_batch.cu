@@ -1615,7 +1615,7 @@ struct g5_batch {
     std::vector<void *> owned;        // degree-ordered graph copies
     // the one-launch form (g5_batch_run; made on its first call)
     void *scratch = nullptr;          // queue arrays of the level graph, or built items
-    int pgrid = 0;                    // its blocks (0: not made yet, -1: the device cannot hold it)
+    int pgrid = 0;                    // its blocks (0: not made, -1: the device cannot hold it)
     PArgs pargs;
     BItem *claimed = nullptr;
     uint8_t *live = nullptr;
@@ -1694,6 +1694,23 @@ g5_status build_batch_graph(g5_batch *b)
     return G5_OK;
 }
 
+// Gives back what the one-launch form holds.
+void drop_one_launch(g5_batch *b)
+{
+    cudaFree(b->claimed);
+    cudaFree(b->live);
+    cudaFree(b->rsums);
+    cudaFree(b->longs);
+    cudaFree(b->stage);
+    cudaFreeHost(b->h_stage);
+    b->claimed = nullptr;
+    b->live = nullptr;
+    b->rsums = nullptr;
+    b->longs = nullptr;
+    b->stage = b->h_stage = nullptr;
+    b->pgrid = 0;
+}
+
 void free_batch(g5_batch *b)
 {
     if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -1704,12 +1721,7 @@ void free_batch(g5_batch *b)
     cudaFree(b->iso);
     cudaFree(b->words);
     cudaFree(b->scratch);
-    cudaFree(b->claimed);
-    cudaFree(b->live);
-    cudaFree(b->rsums);
-    cudaFree(b->longs);
-    cudaFree(b->stage);
-    cudaFreeHost(b->h_stage);
+    drop_one_launch(b);
     cudaFree(b->chunks);
     cudaFree(b->step_graph);
     cudaFree(b->st);
@@ -1808,10 +1820,11 @@ g5_status plan_one_launch(g5_batch *b)
     uint64_t nnz = 0;
     for (const g5_graph *g : b->graphs) nnz += (uint64_t)g->nnz;
     int per_sm = 0;
-    if (cudaFuncSetAttribute(k_bsearch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PShared)) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bsearch, kSB, sizeof(PShared)) != cudaSuccess ||
-        per_sm < 1) {
+    cudaError_t e = cudaFuncSetAttribute(k_bsearch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PShared));
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bsearch, kSB, sizeof(PShared));
+    if (e != cudaSuccess || per_sm < 1) {
         cudaGetLastError();
+        if (e == cudaErrorMemoryAllocation) return G5_ERR_OOM;
         b->pgrid = -1;
         return G5_OK;
     }
@@ -1824,15 +1837,15 @@ g5_status plan_one_launch(g5_batch *b)
     b->zero_at = align16(b->off_at + sizeof(int32_t) * (ng + 1));
     const size_t sums_at = b->zero_at + sizeof(LevelMeet) * kRing, abort_at = sums_at + sizeof(GraphSum) * kRing * ng;
     b->stage_bytes = abort_at + 16;
-    // (a failed call can leave some made: the next one goes on from there)
-    if (!b->claimed) G5_CUDA(cudaMalloc(&b->claimed, sizeof(BItem) * 2 * a.claimed_cap));
-    if (!b->live) G5_CUDA(cudaMalloc(&b->live, vb / 32));
-    if (!b->rsums) G5_CUDA(cudaMalloc(&b->rsums, sizeof(uint64_t) * kRing * 64 * ng));
+    // (a failed call leaves what it has made to drop_one_launch)
+    G5_CUDA(cudaMalloc(&b->claimed, sizeof(BItem) * 2 * a.claimed_cap));
+    G5_CUDA(cudaMalloc(&b->live, vb / 32));
+    G5_CUDA(cudaMalloc(&b->rsums, sizeof(uint64_t) * kRing * 64 * ng));
     // (a row has a piece per kLongRow entries and one for the rest, and more
     // than kLongRow entries to have any)
-    if (!b->longs) G5_CUDA(cudaMalloc(&b->longs, sizeof(LongItem) * (2 * (nnz / kLongRow) + 1)));
-    if (!b->stage) G5_CUDA(cudaMalloc(&b->stage, b->stage_bytes));
-    if (!b->h_stage) G5_CUDA(cudaMallocHost(&b->h_stage, b->stage_bytes));
+    G5_CUDA(cudaMalloc(&b->longs, sizeof(LongItem) * (2 * (nnz / kLongRow) + 1)));
+    G5_CUDA(cudaMalloc(&b->stage, b->stage_bytes));
+    G5_CUDA(cudaMallocHost(&b->h_stage, b->stage_bytes));
     memset(b->h_stage, 0, b->stage_bytes);
     a.gd = reinterpret_cast<const GraphDesc *>(b->stage);
     a.claimed[0] = b->claimed;
@@ -2272,8 +2285,17 @@ g5_status g5_batch_run(g5_batch *b, const int64_t *roots_host, const int *nroots
                        double *device_ms)
 {
     if (!b || !roots_host || !nroots || !pred_out_dev) return G5_ERR_INVALID_ARG;
-    if (!b->pgrid) G5_TRY(plan_one_launch(b));
-    if (b->pgrid < 0) {
+    if (!b->pgrid) {
+        const g5_status st = plan_one_launch(b);
+        if (st != G5_OK) {
+            // (no memory for it now: the level graph needs none, and the next
+            // call tries again)
+            drop_one_launch(b);
+            cudaGetLastError();
+            if (st != G5_ERR_OOM) return st;
+        }
+    }
+    if (b->pgrid <= 0) {
         G5_TRY(g5_batch_launch(b, roots_host, nroots, pred_out_dev));
         int done = 0;
         return g5_batch_poll(b, 1, &done, device_ms);
