@@ -1615,6 +1615,8 @@ struct g5_batch {
     std::vector<void *> owned;        // degree-ordered graph copies
     // the one-launch form (g5_batch_run; made on its first call)
     void *scratch = nullptr;          // queue arrays of the level graph, or built items
+    size_t scratch_bytes = 0;
+    BItem *built = nullptr;           // built items that the scratch has no room for
     int pgrid = 0;                    // its blocks (0: not made, -1: the device cannot hold it)
     PArgs pargs;
     BItem *claimed = nullptr;
@@ -1694,16 +1696,45 @@ g5_status build_batch_graph(g5_batch *b)
     return G5_OK;
 }
 
+// Bytes of the level graph's queue arrays.
+size_t queue_bytes(const BArgs &a)
+{
+    return sizeof(uint64_t) * (2 * a.ntot + 2) + sizeof(uint32_t) * (a.ntot + a.max_tiles);
+}
+
+// Calls f(pointer, bytes) for every device buffer of a workspace but its graph
+// copies and the one-launch form's: one list of what is allocated, freed and
+// charged (from ngraphs, ntot, nchunks, nsteps and max_tiles of its arguments).
+template <typename F>
+void each_buffer(g5_batch *b, F f)
+{
+    const BArgs &a = b->args;
+    const size_t ng = (size_t)a.ngraphs;
+    f(b->gd, sizeof(GraphDesc) * ng);
+    f(b->step_graph, a.nsteps + 1);
+    f(b->chunk_graph, (size_t)a.nchunks);
+    f(b->deg, sizeof(uint32_t) * a.ntot);
+    f(b->iso, sizeof(uint32_t) * (a.ntot / 32));
+    f(b->words, sizeof(uint64_t) * 3 * a.ntot);
+    f(b->scratch, queue_bytes(a));
+    f(b->chunks, sizeof(uint64_t) * 2 * a.nchunks + a.nchunks);
+    f(b->st, sizeof(BState));
+    f(b->roots, sizeof(int64_t) * 64 * ng);
+    f(b->root_off, sizeof(int32_t) * (ng + 1));
+    f(b->level_log, sizeof(uint64_t) * kMaxLevels);
+}
+
 // Gives back what the one-launch form holds.
 void drop_one_launch(g5_batch *b)
 {
     cudaFree(b->claimed);
+    cudaFree(b->built);
     cudaFree(b->live);
     cudaFree(b->rsums);
     cudaFree(b->longs);
     cudaFree(b->stage);
     cudaFreeHost(b->h_stage);
-    b->claimed = nullptr;
+    b->claimed = b->built = nullptr;
     b->live = nullptr;
     b->rsums = nullptr;
     b->longs = nullptr;
@@ -1715,19 +1746,8 @@ void free_batch(g5_batch *b)
 {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
-    cudaFree(b->gd);
-    cudaFree(b->chunk_graph);
-    cudaFree(b->deg);
-    cudaFree(b->iso);
-    cudaFree(b->words);
-    cudaFree(b->scratch);
+    each_buffer(b, [](auto *&p, size_t) { cudaFree(p); });
     drop_one_launch(b);
-    cudaFree(b->chunks);
-    cudaFree(b->step_graph);
-    cudaFree(b->st);
-    cudaFree(b->roots);
-    cudaFree(b->root_off);
-    cudaFree(b->level_log);
     cudaFree(b->adm_dev);
     cudaFreeHost(b->adm_host);
     cudaFreeHost(b->h_roots);
@@ -1839,6 +1859,9 @@ g5_status plan_one_launch(g5_batch *b)
     b->stage_bytes = abort_at + 16;
     // (a failed call leaves what it has made to drop_one_launch)
     G5_CUDA(cudaMalloc(&b->claimed, sizeof(BItem) * 2 * a.claimed_cap));
+    // (more than some 85 entries a vertex: the built items outgrow the queue arrays)
+    const size_t built_bytes = sizeof(BItem) * (vb + nnz / kItemEntries + 1);
+    if (built_bytes > b->scratch_bytes) G5_CUDA(cudaMalloc(&b->built, built_bytes));
     G5_CUDA(cudaMalloc(&b->live, vb / 32));
     G5_CUDA(cudaMalloc(&b->rsums, sizeof(uint64_t) * kRing * 64 * ng));
     // (a row has a piece per kLongRow entries and one for the rest, and more
@@ -1850,7 +1873,7 @@ g5_status plan_one_launch(g5_batch *b)
     a.gd = reinterpret_cast<const GraphDesc *>(b->stage);
     a.claimed[0] = b->claimed;
     a.claimed[1] = b->claimed + a.claimed_cap;
-    a.built = static_cast<BItem *>(b->scratch);
+    a.built = b->built ? b->built : static_cast<BItem *>(b->scratch);
     a.meets = reinterpret_cast<LevelMeet *>(b->stage + b->zero_at);
     a.sums = reinterpret_cast<GraphSum *>(b->stage + sums_at);
     a.abort = reinterpret_cast<unsigned *>(b->stage + abort_at);
@@ -1937,29 +1960,14 @@ g5_status batch_create_impl(g5_graph *const *graphs, int ngraphs, const g5_batch
         sg.insert(sg.end(), steps, (uint8_t)i);
     }
     a.nsteps = sg.size();
-#define B_ALLOC(ptr, bytes) \
-    if (cudaMalloc(&(ptr), (bytes)) != cudaSuccess) return fail(G5_ERR_OOM)
-    B_ALLOC(b->gd, sizeof(GraphDesc) * ngraphs);
-    B_ALLOC(b->step_graph, sg.size() + 1);
-    B_ALLOC(b->chunk_graph, cg.size());
-    B_ALLOC(b->deg, sizeof(uint32_t) * vb);
-    B_ALLOC(b->iso, sizeof(uint32_t) * (vb / 32));
-    B_ALLOC(b->words, sizeof(uint64_t) * 3 * vb);
-    // the queue arrays of the level graph; the one-launch form holds its built
-    // items in the same memory
-    const size_t queue_bytes = sizeof(uint64_t) * (2 * vb + 2) + sizeof(uint32_t) * (vb + a.max_tiles);
-    const size_t item_bytes = sizeof(BItem) * (vb + nnz_max / kItemEntries + 1);
-    B_ALLOC(b->scratch, std::max(queue_bytes, item_bytes));
+    bool room = true;
+    each_buffer(b, [&](auto *&p, size_t bytes) { room = room && cudaMalloc(&p, bytes) == cudaSuccess; });
+    if (!room) return fail(G5_ERR_OOM);
+    b->scratch_bytes = queue_bytes(a);
     b->qoff = static_cast<uint64_t *>(b->scratch);
     b->qbase = reinterpret_cast<int64_t *>(b->qoff + vb + 2);
     b->queue = reinterpret_cast<uint32_t *>(b->qbase + vb);
     b->tile_start = b->queue + vb;
-    B_ALLOC(b->chunks, sizeof(uint64_t) * 2 * a.nchunks + a.nchunks);
-    B_ALLOC(b->st, sizeof(BState));
-    B_ALLOC(b->roots, sizeof(int64_t) * 64 * ngraphs);
-    B_ALLOC(b->root_off, sizeof(int32_t) * (ngraphs + 1));
-    B_ALLOC(b->level_log, sizeof(uint64_t) * kMaxLevels);
-#undef B_ALLOC
     if (cudaMallocHost(&b->h_roots, sizeof(int64_t) * 64 * ngraphs) != cudaSuccess ||
         cudaMallocHost(&b->h_root_off, sizeof(int32_t) * (ngraphs + 1)) != cudaSuccess ||
         cudaMallocHost(&b->h_st, sizeof(BState)) != cudaSuccess)
@@ -2005,16 +2013,26 @@ g5_status batch_create_sharing(g5_batch *owner, g5_batch **out)
 
 size_t batch_workspace_bytes(const g5_graph *g)
 {
-    // per vertex: 3 x 8 B words, degree, queue, edge offset, row base;
-    // per 256 edges a tile start; the fixed parts rounded up
-    return (size_t)g->n * (24 + 4 + 4 + 8 + 8) + (size_t)g->nnz / 64 + ((size_t)1 << 20);
+    g5_batch b;
+    BArgs &a = b.args;
+    memset(&a, 0, sizeof a);
+    a.ngraphs = 1;
+    a.nchunks = (uint32_t)(((uint64_t)g->n + kChunk - 1) / kChunk);
+    a.ntot = (uint64_t)a.nchunks * kChunk;
+    a.nsteps = ((uint64_t)g->n + 31) / 32;
+    a.max_tiles = (uint64_t)g->nnz / kTile + 3;
+    size_t total = 0;
+    each_buffer(&b, [&](auto *&, size_t bytes) { total += device_bytes(bytes); });
+    return total;
 }
 
 size_t batch_copy_bytes(const g5_graph *g)
 {
-    // degree-ordered copy: two id maps, offsets, the list of vertices with edges
-    // (16 bytes for three in four), columns
-    return (size_t)g->n * (4 + 4 + 8 + 12) + (size_t)g->nnz * 4 + ((size_t)1 << 20);
+    // degree-ordered copy: two id maps, offsets, columns and a list of the
+    // vertices with edges, which are not counted here
+    const size_t n = (size_t)g->n, nnz = (size_t)g->nnz;
+    return 2 * device_bytes(sizeof(uint32_t) * n) + device_bytes(sizeof(int64_t) * (n + 1)) +
+           device_bytes(sizeof(uint32_t) * nnz) + device_bytes(sizeof(uint4) * std::min(n, nnz));
 }
 
 }  // namespace g5

@@ -1654,9 +1654,14 @@ g5_status search_status(uint32_t err)
     return err ? G5_ERR_CAPACITY : G5_OK;
 }
 
-g5_status alloc_ws(g5_bfs *b)
+// One launch per search, unless the search encodes its queues, finds its
+// parents in a fix-up sweep or is driven from the host level by level.
+bool one_launch(const g5_bfs_config &cfg) { return cfg.use_graph && !cfg.codec && cfg.parent_mode == 0; }
+
+// The sizes that a workspace's buffers follow from: its graph's, cfg and `one`.
+void plan_sizes(g5_bfs *b)
 {
-    g5_graph *g = b->g;
+    const g5_graph *g = b->g;
     const int64_t n = g->n;
     BfsArgs &a = b->args;
     memset(&a, 0, sizeof a);
@@ -1676,58 +1681,87 @@ g5_status alloc_ws(g5_bfs *b)
     a.bu_serial = b->cfg.bu_serial;
     a.max_tiles = (uint64_t)g->nnz / a.tile + 2;
     a.max_levels = b->cfg.max_levels;
-    G5_CUDA(cudaMalloc(&b->deg, sizeof(uint32_t) * (size_t)n));
-    G5_CUDA(cudaMalloc(&b->bitmaps, sizeof(uint32_t) * (b->one ? 4 * ((a.nwords + 3) & ~(uint64_t)3) : 3 * a.nwords)));
-    G5_CUDA(cudaMalloc(&b->isolated, sizeof(uint32_t) * a.nwords));
-    G5_CUDA(cudaMalloc(&b->heavy, sizeof(uint32_t) * a.nwords));
+    SearchArgs &sa = b->sargs;
+    memset(&sa, 0, sizeof sa);
+    if (!b->one) return;
+    // each vertex of a frontier has at most one item per whole tile of its row
+    // and one for the rest
+    sa.tile_shift = std::max(a.tile_shift, kMinItemShift);
+    const uint64_t tiles = (uint64_t)g->nnz >> sa.tile_shift;
+    sa.claimed_cap = std::min<uint64_t>(std::min<uint64_t>(n, kClaimMax) + tiles + 1, kClaimedItems);
+    sa.built_cap = (uint64_t)n + tiles + 1;
+}
+
+// Calls f(pointer, bytes) for every device buffer of a workspace but the codec's
+// own: one list of what is allocated, freed and charged.
+template <typename F>
+void each_buffer(g5_bfs *b, F f)
+{
+    const size_t n = (size_t)b->g->n;
+    const BfsArgs &a = b->args;
+    f(b->deg, sizeof(uint32_t) * n);
+    f(b->bitmaps, sizeof(uint32_t) * (b->one ? 4 * ((a.nwords + 3) & ~(uint64_t)3) : 3 * a.nwords));
+    f(b->isolated, sizeof(uint32_t) * a.nwords);
+    f(b->heavy, sizeof(uint32_t) * a.nwords);
     // 32-bit offsets while every scan position (row end + one 32-entry step) fits
-    if (g->nnz < ((int64_t)1 << 32) - 64) G5_CUDA(cudaMalloc(&b->ro32, sizeof(uint32_t) * (size_t)(n + 1)));
-    G5_CUDA(cudaMalloc(&b->first, sizeof(uint32_t) * (size_t)n));
-    G5_CUDA(cudaMalloc(&b->pred, sizeof(int64_t) * (size_t)n));
-    if (b->cfg.want_levels) G5_CUDA(cudaMalloc(&b->level, sizeof(int32_t) * (size_t)n));
-    G5_CUDA(cudaMalloc(&b->st, sizeof(BfsState)));
-    G5_CUDA(cudaMalloc(&b->log, sizeof(LevelRec) * (size_t)b->cfg.max_levels));
+    if (b->g->nnz < ((int64_t)1 << 32) - 64) f(b->ro32, sizeof(uint32_t) * (n + 1));
+    f(b->first, sizeof(uint32_t) * n);
+    f(b->pred, sizeof(int64_t) * n);
+    if (b->cfg.want_levels) f(b->level, sizeof(int32_t) * n);
+    f(b->st, sizeof(BfsState));
+    f(b->log, sizeof(LevelRec) * (size_t)a.max_levels);
     if (b->one) {
-        // each vertex of a frontier has at most one item per whole tile of
-        // its row and one for the rest
+        f(b->items, sizeof(Item) * (2 * b->sargs.claimed_cap + b->sargs.built_cap));
+        f(b->sums, sizeof(LevelSum) * (kRing + 1));
+        return;
+    }
+    f(b->multi, sizeof(uint32_t) * a.nwords);
+    f(b->wdeg, sizeof(uint32_t) * a.nwords);
+    f(b->ulist, sizeof(uint32_t) * n + 16);
+    f(b->done, sizeof(unsigned));
+    f(b->queue, sizeof(uint32_t) * n + 16);
+    f(b->qoff, sizeof(uint64_t) * (n + 1));
+    f(b->qbase, sizeof(int64_t) * n);
+    f(b->tile_start, sizeof(uint32_t) * a.max_tiles);
+    f(b->chunks, sizeof(uint64_t) * 3 * a.nchunks);
+    f(b->slist, sizeof(uint32_t) * kSparseCap);
+    f(b->root_dev, sizeof(int64_t));
+    if (b->cfg.codec) {
+        f(b->dqueue, sizeof(uint32_t) * n + 16);
+        f(b->codec_stream, sizeof(uint32_t) * g5::codec_bound(n));
+        f(b->ccap, sizeof(CodecCapture));
+    }
+}
+
+g5_status alloc_ws(g5_bfs *b)
+{
+    g5_graph *g = b->g;
+    const int64_t n = g->n;
+    BfsArgs &a = b->args;
+    plan_sizes(b);
+    cudaError_t err = cudaSuccess;
+    each_buffer(b, [&](auto *&p, size_t bytes) {
+        if (err == cudaSuccess) err = cudaMalloc(&p, bytes);
+    });
+    G5_CUDA(err);
+    if (b->one) {
         SearchArgs &sa = b->sargs;
-        memset(&sa, 0, sizeof sa);
-        sa.tile_shift = std::max(a.tile_shift, kMinItemShift);
-        const uint64_t tiles = (uint64_t)g->nnz >> sa.tile_shift;
-        sa.claimed_cap = std::min<uint64_t>(std::min<uint64_t>(n, kClaimMax) + tiles + 1, kClaimedItems);
-        sa.built_cap = (uint64_t)n + tiles + 1;
-        G5_CUDA(cudaMalloc(&b->items, sizeof(Item) * (2 * sa.claimed_cap + sa.built_cap)));
         sa.claimed[0] = b->items;
         sa.claimed[1] = b->items + sa.claimed_cap;
         sa.built = b->items + 2 * sa.claimed_cap;
-        G5_CUDA(cudaMalloc(&b->sums, sizeof(LevelSum) * (kRing + 1)));
         G5_CUDA(cudaMemset(b->sums, 0, sizeof(LevelSum) * (kRing + 1)));
         G5_CUDA(cudaMallocHost(&b->h_out, sizeof(SearchState)));
         memset(b->h_out, 0, sizeof(SearchState));
     } else {
-        G5_CUDA(cudaMalloc(&b->multi, sizeof(uint32_t) * a.nwords));
-        G5_CUDA(cudaMalloc(&b->wdeg, sizeof(uint32_t) * a.nwords));
         G5_CUDA(cudaMemset(b->wdeg, 0, sizeof(uint32_t) * a.nwords));
-        G5_CUDA(cudaMalloc(&b->ulist, sizeof(uint32_t) * (size_t)n + 16));
-        G5_CUDA(cudaMalloc(&b->done, sizeof(unsigned)));
         G5_CUDA(cudaMemset(b->done, 0, sizeof(unsigned)));
         G5_CUDA(cudaMemset(b->multi, 0, sizeof(uint32_t) * a.nwords));
-        G5_CUDA(cudaMalloc(&b->queue, sizeof(uint32_t) * (size_t)n + 16));
-        G5_CUDA(cudaMalloc(&b->qoff, sizeof(uint64_t) * (size_t)(n + 1)));
-        G5_CUDA(cudaMalloc(&b->qbase, sizeof(int64_t) * (size_t)n));
-        G5_CUDA(cudaMalloc(&b->tile_start, sizeof(uint32_t) * a.max_tiles));
-        G5_CUDA(cudaMalloc(&b->chunks, sizeof(uint64_t) * 3 * a.nchunks));
-        G5_CUDA(cudaMalloc(&b->slist, sizeof(uint32_t) * kSparseCap));
-        G5_CUDA(cudaMalloc(&b->root_dev, sizeof(int64_t)));
     }
     G5_CUDA(cudaMallocHost(&b->h_root, sizeof(int64_t)));
     G5_CUDA(cudaMallocHost(&b->h_st, sizeof(BfsState)));
     G5_CUDA(cudaMallocHost(&b->h_log, sizeof(LevelRec) * (size_t)b->cfg.max_levels));
     if (b->cfg.codec) {
-        G5_CUDA(cudaMalloc(&b->dqueue, sizeof(uint32_t) * (size_t)n + 16));
-        G5_CUDA(cudaMalloc(&b->codec_stream, sizeof(uint32_t) * g5::codec_bound((size_t)n)));
         G5_TRY(g5::codec_work_alloc(b->cw, (size_t)n));
-        G5_CUDA(cudaMalloc(&b->ccap, sizeof(CodecCapture)));
         G5_CUDA(cudaMemset(b->ccap, 0, sizeof(CodecCapture)));
     }
     a.row_off = g->row_off;
@@ -1833,34 +1867,12 @@ void free_ws(g5_bfs *b)
     for (cudaEvent_t e : b->tev) cudaEventDestroy(e);
     cudaFreeHost(b->h_roots);
     cudaFreeHost(b->h_errs);
-    cudaFree(b->deg);
-    cudaFree(b->bitmaps);
-    cudaFree(b->isolated);
-    cudaFree(b->heavy);
-    cudaFree(b->ro32);
-    cudaFree(b->first);
-    cudaFree(b->multi);
-    cudaFree(b->wdeg);
-    cudaFree(b->ulist);
-    cudaFree(b->done);
-    cudaFree(b->pred);
-    cudaFree(b->level);
-    cudaFree(b->queue);
-    cudaFree(b->dqueue);
-    cudaFree(b->qoff);
-    cudaFree(b->qbase);
-    cudaFree(b->tile_start);
-    cudaFree(b->chunks);
-    cudaFree(b->slist);
-    cudaFree(b->items);
-    cudaFree(b->sums);
+    each_buffer(b, [](auto *&p, size_t) {
+        cudaFree(p);
+        p = nullptr;
+    });
     cudaFreeHost(b->h_out);
     cudaFreeHost(b->h_outs);
-    cudaFree(b->st);
-    cudaFree(b->log);
-    cudaFree(b->root_dev);
-    cudaFree(b->codec_stream);
-    cudaFree(b->ccap);
     cudaFreeHost(b->h_root);
     cudaFreeHost(b->h_st);
     cudaFreeHost(b->h_log);
@@ -1902,6 +1914,22 @@ int64_t alg_bytes(const LevelRec *log, int nlev, int64_t n, int64_t with_edges, 
 }
 
 }  // namespace
+
+namespace g5 {
+
+size_t search_workspace_bytes(const g5_graph *g, const g5_bfs_config &cfg)
+{
+    g5_bfs b;
+    b.g = const_cast<g5_graph *>(g);
+    b.cfg = cfg;
+    b.one = one_launch(cfg);
+    plan_sizes(&b);
+    size_t total = 0;
+    each_buffer(&b, [&](auto *&, size_t bytes) { total += device_bytes(bytes); });
+    return total;
+}
+
+}  // namespace g5
 
 extern "C" {
 
@@ -1945,9 +1973,7 @@ g5_status g5_bfs_create(g5_graph *g, const g5_bfs_config *cfg, g5_bfs **out)
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(G5_ERR_CUDA);
     cudaEventCreate(&b->ev0);
     cudaEventCreate(&b->ev1);
-    // one launch per search, unless the search encodes its queues, finds its
-    // parents in a fix-up sweep or is driven from the host level by level
-    if (b->cfg.use_graph && !b->cfg.codec && b->cfg.parent_mode == 0) {
+    if (one_launch(b->cfg)) {
         b->one = g->nnz < ((int64_t)1 << 32) - 64 ? plan_search<uint32_t>(b) : plan_search<int64_t>(b);
     }
     if ((st = alloc_ws(b)) != G5_OK) return fail(st);

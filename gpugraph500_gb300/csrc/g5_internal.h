@@ -24,6 +24,17 @@ namespace g5 {
 // 25 entries each (row-major 5x5 mod 2^31-1).
 const uint32_t *mrg_skip_table_host();
 
+// Device memory that an allocation of x bytes takes: the driver gives out pages
+// of 2 MB, and shares them between allocations of up to 1 MB.
+inline size_t device_bytes(size_t x)
+{
+    const size_t unit = x > ((size_t)1 << 20) ? (size_t)1 << 21 : 512;
+    return (x + unit - 1) / unit * unit;
+}
+
+// Device bytes of a search workspace on one graph (without codec).
+size_t search_workspace_bytes(const g5_graph *g, const g5_bfs_config &cfg);
+
 // Degree of vertex v of a device graph (reads two row offsets).
 g5_status graph_degree(const g5_graph *g, int64_t v, int64_t *deg);
 

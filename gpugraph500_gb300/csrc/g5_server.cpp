@@ -87,6 +87,20 @@ struct Query {
     Clock::time_point t_submit, t_start, t_done;
 };
 
+// What admission charges, in device bytes: a search or batch workspace, and a
+// batch's copy of the graph.  Never less than 48 bytes a vertex, a 64th of the
+// entries and 1 MB (28, four bytes an entry and 1 MB for the copy), which small
+// graphs do not need but callers size their budgets by.
+uint64_t workspace_charge(const g5_graph *g, size_t bytes)
+{
+    return std::max<uint64_t>(48ull * (uint64_t)g->n + (uint64_t)g->nnz / 64 + (1u << 20), bytes);
+}
+
+uint64_t copy_charge(const g5_graph *g)
+{
+    return std::max<uint64_t>(28ull * (uint64_t)g->n + 4ull * (uint64_t)g->nnz + (1u << 20), g5::batch_copy_bytes(g));
+}
+
 }  // namespace
 
 struct g5_server {
@@ -488,7 +502,7 @@ g5_status g5_server_create_modes(g5_graph *const *graphs, int ngraphs, size_t me
             continue;
         }
         if (sv->kind[i] == G5_SERVE_STREAMS) {
-            const uint64_t per = 48ull * n + (uint64_t)graphs[i]->nnz / 64 + (1u << 20);
+            const uint64_t per = workspace_charge(graphs[i], g5::search_workspace_bytes(graphs[i], cfg));
             k = std::min<uint64_t>(64, share / per);
             if (k == 0) return fail(G5_ERR_OOM);
             other_used += k * per;
@@ -520,9 +534,9 @@ g5_status g5_server_create_modes(g5_graph *const *graphs, int ngraphs, size_t me
         const uint64_t n = (uint64_t)graphs[i]->n;
         col_n = std::max(col_n, n);
         const uint64_t gshare = (uint64_t)((double)left * (double)n / (double)cohort_n);
-        const uint64_t per_plain = 48ull * n + (uint64_t)graphs[i]->nnz / 64 + (1u << 20);
-        const uint64_t fixed = g5::batch_copy_bytes(graphs[i]) + kCohortPlain * per_plain;
-        const uint64_t per_ws = g5::batch_workspace_bytes(graphs[i]);
+        const uint64_t per_plain = workspace_charge(graphs[i], g5::search_workspace_bytes(graphs[i], cfg));
+        const uint64_t fixed = copy_charge(graphs[i]) + kCohortPlain * per_plain;
+        const uint64_t per_ws = workspace_charge(graphs[i], g5::batch_workspace_bytes(graphs[i]));
         // as many workspaces (up to kCohortWorkspaces) as leave room for at
         // least 8 root slots each, and every workspace the slots that fit
         int nw = kCohortWorkspaces;
