@@ -1733,6 +1733,23 @@ void each_buffer(g5_bfs *b, F f)
     }
 }
 
+// Gives back what alloc_ws allocates but the codec's own.
+void free_buffers(g5_bfs *b)
+{
+    each_buffer(b, [](auto *&p, size_t) {
+        cudaFree(p);
+        p = nullptr;
+    });
+    cudaFreeHost(b->h_out);
+    cudaFreeHost(b->h_root);
+    cudaFreeHost(b->h_st);
+    cudaFreeHost(b->h_log);
+    b->h_out = nullptr;
+    b->h_root = nullptr;
+    b->h_st = nullptr;
+    b->h_log = nullptr;
+}
+
 g5_status alloc_ws(g5_bfs *b)
 {
     g5_graph *g = b->g;
@@ -1867,15 +1884,8 @@ void free_ws(g5_bfs *b)
     for (cudaEvent_t e : b->tev) cudaEventDestroy(e);
     cudaFreeHost(b->h_roots);
     cudaFreeHost(b->h_errs);
-    each_buffer(b, [](auto *&p, size_t) {
-        cudaFree(p);
-        p = nullptr;
-    });
-    cudaFreeHost(b->h_out);
+    free_buffers(b);
     cudaFreeHost(b->h_outs);
-    cudaFreeHost(b->h_root);
-    cudaFreeHost(b->h_st);
-    cudaFreeHost(b->h_log);
     if (b->cfg.codec) g5::codec_work_free(b->cw);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
@@ -1976,7 +1986,16 @@ g5_status g5_bfs_create(g5_graph *g, const g5_bfs_config *cfg, g5_bfs **out)
     if (one_launch(b->cfg)) {
         b->one = g->nnz < ((int64_t)1 << 32) - 64 ? plan_search<uint32_t>(b) : plan_search<int64_t>(b);
     }
-    if ((st = alloc_ws(b)) != G5_OK) return fail(st);
+    st = alloc_ws(b);
+    if (st == G5_ERR_OOM && b->one) {
+        // up to about 2^20 vertices, and on dense graphs, the level loop takes
+        // less memory (a graph of 2^18 vertices and 90 M entries: 20 MB for 34)
+        cudaGetLastError();
+        free_buffers(b);
+        b->one = false;
+        st = alloc_ws(b);
+    }
+    if (st != G5_OK) return fail(st);
     k_degrees<<<g5::grid_for(8), kBlock, 0, b->stream>>>(g->row_off, g->col, g->n, b->deg, b->isolated,
                                                           b->heavy, b->ro32, b->first);
     if (cudaStreamSynchronize(b->stream) != cudaSuccess) return fail(G5_ERR_CUDA);

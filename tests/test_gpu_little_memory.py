@@ -1,5 +1,5 @@
-"""g5_batch_run on a device with no memory left for its one-launch form: the level
-graph, whose buffers the workspace has from the start, gives the same parents."""
+"""Little device memory: where there is none left for the one-launch form of a
+search or a batch, the level graph, which needs less, gives the same parents."""
 import numpy as np
 import pytest
 
@@ -53,3 +53,31 @@ def test_first_run_without_memory():
     first.close()
     for g in graphs:
         g.close()
+
+
+def test_search_workspace_in_little_memory():
+    g = g5.Graph.kronecker(18, 256)  # (dense: many work items)
+    roots = g5.select_roots(g, 3)
+    outs = [torch.zeros(g.n, dtype=torch.int64, device="cuda") for _ in roots]
+    first, loop = g5.CudaBFS(g), g5.CudaBFS(g, parent_mode=1)  # (the kernels of both are loaded)
+    want = []
+    for r, o in zip(roots, outs):
+        assert loop.run(int(r), o) == 0 and first.run(int(r), o) == 0
+        want.append(o.cpu().numpy())
+    first.close()
+    loop.close()
+    torch.cuda.empty_cache()
+    hole = torch.empty(28 << 20, dtype=torch.uint8, device="cuda")
+    held = fill_device()
+    del hole
+    torch.cuda.empty_cache()
+    try:
+        b = g5.CudaBFS(g)
+        for r, o, w in zip(roots, outs, want):
+            assert b.run(int(r), o) == 0
+            assert np.array_equal(o.cpu().numpy(), w)
+        b.close()
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    g.close()
