@@ -146,7 +146,12 @@ constexpr int kList = 128;               // bottom-up candidates a warp lists at
 constexpr uint64_t kClaimMax = 1u << 18;  // frontier entries up to which top-down claims vertices
 constexpr uint64_t kThin = 8;            // candidates per bitmap word below which a bottom-up level is thin
 constexpr uint64_t kClaimedItems = 1u << 19;  // items a claimed frontier may have (else it is built from its bitmap)
-constexpr int kMinItemShift = 8;         // an item holds 256 entries at least (the tile size if that is larger)
+// An item holds 256 entries at least (the tile size if that is larger): items of
+// 128, 64 and 32 cost memory and gain nothing, as short levels are cut further
+// anyway (us per search for 256 / 128 / 64 / 32: scale 16 44.0 / 44.7 / 45.7 /
+// 46.3, 20 69.5 / 71.0 / 71.8 / 73.8, 24 391 / 393 / 396 / 401, 26 1487 / 1490 /
+// 1497 / 1520; 512 and 1024 within 1 % of 256).
+constexpr int kMinItemShift = 8;
 constexpr uint64_t kBuildWarp = 8192;    // frontier vertices up to which a thin bitmap's items are allocated by warps
 constexpr int kClusterBlocks = 16;       // blocks of the cluster form
 

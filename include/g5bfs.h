@@ -150,7 +150,9 @@ typedef struct g5_bfs_config {
                             2 as 1, but the first discoverer's atomicMin stands
                             unless the vertex is reached twice               */
     uint32_t tile_edges; /* frontier edges per top-down warp tile: a power of
-                            two from 32 to 4096 (default 256)                  */
+                            two from 32 to 4096 (default 256).  The one-launch
+                            search takes 256 where it is given less, and cuts
+                            the tiles of short levels by itself               */
     int bu_serial;       /* adjacency entries a bottom-up lane scans alone
                             before its warp scans the rest together: 1..64
                             (default 8)                                        */
