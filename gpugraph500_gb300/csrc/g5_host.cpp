@@ -83,6 +83,14 @@ bool narrow(const int64_t *in, size_t n, uint32_t *out)
     return seen >> 32 == 0;
 }
 
+// Whether narrow would succeed.
+bool fits(const int64_t *in, size_t n)
+{
+    uint64_t seen = 0;
+    for (size_t i = 0; i < n; ++i) seen |= (uint64_t)in[i];
+    return seen >> 32 == 0;
+}
+
 g5_status ensure(PluginState &p, size_t n, size_t words)
 {
     const g5_status s = grow(p, n, words);
@@ -143,7 +151,8 @@ g5_status g5_plugin_compress(const int64_t *fq_host, size_t size, uint32_t **com
     PluginState &p = plugin();
     std::lock_guard<std::mutex> lk(p.mu);
     g5_status s = ensure(p, size, g5_codec_bound(size));
-    if (s != G5_OK) return s;
+    // (an id that does not fit comes before what the device has to say)
+    if (s != G5_OK) return fits(fq_host, size) ? s : G5_ERR_INVALID_ARG;
     if (!narrow(fq_host, size, p.vals)) return G5_ERR_INVALID_ARG;
     size_t words = 0;
     s = g5_codec_encode(p.codec, p.vals, size, p.stream, &words, mode, nullptr);
