@@ -1881,9 +1881,9 @@ g5_status plan_one_launch(g5_batch *b)
     a.rsums = b->rsums;
     a.longs = b->longs;
     a.out = b->h_st;
-    // a block per SM, fewer where their warps would have no words or entries
+    // a block per SM (but those left out), fewer where their warps would have no words or entries
     const uint64_t warps = std::max<uint64_t>(vb / 32, nnz / 64);
-    b->pgrid = (int)std::min<uint64_t>((uint64_t)std::min(g5::num_sms(), kMaxBlocks), (warps + kSW - 1) / kSW);
+    b->pgrid = (int)std::min<uint64_t>((uint64_t)std::min(g5::meeting_sms(), kMaxBlocks), (warps + kSW - 1) / kSW);
     a.unit = 256;
     while (a.unit > 32 && vb / a.unit < (uint64_t)b->pgrid * kSW) a.unit /= 2;
     a.vps_shift = 5;

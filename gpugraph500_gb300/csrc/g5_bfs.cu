@@ -1575,7 +1575,7 @@ bool plan_search(g5_bfs *b)
         b->sform = form;
         b->sgrid = form == SEARCH_BLOCK     ? 1
                    : form == SEARCH_CLUSTER ? kClusterBlocks
-                                            : std::min(g5::grid_for(per_sm), kMaxBlocks);
+                                            : std::min(g5::meeting_sms() * per_sm, kMaxBlocks);
         // an asynchronous search shares the GPU with those of other
         // workspaces: two grids of half the blocks serve more queries than one
         // that has every SM to itself (us per query of a full server, a grid of

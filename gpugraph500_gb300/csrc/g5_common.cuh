@@ -47,6 +47,17 @@ bool is_device_ptr(const void *p);
 // Grid of `per_sm` blocks per SM.
 inline int grid_for(int per_sm) { return num_sms() * per_sm; }
 
+// SMs of a cooperative grid that would otherwise take them all.  Such a grid
+// begins when every block of it has its place, so one block of some other
+// stream's long kernel (one that polls a flag, say) would hold it up until that
+// kernel ends: 49 ms for a search of 0.2 ms beside a kernel of 50.  Two SMs are
+// left out; us per search with 0, 2, 4 and 8 left out: scale 16 44.1, 43.8, 43.9,
+// 44.1; 20 70.2, 70.6, 70.5, 71.2; 22 148.5, 149.1, 149.0, 149.2; 24 375, 378,
+// 378, 382; 26 1266, 1279, 1285, 1312; per batch of 64 roots scale 22 2074, 2088,
+// 2112, 2153; 24 5710, 5740, 5799, 5892.
+constexpr int kSpareSms = 2;
+inline int meeting_sms() { return num_sms() > 4 * kSpareSms ? num_sms() - kSpareSms : num_sms(); }
+
 // Owning device buffer (freed on scope exit unless released).
 template <class T>
 struct DevBuf {
