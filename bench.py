@@ -510,7 +510,8 @@ def main():
                          "frac": kern["achieved"] / peak, "traffic": kern["traffic"],
                          "peak_kind": peak_kind + " (copy, burst)", "kernel": kern,
                          "search": {"achieved": achieved, "frac": achieved / peak,
-                                    "scope": "whole search (every kernel of the level loop), algorithmic bytes"},
+                                    "scope": "whole search (one launch of k_search; host-driven: every kernel of the "
+                                             "level loop), by the level loop's algorithmic bytes"},
                          "dram_measured": dram_measured(g.scale, peak),
                          # the headline traffic comes from the per-kind capture
                          "traffic_settings": capture_settings("k_bu_kinds", g.scale, alpha, beta, sizes or {})},
@@ -682,7 +683,8 @@ def kernel_roofline(g5, g, roots, alpha, beta, peak, sizes=None):
     key = max(kinds, key=lambda k: acc[k][1])
     name = TD_KERNEL if key == "td" else BU_KERNEL
     head = kinds[key]
-    return {"name": name, "kind": key, "launches": head["launches"], "ms_per_launch": head["ms_per_launch"],
+    return {"name": name, "pass": "untimed, host-driven level loop; the timed searches are one launch of k_search each",
+            "kind": key, "launches": head["launches"], "ms_per_launch": head["ms_per_launch"],
             "bytes_per_launch": head["bytes_per_launch"], "achieved": head["achieved"],
             "share_of_search": head["share_of_search"],
             "traffic": kind_traffic(key, g.scale),

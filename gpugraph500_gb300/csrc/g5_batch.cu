@@ -910,8 +910,8 @@ __global__ void __launch_bounds__(kB, 4) k_bwrite(BArgs a)
 // ---- the whole batch as one launch -----------------------------------------------------
 //
 // g5_batch_run's form (the asynchronous and serving forms keep the level graph
-// below, whose kernels other work on the GPU runs between): one cooperative
-// grid of a block per SM, whose blocks meet twice a level.
+// above, whose kernels other work on the GPU runs between): one cooperative
+// grid of a block per SM but two, whose blocks meet twice a level.
 //   expand  top-down graphs by work items of up to kItemEntries entries,
 //           bottom-up ones as in k_bbu
 //   commit  visited |= next, next -> front, the next frontier's sums per graph
@@ -926,7 +926,7 @@ __global__ void __launch_bounds__(kB, 4) k_bwrite(BArgs a)
 // graphs, 16 edges a vertex, before and after: scale 8, 4 roots, 230 and 71;
 // scale 13, 64 roots, 410 and 138; scale 16 479 and 230; scale 20 1281 and 627;
 // scale 24 10267 and 6140; eight graphs of scales 14 to 20, 16 roots each, 1820
-// and 890.  What bounds it: the bottom-up sweeps, half by instructions and half
+// and 890 (with every SM; leaving two out costs at most 0.9 %).  What bounds it: the bottom-up sweeps, half by instructions and half
 // by the latency of their gathers (39 % of the issue slots, 39 % of the memory
 // bandwidth at 64 registers, which two windows of loads and 64-bit roots need;
 // 48 registers and a quarter more warps measured slower).

@@ -1337,8 +1337,11 @@ struct Prof {
 // scale 22 - / 844 / 845; scale 24 3145 / 2914 / -.  With few long searches the
 // copies of the parents to the host have nothing left to hide behind (4 M
 // vertices, 4 roots 1400 / 1385 / 1431; 8 roots - / 2503 / 2330); on the largest
-// graphs they take longer than the searches, whose pairs only start them later
-// (scale 26, 16 roots, 2856 / 2883 us a search).
+// graphs they take longer than the searches, whose pairs only start them later.
+// us a search, one at a time / two, to pinned memory: scale 23, 4 roots 406 / 429,
+// 16 roots 363 / 370; 24 838 / 914, 731 / 750; 25 1521 / 1604, 1422 / 1451; 26
+// 2999 / 3207, 2856 / 3032.  (To device memory two are ahead up to scale 25 with
+// 4 roots and 24 with 16: 24 447 / 408, 434 / 392; 26 1162 / 1166, 1643 / 1803.)
 constexpr int kLanes = 4;
 constexpr int64_t kCopyBound = 1 << 24;
 inline int run_lanes(int64_t n, int k, bool to_host)
@@ -1893,7 +1896,9 @@ void free_ws(g5_bfs *b)
     if (b->stream) cudaStreamDestroy(b->stream);
 }
 
-// Algorithmic HBM bytes of one search from the level log.  With C the
+// Algorithmic HBM bytes of one search from the level log: the level loop's, by
+// which a one-launch search, with its work items for queues and no list of
+// unvisited vertices, is measured as well.  With C the
 // candidates of a bottom-up level (vertices with edges not yet visited) and
 // off the bytes of a row offset, per level: top-down 20|F| + 4 E_td + N/8
 // (queue entry, edge offset and row base per frontier vertex, adjacency,

@@ -7,8 +7,8 @@
 // 2000 entries take none of that).  What a level costs now is its chain of
 // dependent loads and one meeting: 1-3 us in a block, 2-5 in a cluster, 3-8
 // over the grid.  Device time per search, before and after (thresholds at
-// their defaults): scale 10 108 -> 22 us, 16 164 -> 44, 20 193 -> 70, 22 280 ->
-// 147, 24 619 -> 392, 26 (tuned) 1451 -> 1187.
+// their defaults): scale 10 108 -> 22 us, 16 164 -> 44, 20 193 -> 71, 22 280 ->
+// 149, 24 619 -> 392, 26 (tuned) 1451 -> 1219.
 // Four forms (enum below), by the graph's size: see search_form().
 //
 // The level's result is accounted while it is produced, so no counting or
@@ -157,7 +157,7 @@ constexpr int kClusterBlocks = 16;       // blocks of the cluster form
 
 // Where the blocks of a search meet: one block whose bitmaps and sums live in
 // shared memory, one cluster, or a cooperative grid of one block per SM (64
-// registers) or two (32 registers, twice the loads in flight).
+// registers) or two (32 registers, twice the loads in flight), two SMs left out.
 enum { SEARCH_BLOCK, SEARCH_CLUSTER, SEARCH_GRID1, SEARCH_GRID2 };
 
 // The form for a graph, and where each pays (us per search, mean of 8 roots):
@@ -207,7 +207,7 @@ inline bool cluster_fits(const void *kern, int blocks, size_t smem)
 // that pipelines over its own rounds only, and a last round of steps that half
 // of the warps take costs the other half the same.  us per search, against
 // powers of two of which each warp took about eight steps: scale 19 66 -> 60,
-// 20 79 -> 71, 21 96 -> 89, 22 159 -> 149, 24 399 -> 393, 26 1435 -> 1385; two
+// 20 79 -> 71, 21 96 -> 89, 22 159 -> 149, 24 399 -> 393, 26 1435 -> 1424; two
 // or three times as many steps: scale 20 75 and 78, 22 154 and 156, 26 1405 and
 // 1409.
 inline uint32_t bu_step_words(uint64_t nwords, uint64_t warps)

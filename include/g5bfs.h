@@ -136,8 +136,9 @@ typedef struct g5_bfs_config {
     double beta;         /* bottom-up -> top-down when n_f < n / beta           */
     int codec;           /* G5_CODEC_*: round-trip every level's sorted queue   */
     uint32_t codec_threshold; /* raw below or at this length (cpusimd.hh:27,44) */
-    int use_graph;       /* 1: the whole search on the device (one kernel, or with
-                            codec or parent_mode 1 and 2 one CUDA graph with a
+    int use_graph;       /* 1: the whole search on the device (one kernel; with
+                            codec or parent_mode 1 and 2, or without memory for
+                            the kernel's work items, one CUDA graph with a
                             conditional while node); 0: host-driven loop, one sync
                             per level                                            */
     int max_levels;      /* safety cap on levels (G5_ERR_TIMEOUT past it)       */
@@ -176,7 +177,8 @@ typedef struct g5_bfs_stats {
     int64_t queue_total;      /* sum of frontier queue lengths                    */
     int64_t codec_words;      /* sum of encoded words over levels                 */
     int64_t codec_values;     /* sum of values that went through the codec        */
-    int64_t alg_bytes;        /* algorithmic HBM bytes of the search: per level,
+    int64_t alg_bytes;        /* algorithmic HBM bytes of the search, by the level
+                                 loop's measure whichever form ran: per level,
                                  top-down 20|F| + 4 E + N/8; bottom-up (a sweep
                                  of the unvisited list) (2 off + 8) C + 4 E +
                                  N/8 (C candidates, off row-offset bytes); + 13
@@ -196,7 +198,13 @@ typedef struct g5_bfs_stats {
  * vertex of the previous level adjacent to the vertex (the parent
  * CPUBFS_bin's ascending first-writer sweep picks, cpu_2d/cpubfs_bin.cpp:
  * 143-180).  level_out (host or device, may be NULL; needs want_levels)
- * receives levels, -1 unvisited.  stats may be NULL. */
+ * receives levels, -1 unvisited.  stats may be NULL.
+ * The one-kernel search begins once all of its blocks have their places: one
+ * SM (graphs of up to 2^12 vertices and 2^16 adjacency entries), 16 together
+ * (2^15 and 2^20), or all SMs but two; kernels of other streams that hold more
+ * than those two hold it up until they end.
+ * g5_bfs_launch takes half the SMs, and the searches with use_graph = 0 begin
+ * beside any kernel that leaves room for a block of theirs. */
 g5_status g5_bfs_run(g5_bfs *b, int64_t root, int64_t *pred_out, int32_t *level_out,
                      g5_bfs_stats *stats);
 
@@ -220,7 +228,8 @@ g5_status g5_bfs_poll(g5_bfs *b, int *done, double *device_ms);
  * g5_bfs_device_pred, g5_bfs_teps_edges and g5_bfs_validate refer to the
  * last root.  Where a search is one launch and needs no levels, two to four run
  * at a time (a search's device time is then its share of the GPU's); the first
- * call allocates what each writes (25n bytes and a sixteenth of the edges), or
+ * call allocates what each writes (24.5n bytes, a sixteenth of the adjacency
+ * entries and up to 16 MB), which the workspace keeps until it is destroyed, or
  * searches one at a time if there is no memory for it.  Else it allocates the
  * second parent buffer (8n bytes) and builds its CUDA graph. */
 g5_status g5_bfs_run_many(g5_bfs *b, const int64_t *roots, int k, int64_t *const *pred_out, double *device_ms);
@@ -301,7 +310,11 @@ g5_status g5_batch_set_direction(g5_batch *bt, double alpha, double beta);
  * parent of vertex v for root j at [v * nroots[0] + j]; graph 1 follows.
  * (Each vertex's parents are contiguous, so a level's writes are
  * contiguous per warp.)  g5_batch_root_parents extracts one root's array.
- * Same parent choice as g5_bfs_run. */
+ * Same parent choice as g5_bfs_run.  Runs as one kernel on all SMs but two
+ * (g5_bfs_run says what that means); its first call allocates an eighth of a
+ * byte per adjacency entry and up to 17 MB (16 bytes a vertex and a sixteenth of
+ * the entries more on graphs of over 85 entries a vertex), and without memory
+ * for that it runs the level loop of g5_batch_launch. */
 g5_status g5_batch_run(g5_batch *bt, const int64_t *roots_host, const int *nroots,
                        uint32_t *pred_out_dev, double *device_ms);
 
@@ -418,7 +431,8 @@ g5_status g5_codec_encode(g5_codec *c, const uint32_t *in_dev, size_t n, uint32_
 
 /* IntegerCODEC::decodeArray (compositecodec.h:52-71): decodes a stream of
  * `words` words into out_dev (capacity out_cap values); *out_n = values.
- * Streams that fail validation give G5_ERR_CORRUPT_STREAM. */
+ * Streams that fail validation give G5_ERR_CORRUPT_STREAM.  (The width bytes past
+ * the last group's miniblocks are not looked at, as in the reference's decoder.) */
 g5_status g5_codec_decode(g5_codec *c, const uint32_t *in_dev, size_t words, uint32_t *out_dev,
                           size_t out_cap, size_t *out_n, int mode, void *stream);
 
